@@ -845,6 +845,61 @@ __global__ void k_wide_emit(const BvhNode* bin, const int4* items, uint32_t n, c
 }
 
 // ---------------------------------------------------------------------------------------------
+// four-child nodes, one thread per two-child node
+
+struct QEnt {
+    int ref;
+    float b[6];
+};
+// The children of two-child node `node` replace e[at] and go to e[n].
+__device__ __forceinline__ void quad_children(const BvhNode* bin, int node, QEnt (&e)[4], int& n, int at) {
+    const float4* f = reinterpret_cast<const float4*>(bin + node);
+    const float4 a = f[0], b = f[1], c = f[2];
+    const int4 r = reinterpret_cast<const int4*>(f)[3];
+    const QEnt c0{r.x, {a.x, a.y, a.z, a.w, b.x, b.y}}, c1{r.y, {b.z, b.w, c.x, c.y, c.z, c.w}};
+    const bool two = r.y != kRefPop;   // the empty half of a single-leaf root
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {      // constant indices: the entries stay in registers
+        if (j == at) e[j] = c0;
+        if (two && j == n) e[j] = c1;
+    }
+    n += two ? 1 : 0;
+}
+__device__ __forceinline__ float quad_area(const QEnt& e) {
+    const float x = e.b[3] - e.b[0], y = e.b[4] - e.b[1], z = e.b[5] - e.b[2];
+    return x * y + y * z + z * x;
+}
+
+__global__ void __launch_bounds__(128) k_quads(const BvhNode* nodes, QuadNode* quad, uint32_t base, uint32_t count) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const float lim = kFar;
+    QEnt e[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) e[j] = QEnt{kRefPop, {lim, lim, lim, -lim, -lim, -lim}};
+    int n = 1;
+    quad_children(nodes, (int)(base + i), e, n, 0);
+    const int r0 = e[0].ref, r1 = n > 1 ? e[1].ref : -1;
+    if (r0 >= 0) quad_children(nodes, r0, e, n, 0);
+    if (r1 >= 0) quad_children(nodes, r1, e, n, 1);
+    if (n == 3) {   // one child was a leaf: the largest interior grandchild gives way to its children
+        int best = -1, br = 0;
+        float ba = -1.0f;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (e[j].ref >= 0 && quad_area(e[j]) > ba) { ba = quad_area(e[j]); best = j; br = e[j].ref; }
+        if (best >= 0) quad_children(nodes, br, e, n, best);
+    }
+    float4* q = reinterpret_cast<float4*>(quad + base + i);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        q[2 * a] = make_float4(e[0].b[a], e[1].b[a], e[2].b[a], e[3].b[a]);
+        q[2 * a + 1] = make_float4(e[0].b[3 + a], e[1].b[3 + a], e[2].b[3 + a], e[3].b[3 + a]);
+    }
+    reinterpret_cast<int4*>(q)[6] = make_int4(e[0].ref, e[1].ref, e[2].ref, e[3].ref);
+}
+
+// ---------------------------------------------------------------------------------------------
 // refit of the instance level, topology kept
 //
 // One thread per instance climbs from its leaf: it writes its box into its slot (widened, as
@@ -1959,6 +2014,11 @@ cudaError_t gpu_bvh_collapse(GpuBvh* B, const BvhNode* bin, const std::vector<in
                              WideNode* out, size_t out_cap, std::vector<int>& wroots, uint32_t* count, int* depth,
                              cudaStream_t st, const RefitLinks* links) {
     return B->collapse(bin, roots, wide_base, out, out_cap, wroots, count, depth, st, links);
+}
+
+cudaError_t gpu_bvh_quads(const BvhNode* nodes, QuadNode* quad, uint32_t base, uint32_t count, cudaStream_t st) {
+    if (count) k_quads<<<(count + 127) / 128, 128, 0, st>>>(nodes, quad, base, count);
+    return cudaGetLastError();
 }
 
 cudaError_t gpu_bvh_refit_instances(const RefitLinks& lk, const GpuInstBox* inst, const float* mesh_box,

@@ -41,6 +41,12 @@ struct Vtx {
     uint32_t mat;
     uint32_t inst;
 };
+// A hit's vertex, and where its other attributes come from: the triangle's vertices and the
+// barycentrics of the second and third.
+struct HitVtx : Vtx {
+    uint32_t i0, i1, i2;
+    float b1, b2;
+};
 
 struct MatV {
     f4 diffuse;
@@ -68,7 +74,7 @@ GK_D MatV load_mat(const ShadeScene& sc, uint32_t i) {
 
 // FHardwareRayTracerV2::TraceRay after the query (Shading.slang:801-823): position,
 // interpolated shading normal through WorldToObject, and the material of vertex 0's slot.
-static __device__ __noinline__ Vtx hit_vertex(const ShadeScene& sc, f3 o, f3 d, uint32_t inst, uint32_t prim, uint32_t tri) {
+static __device__ __noinline__ HitVtx hit_vertex(const ShadeScene& sc, f3 o, f3 d, uint32_t inst, uint32_t prim, uint32_t tri) {
     const HitShade h = hit_shade(sc.S, o, d, inst, tri);
     const DevInst* ip = sc.S.inst + inst;
     const uint32_t ioff = __ldg(&ip->index_offset) + 3u * prim, voff = __ldg(&ip->vertex_offset);
@@ -79,9 +85,10 @@ static __device__ __noinline__ Vtx hit_vertex(const ShadeScene& sc, f3 o, f3 d, 
     const f3 nobj = F3(fmaf_(e2.x, h.b2, fmaf_(e1.x, h.b1, n0.x)), fmaf_(e2.y, h.b2, fmaf_(e1.y, h.b1, n0.y)),
                        fmaf_(e2.z, h.b2, fmaf_(e1.z, h.b1, n0.z)));
     float w[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) w[k] = __ldg(&ip->winv[k]);
-    Vtx out;
+    load_winv(ip, w);
+    HitVtx out;
+    out.i0 = i0; out.i1 = i1; out.i2 = i2;
+    out.b1 = h.b1; out.b2 = h.b2;
     out.N = normalize3(xnormal(w, nobj));
     out.P = fma3(d, h.t, o);
     out.mat = __ldg(&sc.inst_mat[16u * inst + (__ldg(&sc.slots[i0]) & 15u)]);
@@ -96,10 +103,19 @@ GK_D f4 sky(const GkrtFrameConstants& fc) {
 }
 
 // ---- textures (the pool's sampler at level 0: Vulkan's linear filter, repeat addressing) ----
-// Texel index of the integral float f modulo n (exact: fmodf is exact).
+// Texel index of the integral float f modulo n. Up to 2^20 the quotient is estimated by an
+// approximate reciprocal, at most one off, and the remainder follows exactly (integers below
+// 2^24); fmodf, exact too, is a long division.
 GK_D uint32_t wrap_repeat(float f, uint32_t n) {
-    float m = fmodf(f, (float)n);
-    if (m < 0.0f) m = m + (float)n;
+    const float fn = (float)n;
+    float m;
+    if (fabsf(f) <= 1048576.0f) {
+        m = fmaf_(-floorf(f * rcp_approx(fn)), fn, f);
+        if (m >= fn) m = m - fn;
+    } else {
+        m = fmodf(f, fn);
+    }
+    if (m < 0.0f) m = m + fn;
     const uint32_t i = (uint32_t)m;
     return i < n ? i : 0u;
 }
@@ -153,33 +169,28 @@ struct HitAttr {
     f3 ln;
     f4 lt;
 };
-static __device__ __noinline__ HitAttr hit_attr(const ShadeScene& sc, f3 o, f3 d, uint32_t inst, uint32_t prim,
-                                                uint32_t tri) {
-    const HitShade h = hit_shade(sc.S, o, d, inst, tri);
-    const DevInst* ip = sc.S.inst + inst;
-    const uint32_t ioff = __ldg(&ip->index_offset) + 3u * prim, voff = __ldg(&ip->vertex_offset);
-    const uint32_t i0 = __ldg(&sc.indices[ioff]) + voff, i1 = __ldg(&sc.indices[ioff + 1]) + voff,
-                   i2 = __ldg(&sc.indices[ioff + 2]) + voff;
+static __device__ __noinline__ HitAttr hit_attr(const ShadeScene& sc, uint32_t i0, uint32_t i1, uint32_t i2, float b1,
+                                                float b2) {
     HitAttr r;
     r.u = 0.0f; r.v = 0.0f;
     r.lt = F4(0.0f, 0.0f, 0.0f, 0.0f);
     if (sc.uv) {
         const float2 a = __ldg(&sc.uv[i0]), b = __ldg(&sc.uv[i1]), c = __ldg(&sc.uv[i2]);
-        r.u = fmaf_(c.x - a.x, h.b2, fmaf_(b.x - a.x, h.b1, a.x));
-        r.v = fmaf_(c.y - a.y, h.b2, fmaf_(b.y - a.y, h.b1, a.y));
+        r.u = fmaf_(c.x - a.x, b2, fmaf_(b.x - a.x, b1, a.x));
+        r.v = fmaf_(c.y - a.y, b2, fmaf_(b.y - a.y, b1, a.y));
     }
     {
         const float4 a = __ldg(&sc.normals[i0]), b = __ldg(&sc.normals[i1]), c = __ldg(&sc.normals[i2]);
-        r.ln = F3(fmaf_(c.x - a.x, h.b2, fmaf_(b.x - a.x, h.b1, a.x)), fmaf_(c.y - a.y, h.b2, fmaf_(b.y - a.y, h.b1, a.y)),
-                  fmaf_(c.z - a.z, h.b2, fmaf_(b.z - a.z, h.b1, a.z)));
+        r.ln = F3(fmaf_(c.x - a.x, b2, fmaf_(b.x - a.x, b1, a.x)), fmaf_(c.y - a.y, b2, fmaf_(b.y - a.y, b1, a.y)),
+                  fmaf_(c.z - a.z, b2, fmaf_(b.z - a.z, b1, a.z)));
     }
     if (sc.tangents) {
         float4 a = __ldg(&sc.tangents[i0]), b = __ldg(&sc.tangents[i1]), c = __ldg(&sc.tangents[i2]);
         a.w = a.w > 0.0f ? 2.0f : 0.0f;
         b.w = b.w > 0.0f ? 2.0f : 0.0f;
         c.w = c.w > 0.0f ? 2.0f : 0.0f;
-        r.lt = F4(fmaf_(c.x - a.x, h.b2, fmaf_(b.x - a.x, h.b1, a.x)), fmaf_(c.y - a.y, h.b2, fmaf_(b.y - a.y, h.b1, a.y)),
-                  fmaf_(c.z - a.z, h.b2, fmaf_(b.z - a.z, h.b1, a.z)), fmaf_(c.w - a.w, h.b2, fmaf_(b.w - a.w, h.b1, a.w)));
+        r.lt = F4(fmaf_(c.x - a.x, b2, fmaf_(b.x - a.x, b1, a.x)), fmaf_(c.y - a.y, b2, fmaf_(b.y - a.y, b1, a.y)),
+                  fmaf_(c.z - a.z, b2, fmaf_(b.z - a.z, b1, a.z)), fmaf_(c.w - a.w, b2, fmaf_(b.w - a.w, b1, a.w)));
     }
     return r;
 }

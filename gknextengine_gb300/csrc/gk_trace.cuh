@@ -3,9 +3,8 @@
 // Replaces the RT-core RayQuery of FHardwareRayTracerV2 (assets/shaders/common/
 // Shading.slang:737-826). GB300 has no RT cores, so traversal is software, over either of
 // the two node formats the builders produce from the same SAH trees:
-//   * two-child nodes (64 bytes, four 16-byte loads per node, a stack of node refs): used by
-//     the rt pass, whose per-pixel megakernel interleaves shading with traversal and runs
-//     fastest with the short node step;
+//   * four-child nodes (128 bytes, one cache line, seven 16-byte loads per node, a stack of
+//     node refs): used by the rt pass and the adjoint, whose node step stays short;
 //   * compressed 8-wide nodes (96 bytes, six loads test eight 8-bit child boxes, a stack of
 //     sorted node groups): used by the ray-query kernels, where traversal runs alone and the
 //     wide nodes halve the node steps of incoherent rays.
@@ -21,8 +20,8 @@
 //   * t within its error bound of tmin/tmax -> FP64 t;
 //   * two hits whose t-intervals overlap -> both are decided in FP64 (the incumbent's
 //     triangle is fetched again) and the key is compared exactly.
-// Box tests widen the slab interval by 1e-6 relative (> 2.5 gamma_3), so no box holding
-// the FP64 winner is culled. A ray component of exactly zero lying on a box face is the one
+// Box tests widen the slab interval by 1e-6 relative (> 2.5 gamma_3; quad_slabs adds what its
+// fused form needs), so no box holding the FP64 winner is culled. A ray component of exactly zero lying on a box face is the one
 // case a t-interval widening cannot cover ((hi - o) * inv is 0 there), so the builders store
 // every node box widened in space as well (widen_lo / widen_hi): a triangle edge on the
 // face stays inside the box the ray is tested against. The 8-bit child boxes of the wide
@@ -34,12 +33,27 @@
 
 namespace gk {
 
-// Two-child node: the output of the SAH builders, collapsed into WideNode for traversal.
+// Two-child node: the output of the SAH builders, collapsed into QuadNode and WideNode for
+// traversal.
 struct __align__(16) BvhNode {
     float4 a;   // c0.lo.x c0.lo.y c0.lo.z c0.hi.x
     float4 b;   // c0.hi.y c0.hi.z c1.lo.x c1.lo.y
     float4 c;   // c1.lo.z c1.hi.x c1.hi.y c1.hi.z
     int4 d;     // ref0 ref1 - -   (ref >= 0: interior node; ref < 0: ~(payload << 3 | count-1))
+};
+
+// Four-child node: the quad of two-child node n is quad n, so that a collapse needs no
+// compaction and a refit rewrites quads in place (half of the slots are never visited). Its
+// children are n's grandchildren, a leaf child of n staying as it is (and its place taken by a
+// child of the largest interior grandchild), so every interior child lies at least two levels
+// below n and a ray needs at most 3 stack entries per two levels. Planes are stored per axis and
+// side for the four children, so that a ray loads its near and far planes by the sign of its
+// direction instead of ordering them. A slot without a child has ref kRefPop and a box that no
+// finite ray meets; popping it pops again.
+struct __align__(16) QuadNode {
+    float4 p[6];    // lo.x hi.x lo.y hi.y lo.z hi.z, child j in component j
+    int4 ref;       // BvhNode encoding
+    int4 pad;       // one node per 128-byte line
 };
 
 // Compressed 8-wide node. Per axis a scale s = 2^e (-100 <= e <= 38) and an integer origin k
@@ -58,7 +72,7 @@ struct __align__(16) WideNode {
 
 struct __align__(16) DevInst {
     float winv[12];       // world -> object rows
-    int blas_root;        // root BvhNode index of the mesh BVH
+    int blas_root;        // root node index of the mesh BVH
     uint32_t index_offset;
     uint32_t vertex_offset;
     uint32_t instance_id;
@@ -71,7 +85,14 @@ GK_HD float widen_lo(float v) { return v - (fabsf(v) * 1e-6f + 1e-10f); }
 GK_HD float widen_hi(float v) { return v + (fabsf(v) * 1e-6f + 1e-10f); }
 
 constexpr int kStackEntries = 24;                // wide node-group entries per thread (3 words each)
-constexpr int kStackSize = 3 * kStackEntries;    // 32-bit words per thread; two-child refs: one word each
+constexpr int kStackSize = 3 * kStackEntries;    // 32-bit words per thread
+constexpr int kMaxBinLevels = kStackSize - 3;    // two-child levels of both trees a build may have
+// Stack words of a ray over quad nodes for trees of the given two-child depths (root = 0): three
+// refs per two levels of each tree, and the marker.
+GK_HD constexpr int quad_stack_words(int blas_depth, int tlas_depth) {
+    return 3 * (blas_depth / 2 + 1) + 3 * (tlas_depth / 2 + 1) + 1;
+}
+constexpr int kQuadStackMax = 3 * (kMaxBinLevels / 2 + 2) + 1;
 constexpr int kRefPop = 0x7FFFFFFE;
 constexpr int kRefMarker = 0x7FFFFFFF;
 constexpr int kIterCap = 1 << 22;
@@ -111,11 +132,11 @@ struct Counters {
 };
 
 struct SceneView {
-    const BvhNode* nodes;   // two-child nodes
+    const float4* quad;     // QuadNode array
     const WideNode* wide;   // the same trees collapsed into 8-wide nodes
     const float4* tris;     // 3 float4 per triangle, v0.w = primitive index bits
     const DevInst* inst;
-    int tlas_root;          // two-child root of the instance level, -1: empty scene
+    int tlas_root;          // quad root of the instance level, -1: empty scene
     int tlas_wide_root;     // wide root of the instance level
     uint32_t* error;
     uint32_t node_count, wide_count, tri_count, inst_count;   // array sizes (checked builds)
@@ -125,6 +146,14 @@ struct Shear {
     int kx, ky, kz;
     float Sx, Sy, Sz;
 };
+
+GK_D float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+GK_D float max3f(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+GK_D float min3f(float a, float b, float c) { return fminf(fminf(a, b), c); }
 
 GK_D float pick(f3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
@@ -161,9 +190,11 @@ GK_D ShearD shear_d(f3 d, const Shear& s) {
 struct ExactHit { bool hit; double t, b1, b2; };
 
 // FP64 watertight test; products and sums rounded in double, nothing fused.
-// Out of line: taken rarely, and inlining it at every call site bloats the hot kernel.
-static __device__ __noinline__ ExactHit exact_test(f3 o, f3 d, Shear s, f3 v0, f3 v1, f3 v2) {
+// Out of line, shear included: taken rarely, and inlining it at every call site bloats the hot
+// kernels.
+static __device__ __noinline__ ExactHit exact_test(f3 o, f3 d, f3 v0, f3 v1, f3 v2) {
     ExactHit r; r.hit = false; r.t = 0.0; r.b1 = 0.0; r.b2 = 0.0;
+    const Shear s = make_shear(d);
     const ShearD sd = shear_d(d, s);
     double Ak = (double)pick(v0, s.kz) - (double)pick(o, s.kz);
     double Bk = (double)pick(v1, s.kz) - (double)pick(o, s.kz);
@@ -246,38 +277,58 @@ GK_D Fp32Hit fp32_test(f3 o, const Shear& s, f3 v0, f3 v1, f3 v2) {
     return r;
 }
 
-// Certified interval for the exact hit distance, from the plane of the triangle:
-// t = dot(n, v0 - o) / dot(n, d), n = (v1 - v0) x (v2 - v0). Its error grows like
-// u |t| / cos(theta), while the bound carried by the sheared edge functions grows like
-// u |t| * distance / size, far too wide for small distant triangles. Used only to order
-// candidates and to check [tmin, tmax]; the shading t stays the sheared FP32 value.
-// e_woop (the sheared bound) scaled by 2^-28 covers the FP64 evaluation's own error.
-// Returns false when dot(n, d) is not bounded away from zero (grazing).
-GK_D bool plane_interval(f3 o, f3 d, f3 v0, f3 v1, f3 v2, float e_woop, float& tp, float& ep) {
+// The traversal's ray / triangle test: which side of certain the FP64 test's answer lies, and a
+// certified interval [t - e, t + e] of its distance. Only this classification and the FP64
+// fallback decide hits, so any formula with a certified bound serves; the edge form (Moeller and
+// Trumbore 1997) needs no shear and no axis permutation, and its scalar triple products give the
+// distance as well. With w = o - v0, e1 = v1 - v0, e2 = v2 - v0, p = d x e2, q = w x e1:
+//   u = w . p, v = d . q, x = det - u - v (the three edges), det = e1 . p, t = (e2 . q) / det.
+// Errors, in units of u = 2^-24 times the sum of the absolute products: the differences carry 1
+// each, a cross product's component 3 (p) or 4 (q) with them, a dot product 3 more: det, u and v
+// 7, e2 . q 8; the constants below are rounded up for the second order and the sums' own
+// rounding (and 1e-37 covers products that underflow). x adds the three errors and 2 roundings. As in the FP32 shading test, edges that are
+// not certain, or errors above half of det, leave the decision to FP64. The reciprocals are
+// approximate (2 ulps, inside the slack of 1.25 and 8u |t|). The last term covers the FP64
+// test's own error: 2^-29 of an FP32 evaluation's, itself below the farthest vertex's distance.
+struct TriTest { int kind; float t, e; };   // kind: 0 certain miss, 1 certain hit, 2 undecided
+GK_D TriTest tri_test(f3 o, f3 d, f3 v0, f3 v1, f3 v2) {
     const float kU = 5.9604645e-08f;
-    const f3 e1 = v1 - v0, e2 = v2 - v0, w = v0 - o;
-    const float nx = fmaf_(e1.y, e2.z, -(e1.z * e2.y));
-    const float ny = fmaf_(e1.z, e2.x, -(e1.x * e2.z));
-    const float nz = fmaf_(e1.x, e2.y, -(e1.y * e2.x));
-    // |n_i - n_i*| <= 3u (|a b| + |c d|) + u |n_i|, rounded up to 4u and 2u
-    const float enx = fmaf_(4.0f * kU, fabsf(e1.y * e2.z) + fabsf(e1.z * e2.y), (2.0f * kU) * fabsf(nx));
-    const float eny = fmaf_(4.0f * kU, fabsf(e1.z * e2.x) + fabsf(e1.x * e2.z), (2.0f * kU) * fabsf(ny));
-    const float enz = fmaf_(4.0f * kU, fabsf(e1.x * e2.y) + fabsf(e1.y * e2.x), (2.0f * kU) * fabsf(nz));
-    const float num = fmaf_(nz, w.z, fmaf_(ny, w.y, nx * w.x));
-    const float den = fmaf_(nz, d.z, fmaf_(ny, d.y, nx * d.x));
-    const float anx = fabsf(nx), any_ = fabsf(ny), anz = fabsf(nz);
-    const float awx = fabsf(w.x), awy = fabsf(w.y), awz = fabsf(w.z);
-    const float adx = fabsf(d.x), ady = fabsf(d.y), adz = fabsf(d.z);
-    const float enum_ = fmaf_(5.0f * kU, fmaf_(anz, awz, fmaf_(any_, awy, anx * awx)),
-                              fmaf_(enz, awz, fmaf_(eny, awy, enx * awx)));
-    const float eden = fmaf_(4.0f * kU, fmaf_(anz, adz, fmaf_(any_, ady, anx * adx)),
-                             fmaf_(enz, adz, fmaf_(eny, ady, enx * adx)));
-    const float aden = fabsf(den);
-    if (!(aden > 2.0f * eden)) return false;
-    tp = div_(num, den);
-    const float atp = fabsf(tp);
-    ep = fmaf_(1.25f, div_(fmaf_(atp, eden, enum_), aden - eden), fmaf_(4.0f * kU, atp, 3.7252903e-09f * e_woop));
-    return true;
+    TriTest r; r.kind = 0; r.t = 0.0f; r.e = 0.0f;
+    const f3 w = o - v0, e1 = v1 - v0, e2 = v2 - v0;
+    const float p0 = d.z * e2.y, p1 = d.x * e2.z, p2 = d.y * e2.x;
+    const f3 p = F3(fmaf_(d.y, e2.z, -p0), fmaf_(d.z, e2.x, -p1), fmaf_(d.x, e2.y, -p2));
+    const f3 A = F3(fmaf_(fabsf(d.y), fabsf(e2.z), fabsf(p0)), fmaf_(fabsf(d.z), fabsf(e2.x), fabsf(p1)),
+                    fmaf_(fabsf(d.x), fabsf(e2.y), fabsf(p2)));
+    const float q0 = w.z * e1.y, q1 = w.x * e1.z, q2 = w.y * e1.x;
+    const f3 q = F3(fmaf_(w.y, e1.z, -q0), fmaf_(w.z, e1.x, -q1), fmaf_(w.x, e1.y, -q2));
+    const f3 B = F3(fmaf_(fabsf(w.y), fabsf(e1.z), fabsf(q0)), fmaf_(fabsf(w.z), fabsf(e1.x), fabsf(q1)),
+                    fmaf_(fabsf(w.x), fabsf(e1.y), fabsf(q2)));
+    const float det = dot3(e1, p), u = dot3(w, p), v = dot3(d, q);
+    const float x = (det - u) - v;
+    const float sd = fmaf_(fabsf(e1.z), A.z, fmaf_(fabsf(e1.y), A.y, fabsf(e1.x) * A.x));
+    const float su = fmaf_(fabsf(w.z), A.z, fmaf_(fabsf(w.y), A.y, fabsf(w.x) * A.x));
+    const float sv = fmaf_(fabsf(d.z), B.z, fmaf_(fabsf(d.y), B.y, fabsf(d.x) * B.x));
+    const float eu = fmaf_(8.0f * kU, su, 1e-37f), ev = fmaf_(8.0f * kU, sv, 1e-37f),
+                ex = fmaf_(11.0f * kU, (sd + su) + sv, 1e-37f);
+    const bool pos = (u > eu) || (v > ev) || (x > ex);
+    const bool ng = (u < -eu) || (v < -ev) || (x < -ex);
+    if (pos && ng) return r;
+    const bool allpos = (u > eu) && (v > ev) && (x > ex);
+    const bool allneg = (u < -eu) && (v < -ev) && (x < -ex);
+    const float adet = fabsf(det);
+    r.kind = 2;
+    if (!(allpos || allneg) || !(ex < 0.5f * adet)) return r;
+    const float ed = (8.0f * kU) * sd;
+    const float t = dot3(e2, q) * rcp_approx(det);
+    const float et = (10.0f * kU) * fmaf_(fabsf(e2.z), B.z, fmaf_(fabsf(e2.y), B.y, fabsf(e2.x) * B.x));
+    const float at = fabsf(t);
+    const float far = (max3f(fabsf(w.x), fabsf(w.y), fabsf(w.z)) +
+                       fmaxf(max3f(fabsf(e1.x), fabsf(e1.y), fabsf(e1.z)), max3f(fabsf(e2.x), fabsf(e2.y), fabsf(e2.z)))) *
+                      rcp_approx(max3f(fabsf(d.x), fabsf(d.y), fabsf(d.z)));
+    r.kind = 1;
+    r.t = t;
+    r.e = fmaf_(1.25f * fmaf_(at, ed, et), rcp_approx(adet - ed), fmaf_(8.0f * kU, at, 3e-8f * far));
+    return r;
 }
 
 GK_D f3 safe_inv(f3 d) {
@@ -287,16 +338,49 @@ GK_D f3 safe_inv(f3 d) {
     return F3(rcp_(x), rcp_(y), rcp_(z));
 }
 
-// Slab test widened by 1e-6 relative; tcull already carries the same widening.
-GK_D bool slab(float lx, float ly, float lz, float hx, float hy, float hz, f3 o, f3 inv, float tmin, float tcull,
-               float& tnear) {
-    float t0x = (lx - o.x) * inv.x, t1x = (hx - o.x) * inv.x;
-    float t0y = (ly - o.y) * inv.y, t1y = (hy - o.y) * inv.y;
-    float t0z = (lz - o.z) * inv.z, t1z = (hz - o.z) * inv.z;
-    float tn = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fmaxf(fminf(t0z, t1z), tmin));
-    float tf = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fmaxf(t0z, t1z)) * 1.000001f;
-    tnear = tn;
-    return tn <= fminf(tf, tcull);
+// Slab constants of a ray over quad nodes. A plane p is met at t = (p - o) inv, evaluated as one
+// fused multiply-add, near t = fma(p, inv, nn) and far t = fma(p, inv, nf) with nn, nf = -o inv
+// shifted by 4u |o inv|: the product's rounding and the shift's own are at most 2u |o inv|, so nn
+// is at or below -o inv and nf at or above it by what those roundings can cost, and the fused
+// step's u |t| and the reciprocal's error (2 ulps, a common factor of the three terms) are covered
+// by the 1e-6 relative widening. inv: an approximate reciprocal suffices, |d| at least 1e-20.
+struct Slabs {
+    f3 inv, nn, nf;
+};
+GK_D void slab_axis(float o, float d, float& inv, float& nn, float& nf) {
+    inv = rcp_approx(fabsf(d) < 1e-20f ? copysignf(1e-20f, d) : d);
+    const float oi = o * inv, m = fabsf(oi) * 2.3841858e-07f;   // 4u
+    nn = -oi - m;
+    nf = -oi + m;
+}
+GK_D Slabs quad_slabs(f3 o, f3 d) {
+    Slabs s;
+    slab_axis(o.x, d.x, s.inv.x, s.nn.x, s.nf.x);
+    slab_axis(o.y, d.y, s.inv.y, s.nn.y, s.nf.y);
+    slab_axis(o.z, d.z, s.inv.z, s.nn.z, s.nf.z);
+    return s;
+}
+
+// tnear of one child's box over [tmin, tcull] (widened by 1e-6 relative, as tcull is), +inf when
+// the ray misses it.
+GK_D float quad_near(float nx, float ny, float nz, float fx, float fy, float fz, const Slabs& s, float tmin,
+                     float tcull) {
+    const float tn = fmaxf(max3f(fmaf_(nx, s.inv.x, s.nn.x), fmaf_(ny, s.inv.y, s.nn.y), fmaf_(nz, s.inv.z, s.nn.z)),
+                           tmin);
+    const float tf = min3f(fmaf_(fx, s.inv.x, s.nf.x), fmaf_(fy, s.inv.y, s.nf.y), fmaf_(fz, s.inv.z, s.nf.z)) *
+                     1.000001f;
+    return tn <= fminf(tf, tcull) ? tn : __int_as_float(0x7F800000);
+}
+
+// Orders two children by tnear.
+GK_D void quad_cx(float& ta, int& ra, float& tb, int& rb) {
+    const bool s = tb < ta;
+    const float t = s ? tb : ta;
+    tb = s ? ta : tb;
+    ta = t;
+    const int r = s ? rb : ra;
+    rb = s ? ra : rb;
+    ra = r;
 }
 
 struct TraceOut {
@@ -306,6 +390,16 @@ struct TraceOut {
 };
 
 enum { kClosest = 0, kAny = 1 };
+
+// The world -> object rows of an instance, three 16-byte loads.
+GK_D void load_winv(const DevInst* ip, float (&w)[12]) {
+    const float4* p = reinterpret_cast<const float4*>(ip->winv);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float4 v = __ldg(p + k);
+        w[4 * k] = v.x; w[4 * k + 1] = v.y; w[4 * k + 2] = v.z; w[4 * k + 3] = v.w;
+    }
+}
 
 GK_D f3 tri_v(const float4* tris, uint32_t ti, int k, uint32_t* prim = nullptr) {
     float4 v = __ldg(&tris[3 * ti + k]);
@@ -317,8 +411,10 @@ GK_D f3 tri_v(const float4* tris, uint32_t ti, int k, uint32_t* prim = nullptr) 
 // strided); everything else is here, so a ray can be advanced one step at a time and a
 // lane can leave the traversal loop and come back.
 struct Trav {
-    f3 wo, wd, winv;      // world ray and its safe reciprocal direction (restored on leaving an instance)
-    f3 o, d, inv;         // ray in the current space (world or instance)
+    f3 wo, wd;            // world ray (restored on leaving an instance)
+    f3 o, d;              // ray in the current space (world or instance)
+    Slabs sl;             // its slab constants (quad nodes)
+    f3 inv;               // its safe reciprocal direction (8-wide nodes)
     float tmin;           // read by the ray-query kernels (kRayTmin); the rt pass uses kTmin
     float tmax, tcull, best_lo, best_hi;
     double best_td;
@@ -337,8 +433,8 @@ constexpr float kTmin = 1e-3f;   // EPS, assets/shaders/common/PreProcessor.slan
 template <bool kWide = false>
 GK_D void trav_init(Trav& T, const SceneView& S, f3 wo, f3 wd, float tmax, int mode, float tmin = kTmin) {
     T.wo = wo; T.wd = wd; T.o = wo; T.d = wd;
-    T.inv = safe_inv(wd);
-    T.winv = T.inv;
+    if (kWide) T.inv = safe_inv(wd);
+    else T.sl = quad_slabs(wo, wd);
     T.tmin = tmin;
     T.tmax = tmax;
     T.tcull = tmax * 1.000001f;
@@ -354,19 +450,15 @@ GK_D void trav_init(Trav& T, const SceneView& S, f3 wo, f3 wd, float tmax, int m
 
 // FP64 t of the current best candidate: its triangle against its instance's
 // object-space ray (recomputed with the same FP32 operations as during traversal).
-GK_D double exact_t_of(const Trav& T, const SceneView& S, Shear sh) {
+GK_D double exact_t_of(const Trav& T, const SceneView& S) {
     f3 o = T.o, d = T.d;
     if (!T.inblas || T.inst != T.cur) {
-        const DevInst* ip = S.inst + T.inst;
         float w[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) w[k] = __ldg(&ip->winv[k]);
+        load_winv(S.inst + T.inst, w);
         o = xpoint(w, T.wo);
         d = xvector(w, T.wd);
-        sh = make_shear(d);
     }
-    const f3 v0 = tri_v(S.tris, T.tri, 0), v1 = tri_v(S.tris, T.tri, 1), v2 = tri_v(S.tris, T.tri, 2);
-    return exact_test(o, d, sh, v0, v1, v2).t;
+    return exact_test(o, d, tri_v(S.tris, T.tri, 0), tri_v(S.tris, T.tri, 1), tri_v(S.tris, T.tri, 2)).t;
 }
 
 // Test the triangles of one leaf against the current best. Returns true when the ray is
@@ -375,21 +467,18 @@ template <bool kRayTmin = false>
 GK_D bool trav_leaf(Trav& T, const SceneView& S, uint32_t first, uint32_t cnt, Counters& cn) {
     const float tmin = kRayTmin ? T.tmin : kTmin;
     const double tmind = (double)tmin, tmaxd = (double)T.tmax;
-    const Shear sh = make_shear(T.d);
     for (uint32_t k = 0; k < cnt; ++k) {
         const uint32_t ti = first + k;
         uint32_t prim;
         const f3 v0 = tri_v(S.tris, ti, 0, &prim), v1 = tri_v(S.tris, ti, 1), v2 = tri_v(S.tris, ti, 2);
         ++cn.tris;
-        const Fp32Hit f = fp32_test(T.o, sh, v0, v1, v2);
+        const TriTest f = tri_test(T.o, T.d, v0, v1, v2);
         if (f.kind == 0) continue;
-        float t, e;
+        float t = f.t, e = f.e;
         double td = 0.0;
         bool have_td = false;
-        if (f.kind == 1 && plane_interval(T.o, T.d, v0, v1, v2, f.e, t, e)) {
-            // certified interval from the plane equation
-        } else {
-            const ExactHit x = exact_test(T.o, T.d, sh, v0, v1, v2);
+        if (f.kind == 2) {
+            const ExactHit x = exact_test(T.o, T.d, v0, v1, v2);
             ++cn.fallbacks;
             if (!x.hit) continue;
             td = x.t; have_td = true;
@@ -399,7 +488,7 @@ GK_D bool trav_leaf(Trav& T, const SceneView& S, uint32_t first, uint32_t cnt, C
         if (t + e < tmin || t - e > T.tmax) continue;
         if (t - e < tmin || t + e > T.tmax) {
             if (!have_td) {
-                const ExactHit x = exact_test(T.o, T.d, sh, v0, v1, v2);
+                const ExactHit x = exact_test(T.o, T.d, v0, v1, v2);
                 ++cn.fallbacks;
                 td = x.t; have_td = true;
                 t = (float)x.t;
@@ -424,14 +513,14 @@ GK_D bool trav_leaf(Trav& T, const SceneView& S, uint32_t first, uint32_t cnt, C
                     // intervals overlap: decide both in FP64 and compare the key exactly
                     ++cn.retraces;
                     if (!have_td) {
-                        const ExactHit x = exact_test(T.o, T.d, sh, v0, v1, v2);
+                        const ExactHit x = exact_test(T.o, T.d, v0, v1, v2);
                         ++cn.fallbacks;
                         td = x.t; have_td = true;
                         t = (float)x.t;
                         e = 2.384185791e-07f * fabsf(t);
                     }
                     if (!T.best_exact) {
-                        T.best_td = exact_t_of(T, S, sh);
+                        T.best_td = exact_t_of(T, S);
                         T.best_exact = true;
                         ++cn.fallbacks;
                     }
@@ -450,79 +539,91 @@ GK_D bool trav_leaf(Trav& T, const SceneView& S, uint32_t first, uint32_t cnt, C
     return false;
 }
 
-// Node phase over two-child nodes ("while-while", Aila and Laine, HPG 2009). One step
-// resolves the lane's next reference to a node and tests that node: a pop, the hand-back
-// from an instance to the instance level (which pops again: the entries below a marker all
-// belong to the instance level) and an instance entry (whose mesh root is then tested) take
-// no step of their own, so every step of the warp's node loop is one box test per lane.
-// The first triangle leaf found is postponed into T.leaf and the lane waits for the leaf
-// phase; so does a lane about to leave the instance of its postponed leaf. Returns true
-// while the lane can take another node step.
-// cap: the stack's capacity in words (entries); the caller's stack holds at least cap * stride.
-template <bool kRayTmin = false>
-GK_D bool trav_node_step(Trav& T, const SceneView& S, uint32_t* stk, int stride, Counters& cn, int cap = kStackSize) {
-    const float tmin = kRayTmin ? T.tmin : kTmin;
-    if (++T.iter > kIterCap) { atomicOr(S.error, kErrIter); T.done = true; return false; }
-    int ref = T.ref;
-    if (ref == kRefPop) {
-        if (T.sp == 0) { T.done = true; return false; }
+// ---- traversal over quad nodes ----
+// A ray is always in one of four states, so that a warp can run one kind of work at a time for
+// all the lanes that need it: kStNode (T.ref is an interior node to test), kStTrans (an instance
+// to enter, or the marker: the instance just traversed to leave), kStLeaf (a triangle leaf to
+// test) and kStDone.
+enum TravState : int { kStDone = 0, kStNode = 1, kStTrans = 2, kStLeaf = 3 };
+
+// The next reference to visit, `ref` or the top of the stack, and the state it puts the ray in.
+GK_D int trav_next(Trav& T, int ref, const uint32_t* stk, int stride) {
+    while (ref == kRefPop) {
+        if (T.sp == 0) return kStDone;
         --T.sp;
         ref = (int)stk[T.sp * stride];
     }
-    if (ref == kRefMarker) {
-        if (T.has_leaf) { T.ref = kRefMarker; return false; }   // the postponed leaf needs this instance's ray
-        T.o = T.wo; T.d = T.wd; T.inv = T.winv;
+    T.ref = ref;
+    return ref == kRefMarker ? kStTrans : ref >= 0 ? kStNode : T.inblas ? kStLeaf : kStTrans;
+}
+
+// Tests the four children of node T.ref: the nearest met is visited next, the others are pushed,
+// farthest first. cap: the stack's capacity in words; the caller's stack holds cap * stride.
+GK_D int trav_node(Trav& T, const SceneView& S, uint32_t* stk, int stride, Counters& cn, int cap) {
+    if (++T.iter > kIterCap) { atomicOr(S.error, kErrIter); return kStDone; }
+    GK_CHECK_OR_END((uint32_t)T.ref < S.node_count, S, T, kStDone);
+    ++cn.nodes;
+    // plane rows by the direction's signs: near lo and far hi for a positive component
+    const uint32_t row = 8u * (uint32_t)T.ref;
+    const uint32_t ix = row | (__float_as_uint(T.sl.inv.x) >> 31), iy = row | 2u | (__float_as_uint(T.sl.inv.y) >> 31),
+                   iz = row | 4u | (__float_as_uint(T.sl.inv.z) >> 31);
+    const float4 nx = __ldg(S.quad + ix), fx = __ldg(S.quad + (ix ^ 1u));
+    const float4 ny = __ldg(S.quad + iy), fy = __ldg(S.quad + (iy ^ 1u));
+    const float4 nz = __ldg(S.quad + iz), fz = __ldg(S.quad + (iz ^ 1u));
+    const int4 rf = __ldg(reinterpret_cast<const int4*>(S.quad + (row | 6u)));
+    float t0 = quad_near(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, T.sl, kTmin, T.tcull);
+    float t1 = quad_near(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, T.sl, kTmin, T.tcull);
+    float t2 = quad_near(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, T.sl, kTmin, T.tcull);
+    float t3 = quad_near(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, T.sl, kTmin, T.tcull);
+    int r0 = rf.x, r1 = rf.y, r2 = rf.z, r3 = rf.w;
+    quad_cx(t0, r0, t1, r1); quad_cx(t2, r2, t3, r3); quad_cx(t0, r0, t2, r2); quad_cx(t1, r1, t3, r3);
+    quad_cx(t1, r1, t2, r2);
+    const float inf = __int_as_float(0x7F800000);
+    const int more = t3 < inf ? 3 : t2 < inf ? 2 : t1 < inf ? 1 : 0;
+    if (T.sp + more > cap) { atomicOr(S.error, kErrStack); return kStDone; }
+    uint32_t* top = stk + T.sp * stride;
+    if (more > 2) { *top = (uint32_t)r3; top += stride; }
+    if (more > 1) { *top = (uint32_t)r2; top += stride; }
+    if (more > 0) *top = (uint32_t)r1;
+    T.sp += more;
+    return trav_next(T, t0 < inf ? r0 : kRefPop, stk, stride);
+}
+
+// Leaves the instance whose marker T.ref is and enters the next one, or enters instance T.ref.
+GK_D int trav_trans(Trav& T, const SceneView& S, uint32_t* stk, int stride, int cap) {
+    T.o = T.wo;
+    T.d = T.wd;
+    int st = kStTrans;
+    if (T.ref == kRefMarker) {
         T.inblas = false;
-        if (T.sp == 0) { T.done = true; T.ref = kRefPop; return false; }
-        --T.sp;
-        ref = (int)stk[T.sp * stride];
+        st = trav_next(T, kRefPop, stk, stride);
     }
-    if (ref < 0 && !T.inblas) {         // an instance: enter it
-        T.cur = ~(uint32_t)ref >> 3;
-        GK_CHECK_OR_END(T.cur < S.inst_count, S, T, false);
+    if (st == kStTrans) {
+        T.cur = ~(uint32_t)T.ref >> 3;
+        GK_CHECK_OR_END(T.cur < S.inst_count, S, T, kStDone);
         const DevInst* ip = S.inst + T.cur;
         float w[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) w[k] = __ldg(&ip->winv[k]);
+        const int root = __ldg(&ip->blas_root);
+        load_winv(ip, w);
         T.o = xpoint(w, T.wo);
         T.d = xvector(w, T.wd);
-        T.inv = safe_inv(T.d);
-        if (T.sp >= cap) { atomicOr(S.error, kErrStack); T.done = true; return false; }
+        if (T.sp >= cap) { atomicOr(S.error, kErrStack); return kStDone; }
         stk[T.sp * stride] = (uint32_t)kRefMarker;
         ++T.sp;
         T.inblas = true;
-        ref = __ldg(&ip->blas_root);
+        T.ref = root;
+        st = kStNode;
     }
-    if (ref < 0) {                      // a triangle leaf: postpone it
-        if (T.has_leaf) { T.ref = ref; return false; }   // one postponed leaf at a time
-        T.leaf = ~(uint32_t)ref;
-        T.has_leaf = true;
-        T.ref = kRefPop;
-        return kSpeculative;
-    }
-    GK_CHECK_OR_END((uint32_t)ref < S.node_count, S, T, false);
-    ++cn.nodes;
-    const float4* np = reinterpret_cast<const float4*>(S.nodes + ref);
-    const float4 na = __ldg(np), nb = __ldg(np + 1), nc = __ldg(np + 2);
-    const int4 nd = __ldg(reinterpret_cast<const int4*>(np + 3));
-    float tn0, tn1;
-    const bool h0 = slab(na.x, na.y, na.z, na.w, nb.x, nb.y, T.o, T.inv, tmin, T.tcull, tn0);
-    const bool h1 = slab(nb.z, nb.w, nc.x, nc.y, nc.z, nc.w, T.o, T.inv, tmin, T.tcull, tn1);
-    if (h0 && h1) {
-        int nearr = nd.x, farr = nd.y;
-        if (tn1 < tn0) { nearr = nd.y; farr = nd.x; }
-        if (T.sp >= cap) { atomicOr(S.error, kErrStack); T.done = true; return false; }
-        stk[T.sp * stride] = (uint32_t)farr;
-        ++T.sp;
-        T.ref = nearr;
-    } else if (h0) {
-        T.ref = nd.x;
-    } else if (h1) {
-        T.ref = nd.y;
-    } else {
-        T.ref = kRefPop;
-    }
-    return true;
+    T.sl = quad_slabs(T.o, T.d);
+    return st;
+}
+
+// Tests the triangles of leaf T.ref.
+GK_D int trav_tris(Trav& T, const SceneView& S, const uint32_t* stk, int stride, Counters& cn) {
+    const uint32_t leaf = ~(uint32_t)T.ref;
+    GK_CHECK_OR_END((leaf >> 3) + (leaf & 7u) + 1u <= S.tri_count, S, T, kStDone);
+    if (trav_leaf(T, S, leaf >> 3, (leaf & 7u) + 1u, cn)) return kStDone;
+    return trav_next(T, kRefPop, stk, stride);
 }
 
 // t of byte `b` of `word` (a WideNode plane): fma(2^23 + q, C, B').
@@ -537,7 +638,7 @@ GK_D void wide_sort_cx(uint32_t& a, uint32_t& b) {
 }
 
 GK_D void trav_to_world(Trav& T) {
-    T.o = T.wo; T.d = T.wd; T.inv = T.winv;
+    T.o = T.wo; T.d = T.wd; T.inv = safe_inv(T.wd);
     T.inblas = false;
 }
 
@@ -652,8 +753,7 @@ GK_D bool trav_node_step_wide(Trav& T, const SceneView& S, uint32_t* stk, int st
         GK_CHECK_OR_END(T.cur < S.inst_count, S, T, false);
         const DevInst* ip = S.inst + T.cur;
         float w[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) w[k] = __ldg(&ip->winv[k]);
+        load_winv(ip, w);
         T.o = xpoint(w, T.wo);
         T.d = xvector(w, T.wd);
         T.inv = safe_inv(T.d);
@@ -688,19 +788,14 @@ GK_D void trav_leaf_step(Trav& T, const SceneView& S, Counters& cn) {
 
 GK_D bool trav_finished(const Trav& T) { return T.done && !T.has_leaf; }
 
-// Whole-ray traversal on top of the two phases: hits with tmin <= t <= tmax.
-template <int MODE, bool kWide = false>
-GK_D TraceOut traverse(const SceneView& S, f3 wo, f3 wd, float tmin, float tmax, uint32_t* stk, int stride,
-                       Counters& cn) {
+// Whole-ray traversal over the 8-wide nodes: hits with tmin <= t <= tmax.
+template <int MODE>
+GK_D TraceOut traverse_wide(const SceneView& S, f3 wo, f3 wd, float tmin, float tmax, uint32_t* stk, int stride,
+                            Counters& cn) {
     Trav T;
-    trav_init<kWide>(T, S, wo, wd, tmax, MODE, tmin);
+    trav_init<true>(T, S, wo, wd, tmax, MODE, tmin);
     while (!trav_finished(T)) {
-        if (kWide) {
-            while (!T.done && trav_node_step_wide(T, S, stk, stride, cn)) {
-            }
-        } else {
-            while (!T.done && trav_node_step<true>(T, S, stk, stride, cn)) {
-            }
+        while (!T.done && trav_node_step_wide(T, S, stk, stride, cn)) {
         }
         trav_leaf_step<true>(T, S, cn);
     }
@@ -712,25 +807,17 @@ GK_D TraceOut traverse(const SceneView& S, f3 wo, f3 wd, float tmin, float tmax,
 // Float t and barycentrics of the winning triangle (the values shading uses).
 struct HitShade { float t, b1, b2; };
 GK_D HitShade hit_shade(const SceneView& S, f3 wo, f3 wd, uint32_t inst, uint32_t tri) {
-    const DevInst* ip = S.inst + inst;
     float w[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) w[k] = __ldg(&ip->winv[k]);
+    load_winv(S.inst + inst, w);
     f3 o = xpoint(w, wo), d = xvector(w, wd);
     Shear sh = make_shear(d);
     f3 v0 = tri_v(S.tris, tri, 0), v1 = tri_v(S.tris, tri, 1), v2 = tri_v(S.tris, tri, 2);
     Fp32Hit f = fp32_test(o, sh, v0, v1, v2);
     HitShade h;
     if (f.kind == 1) { h.t = f.t; h.b1 = f.b1; h.b2 = f.b2; return h; }
-    ExactHit x = exact_test(o, d, sh, v0, v1, v2);
+    ExactHit x = exact_test(o, d, v0, v1, v2);
     h.t = (float)x.t; h.b1 = (float)x.b1; h.b2 = (float)x.b2;
     return h;
-}
-
-// Closest hit under the contract.
-GK_D TraceOut trace_closest(const SceneView& S, f3 wo, f3 wd, float tmin, float tmax, uint32_t* stk, int stride,
-                            Counters& cn) {
-    return traverse<kClosest>(S, wo, wd, tmin, tmax, stk, stride, cn);
 }
 
 }  // namespace gk

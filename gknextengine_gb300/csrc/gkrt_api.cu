@@ -50,6 +50,8 @@ struct GkrtContext {
     uint32_t W = 0, H = 0, P = 0;     // P: row pitch in pixels (W rounded up to 4: 16-byte rows)
     void* img[GKRT_IMG_COUNT] = {};
     float4* atrous_tmp[2] = {nullptr, nullptr};   // ping-pong of the a-trous passes
+    float4* path_pool = nullptr;      // the rt pass's paths in flight (sized with the images)
+    size_t path_pool_bytes = 0;
     uint32_t* d_output = nullptr;     // presentation image, OW x OH BGRA8 words (gkrt_output_resize)
     uint32_t OW = 0, OH = 0;
 
@@ -85,9 +87,9 @@ struct GkrtContext {
     std::vector<GkrtLight> lights_host;
 
     // acceleration structures: d_nodes holds the builders' two-child mesh-level nodes
-    // [0, blas_node_count) and the instance-level nodes after them; d_wide holds their
-    // collapse into the 8-wide nodes the kernels traverse (mesh level [0, blas_wide_count),
-    // then the instance level)
+    // [0, blas_node_count) and the instance-level nodes after them, d_quad the four-child nodes of
+    // the same slots; d_wide holds their collapse into 8-wide nodes (mesh level
+    // [0, blas_wide_count), then the instance level)
     bool host_build = false;          // GKRT_BUILD_ON_HOST
     GpuBvh* builder = nullptr;
     uint32_t blas_node_count = 0, blas_nodes_used = 0;
@@ -96,6 +98,7 @@ struct GkrtContext {
     std::vector<float> blas_box;      // 6 per mesh
     float* d_blas_box = nullptr;
     BvhNode* d_nodes = nullptr;
+    QuadNode* d_quad = nullptr;       // the four-child node of each two-child node, d_nodes_cap of them
     size_t d_nodes_cap = 0;
     float4* d_tris = nullptr;
     int tlas_root = -1;
@@ -140,6 +143,9 @@ struct GkrtContext {
     uint32_t* d_error = nullptr;
     unsigned int* d_work = nullptr;             // pixel counter of the persistent trace kernel
     int num_sms = 1;
+    // stream-ordered scratch of calls that may overlap on several streams (the adjoint): what is freed
+    // stays reserved for the next call, until the context ends
+    cudaMemPool_t mem_pool = nullptr;
 };
 
 // Scope of one pass on its stream: an NVTX range, and with pass timers the begin and end events.
@@ -213,6 +219,8 @@ void free_images(GkrtContext* c) {
     for (auto& p : c->img) dfree(p);
     dfree(c->atrous_tmp[0]);
     dfree(c->atrous_tmp[1]);
+    dfree(c->path_pool);
+    c->path_pool_bytes = 0;
     c->W = c->H = c->P = 0;
 }
 
@@ -223,7 +231,7 @@ void free_scene(GkrtContext* c) {
     dfree(c->d_inst_mat); dfree(c->d_inst_prev); dfree(c->d_inst); dfree(c->d_cubes); dfree(c->d_voxels);
     dfree(c->d_cubes_prev);
     c->lights_host.clear();
-    dfree(c->d_nodes); dfree(c->d_wide); dfree(c->d_tris); dfree(c->d_blas_box); dfree(c->d_emit); dfree(c->d_emit_alias);
+    dfree(c->d_nodes); dfree(c->d_quad); dfree(c->d_wide); dfree(c->d_tris); dfree(c->d_blas_box); dfree(c->d_emit); dfree(c->d_emit_alias);
     c->nemit = c->emit_cap = 0;
     c->mat_host.clear(); c->slot_tris.clear();
     c->d_nodes_cap = 0;
@@ -360,16 +368,21 @@ int ensure_node_cap(GkrtContext* ctx, size_t total) {
     if (total <= ctx->d_nodes_cap && ctx->d_nodes) return GKRT_OK;
     const size_t cap = std::max<size_t>(total + total / 4, 16);
     BvhNode* q = nullptr;
+    QuadNode* q4 = nullptr;
     GK_CUDA(cudaMalloc((void**)&q, cap * sizeof(BvhNode)));
-    cudaError_t e = cudaSuccess;
-    if (ctx->d_nodes && ctx->blas_node_count)
-        e = cudaMemcpy(q, ctx->d_nodes, (size_t)ctx->blas_node_count * sizeof(BvhNode), cudaMemcpyDeviceToDevice);
+    cudaError_t e = cudaMalloc((void**)&q4, cap * sizeof(QuadNode));
+    const size_t keep = ctx->d_nodes ? ctx->blas_node_count : 0;
+    if (e == cudaSuccess && keep) e = cudaMemcpy(q, ctx->d_nodes, keep * sizeof(BvhNode), cudaMemcpyDeviceToDevice);
+    if (e == cudaSuccess && keep) e = cudaMemcpy(q4, ctx->d_quad, keep * sizeof(QuadNode), cudaMemcpyDeviceToDevice);
     if (e != cudaSuccess) {
         cudaFree(q);
-        return cuda_fail(ctx, e, "cudaMemcpy(nodes)");
+        cudaFree(q4);
+        return cuda_fail(ctx, e, "node arrays");
     }
     dfree(ctx->d_nodes);
+    dfree(ctx->d_quad);
     ctx->d_nodes = q;
+    ctx->d_quad = q4;
     ctx->d_nodes_cap = cap;
     return GKRT_OK;
 }
@@ -397,10 +410,11 @@ int ensure_wide_cap(GkrtContext* ctx, size_t total, size_t keep) {
     return GKRT_OK;
 }
 
-// Stack a ray can need: two-child traversal pushes at most one ref per level of each tree
-// plus the marker; wide traversal one group per wide level plus the marker.
+// Tree depths the traversal stacks are sized for: quad traversal pushes at most three refs per two
+// levels of each tree plus the marker (quad_stack_words); wide traversal one group per wide
+// level plus the marker.
 int check_stack_bound(GkrtContext* ctx) {
-    if (ctx->blas_bin_depth + ctx->tlas_bin_depth + 3 > kStackSize)
+    if (ctx->blas_bin_depth + ctx->tlas_bin_depth > kMaxBinLevels)
         return fail(ctx, GKRT_ERR_DEVICE_LIMIT, "BVH deeper than the traversal stack allows (" +
                                                     std::to_string(ctx->blas_bin_depth) + " mesh + " +
                                                     std::to_string(ctx->tlas_bin_depth) + " instance levels)");
@@ -425,6 +439,7 @@ int finish_blas(GkrtContext* ctx, cudaStream_t st) {
     if (e == cudaErrorInvalidValue)
         return fail(ctx, GKRT_ERR_INVALID_ARG, "mesh BVH collapse failed (non-finite geometry or depth > 64)");
     if (e != cudaSuccess) return cuda_fail(ctx, e, "gpu_bvh_collapse(mesh level)");
+    GK_CUDA(gpu_bvh_quads(ctx->d_nodes, ctx->d_quad, 0, ctx->blas_node_count, st));
     ctx->tlas_wide_depth = 0;
     ctx->tlas_bin_depth = 0;
     if ((rc = check_stack_bound(ctx)) != GKRT_OK) return rc;
@@ -492,6 +507,7 @@ int finish_tlas(GkrtContext* ctx, uint32_t bin_count, cudaStream_t st) {
         return fail(ctx, GKRT_ERR_INVALID_ARG, "instance BVH collapse failed (non-finite transforms or depth > 64)");
     if (e != cudaSuccess) return cuda_fail(ctx, e, "gpu_bvh_collapse(instance level)");
     ctx->tlas_wide_root = wr[0];
+    if (ctx->tlas_root >= 0) GK_CUDA(gpu_bvh_quads(ctx->d_nodes, ctx->d_quad, ctx->blas_node_count, bin_count, st));
     return check_stack_bound(ctx);
 }
 
@@ -620,6 +636,7 @@ int build_tlas(GkrtContext* ctx, cudaStream_t st, int (*during)(GkrtContext*, cu
             GK_CUDA(gpu_bvh_build_instance_level_launch(ctx->builder, ctx->d_refit_inst, m, ctx->d_blas_box, ctx->d_nodes,
                                                         base, slots, ctx->d_wide, ctx->blas_wide_count,
                                                         (uint32_t)ctx->d_wide_cap, &ctx->refit, st));
+            if (m) GK_CUDA(gpu_bvh_quads(ctx->d_nodes, ctx->d_quad, base, slots, st));
             // host work of the caller's (the emitter table) while the build runs
             const int rc_during = during ? during(ctx, st) : GKRT_OK;
             InstLevelResult r;
@@ -712,6 +729,8 @@ int refit_tlas(GkrtContext* ctx, cudaStream_t st) {
     GK_CUDA(gpu_bvh_refit_instances(ctx->refit, ctx->d_refit_inst, ctx->d_blas_box, ctx->d_nodes, ctx->d_refit_ubox,
                                     ctx->d_refit_arrive, ctx->d_wide, ctx->tlas_wide_count, ctx->d_error, kErrRefit,
                                     st));
+    if (ctx->tlas_root >= 0)
+        GK_CUDA(gpu_bvh_quads(ctx->d_nodes, ctx->d_quad, ctx->refit.nbase, ctx->refit.ncap, st));
     ++ctx->tlas_refits;
     return GKRT_OK;
 }
@@ -757,7 +776,7 @@ int ensure_bvh(GkrtContext* ctx, uint32_t flags, cudaStream_t st) {
 
 SceneView scene_view(GkrtContext* c) {
     SceneView S;
-    S.nodes = c->d_nodes;
+    S.quad = reinterpret_cast<const float4*>(c->d_quad);
     S.wide = c->d_wide;
     S.tris = c->d_tris;
     S.inst = c->d_inst;
@@ -1019,6 +1038,7 @@ int gkrt_context_destroy(GkrtContext* ctx) {
     for (cudaEvent_t& ev : ctx->trace_ev)
         if (ev) cudaEventDestroy(ev);
     if (ctx->h_trace_counters) cudaFreeHost(ctx->h_trace_counters);
+    if (ctx->mem_pool) cudaMemPoolDestroy(ctx->mem_pool);
     delete ctx;
     return GKRT_OK;
 }
@@ -1041,6 +1061,9 @@ int gkrt_resize(GkrtContext* ctx, uint32_t width, uint32_t height) {
         GK_CUDA(cudaMalloc((void**)&t, px * sizeof(float4)));
         GK_CUDA(cudaMemset(t, 0, px * sizeof(float4)));
     }
+    const size_t pool = gkrt_trace_pool_bytes(width * height, ctx->num_sms);
+    GK_CUDA(cudaMalloc((void**)&ctx->path_pool, pool));
+    ctx->path_pool_bytes = pool;
     ctx->W = width;
     ctx->H = height;
     ctx->P = pitch;
@@ -1259,10 +1282,9 @@ int gkrt_trace_pass(GkrtContext* ctx, const GkrtFrameConstants* fc, void* stream
     im.hit_inst = (uint32_t*)ctx->img[GKRT_IMG_HIT_INST];
     im.hit_prim = (uint32_t*)ctx->img[GKRT_IMG_HIT_PRIM];
     GK_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), st));
-    // the stack bound check_stack_bound enforced at build time, at least 8 entries
-    const int stack_words = std::max(8, std::min(kStackSize, ctx->blas_bin_depth + ctx->tlas_bin_depth + 3));
+    const int stack_words = quad_stack_words(ctx->blas_bin_depth, ctx->tlas_bin_depth);
     GK_CUDA(gkrt_launch_trace_pass(sc, *fc, (int)ctx->W, (int)ctx->H, (int)ctx->P, im, ctx->d_counters, ctx->d_work,
-                                   ctx->num_sms, stack_words, ctx->textured, st));
+                                   ctx->num_sms, stack_words, ctx->textured, ctx->path_pool, ctx->path_pool_bytes, st));
     if (ctx->h_trace_counters) {   // the refit-or-rebuild policy is in use: this pass's counters
         const int k = (int)(ctx->trace_seq & 1);
         GK_CUDA(cudaMemcpyAsync(ctx->h_trace_counters + 7 * k, ctx->d_counters, 7 * sizeof(unsigned long long),
@@ -1746,6 +1768,26 @@ static uint32_t* standalone_err_word() {
     return words[dev];
 }
 
+static int ensure_mem_pool(GkrtContext* ctx) {
+    if (ctx->mem_pool) return GKRT_OK;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaMemPool_t pool = nullptr;
+    GK_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = UINT64_MAX;
+    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return cuda_fail(ctx, e, "cudaMemPoolSetAttribute");
+    }
+    ctx->mem_pool = pool;
+    return GKRT_OK;
+}
+
 static int adjoint_checks(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_t spp) {
     int rc = check_frame(ctx, fc);
     if (rc != GKRT_OK) return rc;
@@ -1768,10 +1810,12 @@ int gkrt_adjoint_forward(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_
     if (!image) return fail(ctx, GKRT_ERR_INVALID_ARG, "null image");
     DeviceGuard device_guard(ctx->device);
     cudaStream_t st = (cudaStream_t)stream;
+    if ((rc = ensure_mem_pool(ctx)) != GKRT_OK) return rc;
     if ((rc = ensure_bvh(ctx, 0, st)) != GKRT_OK) return rc;
     GK_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), st));
     GK_CUDA(gkrt_launch_adjoint(shade_scene(ctx), *fc, (int)ctx->W, (int)ctx->H, spp, sample_roughness,
-                                (float4*)image, nullptr, nullptr, nullptr, ctx->d_counters, st));
+                                (float4*)image, nullptr, nullptr, nullptr, ctx->d_counters,
+                                quad_stack_words(ctx->blas_bin_depth, ctx->tlas_bin_depth), ctx->num_sms, ctx->mem_pool, st));
     return GKRT_OK;
 }
 
@@ -1782,10 +1826,12 @@ int gkrt_adjoint_backward(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32
     if (!d_image || !grad_albedo || !grad_roughness) return fail(ctx, GKRT_ERR_INVALID_ARG, "null buffer");
     DeviceGuard device_guard(ctx->device);
     cudaStream_t st = (cudaStream_t)stream;
+    if ((rc = ensure_mem_pool(ctx)) != GKRT_OK) return rc;
     if ((rc = ensure_bvh(ctx, 0, st)) != GKRT_OK) return rc;
     GK_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), st));
     GK_CUDA(gkrt_launch_adjoint(shade_scene(ctx), *fc, (int)ctx->W, (int)ctx->H, spp, sample_roughness, nullptr,
-                                (const float4*)d_image, grad_albedo, grad_roughness, ctx->d_counters, st));
+                                (const float4*)d_image, grad_albedo, grad_roughness, ctx->d_counters,
+                                quad_stack_words(ctx->blas_bin_depth, ctx->tlas_bin_depth), ctx->num_sms, ctx->mem_pool, st));
     return GKRT_OK;
 }
 

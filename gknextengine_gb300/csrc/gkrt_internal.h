@@ -12,6 +12,7 @@ struct ShadeScene;
 struct PixelImages;
 struct SceneView;
 struct BvhNode;
+struct QuadNode;
 struct WideNode;
 struct ProbeLight;
 struct SkySH;
@@ -179,6 +180,8 @@ cudaError_t gpu_bvh_build_instance_level_launch(GpuBvh* b, const GpuInstBox* ins
                                                cudaStream_t st);
 cudaError_t gpu_bvh_build_instance_level_finish(GpuBvh* b, InstLevelResult* res, cudaStream_t st);
 bool gpu_bvh_cooperative_supported();   // the current device takes cooperative launches
+// Four-child nodes [base, base + count) of `quad` from the same slots of the two-child array.
+cudaError_t gpu_bvh_quads(const BvhNode* nodes, QuadNode* quad, uint32_t base, uint32_t count, cudaStream_t st);
 // Collapse of two-child trees (device array bin, roots: node refs, -1 for none) into the
 // compressed 8-wide nodes the kernels traverse, at out[wide_base ...) of an array of out_cap
 // nodes. wroots: wide root per tree (-1 for none); count: wide nodes written; depth: levels.
@@ -217,12 +220,18 @@ cudaError_t gkrt_launch_output_fsr(const float4* src, int W, int H, int P, uint3
 cudaError_t gkrt_launch_screenshot(const uint32_t* img, int OW, int x0, int y0, int w, int h, uint8_t* rgb,
                                    cudaStream_t st);
 
-// stack_words: traversal stack entries per thread, at least the scene's two-child depth bound
-// (mesh depth + instance depth + 3) and at most kStackSize. textured: the scene's materials
-// name textures (the textured instantiation also runs when the frame samples a sky texture).
+// stack_words: traversal stack entries per thread (quad_stack_words of the scene's depths).
+// textured: the scene's materials name textures (the textured instantiation also runs when the
+// frame samples a sky texture). pool: device scratch of pool_bytes, at least
+// gkrt_trace_pool_bytes(W x H), private to the pass while it runs.
 cudaError_t gkrt_launch_trace_pass(const gk::ShadeScene& sc, const GkrtFrameConstants& fc, int W, int H, int P,
                                    const gk::PixelImages& im, unsigned long long* counters, unsigned int* work,
-                                   int num_sms, int stack_words, bool textured, cudaStream_t st);
+                                   int num_sms, int stack_words, bool textured, float4* pool, size_t pool_bytes,
+                                   cudaStream_t st);
+// Device memory of the pass's path pools for a frame of `pixels`, at most (15 fields of 16 bytes per
+// path); the pass uses as much of it as its grid has warps.
+constexpr uint32_t kPathPoolFields = 15;
+size_t gkrt_trace_pool_bytes(uint32_t pixels, int num_sms);
 // Probe grid (k_probes.cu): voxel distance data of probes [first, first + count), and one bake
 // step of those probes reading neighbours from cubes_prev (a snapshot of cubes).
 cudaError_t gkrt_launch_probe_voxelize(const gk::ShadeScene& sc, uint32_t first, uint32_t count, uint4* voxels,
@@ -239,9 +248,11 @@ int gkrt_internal_fail(GkrtContext* ctx, int code, const std::string& msg);
 // built; GKRT_ERR_STATE otherwise (nothing is built or allocated here).
 int gkrt_internal_ready_view(GkrtContext* ctx, gk::SceneView* view, unsigned long long** counters, int* device);
 
+// mem: stream-ordered pool of the caller's that the launch takes its scratch from.
 cudaError_t gkrt_launch_adjoint(const gk::ShadeScene& sc, const GkrtFrameConstants& fc, int W, int H, uint32_t spp,
                                 const float* sample_rough, float4* image, const float4* dimage, double* g_alb,
-                                double* g_rough, unsigned long long* counters, cudaStream_t st);
+                                double* g_rough, unsigned long long* counters, int stack_words, int num_sms,
+                                cudaMemPool_t mem, cudaStream_t st);
 cudaError_t gkrt_launch_set_params(GkrtMaterial* mats, const float* alb, const float* rough, uint32_t first,
                                    uint32_t count, cudaStream_t st);
 cudaError_t gkrt_launch_conv3x3(const void* x, const void* w, const gk::ConvArgs& args, cudaStream_t st);

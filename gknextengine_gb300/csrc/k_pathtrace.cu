@@ -1,30 +1,32 @@
 // k_pathtrace.cu — the "rt pass" (Core.PathTracing) and ray-query kernels for sm_103a.
 //
-// The rt pass is one persistent kernel: every lane runs the per-pixel logic of
+// The rt pass is one persistent kernel: every path runs the per-pixel logic of
 // FPathTracingRendererV2 (assets/shaders/common/Shading.slang:1084-1241, with the traced
 // camera ray of FHardwarePrimaryRayCaster, :283-334) as a state machine that stops
-// whenever it needs a ray traced. The warp alternates two phases: all lanes advance their
-// rays through the BVH until every ray of the warp is finished, then every lane runs its
-// state machine to its next ray, or takes the next pixel from a global counter
-// (warp-aggregated atomics, 8 x 4 pixel tiles) when its path has ended. A lane whose path
-// ends early thus refills instead of idling until the longest path of its warp is done.
-// (Refilling in the middle of the traversal phase was measured slower: shading is the
-// divergent, expensive part, and is best run for all lanes at once.) Each path keeps its
-// own RNG stream, so results do not depend on the schedule.
+// whenever it needs a ray traced. Each warp owns a pool of paths in device memory (a few per
+// lane, L2-resident) and alternates two phases over it: all rays of the pool are traced, a lane
+// whose ray is finished taking the next one, then every path runs its state machine to its next
+// ray, 32 paths of one kind at a time, and pixels from a global counter (8 x 4 pixel tiles) take
+// the places of paths that ended. A warp thus waits for its longest ray once per pool instead of
+// once per 32 rays, and neither phase carries the other's state in registers. Each path keeps
+// its own RNG stream, so results do not depend on the schedule.
+#include <algorithm>
+
+#include "gk_pool.cuh"
 #include "gk_shade.cuh"
 #include "gkrt_internal.h"
 
 namespace gk {
 
-constexpr int kPtThreads = 128;
-// Resident blocks per SM, per instantiation: 4 (128 registers, few spills) without emissive
-// NEE, 5 (96 registers, spills) with it, whose shadow rays add a second traversal per vertex
-// that more warps hide better. Same box, current kernel: the 1080p brick trace pass (no NEE)
-// 3 / 4 / 5 / 6 blocks 3.94 / 3.43 / 3.56 / 3.54 ms; the 4K city (alias-table NEE) 116.4 /
-// 102.9 / 97.0 ms for 3 / 4 / 5 blocks.
-template <bool kNee>
-constexpr int pt_blocks() { return kNee ? 5 : 4; }
-constexpr int kRefillBelow = 1;    // shade and refill once every lane of the warp has finished its ray
+constexpr int kPtThreads = kPoolThreads;
+constexpr int kPtWarps = kPoolWarps;
+constexpr int kPtMaxBlocks = 8;    // resident blocks per SM, at most
+// Resident blocks per SM, per instantiation. The traversal phase fits 128 registers; the shading
+// phase, longest with textures and emitters, spills below. Trace pass with 4 / 5 / 6 blocks (ms):
+// 1080p bricks 3.05 / 2.99 / 3.25, a 720p frame on the probe grid 2.04 / 1.73 / 1.80, 4K city
+// (emitters) 53.9 / 54.3 / 58.9, textured 1277 x 713 at 8 samples 8.0 / 9.5 / 11.0.
+template <bool kNee, bool kTex>
+constexpr int pt_blocks() { return kNee || kTex ? 4 : 5; }
 constexpr float kCosCone = 0.999990482f;   // cos(0.25 deg), Shading.slang:897
 
 // Warp-aggregated flush: one atomic per counter per warp. Slots 0-5 are per pass
@@ -49,16 +51,29 @@ enum Stage : uint32_t {
     ST_NEE_FIRST = 5, ST_NEE_BOUNCE = 6   // emissive-triangle shadow ray before the first / a later bounce
 };
 
-// Per-thread slots in shared memory (strided by the block size): the primary vertex,
-// the per-pixel loop bounds, the two accumulators, the pending emissive-NEE sample and, in the
-// textured instantiation, the primary albedo (material diffuse x diffuse texture).
-enum Slot {
-    SL_PX = 0, SL_PY, SL_PZ, SL_NX, SL_NY, SL_NZ, SL_MAT, SL_LOOP, SL_FC, SL_FR = SL_FC + 4, SL_NEE = SL_FR + 4,
-    SL_COUNT = SL_NEE + 4, SL_ALB = SL_COUNT, SL_COUNT_TEX = SL_ALB + 4
+// A path in its warp's pool: fields of 16 bytes, field f of the pool's paths contiguous, so that 32
+// paths are read and written as whole lines. The ray and its hit, the RNG state, the throughput
+// and the state word travel every time; the current vertex and direction only over any-hit rays
+// (a bounce ray's vertex is its hit, its direction its own); the primary vertex, the loop bounds,
+// the two accumulators, the pending emissive-NEE sample and (textured scenes) the primary albedo
+// are read where the logic needs them.
+enum Field {
+    PF_SEED = PF_FIRST_OWN, PF_RC, PF_STATE, PF_VP, PF_VN, PF_DIR, PF_PP, PF_PN, PF_FC, PF_FR, PF_NEE,
+    PF_ALB, PF_COUNT
+};
+static_assert(PF_COUNT == kPathPoolFields, "pool size");
+
+// The ray a path stops at, and its answer.
+struct PathRay {
+    f3 wo, wd;
+    float tmax;
+    bool any;                    // any-hit (shadow) or closest-hit ray
+    bool hit;
+    uint32_t inst, prim, tri;
 };
 
 struct Lane {
-    int pix;          // pixel index, -1 when the lane holds no pixel
+    int pix;          // pixel index
     Rng seed;
     uint32_t stage;
     uint32_t i, b;    // sample and bounce indices
@@ -74,24 +89,27 @@ struct Ctx {
     const GkrtFrameConstants& fc;
     const PixelImages& im;
     int W, H, P;      // P: image row pitch in pixels
-    float* ps;        // this thread's first shared slot
-    int stride;
+    float4* path;     // this path's field 0
+    uint32_t np;      // paths per pool: the stride between fields
     Counters& cn;
-    __device__ float& slot(int k) const { return ps[k * stride]; }
+    __device__ f4 get(int f) const {
+        const float4 v = __ldcg(path + (uint32_t)f * np);
+        return F4(v.x, v.y, v.z, v.w);
+    }
+    __device__ void put(int f, f4 v) const { __stcg(path + (uint32_t)f * np, make_float4(v.x, v.y, v.z, v.w)); }
+    __device__ void put(int f, f3 v, uint32_t w) const { put(f, F4(v.x, v.y, v.z, __uint_as_float(w))); }
 };
 
-__device__ __forceinline__ void emit(Trav& T, const Ctx& c, f3 o, f3 d, int mode, float tmax = 1000.0f) {
+__device__ __forceinline__ void emit(PathRay& R, const Ctx& c, f3 o, f3 d, bool any, float tmax = 1000.0f) {
     ++c.cn.rays;
-    trav_init(T, c.sc.S, o, d, tmax, mode);
+    R.wo = o; R.wd = d; R.tmax = tmax; R.any = any;
 }
 
-__device__ __forceinline__ f3 pv_pos(const Ctx& c) { return F3(c.slot(SL_PX), c.slot(SL_PY), c.slot(SL_PZ)); }
-__device__ __forceinline__ f3 pv_nrm(const Ctx& c) { return F3(c.slot(SL_NX), c.slot(SL_NY), c.slot(SL_NZ)); }
 // primaryAlbedo_ of the reference: the material's diffuse, times its diffuse texture (kTex)
 template <bool kTex>
 __device__ __forceinline__ f4 pv_albedo(const Ctx& c) {
-    if (kTex) return F4(c.slot(SL_ALB), c.slot(SL_ALB + 1), c.slot(SL_ALB + 2), c.slot(SL_ALB + 3));
-    return load_mat(c.sc, __float_as_uint(c.slot(SL_MAT))).diffuse;
+    if (kTex) return c.get(PF_ALB);
+    return load_mat(c.sc, __float_as_uint(c.get(PF_PP).w)).diffuse;
 }
 
 // Run the lane's state machine on the ray that just finished, up to the next ray
@@ -102,18 +120,25 @@ __device__ __forceinline__ f4 pv_albedo(const Ctx& c) {
 //
 // The logic is laid out as guarded sections in one fixed order; every lane passes each
 // section at most once per call, so lanes in different states re-converge after each
-// section and the expensive ones (the sampling before a trace, the hit reconstruction
-// after it) run once per warp for all the lanes that need them.
+// section and the expensive ones (the hit reconstruction after a trace, the sampling before the
+// next) run once per warp for all the lanes that need them.
 // kTex: textured materials and the textured sky compiled in (the scene has texture ids or the
 // frame samples a sky texture).
 template <bool kNee, bool kTex>
-__device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
+__device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
     const GkrtFrameConstants& fc = c.fc;
     const f3 sunDir = F3(fc.sun_direction[0], fc.sun_direction[1], fc.sun_direction[2]);
     const uint32_t stage = L.stage;
     bool emitted = false, need_begin = false, need_pre = false, pre_first = false;
     bool need_end = false, need_after_sun = false, need_finish = false;
     float shadow = 0.0f;
+
+    // 0. the vertex a closest-hit ray met
+    HitVtx hv;
+    if (stage <= ST_BOUNCE && T.hit) {
+        ++c.cn.hits;
+        hv = hit_vertex(c.sc, T.wo, T.wd, T.inst, T.prim, T.tri);
+    }
 
     // 1. the camera ray's hit: G-buffer outputs, motion, sample set-up
     if (stage == ST_PRIMARY) {
@@ -129,10 +154,8 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
             c.im.object_id[pix] = 65535u;
             c.im.prev_depth[pix] = 100000.0f;
             if (want_ids) { c.im.hit_inst[pix] = 0xFFFFFFFFu; c.im.hit_prim[pix] = 0xFFFFFFFFu; }
-            L.pix = -1;
         } else {
-            ++c.cn.hits;
-            Vtx pv = hit_vertex(c.sc, T.wo, T.wd, T.inst, T.prim, T.tri);
+            Vtx pv = hv;
             if (want_ids) { c.im.hit_inst[pix] = T.inst; c.im.hit_prim[pix] = T.prim; }
             const f4 P4 = F4(pv.P.x, pv.P.y, pv.P.z, 1.0f);
             const f4 clip = mat4v(fc.view_projection, P4);
@@ -152,7 +175,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
             f4 palb = pm.diffuse;
             float prough = pm.fuzz;
             if (kTex) {   // FetchGBufferV2 (Shading.slang:82-112)
-                const HitAttr ha = hit_attr(c.sc, T.wo, T.wd, T.inst, T.prim, T.tri);
+                const HitAttr ha = hit_attr(c.sc, hv.i0, hv.i1, hv.i2, hv.b1, hv.b2);
                 const GBufTex g = fetch_gbuffer(c.sc, pm, ha, pv.N, pv.inst);
                 palb = g.albedo;
                 prough = g.rough;
@@ -166,7 +189,6 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
             if (pm.model != GKRT_MAT_DIELECTRIC) pv.P = fma3(normalize3(T.wd), -0.03f, pv.P);
             if (pm.model == GKRT_MAT_DIFFUSE_LIGHT) {
                 c.im.single_diffuse[pix] = make_float4(pm.diffuse.x, pm.diffuse.y, pm.diffuse.z, pm.diffuse.w);
-                L.pix = -1;
             } else {
                 const bool pdiel = pm.model == GKRT_MAT_DIELECTRIC;
                 int samples = (int)fc.number_of_samples * (mom > 0u ? 4 : 1);
@@ -174,16 +196,11 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
                 if (samples > 0xFFFF) samples = 0xFFFF;
                 uint32_t maxB = pdiel ? fc.max_number_of_bounces : fc.number_of_bounces;
                 if (maxB > 0x7FFFu) maxB = 0x7FFFu;
-                c.slot(SL_PX) = pv.P.x; c.slot(SL_PY) = pv.P.y; c.slot(SL_PZ) = pv.P.z;
-                c.slot(SL_NX) = pv.N.x; c.slot(SL_NY) = pv.N.y; c.slot(SL_NZ) = pv.N.z;
-                c.slot(SL_MAT) = __uint_as_float(pv.mat);
-                c.slot(SL_LOOP) = __uint_as_float((uint32_t)samples | (maxB << 16) | (pdiel ? 0x80000000u : 0u));
-#pragma unroll
-                for (int q = 0; q < 4; ++q) { c.slot(SL_FC + q) = 0.0f; c.slot(SL_FR + q) = 0.0f; }
-                if (kTex) {
-                    c.slot(SL_ALB) = palb.x; c.slot(SL_ALB + 1) = palb.y;
-                    c.slot(SL_ALB + 2) = palb.z; c.slot(SL_ALB + 3) = palb.w;
-                }
+                c.put(PF_PP, pv.P, pv.mat);
+                c.put(PF_PN, pv.N, (uint32_t)samples | (maxB << 16) | (pdiel ? 0x80000000u : 0u));
+                c.put(PF_FC, F4(0.0f, 0.0f, 0.0f, 0.0f));
+                c.put(PF_FR, F4(0.0f, 0.0f, 0.0f, 0.0f));
+                if (kTex) c.put(PF_ALB, palb);
                 L.i = 0;
                 need_begin = true;
             }
@@ -194,8 +211,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
     if (stage == ST_FIRST || stage == ST_BOUNCE) {
         bool term;
         if (T.hit) {
-            ++c.cn.hits;
-            L.vs = hit_vertex(c.sc, T.wo, T.wd, T.inst, T.prim, T.tri);
+            L.vs = hv;
             const MatV hm = load_mat(c.sc, L.vs.mat);
             if (kNee && L.neeLobe && hm.model == GKRT_MAT_DIFFUSE_LIGHT) {
                 // the emitter this diffuse bounce reached was sampled by the vertex's NEE
@@ -204,7 +220,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
             } else {
                 f4 halb = hm.diffuse;
                 if (kTex && hm.dtex >= 0) {   // the hit's diffuse texture (Shading.slang:1046-1050)
-                    const HitAttr ha = hit_attr(c.sc, T.wo, T.wd, T.inst, T.prim, T.tri);
+                    const HitAttr ha = hit_attr(c.sc, hv.i0, hv.i1, hv.i2, hv.b1, hv.b2);
                     halb = halb * tex_sample(c.sc.tex, hm.dtex, ha.u, ha.v);
                 }
                 if (hm.model == GKRT_MAT_DIFFUSE_LIGHT || !L.chanceReflect) L.rc = L.rc * halb;
@@ -215,7 +231,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
             L.rc = L.rc * (kTex ? sky_dir(c.sc, fc, T.wd) : sky(fc));
             term = true;
         }
-        const uint32_t loop = __float_as_uint(c.slot(SL_LOOP));
+        const uint32_t loop = __float_as_uint(c.get(PF_PN).w);
         if (term) {
             need_end = true;
         } else if (stage == ST_FIRST) {
@@ -232,7 +248,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
         } else if (fc.has_sun && rnd1(L.seed) < 0.5f) {
             const f3 cd = align_normal(cone(L.seed, kCosCone), sunDir);
             L.stage = ST_SUN;
-            emit(T, c, L.vs.P, cd, kAny);
+            emit(T, c, L.vs.P, cd, true);
             emitted = true;
         } else {
             need_after_sun = true;
@@ -251,7 +267,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
 
     // 4. early exit or last bounce: probe termination, else the next bounce
     if (need_after_sun) {
-        const uint32_t loop = __float_as_uint(c.slot(SL_LOOP));
+        const uint32_t loop = __float_as_uint(c.get(PF_PN).w);
         const uint32_t maxB = (loop >> 16) & 0x7FFFu;
         const bool pdiel = (loop >> 31) != 0u;
         const bool early = !pdiel && rnd1(L.seed) < 0.5f;
@@ -267,30 +283,19 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
     // 5. end of a sample (Shading.slang:1159-1176), then the next sample or DirectIlluminate
     if (need_end) {
         if (L.hitMetal) L.rc = L.rc * pv_albedo<kTex>(c);
-        const int acc = L.hitReflect ? SL_FR : SL_FC;
-        c.slot(acc) = c.slot(acc) + L.rc.x;
-        c.slot(acc + 1) = c.slot(acc + 1) + L.rc.y;
-        c.slot(acc + 2) = c.slot(acc + 2) + L.rc.z;
-        c.slot(acc + 3) = c.slot(acc + 3) + L.rc.w;
-        const uint32_t samples = __float_as_uint(c.slot(SL_LOOP)) & 0xFFFFu;
+        const int acc = L.hitReflect ? PF_FR : PF_FC;
+        c.put(acc, c.get(acc) + L.rc);
+        const uint32_t samples = __float_as_uint(c.get(PF_PN).w) & 0xFFFFu;
         if (++L.i < samples) {
             need_begin = true;
+        } else if (fc.has_sun) {
+            const f3 cd = align_normal(cone(L.seed, kCosCone), sunDir);
+            L.stage = ST_DIRECT;
+            emit(T, c, xyz(c.get(PF_PP)), cd, true);
+            emitted = true;
         } else {
-            const float fs = (float)samples;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                c.slot(SL_FC + q) = div_(c.slot(SL_FC + q), fs);
-                c.slot(SL_FR + q) = div_(c.slot(SL_FR + q), fs);
-            }
-            if (fc.has_sun) {
-                const f3 cd = align_normal(cone(L.seed, kCosCone), sunDir);
-                L.stage = ST_DIRECT;
-                emit(T, c, pv_pos(c), cd, kAny);
-                emitted = true;
-            } else {
-                shadow = 0.0f;
-                need_finish = true;
-            }
+            shadow = 0.0f;
+            need_finish = true;
         }
     }
 
@@ -303,34 +308,37 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
     // 6b. an emissive-NEE shadow ray's answer, then the bounce ray its vertex sampled
     if (kNee && (stage == ST_NEE_FIRST || stage == ST_NEE_BOUNCE)) {
         if (!T.hit) {
-            const int acc = L.hitReflect ? SL_FR : SL_FC;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) c.slot(acc + q) = c.slot(acc + q) + c.slot(SL_NEE + q);
+            const int acc = L.hitReflect ? PF_FR : PF_FC;
+            c.put(acc, c.get(acc) + c.get(PF_NEE));
         }
         L.stage = stage == ST_NEE_FIRST ? ST_FIRST : ST_BOUNCE;
-        emit(T, c, fma3(L.vs.N, 0.001f, L.vs.P), L.dir, kClosest);
+        emit(T, c, fma3(L.vs.N, 0.001f, L.vs.P), L.dir, false);
         emitted = true;
     }
 
     // 7. the pixel's outputs (Shading.slang:1175-1183)
     if (need_finish) {
-        const float dd = mx(dot3(sunDir, normalize3(pv_nrm(c))), 0.0f) * 0.318309886183790671538f;
-        f4 fcol = F4(c.slot(SL_FC), c.slot(SL_FC + 1), c.slot(SL_FC + 2), c.slot(SL_FC + 3));
-        const f4 frefl = F4(c.slot(SL_FR), c.slot(SL_FR + 1), c.slot(SL_FR + 2), c.slot(SL_FR + 3));
+        const f4 pn = c.get(PF_PN);
+        const float dd = mx(dot3(sunDir, normalize3(xyz(pn))), 0.0f) * 0.318309886183790671538f;
+        // the means over the samples (Shading.slang:1171-1172)
+        const float fs = (float)(__float_as_uint(pn.w) & 0xFFFFu);
+        f4 fcol = c.get(PF_FC), frefl = c.get(PF_FR);
+        fcol = F4(div_(fcol.x, fs), div_(fcol.y, fs), div_(fcol.z, fs), div_(fcol.w, fs));
+        frefl = F4(div_(frefl.x, fs), div_(frefl.y, fs), div_(frefl.z, fs), div_(frefl.w, fs));
         fcol = fcol + F4((fc.sun_color[0] * dd) * shadow, (fc.sun_color[1] * dd) * shadow,
                          (fc.sun_color[2] * dd) * shadow, (fc.sun_color[3] * dd) * shadow);
         c.im.single_diffuse[L.pix] = make_float4(fcol.x, fcol.y, fcol.z, fcol.w);
         c.im.single_specular[L.pix] = make_float4(frefl.x, frefl.y, frefl.z, frefl.w);
-        L.pix = -1;
     }
 
     // 8. start of a sample (Shading.slang:1103-1117)
     if (need_begin) {
         const f4 eye = mat4v(fc.model_view_inverse, F4(0.0f, 0.0f, 0.0f, 1.0f));
         L.rc = F4(1.0f, 1.0f, 1.0f, 1.0f);
-        L.vs.P = pv_pos(c);
-        L.vs.N = pv_nrm(c);
-        L.vs.mat = __float_as_uint(c.slot(SL_MAT));
+        const f4 pp = c.get(PF_PP);
+        L.vs.P = xyz(pp);
+        L.vs.N = xyz(c.get(PF_PN));
+        L.vs.mat = __float_as_uint(pp.w);
         L.dir = normalize3(L.vs.P - xyz(eye));
         L.hitReflect = false;
         L.hitMetal = false;
@@ -366,13 +374,12 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
         if (kNee && L.neeLobe && nee_sample(c.sc, L.seed, L.vs.P, L.vs.N, L.rc, ns)) {
             f4 contrib = ns.contrib;
             if (L.hitMetal) contrib = contrib * pv_albedo<kTex>(c);
-            c.slot(SL_NEE) = contrib.x; c.slot(SL_NEE + 1) = contrib.y;
-            c.slot(SL_NEE + 2) = contrib.z; c.slot(SL_NEE + 3) = contrib.w;
+            c.put(PF_NEE, contrib);
             L.stage = pre_first ? ST_NEE_FIRST : ST_NEE_BOUNCE;
-            emit(T, c, ns.o, ns.dir, kAny, ns.tmax);
+            emit(T, c, ns.o, ns.dir, true, ns.tmax);
         } else {
             L.stage = pre_first ? ST_FIRST : ST_BOUNCE;
-            emit(T, c, fma3(L.vs.N, 0.001f * startPosOffset, L.vs.P), tdir, kClosest);
+            emit(T, c, fma3(L.vs.N, 0.001f * startPosOffset, L.vs.P), tdir, false);
         }
         emitted = true;
     }
@@ -380,7 +387,7 @@ __device__ bool advance(Lane& L, Trav& T, const Ctx& c) {
 }
 
 // Camera ray of FHardwarePrimaryRayCaster (Shading.slang:286-304) for pixel index pix.
-__device__ void start_pixel(Lane& L, Trav& T, const Ctx& c, int x, int y) {
+__device__ __forceinline__ void start_pixel(Lane& L, PathRay& T, const Ctx& c, int x, int y) {
     const GkrtFrameConstants& fc = c.fc;
     L.pix = y * c.P + x;
     L.seed.v[0] = (uint32_t)x; L.seed.v[1] = (uint32_t)y; L.seed.v[2] = fc.total_frames; L.seed.v[3] = 0u;
@@ -400,72 +407,149 @@ __device__ void start_pixel(Lane& L, Trav& T, const Ctx& c, int x, int y) {
                                 target.z * fc.focus_distance));
     const f4 direction = mat4v(fc.model_view_inverse, F4(tn.x, tn.y, tn.z, 0.0f));
     L.stage = ST_PRIMARY;
-    emit(T, c, xyz(origin), xyz(direction), kClosest);
+    emit(T, c, xyz(origin), xyz(direction), false);
+}
+
+// State word pair of a path: stage and flags, sample and bounce indices.
+__device__ __forceinline__ void store_path(const Ctx& c, const Lane& L, const PathRay& R) {
+    c.put(PF_RAYO, F4(R.wo.x, R.wo.y, R.wo.z, R.tmax));
+    c.put(PF_RAYD, R.wd, R.any ? kRayAny : L.stage == ST_PRIMARY ? kRayCamera : kRayBounce);
+    c.put(PF_SEED, F4(__uint_as_float(L.seed.v[0]), __uint_as_float(L.seed.v[1]), __uint_as_float(L.seed.v[2]),
+                      __uint_as_float(L.seed.v[3])));
+    const uint32_t flags = L.stage | (L.chanceReflect ? 8u : 0u) | (L.back ? 16u : 0u) | (L.diel ? 32u : 0u) |
+                           (L.hitReflect ? 64u : 0u) | (L.hitMetal ? 128u : 0u) | (L.neeLobe ? 256u : 0u);
+    c.put(PF_STATE, F4(__int_as_float(L.pix), __uint_as_float(flags), __uint_as_float(L.i), __uint_as_float(L.b)));
+    if (L.stage != ST_PRIMARY) c.put(PF_RC, L.rc);
+    if (R.any && L.stage != ST_DIRECT) {   // the logic goes on from the vertex the ray left
+        c.put(PF_VP, L.vs.P, L.vs.mat);
+        c.put(PF_VN, L.vs.N, 0u);
+        c.put(PF_DIR, L.dir, 0u);
+    }
+}
+
+__device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
+    const f4 o = c.get(PF_RAYO), d = c.get(PF_RAYD), h = c.get(PF_HIT), sd = c.get(PF_SEED), st = c.get(PF_STATE);
+    R.wo = xyz(o); R.wd = xyz(d); R.tmax = o.w; R.any = __float_as_uint(d.w) == kRayAny;
+    R.inst = __float_as_uint(h.x); R.prim = __float_as_uint(h.y); R.tri = __float_as_uint(h.z);
+    R.hit = R.inst != 0xFFFFFFFFu;
+    L.seed.v[0] = __float_as_uint(sd.x); L.seed.v[1] = __float_as_uint(sd.y);
+    L.seed.v[2] = __float_as_uint(sd.z); L.seed.v[3] = __float_as_uint(sd.w);
+    L.pix = __float_as_int(st.x);
+    const uint32_t f = __float_as_uint(st.y);
+    L.stage = f & 7u;
+    L.chanceReflect = (f & 8u) != 0u; L.back = (f & 16u) != 0u; L.diel = (f & 32u) != 0u;
+    L.hitReflect = (f & 64u) != 0u; L.hitMetal = (f & 128u) != 0u; L.neeLobe = (f & 256u) != 0u;
+    L.i = __float_as_uint(st.z); L.b = __float_as_uint(st.w);
+    L.rc = F4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (L.stage != ST_PRIMARY) L.rc = c.get(PF_RC);
+    L.dir = R.wd;
+    if (R.any && L.stage != ST_DIRECT) {
+        const f4 p = c.get(PF_VP);
+        L.vs.P = xyz(p);
+        L.vs.mat = __float_as_uint(p.w);
+        L.vs.N = xyz(c.get(PF_VN));
+        L.dir = xyz(c.get(PF_DIR));
+    }
 }
 
 // kNee: emissive-triangle NEE compiled in (GKRT_NEE_EMISSIVE with a non-empty table); the
 // reference mode runs the instantiation without it.
 //
+// What bounds it: instruction issue with too few warps to cover it (1080p bricks: 310 warp
+// instructions per ray at 16.3 of 32 lanes, 419 at 12.4 when a warp traced its 32 rays to the end
+// before shading them all in registers; an issue in 38 % of the cycles, waits for instruction
+// fetch, node loads and fixed latencies in equal parts). Trace pass before / now, ms: 1080p bricks
+// 3.43 / 2.99, 4K city 91.9 / 53.3, textured 17.7 / 8.0, Cornell 256 x 256 0.164 / 0.150.
+//
 // Shared memory (dynamic): per-thread traversal stacks of stack_words entries (the scene's
-// two-child depth bound), then the per-pixel slots. A stack no larger than the scene needs
-// leaves the rest of the SM's 256 KB to L1, which serves the node fetches (measured on 1080p
-// bricks: 72-word stacks 4.15 ms, 36-word 4.01 ms).
+// depth bound), the world rays in flight, then each warp's path lists. A stack no larger than the
+// scene needs leaves the rest of the SM's 256 KB to L1, which serves the node fetches.
 template <bool kNee, bool kTex>
-__global__ void __launch_bounds__(kPtThreads, pt_blocks<kNee>()) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
+__global__ void __launch_bounds__(kPtThreads, pt_blocks<kNee, kTex>()) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
                                                            int P, PixelImages im, unsigned long long* counters,
-                                                           unsigned int* work, int stack_words) {
+                                                           unsigned int* work, int stack_words, float4* pools,
+                                                           uint32_t np) {
     extern __shared__ uint32_t dyn_smem[];
-    uint32_t* stack = dyn_smem;
-    float* pslots = reinterpret_cast<float*>(dyn_smem + stack_words * kPtThreads);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = tid & 31u;
+    uint32_t* stack = dyn_smem + tid;
+    float* wray = reinterpret_cast<float*>(dyn_smem + stack_words * kPtThreads) + tid;
+    PathId* lists = reinterpret_cast<PathId*>(dyn_smem + (stack_words + kPoolRayWords) * kPtThreads) + (uint32_t)warp * 5u * np;
+    float4* pool = pools + (size_t)(blockIdx.x * kPtWarps + warp) * (PF_COUNT * np + kStashFields * 32u);
+    float4* stash = pool + PF_COUNT * np + lane;
     Counters cn;
     cn.rays = 0; cn.fallbacks = 0; cn.retraces = 0; cn.nodes = 0; cn.tris = 0; cn.hits = 0;
-    const Ctx c{sc, fc, im, W, H, P, pslots + tid, kPtThreads, cn};
     const int tiles_x = (W + 7) / 8, tiles_y = (H + 3) / 4;
     const unsigned total = (unsigned)tiles_x * (unsigned)tiles_y * 32u;
-    Lane L;
-    L.pix = -1;
-    L.stage = ST_PRIMARY;
-    L.neeLobe = false;
-    Trav T;
-    T.done = true;
-    bool tracing = false, exhausted = false;
+    PathList spare{lists + 4u * np, (int)np};      // paths without a pixel
+    for (uint32_t k = lane; k < np; k += 32u) spare.l[k] = (PathId)k;
+    PathList queue{lists + 3u * np, 0};
+    DoneLists done{lists, np, {0, 0, 0}};
+    stash_empty(stash, sc.S);
+    __syncwarp();
+    bool exhausted = false;
+    int live = 0;                                  // paths with a ray queued, in flight or finished
     for (;;) {
-        if (!tracing) {
-            if (L.pix >= 0) tracing = advance<kNee, kTex>(L, T, c);
-            while (!tracing && !exhausted) {
-                // next pixel: warp-aggregated fetch over 8 x 4 tiles
-                const unsigned m = __activemask();
-                const int leader = __ffs(m) - 1;
-                const unsigned rank = __popc(m & ((1u << lane) - 1u));
-                unsigned base = 0;
-                if ((int)lane == leader) base = atomicAdd(work, (unsigned)__popc(m));
-                base = __shfl_sync(m, base, leader);
-                const unsigned k = base + rank;
-                if (k >= total) { exhausted = true; break; }
+        // shading phase: the paths whose rays are finished, up to their next rays
+        int take[3];
+        const bool pure = done.largest() >= 32;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) take[q] = pure ? done.n[q] & ~31 : done.n[q];
+        const int n = take[0] + take[1] + take[2];
+        live -= n;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const int k = k0 + (int)lane;
+            bool ray = false;
+            uint32_t slot = 0;
+            if (k < n) {
+                slot = done.at(k, take);
+                const Ctx c{sc, fc, im, W, H, P, pool + slot, np, cn};
+                Lane L;
+                PathRay R;
+                load_path(c, L, R);
+                ray = advance<kNee, kTex>(L, R, c);
+                if (ray) store_path(c, L, R);
+            }
+            __syncwarp();
+            queue.add(ray, slot);
+            spare.add(k < n && !ray, slot);
+        }
+        done.drop(take);
+        // pixels into the spare paths, 32 at a time
+        while (spare.n > 0 && !exhausted) {
+            const int take = min(spare.n, 32);
+            unsigned base = 0;
+            if (lane == 0) base = atomicAdd(work, (unsigned)take);
+            base = __shfl_sync(0xFFFFFFFFu, base, 0);
+            const unsigned k = base + lane;
+            exhausted = base + (unsigned)take >= total;
+            bool ray = false;
+            uint32_t slot = 0;
+            if ((int)lane < take) {
+                slot = spare.l[spare.n - take + (int)lane];
                 const unsigned tile = k >> 5, in = k & 31u;
                 const int x = (int)((tile % (unsigned)tiles_x) * 8u + (in & 7u));
                 const int y = (int)((tile / (unsigned)tiles_x) * 4u + (in >> 3));
-                if (x >= W || y >= H) continue;
-                start_pixel(L, T, c, x, y);
-                tracing = true;
+                ray = k < total && x < W && y < H;
+                if (ray) {
+                    const Ctx c{sc, fc, im, W, H, P, pool + slot, np, cn};
+                    Lane L;
+                    PathRay R;
+                    start_pixel(L, R, c, x, y);
+                    L.i = 0; L.b = 0;
+                    L.chanceReflect = L.back = L.diel = L.hitReflect = L.hitMetal = L.neeLobe = false;
+                    store_path(c, L, R);
+                }
             }
+            spare.n -= take;
+            __syncwarp();
+            queue.add(ray, slot);
+            spare.add((int)lane < take && !ray, slot);
+            __syncwarp();
         }
-        if (__ballot_sync(0xFFFFFFFFu, tracing) == 0u) break;
-        // traversal phase: node steps while any lane can take one, then the postponed leaves
-        // of all lanes together, until every ray of the warp is finished
-        for (;;) {
-            bool can = tracing && !T.done;
-            while (__any_sync(0xFFFFFFFFu, can)) {
-                if (can) can = trav_node_step(T, sc.S, stack + tid, kPtThreads, cn, stack_words);
-            }
-            if (tracing) {
-                trav_leaf_step(T, sc.S, cn);
-                if (trav_finished(T)) tracing = false;
-            }
-            if (__popc(__ballot_sync(0xFFFFFFFFu, tracing)) < kRefillBelow) break;
-        }
+        live += queue.n;
+        if (live == 0) break;
+        trace_queue(sc.S, queue, done, pool, np, stash, wray, stack, stack_words, cn);
     }
     flush_counters(cn, counters);
 }
@@ -488,8 +572,8 @@ __global__ void __launch_bounds__(kRqThreads) k_trace_rays(SceneView S, const Gk
         cn.rays = 1;
         // hits with r.tmin <= t <= r.tmax (the reference's shaders pass EPS as TMin)
         const TraceOut t = mode == GKRT_TRACE_ANY
-                               ? traverse<kAny, true>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kRqThreads, cn)
-                               : traverse<kClosest, true>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kRqThreads, cn);
+                               ? traverse_wide<kAny>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kRqThreads, cn)
+                               : traverse_wide<kClosest>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kRqThreads, cn);
         if (t.hit) {
             ++cn.hits;
             const HitShade s = hit_shade(S, o, d, t.inst, t.tri);
@@ -505,43 +589,51 @@ __global__ void __launch_bounds__(kRqThreads) k_trace_rays(SceneView S, const Gk
 
 using namespace gk;
 
+// Paths per pool and the pools' size: as many paths per warp as the frame has pixels for, in whole
+// warps, up to kPoolMax.
+static uint32_t paths_per_pool(uint32_t pixels, uint32_t warps) {
+    const uint32_t want = (pixels / std::max(1u, warps) + 31u) / 32u * 32u;
+    return std::max(32u, std::min(kPoolMax, want));
+}
+size_t gkrt_trace_pool_bytes(uint32_t pixels, int num_sms) {
+    const size_t warps = std::min<size_t>((size_t)num_sms * kPtMaxBlocks, (size_t)pixels / kPtThreads + 1u) * kPtWarps;
+    return (std::min<size_t>(warps * kPoolMax, (size_t)pixels + 32u * warps) * PF_COUNT + warps * kStashFields * 32u) *
+           sizeof(float4);
+}
+
 cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstants& fc, int W, int H, int P,
                                    const PixelImages& im, unsigned long long* counters, unsigned int* work,
-                                   int num_sms, int stack_words, bool textured, cudaStream_t st) {
-    if (stack_words < 1 || stack_words > kStackSize) return cudaErrorInvalidValue;
+                                   int num_sms, int stack_words, bool textured, float4* pool, size_t pool_bytes,
+                                   cudaStream_t st) {
+    if (stack_words < 1 || stack_words > kQuadStackMax) return cudaErrorInvalidValue;
     const bool nee = fc.nee_mode == GKRT_NEE_EMISSIVE && sc.nemit > 0u;
     const bool tex = textured || (fc.has_sky && (fc.flags & GKRT_FRAME_SKY_TEXTURE));
     if (tex && !sc.tex) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)(stack_words + (tex ? SL_COUNT_TEX : SL_COUNT)) * kPtThreads * 4u;
+    const size_t smem = (size_t)(stack_words + kPoolRayWords) * kPtThreads * 4u + pool_list_bytes(kPoolMax);
+    using Kernel = void (*)(ShadeScene, GkrtFrameConstants, int, int, int, PixelImages, unsigned long long*, unsigned int*,
+                            int, float4*, uint32_t);
+    const Kernel f = nee ? (tex ? k_trace_pass<true, true> : k_trace_pass<true, false>)
+                         : (tex ? k_trace_pass<false, true> : k_trace_pass<false, false>);
     // resident blocks per SM of each instantiation and stack size, queried once per device
-    static int occ[kMaxDevices][2][2][kStackSize + 1] = {};
+    static int occ[kMaxDevices][2][2][kQuadStackMax + 1] = {};
     const int dev = current_device_slot();
     if (dev < 0) return cudaErrorInvalidDevice;
     int* o = &occ[dev][nee][tex][stack_words];
     cudaError_t e = cudaSuccess;
     if (!*o) {
-        e = nee ? (tex ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, k_trace_pass<true, true>, kPtThreads, smem)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, k_trace_pass<true, false>, kPtThreads, smem))
-                : (tex ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, k_trace_pass<false, true>, kPtThreads, smem)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, k_trace_pass<false, false>, kPtThreads, smem));
+        const int most = (kQuadStackMax + kPoolRayWords) * kPtThreads * 4 + (int)pool_list_bytes(kPoolMax);   // the deepest trees a build accepts
+        e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, f, kPtThreads, smem);
         if (e != cudaSuccess) return e;
     }
-    int per_sm = *o;
-    if (per_sm < 1) per_sm = 1;
-    const int pixels = W * H;
-    int blocks = num_sms * per_sm;
-    const int need = (pixels + kPtThreads - 1) / kPtThreads;
-    if (blocks > need) blocks = need;
+    const uint32_t pixels = (uint32_t)W * (uint32_t)H;
+    uint32_t blocks = (uint32_t)(num_sms * std::max(1, std::min(*o, kPtMaxBlocks)));
+    blocks = std::min(blocks, (pixels + kPtThreads - 1) / kPtThreads);
+    const uint32_t np = paths_per_pool(pixels, blocks * kPtWarps);
+    if ((size_t)blocks * kPtWarps * (np * PF_COUNT + kStashFields * 32u) * sizeof(float4) > pool_bytes) return cudaErrorInvalidValue;
     e = cudaMemsetAsync(work, 0, sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
-    if (nee && tex)
-        k_trace_pass<true, true><<<blocks, kPtThreads, smem, st>>>(sc, fc, W, H, P, im, counters, work, stack_words);
-    else if (nee)
-        k_trace_pass<true, false><<<blocks, kPtThreads, smem, st>>>(sc, fc, W, H, P, im, counters, work, stack_words);
-    else if (tex)
-        k_trace_pass<false, true><<<blocks, kPtThreads, smem, st>>>(sc, fc, W, H, P, im, counters, work, stack_words);
-    else
-        k_trace_pass<false, false><<<blocks, kPtThreads, smem, st>>>(sc, fc, W, H, P, im, counters, work, stack_words);
+    f<<<blocks, kPtThreads, smem, st>>>(sc, fc, W, H, P, im, counters, work, stack_words, pool, np);
     return cudaGetLastError();
 }
 

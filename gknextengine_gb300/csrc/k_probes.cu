@@ -79,7 +79,7 @@ GK_D ProbeHit probe_trace(const ShadeScene& sc, f3 o, f3 d, float tmax, bool wan
     ProbeHit r;
     r.hit = false; r.back = false; r.t = 0.0f; r.mat = 0u; r.tu = 0.0f; r.tv = 0.0f;
     ++cn.rays;
-    const TraceOut t = traverse<kClosest, true>(sc.S, o, d, kTmin, tmax, stk, stride, cn);
+    const TraceOut t = traverse_wide<kClosest>(sc.S, o, d, kTmin, tmax, stk, stride, cn);
     if (!t.hit) return r;
     r.hit = true;
     const HitShade h = hit_shade(sc.S, o, d, t.inst, t.tri);
@@ -91,14 +91,14 @@ GK_D ProbeHit probe_trace(const ShadeScene& sc, f3 o, f3 d, float tmax, bool wan
     const f3 a = v1 - v0, b = v2 - v1;
     const f3 n = F3(fmaf_(a.y, b.z, -(a.z * b.y)), fmaf_(a.z, b.x, -(a.x * b.z)), fmaf_(a.x, b.y, -(a.y * b.x)));
     float w[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) w[k] = __ldg(&ip->winv[k]);
+    load_winv(ip, w);
     const f3 dl = xvector(w, d);
     r.back = fmaf_(n.z, dl.z, fmaf_(n.y, dl.y, n.x * dl.x)) > 0.0f;
     if (want_vertex) {
-        r.v = hit_vertex(sc, o, d, t.inst, t.prim, t.tri);
+        const HitVtx hv = hit_vertex(sc, o, d, t.inst, t.prim, t.tri);
+        r.v = hv;
         if (sc.uv) {
-            const HitAttr a = hit_attr(sc, o, d, t.inst, t.prim, t.tri);
+            const HitAttr a = hit_attr(sc, hv.i0, hv.i1, hv.i2, hv.b1, hv.b2);
             r.tu = a.u;
             r.tv = a.v;
         }
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kBakeThreads) k_probe_bake(ShadeScene sc, Gkrt
             const float len = len3(dv);
             const f3 dn = F3(div_(dv.x, len), div_(dv.y, len), div_(dv.z, len));
             ++cn.rays;
-            const TraceOut s = traverse<kAny, true>(sc.S, fma3(dn, kCubeUnit * 0.5f, o), dn, kTmin,
+            const TraceOut s = traverse_wide<kAny>(sc.S, fma3(dn, kCubeUnit * 0.5f, o), dn, kTmin,
                                                     len - kCubeUnit, stack + threadIdx.x, kBakeThreads, cn);
             const float atten = s.hit ? 0.0f : 1.0f;
             const f3 ldir = normalize3(dv);
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kBakeThreads) k_probe_bake(ShadeScene sc, Gkrt
         if (fc.has_sun) {
             const f3 sd = F3(fc.sun_direction[0], fc.sun_direction[1], fc.sun_direction[2]);
             ++cn.rays;
-            const TraceOut s = traverse<kAny, true>(sc.S, o, sd, kTmin, kOcclusionMax, stack + threadIdx.x,
+            const TraceOut s = traverse_wide<kAny>(sc.S, o, sd, kTmin, kOcclusionMax, stack + threadIdx.x,
                                                     kBakeThreads, cn);
             const float atten = s.hit ? 0.0f : 1.0f;
             const float ndotl = mn(mx(dot3(basis, sd), 0.0f), 1.0f);
