@@ -559,10 +559,13 @@ GK_D int trav_next(Trav& T, int ref, const uint32_t* stk, int stride) {
 
 // Tests the four children of node T.ref: the nearest met is visited next, the others are pushed,
 // farthest first. cap: the stack's capacity in words; the caller's stack holds cap * stride.
+// kRayTmin: the ray's own tmin, else the constant EPS.
+template <bool kRayTmin = false>
 GK_D int trav_node(Trav& T, const SceneView& S, uint32_t* stk, int stride, Counters& cn, int cap) {
     if (++T.iter > kIterCap) { atomicOr(S.error, kErrIter); return kStDone; }
     GK_CHECK_OR_END((uint32_t)T.ref < S.node_count, S, T, kStDone);
     ++cn.nodes;
+    const float tmin = kRayTmin ? T.tmin : kTmin;
     // plane rows by the direction's signs: near lo and far hi for a positive component
     const uint32_t row = 8u * (uint32_t)T.ref;
     const uint32_t ix = row | (__float_as_uint(T.sl.inv.x) >> 31), iy = row | 2u | (__float_as_uint(T.sl.inv.y) >> 31),
@@ -571,10 +574,10 @@ GK_D int trav_node(Trav& T, const SceneView& S, uint32_t* stk, int stride, Count
     const float4 ny = __ldg(S.quad + iy), fy = __ldg(S.quad + (iy ^ 1u));
     const float4 nz = __ldg(S.quad + iz), fz = __ldg(S.quad + (iz ^ 1u));
     const int4 rf = __ldg(reinterpret_cast<const int4*>(S.quad + (row | 6u)));
-    float t0 = quad_near(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, T.sl, kTmin, T.tcull);
-    float t1 = quad_near(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, T.sl, kTmin, T.tcull);
-    float t2 = quad_near(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, T.sl, kTmin, T.tcull);
-    float t3 = quad_near(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, T.sl, kTmin, T.tcull);
+    float t0 = quad_near(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, T.sl, tmin, T.tcull);
+    float t1 = quad_near(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, T.sl, tmin, T.tcull);
+    float t2 = quad_near(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, T.sl, tmin, T.tcull);
+    float t3 = quad_near(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, T.sl, tmin, T.tcull);
     int r0 = rf.x, r1 = rf.y, r2 = rf.z, r3 = rf.w;
     quad_cx(t0, r0, t1, r1); quad_cx(t2, r2, t3, r3); quad_cx(t0, r0, t2, r2); quad_cx(t1, r1, t3, r3);
     quad_cx(t1, r1, t2, r2);
@@ -619,10 +622,11 @@ GK_D int trav_trans(Trav& T, const SceneView& S, uint32_t* stk, int stride, int 
 }
 
 // Tests the triangles of leaf T.ref.
+template <bool kRayTmin = false>
 GK_D int trav_tris(Trav& T, const SceneView& S, const uint32_t* stk, int stride, Counters& cn) {
     const uint32_t leaf = ~(uint32_t)T.ref;
     GK_CHECK_OR_END((leaf >> 3) + (leaf & 7u) + 1u <= S.tri_count, S, T, kStDone);
-    if (trav_leaf(T, S, leaf >> 3, (leaf & 7u) + 1u, cn)) return kStDone;
+    if (trav_leaf<kRayTmin>(T, S, leaf >> 3, (leaf & 7u) + 1u, cn)) return kStDone;
     return trav_next(T, kRefPop, stk, stride);
 }
 

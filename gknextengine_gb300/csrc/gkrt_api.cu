@@ -952,12 +952,15 @@ cudaError_t gkrt_encode_tmap_bf16_dense(CUtensorMap* map, const void* base, uint
     return encode_tmap_bf16(map, base, rank, dims, strides_bytes, box, 0);
 }
 
-int gkrt_internal_ready_view(GkrtContext* ctx, SceneView* view, unsigned long long** counters, int* device) {
+int gkrt_internal_ready_view(GkrtContext* ctx, SceneView* view, unsigned long long** counters, int* device,
+                             int* stack_words, int* num_sms) {
     if (!ctx->has_scene || !ctx->blas_ready || !ctx->tlas_ready)
         return fail(ctx, GKRT_ERR_STATE, "scene and BVH must be built before this call (it allocates nothing)");
     *view = scene_view(ctx);
     *counters = ctx->d_counters;
     *device = ctx->device;
+    *stack_words = quad_stack_words(ctx->blas_bin_depth, ctx->tlas_bin_depth);
+    *num_sms = ctx->num_sms;
     return GKRT_OK;
 }
 
@@ -1641,7 +1644,8 @@ int gkrt_trace_rays(GkrtContext* ctx, const GkrtRay* rays, GkrtHit* hits, uint32
     int rc = ensure_bvh(ctx, 0, st);
     if (rc != GKRT_OK) return rc;
     GK_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), st));
-    GK_CUDA(gkrt_launch_trace_rays(scene_view(ctx), rays, hits, count, mode, ctx->d_counters, st));
+    GK_CUDA(gkrt_launch_trace_rays(scene_view(ctx), rays, hits, count, mode, ctx->d_counters,
+                                   quad_stack_words(ctx->blas_bin_depth, ctx->tlas_bin_depth), ctx->num_sms, st));
     return GKRT_OK;
 }
 

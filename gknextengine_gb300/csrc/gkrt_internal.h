@@ -240,13 +240,15 @@ cudaError_t gkrt_launch_probe_bake(const gk::ShadeScene& sc, const GkrtFrameCons
                                    const gk::SkySH& sh, uint32_t first, uint32_t count, const uint32_t* cubes_prev, uint32_t* cubes,
                                    uint4* voxels, unsigned long long* counters, cudaStream_t st);
 cudaError_t gkrt_launch_trace_rays(const gk::SceneView& S, const GkrtRay* rays, GkrtHit* hits, uint32_t n,
-                                   uint32_t mode, unsigned long long* counters, cudaStream_t st);
+                                   uint32_t mode, unsigned long long* counters, int stack_words, int num_sms,
+                                   cudaStream_t st);
 // Internal helpers for entry points defined outside gkrt_api.cu.
 #include <string>
 int gkrt_internal_fail(GkrtContext* ctx, int code, const std::string& msg);
-// Scene view, statistics counters and device of a context whose scene and BVH are already
-// built; GKRT_ERR_STATE otherwise (nothing is built or allocated here).
-int gkrt_internal_ready_view(GkrtContext* ctx, gk::SceneView* view, unsigned long long** counters, int* device);
+// Scene view, statistics counters, device, traversal stack words and SM count of a context whose
+// scene and BVH are already built; GKRT_ERR_STATE otherwise (nothing is built or allocated here).
+int gkrt_internal_ready_view(GkrtContext* ctx, gk::SceneView* view, unsigned long long** counters, int* device,
+                             int* stack_words, int* num_sms);
 
 // mem: stream-ordered pool of the caller's that the launch takes its scratch from.
 cudaError_t gkrt_launch_adjoint(const gk::ShadeScene& sc, const GkrtFrameConstants& fc, int W, int H, uint32_t spp,

@@ -7,7 +7,8 @@
 // nothing. Its scratch memory (per-block partial sums of the query statistics) is a
 // file-scope __device__ array of fixed size: 32768 blocks x 8 counters x 8 bytes = 2 MiB,
 // which every GPU that loads the library holds until the process exits. The size caps one
-// call at 32768 blocks of 128 rays = 4,194,304 rays; larger counts are rejected.
+// call at 32768 blocks of 128 rays = 4,194,304 rays; larger counts are rejected. (The kernel's
+// persistent warps need far fewer blocks; the limit is part of the interface.)
 //
 // All calls share the one array. Every block writes all 8 of its slots on each call, so
 // nothing has to be cleared first, and the last call's values stay in it. Two calls that
@@ -20,13 +21,14 @@
 // them: do not use the library across a device reset.
 #include <mutex>
 
-#include "gk_shade.cuh"
+#include "gk_query.cuh"
 #include "gkrt_internal.h"
 
 namespace gk {
 namespace {
 
-constexpr uint32_t kNaThreads = 128;
+constexpr uint32_t kNaThreads = kQueryThreads;
+constexpr int kNaBlocks = 5;       // resident blocks per SM, as k_trace_rays
 constexpr uint32_t kNaMaxBlocks = 32768;
 constexpr uint32_t kNaSlots = 8;   // rays, fp64 fallbacks, resolved pairs, nodes, triangles, hits, 2 unused
 constexpr uint32_t kNaMaxRays = kNaMaxBlocks * kNaThreads;
@@ -40,32 +42,15 @@ static __device__ __align__(256) unsigned long long g_noalloc_scratch[gk::kNaMax
 namespace gk {
 namespace {
 
-__global__ void __launch_bounds__(kNaThreads) k_trace_rays_noalloc(SceneView S, const GkrtRay* rays, GkrtHit* hits,
-                                                                   uint32_t n, uint32_t mode,
-                                                                   unsigned long long* partials) {
-    __shared__ uint32_t stack[kStackSize * kNaThreads];
+__global__ void __launch_bounds__(kNaThreads, kNaBlocks) k_trace_rays_noalloc(SceneView S, const GkrtRay* rays,
+                                                                              GkrtHit* hits, uint32_t n, uint32_t mode,
+                                                                              uint32_t per, int cap,
+                                                                              unsigned long long* partials) {
+    extern __shared__ __align__(16) uint32_t na_smem[];
     __shared__ unsigned long long red[kNaThreads / 32][6];
-    const uint32_t i = blockIdx.x * kNaThreads + threadIdx.x;
     Counters cn;
     cn.rays = 0; cn.fallbacks = 0; cn.retraces = 0; cn.nodes = 0; cn.tris = 0; cn.hits = 0;
-    if (i < n) {
-        const GkrtRay r = rays[i];
-        const f3 o = F3(r.origin[0], r.origin[1], r.origin[2]), d = F3(r.dir[0], r.dir[1], r.dir[2]);
-        GkrtHit h;
-        h.t = -1.0f; h.b1 = 0.0f; h.b2 = 0.0f; h.inst = 0xFFFFFFFFu; h.prim = 0xFFFFFFFFu;
-        h.pad[0] = h.pad[1] = h.pad[2] = 0u;
-        cn.rays = 1;
-        const TraceOut t = mode == GKRT_TRACE_ANY
-                               ? traverse_wide<kAny>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kNaThreads, cn)
-                               : traverse_wide<kClosest>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kNaThreads, cn);
-        if (t.hit) {
-            ++cn.hits;
-            const HitShade s = hit_shade(S, o, d, t.inst, t.tri);
-            h.t = s.t; h.inst = t.inst; h.prim = t.prim;
-            if (mode != GKRT_TRACE_ANY) { h.b1 = s.b1; h.b2 = s.b2; }
-        }
-        hits[i] = h;
-    }
+    query_rays(S, rays, hits, n, mode, per, cap, na_smem, cn);
     unsigned long long v[6] = {cn.rays, cn.fallbacks, cn.retraces, cn.nodes, cn.tris, cn.hits};
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -111,7 +96,6 @@ __global__ void __launch_bounds__(256) k_noalloc_reduce(const unsigned long long
 // Device address of the scratch array, looked up once per device (with that device
 // current) and cached; the host-side name of a __device__ variable is not a device address.
 // The cache holds until process exit (a device reset invalidates it, as it does every context).
-constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mu;
 void* g_scratch_addr[kMaxDevices] = {};
 
@@ -145,8 +129,8 @@ extern "C" int gkrt_trace_rays_noalloc(GkrtContext* ctx, const GkrtRay* rays, Gk
                                   "per call; split the batch");
     SceneView S;
     unsigned long long* counters = nullptr;
-    int device = 0;
-    int rc = gkrt_internal_ready_view(ctx, &S, &counters, &device);
+    int device = 0, stack_words = 0, num_sms = 0;
+    int rc = gkrt_internal_ready_view(ctx, &S, &counters, &device, &stack_words, &num_sms);
     if (rc != GKRT_OK) return rc;
     DeviceGuard device_guard(device);
     cudaError_t e = device_guard.status;
@@ -155,11 +139,25 @@ extern "C" int gkrt_trace_rays_noalloc(GkrtContext* ctx, const GkrtRay* rays, Gk
     if (e != cudaSuccess)
         return gkrt_internal_fail(ctx, GKRT_ERR_CUDA,
                                   std::string("gkrt_trace_rays_noalloc: scratch address: ") + cudaGetErrorString(e));
-    const uint32_t blocks = (count + kNaThreads - 1) / kNaThreads;
+    uint32_t blocks = 0, per = 1;
     cudaStream_t st = (cudaStream_t)stream;
-    if (blocks)
-        k_trace_rays_noalloc<<<blocks, kNaThreads, 0, st>>>(S, rays, hits, count, mode,
-                                                             (unsigned long long*)scratch);
+    if (count) {
+        static int occ[kMaxDevices][kQuadStackMax + 1] = {};
+        int* o = &occ[device][stack_words];
+        const size_t smem = query_smem(stack_words);
+        if (!*o) {
+            e = cudaFuncSetAttribute(k_trace_rays_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)query_smem(kQuadStackMax));
+            if (e == cudaSuccess)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, k_trace_rays_noalloc, kNaThreads, smem);
+            if (e != cudaSuccess)
+                return gkrt_internal_fail(ctx, GKRT_ERR_CUDA,
+                                          std::string("gkrt_trace_rays_noalloc: ") + cudaGetErrorString(e));
+        }
+        query_grid(count, num_sms, *o, blocks, per);
+        k_trace_rays_noalloc<<<blocks, kNaThreads, smem, st>>>(S, rays, hits, count, mode, per, stack_words,
+                                                               (unsigned long long*)scratch);
+    }
     // an empty batch still resets the per-call statistics (zero blocks sum to zero), as
     // gkrt_trace_rays does
     k_noalloc_reduce<<<1, 256, 0, st>>>((const unsigned long long*)scratch, blocks, counters);

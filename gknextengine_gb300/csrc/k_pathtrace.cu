@@ -12,7 +12,7 @@
 // its own RNG stream, so results do not depend on the schedule.
 #include <algorithm>
 
-#include "gk_pool.cuh"
+#include "gk_query.cuh"
 #include "gk_shade.cuh"
 #include "gkrt_internal.h"
 
@@ -554,34 +554,19 @@ __global__ void __launch_bounds__(kPtThreads, pt_blocks<kNee, kTex>()) k_trace_p
     flush_counters(cn, counters);
 }
 
-constexpr int kRqThreads = 128;
-
-__global__ void __launch_bounds__(kRqThreads) k_trace_rays(SceneView S, const GkrtRay* rays, GkrtHit* hits,
-                                                           uint32_t n, uint32_t mode,
-                                                           unsigned long long* counters) {
-    __shared__ uint32_t stack[kStackSize * kRqThreads];
-    const uint32_t i = blockIdx.x * kRqThreads + threadIdx.x;
+// What bounds it: instruction issue and the latency of each ray's chain of nodes. 2 M incoherent rays
+// of the 10 M-triangle city 2543 -> 1354 us (any-hit 2060 -> 853), of the bricks 1472 -> 943, of the
+// Cornell box 680 -> 423; 1000 rays 35 -> 21 us. Before, one ray per thread over the 8-wide nodes
+// with 72-word stacks, each warp waiting for its longest ray. 3 / 4 / 5 / 6 resident blocks: city 2 M
+// 1375 / 1390 / 1354 / 1446, bricks 970 / 986 / 943 / 1001 us.
+constexpr int kRqBlocks = 5;
+__global__ void __launch_bounds__(kQueryThreads, kRqBlocks) k_trace_rays(SceneView S, const GkrtRay* rays, GkrtHit* hits,
+                                                                         uint32_t n, uint32_t mode, uint32_t per, int cap,
+                                                                         unsigned long long* counters) {
+    extern __shared__ __align__(16) uint32_t rq_smem[];
     Counters cn;
     cn.rays = 0; cn.fallbacks = 0; cn.retraces = 0; cn.nodes = 0; cn.tris = 0; cn.hits = 0;
-    if (i < n) {
-        GkrtRay r = rays[i];
-        f3 o = F3(r.origin[0], r.origin[1], r.origin[2]), d = F3(r.dir[0], r.dir[1], r.dir[2]);
-        GkrtHit h;
-        h.t = -1.0f; h.b1 = 0.0f; h.b2 = 0.0f; h.inst = 0xFFFFFFFFu; h.prim = 0xFFFFFFFFu;
-        h.pad[0] = h.pad[1] = h.pad[2] = 0u;
-        cn.rays = 1;
-        // hits with r.tmin <= t <= r.tmax (the reference's shaders pass EPS as TMin)
-        const TraceOut t = mode == GKRT_TRACE_ANY
-                               ? traverse_wide<kAny>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kRqThreads, cn)
-                               : traverse_wide<kClosest>(S, o, d, r.tmin, r.tmax, stack + threadIdx.x, kRqThreads, cn);
-        if (t.hit) {
-            ++cn.hits;
-            const HitShade s = hit_shade(S, o, d, t.inst, t.tri);
-            h.t = s.t; h.inst = t.inst; h.prim = t.prim;
-            if (mode != GKRT_TRACE_ANY) { h.b1 = s.b1; h.b2 = s.b2; }
-        }
-        hits[i] = h;
-    }
+    query_rays(S, rays, hits, n, mode, per, cap, rq_smem, cn);
     flush_counters(cn, counters);
 }
 
@@ -638,8 +623,23 @@ cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstant
 }
 
 cudaError_t gkrt_launch_trace_rays(const SceneView& S, const GkrtRay* rays, GkrtHit* hits, uint32_t n,
-                                   uint32_t mode, unsigned long long* counters, cudaStream_t st) {
+                                   uint32_t mode, unsigned long long* counters, int stack_words, int num_sms,
+                                   cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_trace_rays<<<(n + kRqThreads - 1) / kRqThreads, kRqThreads, 0, st>>>(S, rays, hits, n, mode, counters);
+    if (stack_words < 1 || stack_words > kQuadStackMax) return cudaErrorInvalidValue;
+    static int occ[kMaxDevices][kQuadStackMax + 1] = {};
+    const int dev = current_device_slot();
+    if (dev < 0) return cudaErrorInvalidDevice;
+    int* o = &occ[dev][stack_words];
+    const size_t smem = query_smem(stack_words);
+    if (!*o) {
+        cudaError_t e = cudaFuncSetAttribute(k_trace_rays, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)query_smem(kQuadStackMax));
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, k_trace_rays, kQueryThreads, smem);
+        if (e != cudaSuccess) return e;
+    }
+    uint32_t blocks, per;
+    query_grid(n, num_sms, *o, blocks, per);
+    k_trace_rays<<<blocks, kQueryThreads, smem, st>>>(S, rays, hits, n, mode, per, stack_words, counters);
     return cudaGetLastError();
 }
