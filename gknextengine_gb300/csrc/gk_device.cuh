@@ -21,6 +21,18 @@ struct f4 { float x, y, z, w; };
 GK_D float fmaf_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 GK_D float div_(float a, float b) { return __fdiv_rn(a, b); }
 GK_D float rcp_(float a) { return __frcp_rn(a); }
+// x / 1023 and x / 255 of the 10-bit and 8-bit integers x, correctly rounded: the product with the
+// rounded reciprocal, corrected by the exact remainder (division by a constant, Brisebarre, Muller
+// and Raina 2004; every value of the two ranges was checked). Three operations; the IEEE division
+// has a special-case branch.
+GK_D float div1023(float x) {
+    const float q = x * 0x1.00401p-10f;
+    return __fmaf_rn(__fmaf_rn(-q, 1023.0f, x), 0x1.00401p-10f, q);
+}
+GK_D float div255(float x) {
+    const float q = x * 0x1.010102p-8f;
+    return __fmaf_rn(__fmaf_rn(-q, 255.0f, x), 0x1.010102p-8f, q);
+}
 GK_D float sqrt_(float a) { return __fsqrt_rn(a); }
 
 GK_D f3 F3(float x, float y, float z) { f3 r; r.x = x; r.y = y; r.z = z; return r; }

@@ -44,12 +44,19 @@ __device__ __forceinline__ void query_load(const GkrtRay* rays, uint32_t i, bool
     }
 }
 
-// Completes entries [0, m) of the ring (m <= 32), one per lane.
-__device__ __forceinline__ void query_write(const SceneView& S, const GkrtRay* rays, GkrtHit* hits, const uint4* ring, int m,
-                                            bool any, bool wide, Counters& cn) {
-    const int lane = threadIdx.x & 31;
-    if (lane < m) {
-        const uint4 e = ring[lane];     // ray, instance, primitive, triangle
+// The arrays of a ray query as a source of query_run.
+struct QueryRays {
+    const SceneView& S;
+    const GkrtRay* rays;
+    GkrtHit* hits;
+    bool any, wide;
+    // Ray k: origin and tmin, direction and tmax; true for an any-hit ray.
+    __device__ bool load(uint32_t k, float4& o, float4& d) const {
+        query_load(rays, k, wide, o, d);
+        return any;
+    }
+    // The answer e = (ray, instance or 0xFFFFFFFF, primitive, triangle).
+    __device__ void write(const uint4& e, Counters& cn) const {
         float t = -1.0f, b1 = 0.0f, b2 = 0.0f;
         uint32_t prim = 0xFFFFFFFFu;
         if (e.y != 0xFFFFFFFFu) {
@@ -71,18 +78,17 @@ __device__ __forceinline__ void query_write(const SceneView& S, const GkrtRay* r
             h.pad[0] = h.pad[1] = h.pad[2] = 0u;
         }
     }
-    __syncwarp();
-}
+};
 
-// smem: query_smem(cap) bytes of the block's dynamic shared memory, 16-byte aligned.
-__device__ __forceinline__ void query_rays(const SceneView& S, const GkrtRay* rays, GkrtHit* hits, uint32_t n, uint32_t mode,
-                                           uint32_t per, int cap, uint32_t* smem, Counters& cn) {
+// smem: query_smem(cap) bytes of the block's dynamic shared memory, 16-byte aligned. src.load is called
+// once per ray, src.write by up to 32 lanes together, for rays that load was called for before.
+template <class Source>
+__device__ __forceinline__ void query_run(const SceneView& S, const Source& src, uint32_t n, uint32_t per, int cap,
+                                          uint32_t* smem, Counters& cn) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint4* ring = reinterpret_cast<uint4*>(smem) + warp * kQueryRing;
     uint32_t* stk = smem + kQueryWarps * kQueryRing * 4 + tid;
     float* wray = reinterpret_cast<float*>(smem + kQueryWarps * kQueryRing * 4 + cap * kQueryThreads) + tid;
-    const bool any = mode == GKRT_TRACE_ANY;
-    const bool wide = ((reinterpret_cast<uintptr_t>(rays) | reinterpret_cast<uintptr_t>(hits)) & 15u) == 0u;
     const uint64_t warps = (uint64_t)gridDim.x * kQueryWarps, me = (uint64_t)blockIdx.x * kQueryWarps + warp;
     // ray s of this warp is ray ((s / per) warps + me) per + s mod per of the array
     uint64_t run = me * per;            // first ray of the current run
@@ -114,7 +120,8 @@ __device__ __forceinline__ void query_rays(const SceneView& S, const GkrtRay* ra
             ringn += __popc(mf);
             __syncwarp();
             if (ringn >= 32) {
-                query_write(S, rays, hits, ring, 32, any, wide, cn);
+                src.write(ring[lane], cn);
+                __syncwarp();
                 const int left = ringn - 32;
                 uint4 e = make_uint4(0u, 0u, 0u, 0u);
                 if (lane < left) e = ring[32 + lane];
@@ -129,7 +136,7 @@ __device__ __forceinline__ void query_rays(const SceneView& S, const GkrtRay* ra
                 if (st == kStDone && k < per && r < n) {
                     ray = (uint32_t)r;
                     float4 o, d;
-                    query_load(rays, ray, wide, o, d);
+                    const bool any = src.load(ray, o, d);
                     ++cn.rays;
                     trav_init(T, S, F3(o.x, o.y, o.z), F3(d.x, d.y, d.z), d.w, any ? kAny : kClosest, o.w);
                     wray[0] = o.x; wray[kQueryThreads] = o.y; wray[2 * kQueryThreads] = o.z;
@@ -164,7 +171,15 @@ __device__ __forceinline__ void query_rays(const SceneView& S, const GkrtRay* ra
             st = trav_node<true>(T, S, stk, kQueryThreads, cn, cap);
         }
     }
-    query_write(S, rays, hits, ring, ringn, any, wide, cn);
+    if (lane < ringn) src.write(ring[lane], cn);
+    __syncwarp();
+}
+
+__device__ __forceinline__ void query_rays(const SceneView& S, const GkrtRay* rays, GkrtHit* hits, uint32_t n, uint32_t mode,
+                                           uint32_t per, int cap, uint32_t* smem, Counters& cn) {
+    const bool wide = ((reinterpret_cast<uintptr_t>(rays) | reinterpret_cast<uintptr_t>(hits)) & 15u) == 0u;
+    const QueryRays src{S, rays, hits, mode == GKRT_TRACE_ANY, wide};
+    query_run(S, src, n, per, cap, smem, cn);
 }
 
 }  // namespace gk

@@ -280,8 +280,8 @@ GK_D f4 sky_sh(const SkySH& s, const GkrtFrameConstants& fc, f3 n) {
     return F4(r, g, bl, 1.0f) * (fc.has_sky ? fc.sky_intensity : 0.0f);
 }
 GK_D f4 unpack10(uint32_t p) {
-    float r = div_((float)(p & 0x3FFu), 1023.0f), g = div_((float)((p >> 10) & 0x3FFu), 1023.0f),
-          b = div_((float)((p >> 20) & 0x3FFu), 1023.0f);
+    float r = div1023((float)(p & 0x3FFu)), g = div1023((float)((p >> 10) & 0x3FFu)),
+          b = div1023((float)((p >> 20) & 0x3FFu));
     return F4(r * 512.0f, g * 512.0f, b * 512.0f, 0.0f * 512.0f);
 }
 GK_D f4 cube_sample(const uint32_t* cube, f3 n) {
@@ -296,11 +296,17 @@ GK_D f4 cube_sample(const uint32_t* cube, f3 n) {
     sk = sk + (float)((s0 >> 24) & 0xFFu) * wny;
     sk = sk + (float)(s1 & 0xFFu) * wx;
     sk = sk + (float)((s1 >> 8) & 0xFFu) * wnx;
-    const int ord[12] = {10, 11, 8, 9, 6, 7, 4, 5, 2, 3, 0, 1};
-    const float w[12] = {wx, wnx, wy, wny, wz, wnz, wx, wnx, wy, wny, wz, wnz};
+    // direct colours, then indirect ones, +x -x +y -y +z -z: of each pair of directions only the one
+    // the normal faces has a weight (the other would add exact zeros)
+    const int ox = n.x > 0.0f ? 10 : 11, oy = n.y > 0.0f ? 8 : 9, oz = n.z > 0.0f ? 6 : 7;
+    const float sx = n.x > 0.0f ? wx : wnx, sy = n.y > 0.0f ? wy : wny, sz = n.z > 0.0f ? wz : wnz;
     f4 col = F4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-    for (int i = 0; i < 12; ++i) col = col + unpack10(__ldg(&cube[ord[i]])) * w[i];
+    col = col + unpack10(__ldg(&cube[ox])) * sx;
+    col = col + unpack10(__ldg(&cube[oy])) * sy;
+    col = col + unpack10(__ldg(&cube[oz])) * sz;
+    col = col + unpack10(__ldg(&cube[ox - 6])) * sx;
+    col = col + unpack10(__ldg(&cube[oy - 6])) * sy;
+    col = col + unpack10(__ldg(&cube[oz - 6])) * sz;
     float k = sum > 0.0f ? div_(1.0f, sum) : 1.0f;
     col.x = col.x * k; col.y = col.y * k; col.z = col.z * k;
     sk = sk * k;
@@ -309,7 +315,7 @@ GK_D f4 cube_sample(const uint32_t* cube, f3 n) {
 }
 static __device__ __noinline__ f4 probe_grid(const ShadeScene& sc, float npx, float npy, float npz, f3 n);
 GK_D f4 probe_term(const ShadeScene& sc, f3 p, f3 n) {
-    float npx = div_(p.x - -24.0f, 0.25f), npy = div_(p.y - -0.34375f, 0.25f), npz = div_(p.z - -24.0f, 0.25f);
+    float npx = (p.x - -24.0f) * 4.0f, npy = (p.y - -0.34375f) * 4.0f, npz = (p.z - -24.0f) * 4.0f;
     // written as !(>=) so that a NaN position takes the early out
     if (!(npx >= 0.0f) || !(npy >= 0.0f) || !(npz >= 0.0f) || npx > 190.0f || npy > 46.0f || npz > 190.0f)
         return F4(0.0f, 0.0f, 0.0f, 1.0f);
@@ -327,20 +333,19 @@ static __device__ __noinline__ f4 probe_grid(const ShadeScene& sc, float npx, fl
         int ox = i & 1, oy = (i >> 1) & 1, oz = (i >> 2) & 1;
         size_t id = (size_t)(by + oy) * 192 * 192 + (size_t)(bz + oz) * 192 + (size_t)(bx + ox);
         uint32_t u0 = __ldg(&sc.voxels[id * 4 + 2]), u1 = __ldg(&sc.voxels[id * 4 + 3]);
-        float d0y = div_((float)((u0 >> 8) & 0xFFu), 255.0f);
+        float d0y = div255((float)((u0 >> 8) & 0xFFu));
         if (d0y < 0.01f) continue;
-        float d0z = div_((float)((u0 >> 16) & 0xFFu), 255.0f), d0w = div_((float)((u0 >> 24) & 0xFFu), 255.0f);
-        float d1x = div_((float)(u1 & 0xFFu), 255.0f), d1y = div_((float)((u1 >> 8) & 0xFFu), 255.0f);
-        float d1z = div_((float)((u1 >> 16) & 0xFFu), 255.0f), d1w = div_((float)((u1 >> 24) & 0xFFu), 255.0f);
+        float d0z = div255((float)((u0 >> 16) & 0xFFu)), d0w = div255((float)((u0 >> 24) & 0xFFu));
+        float d1x = div255((float)(u1 & 0xFFu)), d1y = div255((float)((u1 >> 8) & 0xFFu));
+        float d1z = div255((float)((u1 >> 16) & 0xFFu)), d1w = div255((float)((u1 >> 24) & 0xFFu));
         f3 pl = F3(frx - (float)ox, fry - (float)oy, frz - (float)oz);
         float dist = len3(pl);
         f3 dir = normalize3(pl);
-        float hl = sqrt_(mx(dir.x, 0.0f)) * d1x;
-        hl = hl + sqrt_(mx(-dir.x, 0.0f)) * d1y;
-        hl = hl + sqrt_(mx(dir.y, 0.0f)) * d1z;
-        hl = hl + sqrt_(mx(-dir.y, 0.0f)) * d1w;
-        hl = hl + sqrt_(mx(dir.z, 0.0f)) * d0z;
-        hl = hl + sqrt_(mx(-dir.z, 0.0f)) * d0w;
+        // the distance along the three directions it faces (the other three would add exact zeros; a NaN
+        // direction, at the probe itself, counts as none)
+        float hl = sqrt_(mx(fabsf(dir.x), 0.0f)) * (dir.x > 0.0f ? d1x : d1y);
+        hl = hl + sqrt_(mx(fabsf(dir.y), 0.0f)) * (dir.y > 0.0f ? d1z : d1w);
+        hl = hl + sqrt_(mx(fabsf(dir.z), 0.0f)) * (dir.z > 0.0f ? d0z : d0w);
         if (dist > hl + 0.05f) continue;
         float wx = ox == 0 ? 1.0f - frx : frx, wy = oy == 0 ? 1.0f - fry : fry, wz = oz == 0 ? 1.0f - frz : frz;
         float wgt = (wx * wy) * wz;

@@ -79,7 +79,7 @@ struct GkrtContext {
     DevInst* d_inst = nullptr;
     uint32_t* d_cubes = nullptr;                // probe grid (uploaded, or made by gkrt_probe_voxelize)
     uint32_t* d_voxels = nullptr;
-    uint32_t* d_cubes_prev = nullptr;           // snapshot the bake interpolates from
+    uint32_t* d_cubes_prev = nullptr;           // snapshot that a bake of many probes interpolates from
     // page-locked staging of the per-update tables (instance tables, emitter table, refit
     // transforms), so that their uploads are asynchronous on the caller's stream: two buffers
     // per table, each with the event recorded after its last upload
@@ -143,7 +143,7 @@ struct GkrtContext {
     uint32_t* d_error = nullptr;
     unsigned int* d_work = nullptr;             // pixel counter of the persistent trace kernel
     int num_sms = 1;
-    // stream-ordered scratch of calls that may overlap on several streams (the adjoint): what is freed
+    // stream-ordered scratch of calls that may overlap on several streams (adjoint, bake): what is freed
     // stays reserved for the next call, until the context ends
     cudaMemPool_t mem_pool = nullptr;
 };
@@ -1649,6 +1649,26 @@ int gkrt_trace_rays(GkrtContext* ctx, const GkrtRay* rays, GkrtHit* hits, uint32
     return GKRT_OK;
 }
 
+static int ensure_mem_pool(GkrtContext* ctx) {
+    if (ctx->mem_pool) return GKRT_OK;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    cudaMemPool_t pool = nullptr;
+    GK_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = UINT64_MAX;
+    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return cuda_fail(ctx, e, "cudaMemPoolSetAttribute");
+    }
+    ctx->mem_pool = pool;
+    return GKRT_OK;
+}
+
 // ---- ambient-cube probe grid ----
 
 namespace {
@@ -1683,9 +1703,14 @@ int gkrt_probe_bake(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_t fir
     cudaStream_t st = (cudaStream_t)stream;
     int rc = ensure_bvh(ctx, 0, st);
     if (rc != GKRT_OK) return rc;
-    if (!ctx->d_cubes_prev) GK_CUDA(cudaMalloc((void**)&ctx->d_cubes_prev, kProbeCount * 14 * sizeof(uint32_t)));
-    GK_CUDA(cudaMemcpyAsync(ctx->d_cubes_prev, ctx->d_cubes, kProbeCount * 14 * sizeof(uint32_t),
-                            cudaMemcpyDeviceToDevice, st));
+    if ((rc = ensure_mem_pool(ctx)) != GKRT_OK) return rc;
+    const uint32_t* cubes_read = ctx->d_cubes;
+    if (gkrt_probe_bake_needs_snapshot(count)) {
+        if (!ctx->d_cubes_prev) GK_CUDA(cudaMalloc((void**)&ctx->d_cubes_prev, kProbeCount * 14 * sizeof(uint32_t)));
+        GK_CUDA(cudaMemcpyAsync(ctx->d_cubes_prev, ctx->d_cubes, kProbeCount * 14 * sizeof(uint32_t),
+                                cudaMemcpyDeviceToDevice, st));
+        cubes_read = ctx->d_cubes_prev;
+    }
     ProbeLight lt;
     std::memset(&lt, 0, sizeof(lt));
     if (!ctx->lights_host.empty()) {
@@ -1708,8 +1733,10 @@ int gkrt_probe_bake(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_t fir
         if (!ctx->tex_sh.empty())
             std::memcpy(sh.c, ctx->tex_sh.data() + (size_t)fc->sky_index * 27u, sizeof(sh.c));
     }
-    GK_CUDA(gkrt_launch_probe_bake(shade_scene(ctx), *fc, lt, sh, first, count, ctx->d_cubes_prev, ctx->d_cubes,
-                                   (uint4*)ctx->d_voxels, ctx->d_counters, st));
+    GK_CUDA(gkrt_launch_probe_bake(shade_scene(ctx), *fc, lt, sh, first, count, cubes_read, ctx->d_cubes,
+                                   (uint4*)ctx->d_voxels, ctx->d_counters,
+                                   quad_stack_words(ctx->blas_bin_depth, ctx->tlas_bin_depth), ctx->num_sms, ctx->mem_pool,
+                                   st));
     return GKRT_OK;
 }
 
@@ -1770,26 +1797,6 @@ static uint32_t* standalone_err_word() {
     if (dev < 0) return nullptr;
     if (!words[dev] && cudaMalloc((void**)&words[dev], 4) != cudaSuccess) return nullptr;
     return words[dev];
-}
-
-static int ensure_mem_pool(GkrtContext* ctx) {
-    if (ctx->mem_pool) return GKRT_OK;
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = ctx->device;
-    cudaMemPool_t pool = nullptr;
-    GK_CUDA(cudaMemPoolCreate(&pool, &props));
-    uint64_t keep = UINT64_MAX;
-    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-        cudaMemPoolDestroy(pool);
-        return cuda_fail(ctx, e, "cudaMemPoolSetAttribute");
-    }
-    ctx->mem_pool = pool;
-    return GKRT_OK;
 }
 
 static int adjoint_checks(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_t spp) {

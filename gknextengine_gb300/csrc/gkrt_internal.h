@@ -233,12 +233,16 @@ cudaError_t gkrt_launch_trace_pass(const gk::ShadeScene& sc, const GkrtFrameCons
 constexpr uint32_t kPathPoolFields = 15;
 size_t gkrt_trace_pool_bytes(uint32_t pixels, int num_sms);
 // Probe grid (k_probes.cu): voxel distance data of probes [first, first + count), and one bake
-// step of those probes reading neighbours from cubes_prev (a snapshot of cubes).
+// step of those probes.
 cudaError_t gkrt_launch_probe_voxelize(const gk::ShadeScene& sc, uint32_t first, uint32_t count, uint4* voxels,
                                        unsigned long long* counters, cudaStream_t st);
+// cubes_read: the grid before the step, `cubes` itself unless gkrt_probe_bake_needs_snapshot(count).
+// mem: stream-ordered pool of the caller's that the launch takes its scratch from.
+bool gkrt_probe_bake_needs_snapshot(uint32_t count);
 cudaError_t gkrt_launch_probe_bake(const gk::ShadeScene& sc, const GkrtFrameConstants& fc, const gk::ProbeLight& lt,
-                                   const gk::SkySH& sh, uint32_t first, uint32_t count, const uint32_t* cubes_prev, uint32_t* cubes,
-                                   uint4* voxels, unsigned long long* counters, cudaStream_t st);
+                                   const gk::SkySH& sh, uint32_t first, uint32_t count, const uint32_t* cubes_read,
+                                   uint32_t* cubes, uint4* voxels, unsigned long long* counters, int stack_words,
+                                   int num_sms, cudaMemPool_t mem, cudaStream_t st);
 cudaError_t gkrt_launch_trace_rays(const gk::SceneView& S, const GkrtRay* rays, GkrtHit* hits, uint32_t n,
                                    uint32_t mode, unsigned long long* counters, int stack_words, int num_sms,
                                    cudaStream_t st);

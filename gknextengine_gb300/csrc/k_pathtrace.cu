@@ -21,12 +21,11 @@ namespace gk {
 constexpr int kPtThreads = kPoolThreads;
 constexpr int kPtWarps = kPoolWarps;
 constexpr int kPtMaxBlocks = 8;    // resident blocks per SM, at most
-// Resident blocks per SM, per instantiation. The traversal phase fits 128 registers; the shading
-// phase, longest with textures and emitters, spills below. Trace pass with 4 / 5 / 6 blocks (ms):
-// 1080p bricks 3.05 / 2.99 / 3.25, a 720p frame on the probe grid 2.04 / 1.73 / 1.80, 4K city
-// (emitters) 53.9 / 54.3 / 58.9, textured 1277 x 713 at 8 samples 8.0 / 9.5 / 11.0.
-template <bool kNee, bool kTex>
-constexpr int pt_blocks() { return kNee || kTex ? 4 : 5; }
+// Resident blocks per SM: the traversal phase fits 128 registers, the shading phase spills below.
+// Trace pass with 4 / 5 / 6 blocks (ms): 1080p bricks 2.97 / 3.11 / 3.25, Cornell 256 x 256
+// 0.146 / 0.159 / 0.175, 720p on the probe grid 1.25 / 1.18 / -, 4K city 53.9 / 54.3 / 58.9, textured
+// 1277 x 713 at 8 samples 8.0 / 9.5 / 11.0.
+constexpr int kPtBlocks = 4;
 constexpr float kCosCone = 0.999990482f;   // cos(0.25 deg), Shading.slang:897
 
 // Warp-aggregated flush: one atomic per counter per warp. Slots 0-5 are per pass
@@ -459,13 +458,14 @@ __device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
 // instructions per ray at 16.3 of 32 lanes, 419 at 12.4 when a warp traced its 32 rays to the end
 // before shading them all in registers; an issue in 38 % of the cycles, waits for instruction
 // fetch, node loads and fixed latencies in equal parts). Trace pass before / now, ms: 1080p bricks
-// 3.43 / 2.99, 4K city 91.9 / 53.3, textured 17.7 / 8.0, Cornell 256 x 256 0.164 / 0.150.
+// 3.43 / 2.97, 4K city 91.9 / 51.0, textured 17.7 / 8.0, Cornell 256 x 256 0.164 / 0.146, 720p on
+// the probe grid 1.98 / 1.25.
 //
 // Shared memory (dynamic): per-thread traversal stacks of stack_words entries (the scene's
 // depth bound), the world rays in flight, then each warp's path lists. A stack no larger than the
 // scene needs leaves the rest of the SM's 256 KB to L1, which serves the node fetches.
 template <bool kNee, bool kTex>
-__global__ void __launch_bounds__(kPtThreads, pt_blocks<kNee, kTex>()) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
+__global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
                                                            int P, PixelImages im, unsigned long long* counters,
                                                            unsigned int* work, int stack_words, float4* pools,
                                                            uint32_t np) {
