@@ -276,14 +276,22 @@ struct WgradArgs {
 };
 }
 cudaError_t gkrt_launch_conv_wgrad(const gk::WgradArgs& a, cudaStream_t st);
-cudaError_t gkrt_launch_avgpool2_bwd(const void* dout, int dout_c, int dout_off, void* din, int din_c, int din_off,
-                                     int B, int H, int W, int C, int accumulate, cudaStream_t st);
-cudaError_t gkrt_launch_upsample2_bwd(const void* dout, int dout_c, int dout_off, void* din, int din_c, int din_off,
-                                      int B, int h, int w, int C, cudaStream_t st);
-cudaError_t gkrt_launch_relu_bwd(void* dy, int dy_c, int dy_off, const void* y, int y_c, int y_off, long long npix,
-                                 int C, cudaStream_t st);
-cudaError_t gkrt_launch_bias_grad(const void* dp, int dp_c, int dp_off, long long npix, int C, float* db,
-                                  cudaStream_t st);
+// One layer's pre-activation and bias gradients (k_unet.cu). mode 0: dy as it is; 1: with a quarter of
+// src at half resolution added (the 2 x 2 average pooling's gradient); 2: the sums of src's 2 x 2 blocks
+// at double resolution in its place (the nearest upsampling's).
+namespace gk {
+struct LayerGradArgs {
+    int B, H, W, C;                          // dy's pixels and channels
+    __nv_bfloat16* dy;
+    int dy_c, dy_off;
+    const __nv_bfloat16* y;                  // the layer's output for the ReLU's mask, or null
+    int y_c, y_off;
+    const __nv_bfloat16* src;
+    int src_c, src_off;
+    float* db;                               // added to
+};
+}
+cudaError_t gkrt_launch_layer_grad(const gk::LayerGradArgs& a, int mode, cudaStream_t st);
 size_t gkrt_conv_smem_bytes(int cout);
 // The learned denoiser (unet.cu).
 namespace gk {

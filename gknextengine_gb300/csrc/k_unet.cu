@@ -1,10 +1,10 @@
 // k_unet.cu — the learned denoiser's training and inference kernels besides the forward
-// convolution (k_conv.cu): weight gradients on the tensor cores, and the element-wise,
-// pooling, loss and optimiser kernels.
+// convolution (k_conv.cu): weight gradients on the tensor cores, and the element-wise part of each
+// layer's backward pass.
 //
 // The weight gradient of a 3x3 convolution, dW[cout][tap][cin] = sum over pixels of
 // dP[p][cout] * X[p + tap offset][cin], is a GEMM with K = pixels whose operands TMA loads
-// straight from the NHWC tensors in the MN-major layout (k_conv_wgrad_tma, below).
+// straight from the NHWC tensors in the MN-major layout (k_conv_wgrad, below).
 #include <algorithm>
 
 #include "gk_umma.cuh"
@@ -15,66 +15,89 @@ namespace gk {
 namespace {
 
 // ---- weight gradient with TMA-fed MN-major operands ----
-// The same GEMM, dW[cout][tap][cin] = sum over pixels of dP[p][cout] X[p + tap][cin], with K =
-// pixels: NHWC rows hold the channels of one pixel contiguously, which is the MN-major layout
-// of both operands for K along pixels, so TMA loads them unchanged. A K step is a run of
-// kWtK pixels of one image row; per 64-channel group one box {64 channels, kWtK pixels} lands
-// 128-byte swizzled (an atom of 8 pixel rows x 128 bytes, atoms 1024 bytes apart along K). X's
-// box starts at the tap's shift, and TMA's zero fill outside the tensor is the padding. The CTA
-// takes one tap and a run of image rows: warp 0 issues the loads into a ring of stages, warp 1
-// the MMAs (M = 128 rows of dP's channels, zero past cout; N = cin), and all four warps the
-// epilogue (atomics into dW). Every wait is bounded.
+// dW[cout][tap][cin] = sum over pixels of dP[p][cout] X[p + tap][cin] with K = pixels: NHWC rows hold
+// the channels of one pixel contiguously, which is the MN-major layout of both operands for K along
+// pixels, so TMA loads them unchanged, in boxes of 32 channels x 32 pixels x some image rows, 64-byte
+// swizzled (atoms of 8 pixels x 64 bytes). All nine taps of 32 x 32 channels are one MMA of 128 x 96:
+//   M  rows are four boxes of X: the pairs (dx, 32-channel group) in order, four to an M block, each
+//      box loaded at its horizontal shift;
+//   N  columns are the dP rows r - 1, r, r + 1 of one 32-channel group against X's row r (the taps
+//      dy = 1, 0, -1): consecutive rows of one box with a halo row on each side.
+// So an X element is loaded three times (once per dx) instead of nine, a dP element 1.5 times, and no
+// MMA is issued per tap. TMA's zero fill is the padding, and the channels past the tensors' ends. A
+// CTA takes up to kWgCombos pairs of M block and dP group (their accumulators fill the 512 TMEM
+// columns) and a run of tiles; warp 0 issues the loads into a ring of stages, warp 1 the MMAs, and
+// all four warps add the accumulators to dW: a warp's 32 lanes hold 32 consecutive input
+// channels, and through shared memory each lane gets four of them for one 16-byte addition (a
+// quarter of the additions at L2: 224 x 96 took 43.5 us with one value per addition, now 39; a dW that
+// is not 16-byte aligned keeps the single ones). Every wait is bounded.
+// What bounds it: L2 reads of the boxes, the tensor core at three quarters of its rows. One tap of one
+// 64-channel atom per MMA, every operand read once per tap (or dP once per step for up to 32
+// input channels), took 119 us for 32 x 32 channels on 8 x 256 x 256 pixels (now 31), 261 for 96 x 32
+// (90), 75 for 64 x 64 on 8 x 128 x 128 (29), 72 for 224 x 96 on 8 x 64 x 64 (39).
 
 constexpr int kWtThreads = 128;
-constexpr int kWtK = 32;                        // pixels per K step
-constexpr int kWtAtom = kWtK * 128;             // one 64-channel box of a step: 4096 bytes
-constexpr int kWtStages = 4;
-constexpr int kWtGuard = 4096;                  // shared memory after the last stage, never written
+constexpr int kWgPix = 32;                       // pixels of a tile row
+constexpr int kWgRows = 4;                       // X rows of a tile
+constexpr int kWgRow = kWgPix * 64;              // one box row: 32 pixels x 32 channels
+constexpr int kWgXBox = kWgRows * kWgRow;        // 8 KB
+constexpr int kWgDBox = (kWgRows + 2) * kWgRow;  // 12 KB
+constexpr int kWgCombos = 5;
+constexpr int kWgSmem = 200 * 1024;              // stages
+constexpr int kWgMaxStages = 4;
+constexpr int kWgExtra = 1024 + 256 + 4 * 2048;  // alignment, barriers, the epilogue's exchange
 
-// Descriptor of an MN-major, 128-byte-swizzled operand: the leading byte offset is the stride
-// between 64-channel atoms along M (or N), 4096 bytes here, and the stride byte offset the one
-// between 8-row groups along K, 1024 bytes (the weight-gradient test against torch holds this
-// assignment; the swapped one gives wrong sums).
-__device__ __forceinline__ uint64_t wt_desc(uint32_t saddr) {
+// Descriptor of an MN-major, 64-byte-swizzled operand: the leading byte offset is the stride between
+// 32-channel atoms along M (or N), the stride byte offset the one between 8-pixel groups along K.
+__device__ __forceinline__ uint64_t wg_desc(uint32_t saddr, uint32_t atom_stride) {
     uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)(((uint32_t)kWtAtom >> 4) & 0x3FFFu) << 16;   // leading byte offset
-    d |= (uint64_t)((1024u >> 4) & 0x3FFFu) << 32;               // stride byte offset
+    d |= (uint64_t)((atom_stride >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)((512u >> 4) & 0x3FFFu) << 32;
     d |= (uint64_t)1u << 46;   // version
-    d |= (uint64_t)2u << 61;   // SWIZZLE_128B
+    d |= (uint64_t)4u << 61;   // SWIZZLE_64B
     return d;
 }
 
-// kTaps = 1: one tap per CTA (blockIdx.y), N = cin in nb atoms. kTaps = 9: all nine taps in one
-// CTA for cin <= 32 (one B atom per tap, nine accumulators of 32 columns in 512 TMEM columns),
-// so that dP is loaded once per step instead of once per tap.
-template <int kTaps>
-__global__ void __launch_bounds__(kWtThreads) k_conv_wgrad_tma(const __grid_constant__ CUtensorMap mdp,
-                                                               const __grid_constant__ CUtensorMap mx, WgradArgs a,
-                                                               int rows_per_cta, int nb) {
+// How the pairs of M block and dP group are split over CTAs: mb x gb pairs per CTA.
+struct WgPlan {
+    int na;            // 32-channel groups of X
+    int nblk, ng;      // M blocks, dP groups in all
+    int mb, gb;        // per CTA
+    int stages;
+    int xt, yt;        // tiles per image row, row tiles per image
+    int items;         // tiles in all
+    int segs;          // partial sums per CTA: the accumulators are added to dW and restarted
+    int vec;           // dW takes 16-byte additions (16-byte aligned; cin is a multiple of 16)
+};
+
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant__ CUtensorMap mdp,
+                                                           const __grid_constant__ CUtensorMap mx, WgradArgs a, WgPlan p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const int nbt = kTaps == 1 ? nb : 9;           // B atoms per stage
-    const int stage_bytes = (2 + nbt) * kWtAtom;   // A: 2 atoms (M = 128), then the B atoms
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kWtStages * stage_bytes + kWtGuard);
-    uint64_t* empty = full + kWtStages;
-    uint64_t* accb = empty + kWtStages;
+    const int stage_bytes = 4 * p.mb * kWgXBox + p.gb * kWgDBox;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
+    uint64_t* empty = full + kWgMaxStages;
+    uint64_t* accb = empty + kWgMaxStages;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(accb + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tap0 = kTaps == 1 ? (int)blockIdx.y : 0;
-    const int rows = a.B * a.H;
-    const int r0 = blockIdx.x * rows_per_cta, r1 = min(r0 + rows_per_cta, rows);
-    const int xsteps = (a.W + kWtK - 1) / kWtK;
-    const int nk = r1 > r0 ? (r1 - r0) * xsteps : 0;
-    const bool a_two = a.cout > 64;   // dP's second 64-channel atom is loaded, else it stays zero
-    const uint32_t ncols = kTaps == 9 ? 512u : a.cin <= 32 ? 32u : a.cin <= 64 ? 64u : a.cin <= 128 ? 128u : 256u;
+    float* tb = reinterpret_cast<float*>(smem + p.stages * stage_bytes + 256) + warp * 512;   // 2 KB per warp
+    const int msplit = (p.nblk + p.mb - 1) / p.mb;
+    const int blk0 = ((int)blockIdx.y % msplit) * p.mb, g0 = ((int)blockIdx.y / msplit) * p.gb;
+    const int nb = min(p.mb, p.nblk - blk0), ng = min(p.gb, p.ng - g0);
+    const int atoms = min(4 * nb, 3 * p.na - 4 * blk0);   // X boxes of this CTA's blocks
+    const int i0 = (int)((long long)p.items * blockIdx.x / gridDim.x);
+    const int i1 = (int)((long long)p.items * (blockIdx.x + 1) / gridDim.x);
+    const int combos = p.mb * p.gb;
+    const uint32_t ncols = combos == 1 ? 128u : combos == 2 ? 256u : 512u;
 
-    if (!a_two)   // the second A atom of every stage: zero rows of M
-        for (int st = 0; st < kWtStages; ++st)
-            for (int i = tid; i < kWtAtom / 16; i += kWtThreads)
-                reinterpret_cast<uint4*>(smem + st * stage_bytes + kWtAtom)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0) {
-        for (int st = 0; st < kWtStages; ++st) {
+        for (int st = 0; st < p.stages; ++st) {
             mbar_init(&full[st], 1);
             mbar_init(&empty[st], 1);
         }
@@ -82,7 +105,6 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad_tma(const __grid_cons
         *abort_flag = 0;
         mbar_fence_init();
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeroed atoms, for the tensor core
     if (warp == 1) {
         tmem_alloc(tslot, ncols);
         tmem_relinquish();
@@ -92,74 +114,98 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad_tma(const __grid_cons
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    if (warp == 0) {
-        if (lane == 0) {   // producer
-            const uint32_t bytes = (uint32_t)((a_two ? 2 : 1) + nbt) * (uint32_t)kWtAtom;
-            for (int k = 0; k < nk && !*abort_flag; ++k) {
-                const int s = k % kWtStages;
-                const uint32_t use = (uint32_t)(k / kWtStages);
-                if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1u) & 1u, a.err)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                const int row = r0 + k / xsteps, x0 = (k % xsteps) * kWtK;
-                const int img = row / a.H, y = row - img * a.H;
-                uint8_t* st = smem + s * stage_bytes;
-                mbar_expect_tx(&full[s], bytes);
-                tma_load_4d(st, &mdp, 0, x0, y, img, &full[s]);
-                if (a_two) tma_load_4d(st + kWtAtom, &mdp, 64, x0, y, img, &full[s]);
-                if (kTaps == 1) {
-                    const int dy = tap0 / 3 - 1, dx = tap0 % 3 - 1;
-                    for (int j = 0; j < nb; ++j)
-                        tma_load_4d(st + (2 + j) * kWtAtom, &mx, 64 * j, x0 + dx, y + dy, img, &full[s]);
-                } else {
-                    for (int t = 0; t < 9; ++t)
-                        tma_load_4d(st + (2 + t) * kWtAtom, &mx, 0, x0 + t % 3 - 1, y + t / 3 - 1, img, &full[s]);
+    for (int seg = 0; seg < p.segs; ++seg) {
+        const int k0 = (int)((long long)(i1 - i0) * seg / p.segs), k1 = (int)((long long)(i1 - i0) * (seg + 1) / p.segs);
+        if (warp == 0) {
+            if (lane == 0) {   // producer
+                const uint32_t bytes = (uint32_t)(atoms * kWgXBox + ng * kWgDBox);
+                for (int k = k0; k < k1 && !*abort_flag; ++k) {
+                    const int s = k % p.stages;
+                    const uint32_t use = (uint32_t)(k / p.stages);
+                    if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1u) & 1u, a.err)) {
+                        *abort_flag = 1;
+                        break;
+                    }
+                    const int it = i0 + k, per_img = p.xt * p.yt, img = it / per_img, rem = it - img * per_img;
+                    const int y0 = (rem / p.xt) * kWgRows, x0 = (rem % p.xt) * kWgPix;
+                    uint8_t* st = smem + s * stage_bytes;
+                    mbar_expect_tx(&full[s], bytes);
+                    for (int j = 0; j < atoms; ++j) {
+                        const int q = 4 * blk0 + j, dx = q / p.na, c = q - dx * p.na;
+                        tma_load_4d(st + j * kWgXBox, &mx, 32 * c, x0 + dx - 1, y0, img, &full[s]);
+                    }
+                    for (int g = 0; g < ng; ++g)
+                        tma_load_4d(st + 4 * p.mb * kWgXBox + g * kWgDBox, &mdp, 32 * (g0 + g), x0, y0 - 1, img, &full[s]);
                 }
             }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {   // MMA issuer
-            const uint32_t idesc = umma_idesc_bf16(128u, (uint32_t)a.cin) | (1u << 15) | (1u << 16);   // MN-major A, B
-            bool ok = true;
-            for (int k = 0; k < nk && ok; ++k) {
-                const int s = k % kWtStages;
-                if (!mbar_wait_bounded(&full[s], (uint32_t)(k / kWtStages) & 1u, a.err)) {
-                    *abort_flag = 1;
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t sa = smem_u32(smem + s * stage_bytes), sb = sa + 2u * (uint32_t)kWtAtom;
-                for (int t = 0; t < (kTaps == 1 ? 1 : 9); ++t)
-                    for (int kk = 0; kk < kWtK / 16; ++kk)   // 16 pixels (two 8-row groups) per MMA
-                        umma_bf16(tmem + (uint32_t)(t * 32), wt_desc(sa + 2048u * kk),
-                                  wt_desc(sb + (uint32_t)(t * kWtAtom) + 2048u * kk), idesc, (k | kk) != 0 ? 1u : 0u);
-                umma_commit(&empty[s]);
-            }
-        }
-        if (lane == 0) umma_commit(accb);
-    }
-    __syncwarp();
-    const bool ready = mbar_wait_bounded(accb, 0u, a.err) && nk > 0 && !*abort_flag;
-    __syncwarp();
-    tc_fence_after();
-    const int r = warp * 32 + lane;   // TMEM lane = cout row
-    for (int t = 0; t < (kTaps == 1 ? 1 : 9); ++t)
-        for (int c0 = 0; c0 < a.cin; c0 += 16) {
-            uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * 32 + c0), v);
-            tmem_ld_wait();
-            if (!ready || r >= a.cout) continue;
-            float* d = a.dw + ((size_t)r * 9 + (kTaps == 1 ? tap0 : t)) * a.cin + c0;
+        } else if (warp == 1) {
+            if (lane == 0) {   // MMA issuer
+                const uint32_t idesc = umma_idesc_bf16(128u, 96u) | (1u << 15) | (1u << 16);   // MN-major A, B
+                bool ok = true;
+                for (int k = k0; k < k1 && ok; ++k) {
+                    const int s = k % p.stages;
+                    if (!mbar_wait_bounded(&full[s], (uint32_t)(k / p.stages) & 1u, a.err)) {
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sx = smem_u32(smem + s * stage_bytes), sd = sx + (uint32_t)(4 * p.mb * kWgXBox);
+                    for (int m = 0; m < nb; ++m)
+                        for (int g = 0; g < ng; ++g) {
+                            const uint32_t d = tmem + (uint32_t)((m * p.gb + g) * 96);
+                            const uint64_t da = wg_desc(sx + (uint32_t)(4 * m * kWgXBox), (uint32_t)kWgXBox);
+                            const uint64_t db = wg_desc(sd + (uint32_t)(g * kWgDBox), (uint32_t)kWgRow);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float f = __uint_as_float(v[j]);
-                if (f != 0.0f) atomicAdd(d + j, f);
+                            for (int r = 0; r < kWgRows * 2; ++r)   // 16 pixels (two 8-pixel groups) per MMA
+                                umma_bf16(d, da + (uint64_t)(r * 64), db + (uint64_t)(r * 64), idesc,
+                                          k != k0 || r != 0 ? 1u : 0u);
+                        }
+                    umma_commit(&empty[s]);
+                }
+            }
+            if (lane == 0) umma_commit(accb);
+        }
+        __syncwarp();
+        const bool summed = mbar_wait_bounded(accb, (uint32_t)seg & 1u, a.err);
+        if (!summed) *abort_flag = 1;
+        const bool ready = summed && k1 > k0 && !*abort_flag;
+        __syncwarp();
+        tc_fence_after();
+        // lane `lane` of warp w: input channel 32 c + lane of box 4 (blk0 + m) + w
+        for (int part = 0; part < nb * ng * 6; ++part) {
+            const int m = part / (ng * 6), g = (part / 6) % ng, n0 = (part % 6) * 16;
+            const int q = 4 * (blk0 + m) + warp, dx = q / p.na, ci = 32 * (q - dx * p.na) + lane;
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((m * p.gb + g) * 96 + n0), v);
+            tmem_ld_wait();
+            if (!ready || q >= 3 * p.na) continue;   // the same for the whole warp
+            const int dy = 2 - n0 / 32;   // tap row: dP's row r - 1 is tap dy = +1
+            const int co = 32 * (g0 + g) + (n0 & 31);
+            float* d = a.dw + ((size_t)co * 9 + 3 * dy + dx) * a.cin + (ci - lane);
+            if (p.vec) {   // 16 x 32 values as four consecutive input channels per lane and addition
+#pragma unroll
+                for (int j = 0; j < 16; ++j) tb[j * 32 + lane] = __uint_as_float(v[j]);
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int r = 4 * j + (lane >> 3), c4 = 4 * (lane & 7);
+                    const float4 f = *reinterpret_cast<const float4*>(tb + r * 32 + c4);
+                    if (co + r < a.cout && ci - lane + c4 < a.cin) red_add4(d + (size_t)r * 9 * a.cin + c4, f);
+                }
+                __syncwarp();
+            } else if (ci < a.cin) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float f = __uint_as_float(v[j]);
+                    if (f != 0.0f && co + j < a.cout) atomicAdd(d + lane + (size_t)j * 9 * a.cin, f);
+                }
             }
         }
-    tc_fence_before();
-    __syncthreads();
+        tc_fence_before();
+        if (__syncthreads_or(*abort_flag)) break;   // the next sums start in the accumulators read here
+        tc_fence_after();
+    }
     if (warp == 1) tmem_dealloc(tmem, ncols);
 }
 
@@ -185,76 +231,64 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float* v) {
     *reinterpret_cast<uint4*>(p) = u;
 }
 
-// d_in (+)= d_out / 4 for each of the 2x2 inputs (accumulate: add to what is there)
-__global__ void k_avgpool2_bwd(const __nv_bfloat16* dout, int dout_c, int dout_off, __nv_bfloat16* din, int din_c,
-                               int din_off, int B, int H, int W, int C, int accumulate) {   // H, W: input size
-    const int g8 = C / 8;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * H * W * g8) return;
-    const int g = i % g8, p = i / g8;
-    const int x = p % W, y = (p / W) % H, b = p / (W * H);
-    const size_t q = (size_t)(b * (H / 2) + y / 2) * (W / 2) + x / 2;
-    float v[8], d[8];
-    ld8(dout + q * dout_c + dout_off + 8 * g, v);
-    __nv_bfloat16* dst = din + (size_t)p * din_c + din_off + 8 * g;
-    if (accumulate) ld8(dst, d);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = 0.25f * v[j] + (accumulate ? d[j] : 0.0f);
-    st8(dst, v);
-}
-
-// d_in = sum of the 2x2 output gradients it was copied to
-__global__ void k_upsample2_bwd(const __nv_bfloat16* dout, int dout_c, int dout_off, __nv_bfloat16* din, int din_c,
-                                int din_off, int B, int h, int w, int C) {   // h, w: input size
-    const int g8 = C / 8;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * h * w * g8) return;
-    const int g = i % g8, p = i / g8;
-    const int x = p % w, y = (p / w) % h, b = p / (w * h);
-    const int W = 2 * w, H = 2 * h;
-    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, v[8];
-    for (int k = 0; k < 4; ++k) {
-        const size_t q = (size_t)(b * H + 2 * y + (k >> 1)) * W + 2 * x + (k & 1);
-        ld8(dout + q * dout_c + dout_off + 8 * g, v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s[j] += v[j];
-    }
-    st8(din + (size_t)p * din_c + din_off + 8 * g, s);
-}
-
-// dP = dY * (Y > 0) (ReLU), written in place of dY
-__global__ void k_relu_bwd(__nv_bfloat16* dy, int dy_c, int dy_off, const __nv_bfloat16* y, int y_c, int y_off,
-                           int npix, int C) {
-    const int g8 = C / 8;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npix * g8) return;
-    const int g = i % g8, p = i / g8;
-    float a[8], b[8];
-    __nv_bfloat16* d = dy + (size_t)p * dy_c + dy_off + 8 * g;
-    ld8(d, a);
-    ld8(y + (size_t)p * y_c + y_off + 8 * g, b);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if (!(b[j] > 0.0f)) a[j] = 0.0f;
-    st8(d, a);
-}
-
-// db[c] += sum over pixels of dP[p][c]; one block per run of pixels. Thread t owns the 8
-// channels 8 (t % G) .. +7 (G = C / 8, one 16-byte load per pixel) of every (256 / G)-th pixel
-// of the run and sums them in registers; the threads of each channel group are then reduced
-// in shared memory and each channel gets one atomic per block.
-__global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* dp, int dp_c, int dp_off, long long npix,
-                                                   int C, int run, float* db) {
+// One layer's gradient of its pre-activation, dP = dY * (Y > 0), in place of dY, and its bias
+// gradient db[c] += sum over pixels of dP[p][c], in one pass over dY; and on the way there what dY
+// is still to receive:
+//   kPool      dY += d_pool / 4 of the half-resolution pixel (the 2 x 2 average pooling's gradient);
+//   kUpsample  dY = sum of the 2 x 2 double-resolution gradients it was copied to;
+// each rounded to bf16 before the ReLU's mask, as a pass of its own would store it. y null: no ReLU.
+// One block per run of pixels. Thread t owns the 8 channels 8 (t % G) .. +7 (G = C / 8, 16-byte
+// loads and stores) of every (256 / G)-th pixel of the run and sums them in registers; the threads
+// of each channel group are then reduced in shared memory and each channel gets one atomic per
+// block. Three separate passes and a run of 1024 pixels per block (8 blocks for the eighth-resolution
+// layers) took 0.45 ms of an 8 x 256 x 256 training step; now 0.13.
+enum GradMode { kGradPlain = 0, kGradPool = 1, kGradUpsample = 2 };
+template <int kMode>
+__global__ void __launch_bounds__(256) k_layer_grad(LayerGradArgs a, int run) {
     __shared__ float part[256 * 8];
-    const int G = C / 8, per = 256 / G;
+    const int G = a.C / 8, per = 256 / G;
     const int g = threadIdx.x % G, k = threadIdx.x / G;
     float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     if (k < per) {
-        const long long p0 = (long long)blockIdx.x * run;
-        const long long p1 = p0 + run < npix ? p0 + run : npix;
-        for (long long p = p0 + k; p < p1; p += per) {
+        const int p0 = blockIdx.x * run, p1 = min(p0 + run, a.B * a.H * a.W);
+        for (int p = p0 + k; p < p1; p += per) {
             float v[8];
-            ld8(dp + p * dp_c + dp_off + 8 * g, v);
+            __nv_bfloat16* d = a.dy + (size_t)p * a.dy_c + a.dy_off + 8 * g;
+            if (kMode == kGradUpsample) {
+                const int x = p % a.W, y = (p / a.W) % a.H, b = p / (a.W * a.H);
+                float t[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const size_t s = (size_t)(b * 2 * a.H + 2 * y + (q >> 1)) * (2 * a.W) + 2 * x + (q & 1);
+                    ld8(a.src + s * a.src_c + a.src_off + 8 * g, t);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] += t[j];
+                }
+            } else {
+                ld8(d, v);
+                if (kMode == kGradPool) {
+                    const int x = p % a.W, y = (p / a.W) % a.H, b = p / (a.W * a.H);
+                    const size_t s = (size_t)(b * (a.H / 2) + y / 2) * (a.W / 2) + x / 2;
+                    float t[8];
+                    ld8(a.src + s * a.src_c + a.src_off + 8 * g, t);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] = 0.25f * t[j] + v[j];
+                }
+            }
+            if (kMode != kGradPlain) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+            }
+            if (a.y) {
+                float y8[8];
+                ld8(a.y + (size_t)p * a.y_c + a.y_off + 8 * g, y8);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (!(y8[j] > 0.0f)) v[j] = 0.0f;
+            }
+            if (a.y || kMode != kGradPlain) st8(d, v);
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] += v[j];
         }
@@ -262,11 +296,11 @@ __global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* dp, int 
 #pragma unroll
     for (int j = 0; j < 8; ++j) part[threadIdx.x * 8 + j] = acc[j];
     __syncthreads();
-    if (threadIdx.x < C) {
+    if (threadIdx.x < a.C) {
         const int c = threadIdx.x, cg = c / 8, cj = c % 8;
         float sum = 0.0f;
         for (int i = 0; i < per; ++i) sum += part[(i * G + cg) * 8 + cj];
-        if (sum != 0.0f) atomicAdd(&db[c], sum);
+        if (sum != 0.0f) atomicAdd(&a.db[c], sum);
     }
 }
 
@@ -276,11 +310,35 @@ __global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* dp, int 
 
 using namespace gk;
 
-cudaError_t gkrt_encode_tmap_bf16_sw128(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims,
-                                        const uint64_t* strides_bytes, const uint32_t* box);
+cudaError_t gkrt_encode_tmap_bf16(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims,
+                                  const uint64_t* strides_bytes, const uint32_t* box);
 
-static size_t wgrad_tma_smem(int nbt) {   // nbt: B atoms per stage
-    return (size_t)kWtStages * (size_t)(2 + nbt) * kWtAtom + kWtGuard + 256 + 1024;
+// The split that loads least: each CTA of a pixel run loads 4 mb boxes of X and gb of dP (1.5 times
+// as tall), at least two stages in shared memory.
+static WgPlan wgrad_plan(const WgradArgs& a) {
+    WgPlan p{};
+    p.na = (a.cin + 31) / 32;
+    p.nblk = (3 * p.na + 3) / 4;
+    p.ng = (a.cout + 31) / 32;
+    double best = 1e30;
+    for (int mb = 1; mb <= std::min(p.nblk, kWgCombos); ++mb)
+        for (int gb = 1; gb <= std::min(p.ng, kWgCombos / mb); ++gb) {
+            const int bytes = 4 * mb * kWgXBox + gb * kWgDBox;
+            if (2 * bytes > kWgSmem) continue;
+            const int groups = ((p.nblk + mb - 1) / mb) * ((p.ng + gb - 1) / gb);
+            const double cost = groups * (double)bytes;
+            if (cost < best) {
+                best = cost;
+                p.mb = mb;
+                p.gb = gb;
+                p.stages = std::min(kWgMaxStages, kWgSmem / bytes);
+            }
+        }
+    p.xt = (a.W + kWgPix - 1) / kWgPix;
+    p.yt = (a.H + kWgRows - 1) / kWgRows;
+    p.items = a.B * p.xt * p.yt;
+    p.vec = ((uintptr_t)a.dw & 15u) == 0u;
+    return p;
 }
 
 cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
@@ -290,76 +348,52 @@ cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
         a.x_valid > a.cin || a.x_valid % 8 || a.x_off + xv > a.x_c || ((uintptr_t)a.dp & 15u) ||
         ((uintptr_t)a.x & 15u) || a.B < 1 || a.H < 1 || a.W < 1)
         return cudaErrorInvalidValue;
+    if ((long long)a.B * ((a.W + kWgPix - 1) / kWgPix) * ((a.H + kWgRows - 1) / kWgRows) > 0x7FFFFFFFLL)
+        return cudaErrorInvalidValue;
     static int sms_dev[kMaxDevices] = {};
-    static bool attr_set[kMaxDevices] = {};   // set once per device for the largest stage
     const int dev = current_device_slot();
     if (dev < 0) return cudaErrorInvalidDevice;
     if (!sms_dev[dev]) {
-        cudaError_t e = cudaDeviceGetAttribute(&sms_dev[dev], cudaDevAttrMultiProcessorCount, dev);
+        cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem + kWgExtra);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms_dev[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
-    }
-    if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad_tma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)wgrad_tma_smem(4));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_conv_wgrad_tma<9>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)wgrad_tma_smem(9));
-        if (e != cudaSuccess) return e;
-        attr_set[dev] = true;
     }
     const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B;
-    const uint32_t box[4] = {64u, (uint32_t)kWtK, 1u, 1u};
+    const uint32_t dbox[4] = {32u, (uint32_t)kWgPix, (uint32_t)(kWgRows + 2), 1u};
+    const uint32_t xbox[4] = {32u, (uint32_t)kWgPix, (uint32_t)kWgRows, 1u};
     CUtensorMap mdp, mx;
     const uint64_t dd[4] = {(uint64_t)a.cout, W, H, B};
     const uint64_t ds[3] = {(uint64_t)a.dp_c * 2, W * a.dp_c * 2, H * W * a.dp_c * 2};
-    cudaError_t e = gkrt_encode_tmap_bf16_sw128(&mdp, a.dp + a.dp_off, 4, dd, ds, box);
+    cudaError_t e = gkrt_encode_tmap_bf16(&mdp, a.dp + a.dp_off, 4, dd, ds, dbox);
     if (e != cudaSuccess) return e;
     const uint64_t xd[4] = {(uint64_t)xv, W, H, B};   // channels past xv: TMA's zero fill
     const uint64_t xs[3] = {(uint64_t)a.x_c * 2, W * a.x_c * 2, H * W * a.x_c * 2};
-    if ((e = gkrt_encode_tmap_bf16_sw128(&mx, a.x + a.x_off, 4, xd, xs, box)) != cudaSuccess) return e;
-    const int nb = (a.cin + 63) / 64;
-    const long long rows = (long long)a.B * a.H;
-    if (a.cin <= 32) {   // all taps per CTA (512 TMEM columns: one CTA per SM), a run of image rows each
-        const long long target = sms_dev[dev];
-        const int rows_per_cta = (int)std::max(1LL, (rows + target - 1) / target);
-        const dim3 grid((unsigned)((rows + rows_per_cta - 1) / rows_per_cta), 1);
-        k_conv_wgrad_tma<9><<<grid, kWtThreads, wgrad_tma_smem(9), st>>>(mdp, mx, a, rows_per_cta, 1);
-        return cudaGetLastError();
-    }
-    // about two CTAs per SM over the nine taps, each a run of image rows
-    const long long target = 2LL * sms_dev[dev];
-    const int rows_per_cta = (int)std::max(1LL, (rows * 9 + target - 1) / target);
-    const dim3 grid((unsigned)((rows + rows_per_cta - 1) / rows_per_cta), 9);
-    k_conv_wgrad_tma<1><<<grid, kWtThreads, wgrad_tma_smem(nb), st>>>(mdp, mx, a, rows_per_cta, nb);
+    if ((e = gkrt_encode_tmap_bf16(&mx, a.x + a.x_off, 4, xd, xs, xbox)) != cudaSuccess) return e;
+    WgPlan p = wgrad_plan(a);
+    const int stage_bytes = 4 * p.mb * kWgXBox + p.gb * kWgDBox;
+    const int groups = ((p.nblk + p.mb - 1) / p.mb) * ((p.ng + p.gb - 1) / p.gb);
+    // one CTA per SM (its stages fill the shared memory), at least two tiles each. An FP32 sum covers at
+    // most a 34th of the pixels: with 30 CTAs, 224 x 96 on 8 x 64 x 64 was off by 1.3e-6 of the largest
+    // value in one sum each (27 us) and is by 6.2e-7 in two (39 us).
+    const int grid = std::max(1, std::min((p.items + 1) / 2, sms_dev[dev] / groups));
+    p.segs = (34 + grid - 1) / grid;
+    if (p.items < 34 * 4) p.segs = 1;
+    k_conv_wgrad<<<dim3((unsigned)grid, (unsigned)groups), kWtThreads, (size_t)p.stages * stage_bytes + kWgExtra, st>>>(
+        mdp, mx, a, p);
     return cudaGetLastError();
 }
 
-static inline unsigned nblk(long long n) { return (unsigned)((n + 255) / 256); }
-
-cudaError_t gkrt_launch_avgpool2_bwd(const void* dout, int dout_c, int dout_off, void* din, int din_c, int din_off,
-                                     int B, int H, int W, int C, int accumulate, cudaStream_t st) {
-    k_avgpool2_bwd<<<nblk((long long)B * H * W * (C / 8)), 256, 0, st>>>((const __nv_bfloat16*)dout, dout_c, dout_off,
-                                                                   (__nv_bfloat16*)din, din_c, din_off, B, H, W, C,
-                                                                   accumulate);
-    return cudaGetLastError();
-}
-cudaError_t gkrt_launch_upsample2_bwd(const void* dout, int dout_c, int dout_off, void* din, int din_c, int din_off,
-                                      int B, int h, int w, int C, cudaStream_t st) {
-    k_upsample2_bwd<<<nblk((long long)B * h * w * (C / 8)), 256, 0, st>>>((const __nv_bfloat16*)dout, dout_c, dout_off,
-                                                                    (__nv_bfloat16*)din, din_c, din_off, B, h, w, C);
-    return cudaGetLastError();
-}
-cudaError_t gkrt_launch_relu_bwd(void* dy, int dy_c, int dy_off, const void* y, int y_c, int y_off, long long npix,
-                                 int C, cudaStream_t st) {
-    k_relu_bwd<<<nblk(npix * (C / 8)), 256, 0, st>>>((__nv_bfloat16*)dy, dy_c, dy_off, (const __nv_bfloat16*)y, y_c,
-                                                     y_off, (int)npix, C);
-    return cudaGetLastError();
-}
-cudaError_t gkrt_launch_bias_grad(const void* dp, int dp_c, int dp_off, long long npix, int C, float* db,
-                                  cudaStream_t st) {
-    if (C > 256 || C % 8 || dp_c % 8 || dp_off % 8 || ((uintptr_t)dp & 15u)) return cudaErrorInvalidValue;
-    const int run = 1024;
-    k_bias_grad<<<(unsigned)((npix + run - 1) / run), 256, 0, st>>>((const __nv_bfloat16*)dp, dp_c, dp_off, npix, C,
-                                                                   run, db);
+cudaError_t gkrt_launch_layer_grad(const LayerGradArgs& a, int mode, cudaStream_t st) {
+    const long long npix = (long long)a.B * a.H * a.W;
+    if (a.C > 128 || a.C % 8 || a.C < 8 || a.dy_c % 8 || a.dy_off % 8 || ((uintptr_t)a.dy & 15u) ||
+        npix > 0x7FFFFFFFLL / 4)
+        return cudaErrorInvalidValue;
+    // about four blocks per SM, each thread at least four pixels
+    const int per = 256 / (a.C / 8);
+    const int run = (int)std::max<long long>(4 * per, (npix + 607) / 608);
+    const unsigned blocks = (unsigned)((npix + run - 1) / run);
+    if (mode == kGradPool) k_layer_grad<kGradPool><<<blocks, 256, 0, st>>>(a, run);
+    else if (mode == kGradUpsample) k_layer_grad<kGradUpsample><<<blocks, 256, 0, st>>>(a, run);
+    else k_layer_grad<kGradPlain><<<blocks, 256, 0, st>>>(a, run);
     return cudaGetLastError();
 }

@@ -116,37 +116,48 @@ __global__ void __launch_bounds__(256) k_pack_frame(const float4* sd, const floa
     for (int j = threadIdx.x; j < n * (kXc / 8); j += 256) o[j] = packed[j];
 }
 
-// gradient of the loss in log space; loss sum in FP64
-__global__ void k_loss(const float* y, const float* target, long long npix, float gscale, __nv_bfloat16* gy,
-                       double* loss) {
+// The bf16 32-channel gradient of one pixel's raw output: three channels, zeros after them.
+__device__ __forceinline__ void store_grad(__nv_bfloat16* gy, long long p, float a, float b, float c) {
+    const __nv_bfloat162 ab = __floats2bfloat162_rn(a, b), c0 = __floats2bfloat162_rn(c, 0.0f);
+    uint4* o = reinterpret_cast<uint4*>(gy + p * 32);
+    o[0] = make_uint4(*reinterpret_cast<const uint32_t*>(&ab), *reinterpret_cast<const uint32_t*>(&c0), 0u, 0u);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) o[k] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// gradient of the loss in log space; loss sum in FP64 (16-byte accesses: 105 us for 8 x 256 x 256
+// pixels with a 2-byte store per channel, now 12)
+__global__ void __launch_bounds__(256) k_loss(const float4* y, const float* target, long long npix, float gscale,
+                                              __nv_bfloat16* gy, double* loss) {
     __shared__ double part[8];
-    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long p = blockIdx.x * 256LL + threadIdx.x;
     double l = 0.0;
     if (p < npix) {
-        __nv_bfloat16* g = gy + p * 32;
+        const float4 yv = y[p];
+        const float yc[3] = {yv.x, yv.y, yv.z};
+        float g[3];
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const float e = y[p * 4 + c] - log1pf(fmaxf(target[p * 3 + c], 0.0f));
+            const float e = yc[c] - log1pf(fmaxf(target[p * 3 + c], 0.0f));
             l += (double)e * e;
-            g[c] = __float2bfloat16_rn(2.0f * e * gscale);
+            g[c] = 2.0f * e * gscale;
         }
-        for (int c = 3; c < 32; ++c) g[c] = __float2bfloat16_rn(0.0f);
+        store_grad(gy, p, g[0], g[1], g[2]);
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xFFFFFFFFu, l, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = l;
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += part[k];
+        for (int k = 0; k < 8; ++k) s += part[k];
         atomicAdd(loss, s);
     }
 }
 
 // caller-supplied gradient of the raw output (f32, 4 channels) to the bf16 32-channel layout
-__global__ void k_grad_in(const float* d, long long npix, __nv_bfloat16* gy) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= npix * 32) return;
-    const int c = (int)(i % 32);
-    gy[i] = __float2bfloat16_rn(c < 3 ? d[(i / 32) * 4 + c] : 0.0f);
+__global__ void __launch_bounds__(256) k_grad_in(const float* d, long long npix, __nv_bfloat16* gy) {
+    const long long p = blockIdx.x * 256LL + threadIdx.x;
+    if (p < npix) store_grad(gy, p, d[p * 4], d[p * 4 + 1], d[p * 4 + 2]);
 }
 
 __global__ void k_out_linear(const float* y, long long npix, float* out) {
@@ -156,28 +167,43 @@ __global__ void k_out_linear(const float* y, long long npix, float* out) {
     out[p * 4 + 3] = 1.0f;
 }
 
-__global__ void k_adam(float* p, const float* g, float* m, float* v, long long n, float lr, float b1, float b2,
-                       float eps, float c1, float c2) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-}
-
-// bf16 weights in both layouts: wb[co][tap][ci] and wf[ci][8 - tap][co]
-__global__ void k_weights_bf16(const float* w, int cin, int cout, __nv_bfloat16* wb, __nv_bfloat16* wf) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= 9LL * cin * cout) return;
-    const int ci = (int)(i % cin);
-    const int tap = (int)((i / cin) % 9);
-    const int co = (int)(i / (9LL * cin));
-    const __nv_bfloat16 h = __float2bfloat16_rn(w[i]);
-    wb[i] = h;
-    wf[((long long)ci * 9 + (8 - tap)) * cout + co] = h;
+// Where each layer's parameters lie: weights at w, biases at b of the FP32 array, weights at h of the
+// bf16 ones; and its channels.
+struct ParamMap {
+    int w[kUnetLayers], b[kUnetLayers], h[kUnetLayers], cin[kUnetLayers], cout[kUnetLayers];
+    int n;
+};
+struct AdamStep {
+    float lr, b1, b2, eps, c1, c2;
+};
+// One pass over the parameters: with kStep Adam's update, and the weights' bf16 copies in both
+// layouts, wb[co][tap][ci] and wf[ci][8 - tap][co]. (A launch per layer for the copies took 56 us a
+// step.)
+template <bool kStep>
+__global__ void __launch_bounds__(256) k_params(ParamMap map, float* p, const float* g, float* m, float* v, AdamStep s,
+                                                __nv_bfloat16* wb, __nv_bfloat16* wf) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= map.n) return;
+    float w = p[i];
+    if (kStep) {
+        const float gi = g[i];
+        const float mi = s.b1 * m[i] + (1.0f - s.b1) * gi;
+        const float vi = s.b2 * v[i] + (1.0f - s.b2) * gi * gi;
+        m[i] = mi;
+        v[i] = vi;
+        w -= s.lr * (mi * s.c1) / (sqrtf(vi * s.c2) + s.eps);
+        p[i] = w;
+    }
+    int l = 0;
+#pragma unroll
+    for (int k = 1; k < kUnetLayers; ++k) l += i >= map.w[k] ? 1 : 0;
+    const int j = i - map.w[l];
+    if (i >= map.b[l]) return;
+    const int cin = map.cin[l], cout = map.cout[l];
+    const int ci = j % cin, tap = (j / cin) % 9, co = j / (9 * cin);
+    const __nv_bfloat16 h = __float2bfloat16_rn(w);
+    wb[map.h[l] + j] = h;
+    wf[map.h[l] + (ci * 9 + (8 - tap)) * cout + co] = h;
 }
 
 // dec0a's weights (fp32 [32][9][96]; input channels 0-63 the nearest-upsampled dec1b, 64-95
@@ -212,6 +238,12 @@ __global__ void k_weights_subpixel(const float* w, __nv_bfloat16* wup, __nv_bflo
 inline unsigned nb(long long n) { return (unsigned)((n + 255) / 256); }
 
 }  // namespace
+
+// Where an output's gradient comes from besides what dY holds (Unet::layer_bwd).
+struct GradFrom {
+    const __nv_bfloat16 *pooled, *copied;
+    int src_c;
+};
 
 struct Unet {
     size_t woff[kUnetLayers], boff[kUnetLayers], wb_off[kUnetLayers];
@@ -265,13 +297,23 @@ struct Unet {
         return cudaMemset(err, 0, 4);
     }
 
-    // bf16 copies of the weights from the FP32 masters
-    cudaError_t refresh_bf16(cudaStream_t st) {
+    ParamMap param_map() const {
+        ParamMap map;
         for (int l = 0; l < kUnetLayers; ++l) {
-            const long long n = 9LL * kLayers[l].cin * kLayers[l].cout;
-            k_weights_bf16<<<nb(n), 256, 0, st>>>(p + woff[l], kLayers[l].cin, kLayers[l].cout, wb + wb_off[l],
-                                                  wf + wb_off[l]);
+            map.w[l] = (int)woff[l];
+            map.b[l] = (int)boff[l];
+            map.h[l] = (int)wb_off[l];
+            map.cin[l] = kLayers[l].cin;
+            map.cout[l] = kLayers[l].cout;
         }
+        map.n = (int)nparams;
+        return map;
+    }
+
+    // the weights' bf16 copies from the FP32 masters, after an Adam step if given
+    cudaError_t update_params(const AdamStep* s, cudaStream_t st) {
+        if (s) k_params<true><<<nb((long long)nparams), 256, 0, st>>>(param_map(), p, g, m, v, *s, wb, wf);
+        else k_params<false><<<nb((long long)nparams), 256, 0, st>>>(param_map(), p, g, m, v, AdamStep{}, wb, wf);
         k_weights_subpixel<<<nb(128 * 9 * 64), 256, 0, st>>>(p + woff[D0A], wup, we0b);
         return cudaGetLastError();
     }
@@ -393,15 +435,22 @@ struct Unet {
     }
 
     // One layer's backward: dP (in place of dY) = dY * relu', weight and bias gradients, and
-    // (if din) the input gradient through the mirrored weights.
+    // (if din) the input gradient through the mirrored weights. pooled: the gradient of the output's
+    // 2 x 2 averages, still to be added to dY; copied: the gradient of its nearest upsampling, dY
+    // being its 2 x 2 sums (channels from 0 of src_c).
     cudaError_t layer_bwd(int l, __nv_bfloat16* dy, int dy_c, int dy_off, const __nv_bfloat16* y_act, int y_c,
                           int y_off, const __nv_bfloat16* x, int x_c, int x_off, __nv_bfloat16* din, int level,
-                          cudaStream_t st) {
+                          cudaStream_t st, GradFrom from = GradFrom{nullptr, nullptr, 0}) {
         cudaError_t e;
         const int h = H >> level, w = W >> level;
-        const long long npix = (long long)B * h * w;
         const LayerDef& L = kLayers[l];
-        if (L.relu) GK_T(gkrt_launch_relu_bwd(dy, dy_c, dy_off, y_act, y_c, y_off, npix, L.cout, st));
+        LayerGradArgs ga{};
+        ga.B = B; ga.H = h; ga.W = w; ga.C = L.cout;
+        ga.dy = dy; ga.dy_c = dy_c; ga.dy_off = dy_off;
+        ga.y = L.relu ? y_act : nullptr; ga.y_c = y_c; ga.y_off = y_off;
+        ga.src = from.pooled ? from.pooled : from.copied; ga.src_c = from.src_c; ga.src_off = 0;
+        ga.db = g + boff[l];
+        GK_T(gkrt_launch_layer_grad(ga, from.pooled ? 1 : from.copied ? 2 : 0, st));
         WgradArgs wa{};
         wa.B = B; wa.H = h; wa.W = w;
         wa.dp = dy; wa.dp_c = dy_c; wa.dp_off = dy_off; wa.cout = L.cout;
@@ -410,7 +459,6 @@ struct Unet {
         wa.dw = g + woff[l];
         wa.err = err;
         GK_T(gkrt_launch_conv_wgrad(wa, st));
-        GK_T(gkrt_launch_bias_grad(dy, dy_c, dy_off, npix, L.cout, g + boff[l], st));
         if (din) {
             ConvArgs a{};
             a.B = B; a.H = h; a.W = w;
@@ -431,24 +479,18 @@ struct Unet {
         GK_T(layer_bwd(OUT, gy, 32, 0, nullptr, 0, 0, d0b, 32, 0, g_d0b, 0, st));
         GK_T(layer_bwd(D0B, g_d0b, 32, 0, d0b, 32, 0, d0a, 32, 0, g_d0a, 0, st));
         GK_T(layer_bwd(D0A, g_d0a, 32, 0, d0a, 32, 0, cat0, 96, 0, g_cat0, 0, st));
-        GK_T(gkrt_launch_upsample2_bwd(g_cat0, 96, 0, g_d1b, 64, 0, B, H >> 1, W >> 1, 64, st));
-        GK_T(layer_bwd(D1B, g_d1b, 64, 0, d1b, 64, 0, d1a, 64, 0, g_d1a, 1, st));
+        GK_T(layer_bwd(D1B, g_d1b, 64, 0, d1b, 64, 0, d1a, 64, 0, g_d1a, 1, st, GradFrom{nullptr, g_cat0, 96}));
         GK_T(layer_bwd(D1A, g_d1a, 64, 0, d1a, 64, 0, cat1, 160, 0, g_cat1, 1, st));
-        GK_T(gkrt_launch_upsample2_bwd(g_cat1, 160, 0, g_d2b, 96, 0, B, H >> 2, W >> 2, 96, st));
-        GK_T(layer_bwd(D2B, g_d2b, 96, 0, d2b, 96, 0, d2a, 96, 0, g_d2a, 2, st));
+        GK_T(layer_bwd(D2B, g_d2b, 96, 0, d2b, 96, 0, d2a, 96, 0, g_d2a, 2, st, GradFrom{nullptr, g_cat1, 160}));
         GK_T(layer_bwd(D2A, g_d2a, 96, 0, d2a, 96, 0, cat2, 224, 0, g_cat2, 2, st));
-        GK_T(gkrt_launch_upsample2_bwd(g_cat2, 224, 0, g_e3b, 128, 0, B, H >> 3, W >> 3, 128, st));
-        GK_T(layer_bwd(E3B, g_e3b, 128, 0, e3b, 128, 0, e3a, 128, 0, g_e3a, 3, st));
+        GK_T(layer_bwd(E3B, g_e3b, 128, 0, e3b, 128, 0, e3a, 128, 0, g_e3a, 3, st, GradFrom{nullptr, g_cat2, 224}));
         GK_T(layer_bwd(E3A, g_e3a, 128, 0, e3a, 128, 0, p2, 96, 0, g_p2, 3, st));
-        // the encoder output of level 2 feeds both the pool and the skip
-        GK_T(gkrt_launch_avgpool2_bwd(g_p2, 96, 0, g_cat2, 224, 128, B, H >> 2, W >> 2, 96, 1, st));
-        GK_T(layer_bwd(E2B, g_cat2, 224, 128, cat2, 224, 128, e2a, 96, 0, g_e2a, 2, st));
+        // the encoder outputs feed both the pool and the skip
+        GK_T(layer_bwd(E2B, g_cat2, 224, 128, cat2, 224, 128, e2a, 96, 0, g_e2a, 2, st, GradFrom{g_p2, nullptr, 96}));
         GK_T(layer_bwd(E2A, g_e2a, 96, 0, e2a, 96, 0, p1, 64, 0, g_p1, 2, st));
-        GK_T(gkrt_launch_avgpool2_bwd(g_p1, 64, 0, g_cat1, 160, 96, B, H >> 1, W >> 1, 64, 1, st));
-        GK_T(layer_bwd(E1B, g_cat1, 160, 96, cat1, 160, 96, e1a, 64, 0, g_e1a, 1, st));
+        GK_T(layer_bwd(E1B, g_cat1, 160, 96, cat1, 160, 96, e1a, 64, 0, g_e1a, 1, st, GradFrom{g_p1, nullptr, 64}));
         GK_T(layer_bwd(E1A, g_e1a, 64, 0, e1a, 64, 0, p0, 32, 0, g_p0, 1, st));
-        GK_T(gkrt_launch_avgpool2_bwd(g_p0, 32, 0, g_cat0, 96, 64, B, H, W, 32, 1, st));
-        GK_T(layer_bwd(E0B, g_cat0, 96, 64, cat0, 96, 64, e0a, 32, 0, g_e0a, 0, st));
+        GK_T(layer_bwd(E0B, g_cat0, 96, 64, cat0, 96, 64, e0a, 32, 0, g_e0a, 0, st, GradFrom{g_p0, nullptr, 32}));
         GK_T(layer_bwd(E0A, g_e0a, 32, 0, e0a, 32, 0, x0, kXc, 0, nullptr, 0, st));
         return cudaSuccess;
     }
@@ -484,7 +526,7 @@ cudaError_t gkrt_unet_set_params_host(Unet* u, const float* h) {
     for (float* q : {u->g, u->m, u->v})
         if ((e = cudaMemset(q, 0, u->nparams * 4)) != cudaSuccess) return e;
     u->step = 0;
-    if ((e = u->refresh_bf16(0)) != cudaSuccess) return e;
+    if ((e = u->update_params(nullptr, 0)) != cudaSuccess) return e;
     return cudaDeviceSynchronize();
 }
 
@@ -538,7 +580,7 @@ cudaError_t gkrt_unet_backward_dev(Unet* u, const float* d_raw, cudaStream_t st)
     const long long npix = (long long)u->B * u->H * u->W;
     cudaError_t e;
     if (!u->train_acts && (e = u->forward(st, true)) != cudaSuccess) return e;
-    k_grad_in<<<nb(npix * 32), 256, 0, st>>>(d_raw, npix, u->gy);
+    k_grad_in<<<nb(npix), 256, 0, st>>>(d_raw, npix, u->gy);
     return u->backward(st);
 }
 
@@ -550,15 +592,14 @@ cudaError_t gkrt_unet_train_step_dev(Unet* u, const float* input, const float* t
     if ((e = cudaMemsetAsync(u->d_loss, 0, sizeof(double), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(u->g, 0, u->nparams * 4, st)) != cudaSuccess) return e;
     // gradients of the per-image sum of squared log errors (Adam does not see the scale)
-    k_loss<<<nb(npix), 256, 0, st>>>(u->y, target, npix, 1.0f, u->gy, u->d_loss);
+    k_loss<<<nb(npix), 256, 0, st>>>(reinterpret_cast<const float4*>(u->y), target, npix, 1.0f, u->gy, u->d_loss);
     if ((e = u->backward(st)) != cudaSuccess) return e;
     u->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = (float)(1.0 / (1.0 - std::pow((double)b1, u->step)));
     const float c2 = (float)(1.0 / (1.0 - std::pow((double)b2, u->step)));
-    k_adam<<<nb((long long)u->nparams), 256, 0, st>>>(u->p, u->g, u->m, u->v, (long long)u->nparams, lr, b1, b2, 1e-8f,
-                                                     c1, c2);
-    if ((e = u->refresh_bf16(st)) != cudaSuccess) return e;
+    const AdamStep step{lr, b1, b2, 1e-8f, c1, c2};
+    if ((e = u->update_params(&step, st)) != cudaSuccess) return e;
     if (loss_host) {
         double l = 0.0;
         if ((e = cudaMemcpyAsync(&l, u->d_loss, sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
