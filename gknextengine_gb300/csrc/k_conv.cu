@@ -5,8 +5,10 @@
 // are multiples of 32; weights are [Cout][3][3][Cin] bf16; accumulation is FP32 in tensor
 // memory.
 //
-// Persistent, warp-specialised CTAs loop over tiles of 16 x 8 pixels (x by y, M = 128) times
-// all Cout (N <= 256) of one image (outputs of up to 32 channels use the halo-tile kernel below):
+// Three kernels, all persistent and warp-specialised, that take the FP32 sums of an output in the same
+// order: k_conv_rows (row tiles, weights in shared memory) for the layers whose weights fit and whose
+// images are large enough, and for the rest k_conv3x3_halo (outputs of up to 32 channels) and k_conv3x3,
+// whose CTAs loop over tiles of 16 x 8 pixels (x by y, M = 128) times all Cout (N <= 256) of one image:
 //   K loop   9 taps x Cin / 32 chunks. For tap (dy, dx) and chunk c the A operand is the
 //            4D TMA box {32 channels, 16 x, 8 y, 1 image} of the input shifted by the tap;
 //            coordinates outside the image read zeros, which is the zero padding. The B
@@ -33,6 +35,7 @@
 // Every barrier wait is bounded; a wait that runs out records the wait error bit in the
 // device error word and the CTA skips its stores.
 #include <algorithm>
+#include <numeric>
 
 #include <cuda_bf16.h>
 
@@ -588,6 +591,472 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3_halo(const __grid_cons
     if (warp == 1) tmem_dealloc(tmem, ncols);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Row tiles: a CTA keeps the weights of its output channels in shared memory for all its tiles of 128 x
+// kR pixels, whose kR rows of accumulators lie next to each other in TMEM. M = 128 pixels of one input
+// row; that row against the weights of its vertical taps is one MMA of N = up to 3 Cout, which adds to
+// the accumulators of the rows r - 1, r and r + 1: the A operand, whose shared-memory reads bound MMAs
+// of small N (128 rows of 32 bytes take 32 cycles; N = 32 alone 16), is shared by the taps.
+//   stages    the tile's kR + 2 input rows of 130 pixels x 32 channels in one box (64-byte swizzle; 32
+//             for a 16-channel input); the horizontal taps are its windows from pixel 0, 1 and 2.
+//   order     FP32 sums are taken as the other kernels take them: (chunk, dy, dx), or with kDxOuter (dx,
+//             chunk, dy), for which a tile's chunks all stay in shared memory.
+//   issue     a warp's MMAs follow one another only as fast as it issues them (a wait on a barrier costs
+//             about 115 cycles, a commit 36, a dependent instruction 5), so a tile's MMAs are unrolled
+//             with their offsets as constants, a tile has one barrier per chunk for its loads, one for
+//             its sums and one for their release, and two warps issue, for every other tile each: while
+//             one waits or computes addresses, the other's MMAs run.
+//   epilogue  up to four groups of four warps take the rows in turn, kG columns at a time: bias, addend,
+//             ReLU, and through swizzled shared memory out by TMA (the tensor map clips the edges; the
+//             nearest upsampling is four more stores of the same bytes). kMode is a template parameter
+//             because the pooled rows and the addend of a general one lived in local memory: 540
+//             instructions per 32 columns instead of 200, and twice the time of the whole kernel.
+// What bounds it: DRAM at full resolution, the operand reads of shared memory otherwise. Before and after,
+// cold: 32 -> 32 channels on 1080p 72 -> 48 us, 32 -> 4 (FP32) 60 -> 44; on 540 x 960 32 -> 64 44 -> 27,
+// 64 -> 64 55 -> 37, 64 -> 128 88 -> 58; 64 -> 64 on 539 x 963 66 -> 36.
+constexpr int kRowGroups = 4;
+constexpr int kRowThreads = 96 + kRowGroups * kEpiThreads;   // producer, issuer, epilogue, issuer
+constexpr int kRowMaxStages = 8;
+constexpr int kRowMaxSets = 8;
+constexpr int kRowMaxChunks = 8;
+constexpr int kRowPix = 130;
+
+struct RowPlan {
+    int nco;             // output channels of a CTA (blockIdx.y: which)
+    int nxs, nyb;        // tiles per image row and column
+    int items;           // tiles
+    int ring, sets;      // input boxes of each issuer; tiles whose accumulators TMEM holds
+    int groups;          // epilogue groups at work
+};
+
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_5d(const CUtensorMap* map, const void* src, int c0, int c1, int c2, int c3,
+                                             int c4) {
+    asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void tma_store_wait_read() {   // at most kPending groups still read shared memory
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kPending) : "memory");
+}
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// (a, b) += (x, y)
+__device__ __forceinline__ void add2(uint32_t& a, uint32_t& b, float x, float y) {
+    asm("{\n\t.reg .b64 s, t;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 t, {%2, %3};\n\tadd.rn.f32x2 s, s, t;\n\t"
+        "mov.b64 {%0, %1}, s;\n\t}"
+        : "+r"(a), "+r"(b)
+        : "f"(x), "f"(y));
+}
+__device__ __forceinline__ uint32_t relu2(uint32_t v) {
+    __nv_bfloat162 h = *reinterpret_cast<__nv_bfloat162*>(&v);
+    h = __hmax2(h, __nv_bfloat162{__nv_bfloat16_raw{0}, __nv_bfloat16_raw{0}});
+    return *reinterpret_cast<uint32_t*>(&h);
+}
+__host__ __device__ constexpr int row_stage_bytes(int rb, int r) {
+    return ((r + 2) * kRowPix * rb + 511) & ~511;
+}
+
+// The 2 x 2 average of two rows' 32 (kG) stored channels of a warp's pixels: the lanes of a pixel pair
+// swap halves of their channels, and each averages its half, (((0 + v(x, y)) + v(x + 1, y)) +
+// v(x, y + 1)) + v(x + 1, y + 1) times 1/4 rounded to bf16, and stores it.
+template <int kG>
+__device__ __forceinline__ void pool_store(const uint32_t (&r0)[kG / 2], const uint32_t (&r1)[kG / 2], bool inside,
+                                           __nv_bfloat16* dst) {
+    constexpr int kH = kG / 4;   // registers (two channels each) of half the channels
+    const bool odd = (threadIdx.x & 1) != 0;
+    uint32_t o[kH];
+#pragma unroll
+    for (int j = 0; j < kH; ++j) {
+        const uint32_t own0 = odd ? r0[kH + j] : r0[j], own1 = odd ? r1[kH + j] : r1[j];
+        const uint32_t got0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? r0[j] : r0[kH + j], 1);
+        const uint32_t got1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? r1[j] : r1[kH + j], 1);
+        const uint32_t a = odd ? got0 : own0, b = odd ? own0 : got0, c = odd ? got1 : own1, d = odd ? own1 : got1;
+        float lo = 0.0f + __uint_as_float(a << 16), hi = 0.0f + __uint_as_float(a & 0xFFFF0000u);
+        lo = lo + __uint_as_float(b << 16);
+        hi = hi + __uint_as_float(b & 0xFFFF0000u);
+        lo = lo + __uint_as_float(c << 16);
+        hi = hi + __uint_as_float(c & 0xFFFF0000u);
+        lo = lo + __uint_as_float(d << 16);
+        hi = hi + __uint_as_float(d & 0xFFFF0000u);
+        o[j] = pack_bf16x2(lo * 0.25f, hi * 0.25f);
+    }
+    if (!inside) return;
+#pragma unroll
+    for (int j = 0; j < kH; j += 4)
+        reinterpret_cast<uint4*>(dst + (odd ? kG / 2 : 0))[j / 4] = make_uint4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+}
+
+// kMode: what the epilogue does besides bias, ReLU and the store
+enum RowMode { kRowPlain = 0, kRowPool = 1, kRowAdd = 2, kRowF32 = 3 };
+template <int kRb, int kG, int kR, bool kDxOuter, int kMode>
+__global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_constant__ CUtensorMap mx,
+                                                              const __grid_constant__ CUtensorMap mw,
+                                                              const __grid_constant__ CUtensorMap mo,
+                                                              const __grid_constant__ CUtensorMap mu, ConvArgs a,
+                                                              RowPlan p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    constexpr int kStage = row_stage_bytes(kRb, kR);
+    const int kc = a.cin / 32;
+    const int b_bytes = p.nco * 64;   // one tap's weight box
+    uint8_t* wsm = smem;              // box (chunk c, dx, dy) at ((3 c + dx) 3 + 2 - dy) b_bytes
+    uint8_t* stage0 = wsm + 9 * kc * b_bytes;
+    uint8_t* stores = stage0 + 2 * p.ring * kStage;   // 64 kG bytes per epilogue warp
+    float* bsm = reinterpret_cast<float*>(stores + p.groups * 4 * 64 * kG);   // the bias
+    uint64_t* full = reinterpret_cast<uint64_t*>(bsm + 128);
+    uint64_t* empty = full + kRowMaxStages;
+    uint64_t* sfull = empty + kRowMaxStages;   // a set's sums are complete
+    uint64_t* sempty = sfull + kRowMaxSets;    // and have been read
+    uint64_t* wbar = sempty + kRowMaxSets;     // weight boxes of (chunk, dx)
+    uint64_t* fin = wbar + 3 * kRowMaxChunks;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(fin + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int co0 = blockIdx.y * p.nco;
+    if (tid == 0) {
+        for (int s = 0; s < 2 * p.ring; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int i = 0; i < p.sets; ++i) {
+            mbar_init(&sfull[i], 1);
+            mbar_init(&sempty[i], 4 * kR);
+        }
+        for (int i = 0; i < 3 * kc; ++i) mbar_init(&wbar[i], 1);
+        mbar_init(fin, 2);
+        *abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tslot, 512u);
+        tmem_relinquish();
+    }
+    // -0 adds nothing, not even to a -0
+    for (int i = tid; i < p.nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + co0 + i) : -0.0f;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    const int per_img = p.nxs * p.nyb;
+
+    if (warp == 0) {
+        if (lane == 0) {   // producer: the weights in the order of their use, then the tiles' rows
+            for (int i = 0; i < 3 * kc; ++i) {
+                const int c = kDxOuter ? i % kc : i / 3, dx = kDxOuter ? i / kc : i % 3, wi = 3 * c + dx;
+                mbar_expect_tx(&wbar[wi], (uint32_t)(3 * b_bytes));
+                for (int dy = 0; dy < 3; ++dy)
+                    tma_load_2d(wsm + (3 * wi + 2 - dy) * b_bytes, &mw, (3 * dy + dx) * a.cin + 32 * c, co0, &wbar[wi]);
+            }
+            // Each issuer has a ring of its own, so that whoever waits for a stage's next load has waited
+            // for its last one (a barrier tells phases apart by parity alone).
+            int pos = 0, other = 0;   // the next stage of this tile's ring, and of the other one
+            uint32_t use = 0, other_use = 0;
+            int base = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < p.items && ok; t += gridDim.x) {
+                const int img = t / per_img, r = t - img * per_img, yb = r / p.nxs;
+                const int x = (r - yb * p.nxs) * 128 - 1, y = yb * kR - 1;
+                for (int c = 0; c < kc; ++c) {
+                    const int s = base + pos;
+                    if (use > 0) ok = mbar_wait_bounded(&empty[s], (use - 1u) & 1u, a.err);
+                    if (!ok || *abort_flag) {
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full[s], (uint32_t)((kR + 2) * kRowPix * kRb));
+                    tma_load_4d(stage0 + s * kStage, &mx, 32 * c, x, y, img, &full[s]);
+                    if (++pos == p.ring) {
+                        pos = 0;
+                        ++use;
+                    }
+                }
+                if (!ok) break;
+                const int pt = pos;
+                pos = other;
+                other = pt;
+                const uint32_t ut = use;
+                use = other_use;
+                other_use = ut;
+                base = p.ring - base;
+            }
+            // no load may be in flight when the CTA ends, whoever gave up
+            for (int w = 0; w < 2; ++w) {
+                for (int i = 0; i < p.ring; ++i) {
+                    const uint32_t uses = use + (i < pos ? 1u : 0u);
+                    if (uses > 0) mbar_wait_bounded(&full[base + i], (uses - 1u) & 1u, a.err);
+                }
+                pos = other;
+                use = other_use;
+                base = p.ring - base;
+            }
+            for (int i = 0; i < 3 * kc; ++i) mbar_wait_bounded(&wbar[i], 0u, a.err);
+        }
+    } else if (warp == 1 || warp == 2 + 4 * p.groups) {
+        // two MMA issuers take the tiles in turn; the whole warp walks them, so that what an MMA needs is
+        // warp-uniform, and one elected lane issues
+        constexpr uint32_t kHi = (8u * kRb >> 4) | (1u << 14) | ((kRb == 64 ? 4u : 6u) << 29);   // umma_desc_swz
+        constexpr uint32_t kHiB = (512u >> 4) | (1u << 14) | (4u << 29);                         // umma_desc_sw64
+        constexpr uint32_t kRow = kRowPix * kRb / 16, kPixel = kRb / 16;                         // of a box
+        constexpr int nkk = kRb / 32;
+        const bool leader = elect_one();
+        const uint32_t nfield = (uint32_t)(p.nco >> 3) << 17, id1 = umma_idesc_bf16(128u, 0u) + nfield;
+        const uint32_t ids[3] = {id1, id1 + nfield, id1 + 2u * nfield};
+        const uint32_t wlo = (smem_u32(wsm) >> 4) | (1u << 16), slo = (smem_u32(stage0) >> 4) | (1u << 16);
+        const uint32_t bstep = (uint32_t)b_bytes >> 4;
+        const int who = warp == 1 ? 0 : 1;
+        int s0 = 0, set = 0, kt = who;   // the tile's first stage and its set
+        uint32_t use0 = 0, phase = 0;
+        bool ok = true;
+        const uint32_t sring = slo + (uint32_t)(who * p.ring * (kStage >> 4));
+        full += who * p.ring;
+        empty += who * p.ring;
+        auto next_set = [&](int n) {
+            set += n;
+            while (set >= p.sets) {
+                set -= p.sets;
+                phase ^= 1u;
+            }
+        };
+        next_set(who);
+        // all MMAs of input row rr at horizontal taps dx0 .. dx1 - 1 (a: the stage, b: the first tap's
+        // boxes); fresh: row rr of the accumulators gets its first products
+        auto mma_row = [&](uint32_t dt, uint32_t ar, uint32_t b, int rr, int dx0, int dx1, bool fresh) {
+            const int lo = rr < 2 ? 0 : rr - 2, n = (rr < kR ? rr : kR - 1) - lo + 1;   // rows lo ..: tap dy = rr - o
+            const uint32_t d = dt + (uint32_t)(lo * p.nco);
+#pragma unroll
+            for (int dx = dx0; dx < dx1; ++dx)
+#pragma unroll
+                for (int kk = 0; kk < nkk; ++kk) {
+                    const uint32_t al = ar + (uint32_t)dx * kPixel + 2u * (uint32_t)kk;
+                    const uint32_t bx = b + (uint32_t)(3 * (dx - dx0)) * bstep + 2u * (uint32_t)kk;
+                    const uint32_t bo = bx + (uint32_t)(2 - rr + lo) * bstep;
+                    if (dx == dx0 && kk == 0 && rr < kR && fresh) {
+                        if (rr > 0) umma_bf16_lo(d, al, kHi, bo, kHiB, ids[n - 2 < 0 ? 0 : n - 2], 1u);
+                        umma_bf16_lo(dt + (uint32_t)(rr * p.nco), al, kHi, bx + 2u * bstep, kHiB, id1, 0u);
+                    } else {
+                        umma_bf16_lo(d, al, kHi, bo, kHiB, ids[n - 1], 1u);
+                    }
+                }
+        };
+        for (int t = blockIdx.x + who * gridDim.x; t < p.items && ok; t += 2 * gridDim.x, kt += 2) {
+            const uint32_t dt = tmem + (uint32_t)(set * kR * p.nco);
+            if (kt >= p.sets) ok = mbar_wait_bounded(&sempty[set], phase ^ 1u, a.err);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (kDxOuter) {
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) {
+                    int s = s0;
+                    uint32_t use = use0;
+                    for (int c = 0; c < kc && ok; ++c) {
+                        const int wi = 3 * c + dx;
+                        if (kt < 2) ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&wbar[wi], 0u, a.err));
+                        if (dx == 0) ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&full[s], use & 1u, a.err) && ok);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (leader) {
+                            const uint32_t b = wlo + (uint32_t)(3 * wi) * bstep;
+                            const uint32_t as = sring + (uint32_t)s * (uint32_t)(kStage >> 4);
+                            if (dx == 0 && c == 0) {
+#pragma unroll
+                                for (int rr = 0; rr < kR + 2; ++rr)
+                                    mma_row(dt, as + (uint32_t)rr * kRow, b, rr, dx, dx + 1, true);
+                            } else {
+#pragma unroll
+                                for (int rr = 0; rr < kR + 2; ++rr)
+                                    mma_row(dt, as + (uint32_t)rr * kRow, b, rr, dx, dx + 1, false);
+                            }
+                            if (dx == 2) umma_commit(&empty[s]);
+                        }
+                        __syncwarp();
+                        if (++s == p.ring) {
+                            s = 0;
+                            ++use;
+                        }
+                    }
+                }
+            } else {
+                int s = s0;
+                uint32_t use = use0;
+                for (int c = 0; c < kc && ok; ++c) {
+                    if (kt < 2) {
+                        for (int dx = 0; dx < 3; ++dx) ok = mbar_wait_bounded(&wbar[3 * c + dx], 0u, a.err) && ok;
+                    }
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&full[s], use & 1u, a.err) && ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (leader) {
+                        const uint32_t b = wlo + (uint32_t)(9 * c) * bstep;
+                        const uint32_t as = sring + (uint32_t)s * (uint32_t)(kStage >> 4);
+                        if (c == 0) {
+#pragma unroll
+                            for (int rr = 0; rr < kR + 2; ++rr) mma_row(dt, as + (uint32_t)rr * kRow, b, rr, 0, 3, true);
+                        } else {
+#pragma unroll
+                            for (int rr = 0; rr < kR + 2; ++rr) mma_row(dt, as + (uint32_t)rr * kRow, b, rr, 0, 3, false);
+                        }
+                        umma_commit(&empty[s]);
+                    }
+                    __syncwarp();
+                    if (++s == p.ring) {
+                        s = 0;
+                        ++use;
+                    }
+                }
+            }
+            if (!ok) break;
+            if (leader) umma_commit(&sfull[set]);
+            __syncwarp();
+            s0 += kc;
+            while (s0 >= p.ring) {
+                s0 -= p.ring;
+                ++use0;
+            }
+            next_set(2);
+        }
+        if (!ok) *abort_flag = 1;
+        if (leader) {
+            umma_commit(fin);
+            mbar_wait_bounded(fin, 0u, a.err);   // nothing may be in flight when TMEM is freed
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3, group = (warp - 2) >> 2;
+        uint8_t* sbuf = stores + (warp - 2) * 64 * kG;
+        const uint32_t lane0 = tmem + ((uint32_t)(q * 32) << 16);
+        const bool relu = (a.flags & kConvRelu) != 0, leader = elect_one();
+        constexpr int kUnit = kMode == kRowPool ? 2 : 1;   // rows taken together
+        const int sw = kG == 32 ? (lane >> 1) & 3 : (lane >> 2) & 1;
+        uint4* sb = reinterpret_cast<uint4*>(sbuf) + lane * (kG / 8);
+        int set = 0, turn = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.items && ok; t += gridDim.x) {
+            const int img = t / per_img, rt = t - img * per_img, yb = rt / p.nxs;
+            const int x0 = (rt - yb * p.nxs) * 128 + q * 32, x = x0 + lane;
+#pragma unroll 1
+            for (int o0 = 0; o0 < kR; o0 += kUnit) {
+                const bool mine = turn == group;
+                if (++turn == p.groups) turn = 0;
+                if (!mine) continue;
+                uint4 add[kMode == kRowAdd ? kG / 8 : 1];
+                if (kMode == kRowAdd) {   // in flight while the tile's sums are awaited (one column group)
+                    const int y = yb * kR + o0;
+                    const bool in = x < a.W && y < a.H;
+                    const uint4* src = reinterpret_cast<const uint4*>(
+                        reinterpret_cast<const __nv_bfloat16*>(a.add_par) + (in ? pix_add(a, img, x, y) + co0 : 0));
+#pragma unroll
+                    for (int j = 0; j < kG / 8; ++j) add[j] = in ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+                }
+                ok = mbar_wait_bounded(&sfull[set], phase, a.err) && !*abort_flag;
+                ok = __all_sync(0xFFFFFFFFu, ok);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int c0 = 0; c0 < p.nco; c0 += kG) {
+                    uint32_t pk[kUnit][kG / 2];   // the rows' stored values
+#pragma unroll
+                    for (int u = 0; u < kUnit; ++u) {
+                        const int o = o0 + u, y = yb * kR + o;
+                        uint32_t r[kG];
+                        const uint32_t col = lane0 + (uint32_t)((set * kR + o) * p.nco + c0);
+                        if constexpr (kG == 32) tmem_ld32(col, r);
+                        else tmem_ld16(col, r);
+                        tmem_ld_wait();
+                        if (c0 + kG >= p.nco) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (leader) mbar_arrive(&sempty[set]);
+                        }
+                        float v[kG];
+                        const float4* b4 = reinterpret_cast<const float4*>(bsm + c0);
+#pragma unroll
+                        for (int j = 0; j < kG; j += 4) {
+                            const float4 b = b4[j / 4];
+                            v[j] = __uint_as_float(r[j]) + b.x;
+                            v[j + 1] = __uint_as_float(r[j + 1]) + b.y;
+                            v[j + 2] = __uint_as_float(r[j + 2]) + b.z;
+                            v[j + 3] = __uint_as_float(r[j + 3]) + b.w;
+                        }
+                        if (kMode == kRowAdd) {
+#pragma unroll
+                            for (int j = 0; j < kG / 2; ++j) {
+                                const uint4& w4 = add[j / 4];
+                                const uint32_t w = (j & 3) == 0 ? w4.x : (j & 3) == 1 ? w4.y : (j & 3) == 2 ? w4.z : w4.w;
+                                v[2 * j] += __uint_as_float(w << 16);
+                                v[2 * j + 1] += __uint_as_float(w & 0xFFFF0000u);
+                            }
+                        }
+                        if (kMode == kRowF32) {
+                            if (relu) {
+#pragma unroll
+                                for (int j = 0; j < kG; ++j) v[j] = fmaxf(v[j], 0.0f);
+                            }
+                            if (x < a.W && y < a.H) {
+                                float* d = reinterpret_cast<float*>(a.out) +
+                                           (((size_t)img * a.H + y) * a.W + x) * a.out_c + a.out_off + co0 + c0;
+#pragma unroll
+                                for (int h = 0; h < kG; h += 16) {
+                                    float w[16];
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j) w[j] = v[h + j];
+                                    store_f32(d + h, w, min(16, a.n_store - co0 - c0 - h));
+                                }
+                            }
+                            continue;
+                        }
+#pragma unroll
+                        for (int j = 0; j < kG / 2; ++j) pk[u][j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+                        if (relu) {   // of the rounded values: the same (a NaN becomes 0 either way)
+#pragma unroll
+                            for (int j = 0; j < kG / 2; ++j) pk[u][j] = relu2(pk[u][j]);
+                        }
+                        tma_store_wait_read<0>();   // the leader's last store has read the buffer
+                        __syncwarp();
+#pragma unroll
+                        for (int j = 0; j < kG / 8; ++j)
+                            sb[j ^ sw] = make_uint4(pk[u][4 * j], pk[u][4 * j + 1], pk[u][4 * j + 2], pk[u][4 * j + 3]);
+                        fence_async_smem();
+                        __syncwarp();
+                        if (leader && y < a.H && x0 < a.W) {
+                            tma_store_4d(&mo, sbuf, co0 + c0, x0, y, img);
+                            if (a.up_out)
+                                for (int k = 0; k < 4; ++k)
+                                    tma_store_5d(&mu, sbuf, co0 + c0, k & 1, x0, 2 * y + (k >> 1), img);
+                            tma_store_commit();
+                        }
+                    }
+                    if (kMode == kRowPool) {
+                        const int h2 = a.H >> 1, w2 = a.W >> 1, y2 = (yb * kR + o0) >> 1;
+                        pool_store<kG>(pk[0], pk[kUnit - 1], y2 < h2 && (x >> 1) < w2,
+                                       reinterpret_cast<__nv_bfloat16*>(a.pool_out) +
+                                           (((size_t)img * h2 + y2) * w2 + (x >> 1)) * a.pool_c + a.pool_off + co0 + c0);
+                    }
+                }
+            }
+            if (!ok) break;
+            if (++set == p.sets) {
+                set = 0;
+                phase ^= 1u;
+            }
+        }
+        if (leader) tma_store_wait_all();
+    }
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 512u);
+}
+
 }  // namespace
 
 }  // namespace gk
@@ -608,6 +1077,125 @@ cudaError_t gkrt_encode_tmap_bf16_dense(CUtensorMap* map, const void* base, uint
 static bool conv_halo(int cin, int cout) { return cout <= 32 && 9 * cin * cout * 2 <= kHaloWeightMax; }
 static size_t conv_halo_smem(int cin, int cout) {
     return (size_t)9 * cin * cout * 2 + kHaloStages * kHaloStage + (2 * kHaloStages + 6) * 8 + 8 + kEpiBuf + 1024;
+}
+
+constexpr int kRowSmem = 227 * 1024;
+constexpr int kRowSmemMin = 116 * 1024;   // more than half of an SM's: one CTA per SM (it takes all of TMEM)
+// Rows of a tile: 2 where its chunks stay in shared memory together or are several, or rows are pooled in
+// pairs, else 3: four boxes are to fit. (Per output row of 32 -> 32 channels, 2 rows take 528 cycles of
+// operand reads, 3 464, 4 432, taps of its own MMAs 720.)
+static int row_rows(const ConvArgs& a, bool dx_outer) { return dx_outer || a.pool_out || a.cin > 32 ? 2 : 3; }
+
+static size_t row_smem(const ConvArgs& a, const RowPlan& p, int stage) {
+    return (size_t)9 * a.cin * p.nco * 2 + (size_t)2 * p.ring * stage + (size_t)p.groups * 4 * 64 * (p.nco % 32 ? 16 : 32) +
+           128 * 4 + (2 * kRowMaxStages + 2 * kRowMaxSets + 3 * kRowMaxChunks + 1) * 8 + 8 + 1024;
+}
+
+// A barrier tells its phases apart by parity, so an epilogue group has to have seen a set's last use, or
+// a later tile of the same issuer, before it waits for the next: with `units` turns a tile, a group is
+// back at the same place of a tile after groups / gcd(groups, 2 units) of an issuer's tiles, of which
+// there are to be no more than the issuer has sets.
+static bool row_turns_ok(const RowPlan& p, int units) {
+    return p.groups / std::gcd(p.groups, 2 * units) <= p.sets / 2;
+}
+
+// The plan of a convolution on row tiles, or none (items 0) where it does not fit or the other kernels'
+// 16 x 8 tiles are estimated faster. The output channels are split over CTAs until the weights leave room
+// for each issuer's boxes (all of a tile's chunks where they stay, else two).
+// The estimate is in times of one 16 x 8 tile per SM, of which the other kernels take their tiles' number
+// over the SMs; a row tile was measured at 1.0 of those (128 x 2 pixels, sums by horizontal tap; 0.62
+// with the channels split), 1.8 (128 x 3, sums by chunk) and 1.5 (128 x 2), and whole waves count. Over
+// nine layers on 50 sizes from 16 x 32 to 4 x 200 x 500 either side of that line differs by at most 15%
+// (64 -> 64 channels: 200 x 128 pixels 8.2 us by tiles, 7.9 by rows; 4 x 200 x 140 14.8 and 16.4).
+static RowPlan row_plan(const ConvArgs& a, int rb, int sms) {
+    RowPlan p{};
+    const int kc = a.cin / 32;
+    const bool dx_outer = !conv_halo(a.cin, a.cout);
+    const int R = row_rows(a, dx_outer), stage = row_stage_bytes(rb, R), need = dx_outer ? kc : 2;
+    if (a.cout > 128 || kc > kRowMaxChunks || (a.add_par && (a.pool_out || a.cout > 32))) return p;
+    p.nxs = (a.W + 127) / 128;
+    p.nyb = (a.H + R - 1) / R;
+    const long long items = (long long)a.B * p.nxs * p.nyb;
+    if (items > 0x7FFFFFFFLL / 4) return p;
+    for (int split = 1; split <= 4; ++split) {
+        if (split > 1 && a.cout % (32 * split)) continue;
+        p.nco = a.cout / split;
+        p.sets = std::min(kRowMaxSets, 512 / (R * p.nco)) & ~1;   // the issuers' in turn
+        for (p.groups = kRowGroups; p.groups > 0; p.groups /= 2) {
+            p.ring = 0;
+            const size_t fixed = row_smem(a, p, stage);
+            if (fixed < (size_t)kRowSmem)
+                p.ring = std::min(kRowMaxStages / 2, (int)(((size_t)kRowSmem - fixed) / (2 * (size_t)stage)));
+            if (p.ring >= need && row_turns_ok(p, R / (a.pool_out ? 2 : 1))) break;
+        }
+        if (!p.groups) continue;
+        const long long grid = std::max(1, sms / split), waves = (items + grid - 1) / grid;
+        const float rows = dx_outer ? (split == 1 ? 1.0f : 0.62f) * (float)waves + 0.3f
+                                    : (R == 3 ? 1.8f : 1.5f) * (float)waves + 1.6f;
+        const long long tiles = (long long)a.B * ((a.W + kTileX - 1) / kTileX) * ((a.H + kTileY - 1) / kTileY);
+        if (rows < (float)tiles / (float)sms) p.items = (int)items;
+        return p;
+    }
+    return p;
+}
+
+static cudaError_t launch_rows(const void* xbase, int xv, uint64_t xc, const void* w, const ConvArgs& a, const RowPlan& p,
+                               int rb, int sms, int dev, cudaStream_t st) {
+    const bool f32 = (a.flags & kConvF32Out) != 0, dx_outer = !conv_halo(a.cin, a.cout);
+    const int kg = p.nco % 32 ? 16 : 32, R = row_rows(a, dx_outer);
+    const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B;
+    CUtensorMap mx, mw, mo, mu;
+    const uint64_t xd[4] = {(uint64_t)xv, W, H, B};
+    const uint64_t xs[3] = {xc * 2, W * xc * 2, H * W * xc * 2};
+    const uint32_t xb[4] = {(uint32_t)rb / 2, kRowPix, (uint32_t)R + 2, 1};
+    cudaError_t e = rb == 64 ? gkrt_encode_tmap_bf16(&mx, xbase, 4, xd, xs, xb)
+                             : gkrt_encode_tmap_bf16_sw32(&mx, xbase, 4, xd, xs, xb);
+    if (e != cudaSuccess) return e;
+    const uint64_t wd[2] = {(uint64_t)9 * a.cin, (uint64_t)a.cout};
+    const uint64_t ws[1] = {(uint64_t)9 * a.cin * 2};
+    const uint32_t wb[2] = {32, (uint32_t)p.nco};
+    if ((e = gkrt_encode_tmap_bf16(&mw, w, 2, wd, ws, wb)) != cudaSuccess) return e;
+    mo = mu = mw;
+    auto encode = kg == 32 ? gkrt_encode_tmap_bf16 : gkrt_encode_tmap_bf16_sw32;
+    if (!f32) {
+        const uint64_t oc = (uint64_t)a.out_c * 2;
+        const uint64_t od[4] = {(uint64_t)a.cout, W, H, B}, os[3] = {oc, W * oc, H * W * oc};
+        const uint32_t ob[4] = {(uint32_t)kg, 32, 1, 1};
+        if ((e = encode(&mo, static_cast<uint8_t*>(a.out) + (size_t)a.out_off * 2, 4, od, os, ob)) != cudaSuccess) return e;
+    }
+    if (a.up_out) {
+        const uint64_t uc = (uint64_t)a.up_c * 2;
+        const uint64_t ud[5] = {(uint64_t)a.cout, 2, W, 2 * H, B}, us[4] = {uc, 2 * uc, 2 * W * uc, 4 * H * W * uc};
+        const uint32_t ub[5] = {(uint32_t)kg, 1, 32, 1, 1};
+        if ((e = encode(&mu, static_cast<uint8_t*>(a.up_out) + (size_t)a.up_off * 2, 5, ud, us, ub)) != cudaSuccess) return e;
+    }
+    typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ConvArgs, RowPlan);
+    // by pixel bytes, rows and order of the sums; column group; mode
+#define GK_ROWS(rb, kg, r, dxo, add) \
+    {k_conv_rows<rb, kg, r, dxo, kRowPlain>, r % 2 ? nullptr : k_conv_rows<rb, kg, 2, dxo, kRowPool>, \
+     add ? k_conv_rows<rb, kg, r, false, kRowAdd> : nullptr, k_conv_rows<rb, kg, r, dxo, kRowF32>}
+    static const Kernel kernels[5][2][4] = {{GK_ROWS(64, 16, 2, true, false), GK_ROWS(64, 32, 2, true, false)},
+                                            {GK_ROWS(64, 16, 2, false, true), GK_ROWS(64, 32, 2, false, true)},
+                                            {GK_ROWS(64, 16, 3, false, true), GK_ROWS(64, 32, 3, false, true)},
+                                            {GK_ROWS(32, 16, 2, false, true), GK_ROWS(32, 32, 2, false, true)},
+                                            {GK_ROWS(32, 16, 3, false, true), GK_ROWS(32, 32, 3, false, true)}};
+#undef GK_ROWS
+    const int mode = f32 ? kRowF32 : a.add_par ? kRowAdd : a.pool_out ? kRowPool : kRowPlain;
+    const Kernel kernel = kernels[dx_outer ? 0 : R - 1 + (rb == 32 ? 2 : 0)][kg == 32][mode];
+    static bool attr[kMaxDevices] = {};
+    if (!attr[dev]) {
+        for (int i = 0; i < 40; ++i)
+            if ((&kernels[0][0][0])[i] &&
+                (e = cudaFuncSetAttribute((const void*)(&kernels[0][0][0])[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          kRowSmem)) != cudaSuccess)
+                return e;
+        attr[dev] = true;
+    }
+    const int split = a.cout / p.nco;
+    const size_t smem = row_smem(a, p, row_stage_bytes(rb, R));
+    const unsigned grid = (unsigned)std::min(p.items, std::max(1, sms / split));
+    kernel<<<dim3(grid, (unsigned)split), 96 + p.groups * kEpiThreads, std::max(smem, (size_t)kRowSmemMin), st>>>(mx, mw, mo, mu, a, p);
+    return cudaGetLastError();
 }
 
 // Outputs of up to 128 channels use the row-box stages (three vertical taps per box); the
@@ -671,6 +1259,13 @@ cudaError_t gkrt_launch_conv3x3(const void* x, const void* w, const ConvArgs& ar
         if (e0 != cudaSuccess) return e0;
     }
     const int sms = sms_dev[dev];
+    if (!(xv % 32) || xc == 16) {   // (a 16-channel input is the whole pixel)
+        const int rb = xv == 16 ? 32 : 64;
+        const RowPlan plan = row_plan(args, rb, sms);
+        if (plan.items)
+            return launch_rows(static_cast<const uint8_t*>(x) + (size_t)args.x_off * 2, xv, xc, w, args, plan, rb, sms,
+                               dev, st);
+    }
     if (halo) {
         // rows when a chunk is the whole pixel (64 bytes, or 32 for an input of 16 channels),
         // planes when the pixel is wider than the chunk
