@@ -5,9 +5,10 @@
 // are multiples of 32; weights are [Cout][3][3][Cin] bf16; accumulation is FP32 in tensor
 // memory.
 //
-// Three kernels, all persistent and warp-specialised, that take the FP32 sums of an output in the same
+// Four kernels, all persistent and warp-specialised, that take the FP32 sums of an output in the same
 // order: k_conv_rows (row tiles, weights in shared memory) for the layers whose weights fit and whose
-// images are large enough, and for the rest k_conv3x3_halo (outputs of up to 32 channels) and k_conv3x3,
+// images are large enough, k_conv_tiles (16 x 16 tiles, weights streamed) for the others of up to 128
+// channels, and for the rest k_conv3x3_halo (outputs of up to 32 channels) and k_conv3x3,
 // whose CTAs loop over tiles of 16 x 8 pixels (x by y, M = 128) times all Cout (N <= 256) of one image:
 //   K loop   9 taps x Cin / 32 chunks. For tap (dy, dx) and chunk c the A operand is the
 //            4D TMA box {32 channels, 16 x, 8 y, 1 image} of the input shifted by the tap;
@@ -622,7 +623,6 @@ constexpr int kRowMaxChunks = 8;
 constexpr int kRowPix = 130;
 
 struct RowPlan {
-    int nco;             // output channels of a CTA (blockIdx.y: which)
     int nxs, nyb;        // tiles per image row and column
     int items;           // tiles
     int ring, sets;      // input boxes of each issuer; tiles whose accumulators TMEM holds
@@ -707,8 +707,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int kStage = row_stage_bytes(kRb, kR);
-    const int kc = a.cin / 32;
-    const int b_bytes = p.nco * 64;   // one tap's weight box
+    const int kc = a.cin / 32, nco = a.cout;
+    const int b_bytes = nco * 64;   // one tap's weight box
     uint8_t* wsm = smem;              // box (chunk c, dx, dy) at ((3 c + dx) 3 + 2 - dy) b_bytes
     uint8_t* stage0 = wsm + 9 * kc * b_bytes;
     uint8_t* stores = stage0 + 2 * p.ring * kStage;   // 64 kG bytes per epilogue warp
@@ -723,7 +723,6 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int co0 = blockIdx.y * p.nco;
     if (tid == 0) {
         for (int s = 0; s < 2 * p.ring; ++s) {
             mbar_init(&full[s], 1);
@@ -743,7 +742,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
         tmem_relinquish();
     }
     // -0 adds nothing, not even to a -0
-    for (int i = tid; i < p.nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + co0 + i) : -0.0f;
+    for (int i = tid; i < nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + i) : -0.0f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -756,7 +755,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                 const int c = kDxOuter ? i % kc : i / 3, dx = kDxOuter ? i / kc : i % 3, wi = 3 * c + dx;
                 mbar_expect_tx(&wbar[wi], (uint32_t)(3 * b_bytes));
                 for (int dy = 0; dy < 3; ++dy)
-                    tma_load_2d(wsm + (3 * wi + 2 - dy) * b_bytes, &mw, (3 * dy + dx) * a.cin + 32 * c, co0, &wbar[wi]);
+                    tma_load_2d(wsm + (3 * wi + 2 - dy) * b_bytes, &mw, (3 * dy + dx) * a.cin + 32 * c, 0, &wbar[wi]);
             }
             // Each issuer has a ring of its own, so that whoever waits for a stage's next load has waited
             // for its last one (a barrier tells phases apart by parity alone).
@@ -811,7 +810,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
         constexpr uint32_t kRow = kRowPix * kRb / 16, kPixel = kRb / 16;                         // of a box
         constexpr int nkk = kRb / 32;
         const bool leader = elect_one();
-        const uint32_t nfield = (uint32_t)(p.nco >> 3) << 17, id1 = umma_idesc_bf16(128u, 0u) + nfield;
+        const uint32_t nfield = (uint32_t)(nco >> 3) << 17, id1 = umma_idesc_bf16(128u, 0u) + nfield;
         const uint32_t ids[3] = {id1, id1 + nfield, id1 + 2u * nfield};
         const uint32_t wlo = (smem_u32(wsm) >> 4) | (1u << 16), slo = (smem_u32(stage0) >> 4) | (1u << 16);
         const uint32_t bstep = (uint32_t)b_bytes >> 4;
@@ -834,7 +833,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
         // boxes); fresh: row rr of the accumulators gets its first products
         auto mma_row = [&](uint32_t dt, uint32_t ar, uint32_t b, int rr, int dx0, int dx1, bool fresh) {
             const int lo = rr < 2 ? 0 : rr - 2, n = (rr < kR ? rr : kR - 1) - lo + 1;   // rows lo ..: tap dy = rr - o
-            const uint32_t d = dt + (uint32_t)(lo * p.nco);
+            const uint32_t d = dt + (uint32_t)(lo * nco);
 #pragma unroll
             for (int dx = dx0; dx < dx1; ++dx)
 #pragma unroll
@@ -844,14 +843,14 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                     const uint32_t bo = bx + (uint32_t)(2 - rr + lo) * bstep;
                     if (dx == dx0 && kk == 0 && rr < kR && fresh) {
                         if (rr > 0) umma_bf16_lo(d, al, kHi, bo, kHiB, ids[n - 2 < 0 ? 0 : n - 2], 1u);
-                        umma_bf16_lo(dt + (uint32_t)(rr * p.nco), al, kHi, bx + 2u * bstep, kHiB, id1, 0u);
+                        umma_bf16_lo(dt + (uint32_t)(rr * nco), al, kHi, bx + 2u * bstep, kHiB, id1, 0u);
                     } else {
                         umma_bf16_lo(d, al, kHi, bo, kHiB, ids[n - 1], 1u);
                     }
                 }
         };
         for (int t = blockIdx.x + who * gridDim.x; t < p.items && ok; t += 2 * gridDim.x, kt += 2) {
-            const uint32_t dt = tmem + (uint32_t)(set * kR * p.nco);
+            const uint32_t dt = tmem + (uint32_t)(set * kR * nco);
             if (kt >= p.sets) ok = mbar_wait_bounded(&sempty[set], phase ^ 1u, a.err);
             ok = __all_sync(0xFFFFFFFFu, ok);
             if (kDxOuter) {
@@ -950,31 +949,38 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                 const bool mine = turn == group;
                 if (++turn == p.groups) turn = 0;
                 if (!mine) continue;
-                uint4 add[kMode == kRowAdd ? kG / 8 : 1];
-                if (kMode == kRowAdd) {   // in flight while the tile's sums are awaited (one column group)
+                // the addend, in flight while the tile's sums are awaited (one column group): kG / 8 lanes to
+                // a pixel, whole sectors each; every lane gets its own pixel's through the store buffer
+                constexpr int kParts = kG / 8;
+                uint4 add[kMode == kRowAdd ? kParts : 1];
+                if (kMode == kRowAdd) {
                     const int y = yb * kR + o0;
-                    const bool in = x < a.W && y < a.H;
-                    const uint4* src = reinterpret_cast<const uint4*>(
-                        reinterpret_cast<const __nv_bfloat16*>(a.add_par) + (in ? pix_add(a, img, x, y) + co0 : 0));
 #pragma unroll
-                    for (int j = 0; j < kG / 8; ++j) add[j] = in ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+                    for (int j = 0; j < kParts; ++j) {
+                        const int xa = x0 + j * (32 / kParts) + lane / kParts;
+                        const bool in = xa < a.W && y < a.H;
+                        add[j] = in ? __ldg(reinterpret_cast<const uint4*>(
+                                                reinterpret_cast<const __nv_bfloat16*>(a.add_par) +
+                                                pix_add(a, img, xa, y)) + lane % kParts)
+                                    : make_uint4(0u, 0u, 0u, 0u);
+                    }
                 }
                 ok = mbar_wait_bounded(&sfull[set], phase, a.err) && !*abort_flag;
                 ok = __all_sync(0xFFFFFFFFu, ok);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll 1
-                for (int c0 = 0; c0 < p.nco; c0 += kG) {
+                for (int c0 = 0; c0 < nco; c0 += kG) {
                     uint32_t pk[kUnit][kG / 2];   // the rows' stored values
 #pragma unroll
                     for (int u = 0; u < kUnit; ++u) {
                         const int o = o0 + u, y = yb * kR + o;
                         uint32_t r[kG];
-                        const uint32_t col = lane0 + (uint32_t)((set * kR + o) * p.nco + c0);
+                        const uint32_t col = lane0 + (uint32_t)((set * kR + o) * nco + c0);
                         if constexpr (kG == 32) tmem_ld32(col, r);
                         else tmem_ld16(col, r);
                         tmem_ld_wait();
-                        if (c0 + kG >= p.nco) {
+                        if (c0 + kG >= nco) {
                             tc_fence_before();
                             __syncwarp();
                             if (leader) mbar_arrive(&sempty[set]);
@@ -990,12 +996,24 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                             v[j + 3] = __uint_as_float(r[j + 3]) + b.w;
                         }
                         if (kMode == kRowAdd) {
+                            tma_store_wait_read<0>();
+                            __syncwarp();
 #pragma unroll
-                            for (int j = 0; j < kG / 2; ++j) {
-                                const uint4& w4 = add[j / 4];
-                                const uint32_t w = (j & 3) == 0 ? w4.x : (j & 3) == 1 ? w4.y : (j & 3) == 2 ? w4.z : w4.w;
-                                v[2 * j] += __uint_as_float(w << 16);
-                                v[2 * j + 1] += __uint_as_float(w & 0xFFFF0000u);
+                            for (int j = 0; j < kParts; ++j) {
+                                const int px = j * (32 / kParts) + lane / kParts;
+                                const int psw = kG == 32 ? (px >> 1) & 3 : (px >> 2) & 1;
+                                reinterpret_cast<uint4*>(sbuf)[px * kParts + ((lane % kParts) ^ psw)] = add[j];
+                            }
+                            __syncwarp();
+#pragma unroll
+                            for (int j = 0; j < kParts; ++j) {
+                                const uint4 w4 = sb[j ^ sw];
+                                const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    v[8 * j + 2 * k] += __uint_as_float(w[k] << 16);
+                                    v[8 * j + 2 * k + 1] += __uint_as_float(w[k] & 0xFFFF0000u);
+                                }
                             }
                         }
                         if (kMode == kRowF32) {
@@ -1005,13 +1023,13 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                             }
                             if (x < a.W && y < a.H) {
                                 float* d = reinterpret_cast<float*>(a.out) +
-                                           (((size_t)img * a.H + y) * a.W + x) * a.out_c + a.out_off + co0 + c0;
+                                           (((size_t)img * a.H + y) * a.W + x) * a.out_c + a.out_off + c0;
 #pragma unroll
                                 for (int h = 0; h < kG; h += 16) {
                                     float w[16];
 #pragma unroll
                                     for (int j = 0; j < 16; ++j) w[j] = v[h + j];
-                                    store_f32(d + h, w, min(16, a.n_store - co0 - c0 - h));
+                                    store_f32(d + h, w, min(16, a.n_store - c0 - h));
                                 }
                             }
                             continue;
@@ -1030,10 +1048,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                         fence_async_smem();
                         __syncwarp();
                         if (leader && y < a.H && x0 < a.W) {
-                            tma_store_4d(&mo, sbuf, co0 + c0, x0, y, img);
+                            tma_store_4d(&mo, sbuf, c0, x0, y, img);
                             if (a.up_out)
                                 for (int k = 0; k < 4; ++k)
-                                    tma_store_5d(&mu, sbuf, co0 + c0, k & 1, x0, 2 * y + (k >> 1), img);
+                                    tma_store_5d(&mu, sbuf, c0, k & 1, x0, 2 * y + (k >> 1), img);
                             tma_store_commit();
                         }
                     }
@@ -1041,7 +1059,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
                         const int h2 = a.H >> 1, w2 = a.W >> 1, y2 = (yb * kR + o0) >> 1;
                         pool_store<kG>(pk[0], pk[kUnit - 1], y2 < h2 && (x >> 1) < w2,
                                        reinterpret_cast<__nv_bfloat16*>(a.pool_out) +
-                                           (((size_t)img * h2 + y2) * w2 + (x >> 1)) * a.pool_c + a.pool_off + co0 + c0);
+                                           (((size_t)img * h2 + y2) * w2 + (x >> 1)) * a.pool_c + a.pool_off + c0);
                     }
                 }
             }
@@ -1049,6 +1067,257 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
             if (++set == p.sets) {
                 set = 0;
                 phase ^= 1u;
+            }
+        }
+        if (leader) tma_store_wait_all();
+    }
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 512u);
+}
+
+// ---------------------------------------------------------------------------------------------
+// 16 x 16-pixel tiles with streamed weights, for the layers whose weights do not fit in shared memory beside
+// a row tile's chunks (sums by horizontal tap). A stage holds 64 input channels at one horizontal shift: the box {64 channels,
+// 16 x, 18 y} in 128-byte-swizzled rows, whose windows from image row 0, 1 and 2 are the vertical taps,
+// and the three taps' weights {64, Cout}. Both halves of the tile (16 x 8 pixels, M = 128, an accumulator
+// each, with an issuer of its own) use them: 12 MMAs an issuer and stage.
+// What bounds it: the TMA unit, which takes about 1.6 cycles for a box row of 64 bytes and 1.8 for one of
+// 128, and the operand reads. A 16 x 8 tile with stages of 32 channels loads 352 rows for 288 cycles of
+// MMAs (64 output channels); here it is 480 rows for 1152. Before and after, cold: 160 -> 64 channels on 540 x
+// 960 pixels 103 -> 88 us, 224 -> 96 on 270 x 480 54 -> 46, 128 -> 96 on 2 x 300 x 300 44 -> 33.
+constexpr int kBigEdge = 16;
+constexpr int kBigXBytes = kBigEdge * (kBigEdge + 2) * 128;
+constexpr int kBigMaxStages = 4;
+constexpr int kBigThreads = 96 + 2 * kEpiThreads;   // producer, issuer, epilogue, issuer
+
+struct BigPlan {
+    int nx, ny, items;   // tiles per image row and column, in all
+    int stages, groups;  // of four epilogue warps (two: one for each half)
+};
+
+template <int kG, bool kPool>
+__global__ void __launch_bounds__(kBigThreads, 1) k_conv_tiles(const __grid_constant__ CUtensorMap mx,
+                                                               const __grid_constant__ CUtensorMap mw,
+                                                               const __grid_constant__ CUtensorMap mo,
+                                                               const __grid_constant__ CUtensorMap mu, ConvArgs a,
+                                                               BigPlan p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const int kc = a.cin / 32, chunks = (kc + 1) / 2, nco = a.cout;
+    const int b_bytes = nco * 128, stage_bytes = kBigXBytes + 3 * b_bytes;
+    uint8_t* stores = smem + p.stages * stage_bytes;   // 64 kG bytes per epilogue warp
+    float* bsm = reinterpret_cast<float*>(stores + p.groups * 4 * 64 * kG);
+    uint64_t* full = reinterpret_cast<uint64_t*>(bsm + 128);
+    uint64_t* empty = full + kBigMaxStages;
+    uint64_t* sfull = empty + kBigMaxStages;   // a tile's sums are complete (two tiles alternate in TMEM)
+    uint64_t* sempty = sfull + 2;              // and have been read
+    uint64_t* fin = sempty + 2;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(fin + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < p.stages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 2);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&sfull[i], 2);
+            mbar_init(&sempty[i], 8);   // four warps for each half
+        }
+        mbar_init(fin, 2);
+        *abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(tslot, 512u);
+        tmem_relinquish();
+    }
+    for (int i = tid; i < nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + i) : -0.0f;   // -0 adds nothing
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+    const int per_img = p.nx * p.ny;
+
+    if (warp == 0) {
+        if (lane == 0) {   // producer
+            int s = 0;
+            uint32_t use = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < p.items && ok; t += gridDim.x) {
+                const int img = t / per_img, r = t - img * per_img, ty = r / p.nx;
+                const int x = (r - ty * p.nx) * kBigEdge - 1, y = ty * kBigEdge - 1;
+                for (int dx = 0; dx < 3 && ok; ++dx)
+                    for (int c = 0; c < chunks; ++c) {
+                        if (use > 0) ok = mbar_wait_bounded(&empty[s], (use - 1u) & 1u, a.err);
+                        if (!ok || *abort_flag) {
+                            *abort_flag = 1;
+                            ok = false;
+                            break;
+                        }
+                        uint8_t* sa = smem + s * stage_bytes;
+                        mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
+                        tma_load_4d(sa, &mx, 64 * c, x + dx, y, img, &full[s]);
+                        for (int dy = 0; dy < 3; ++dy)
+                            tma_load_2d(sa + kBigXBytes + dy * b_bytes, &mw, (3 * dy + dx) * a.cin + 64 * c, 0, &full[s]);
+                        if (++s == p.stages) {
+                            s = 0;
+                            ++use;
+                        }
+                    }
+            }
+            // no load may be in flight when the CTA ends, whoever gave up
+            for (int i = 0; i < p.stages; ++i) {
+                const uint32_t uses = use + (i < s ? 1u : 0u);
+                if (uses > 0) mbar_wait_bounded(&full[i], (uses - 1u) & 1u, a.err);
+            }
+        }
+    } else if (warp == 1 || warp == 2 + 4 * p.groups) {
+        // one MMA issuer for each half of the tile: the warp walks the stages, one elected lane issues
+        constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // 8-row groups 1 KB apart, SWIZZLE_128B
+        const bool leader = elect_one();
+        const uint32_t idesc = umma_idesc_bf16(128u, (uint32_t)nco), bstep = (uint32_t)b_bytes >> 4;
+        const uint32_t slo = (smem_u32(smem) >> 4) | (1u << 16);
+        int s = 0, kt = 0;
+        uint32_t use = 0;
+        bool ok = true;
+        const int half = warp == 1 ? 0 : 1;
+        // the taps dy of one 32-channel half of a stage
+        auto chunk = [&](uint32_t d, uint32_t al, uint32_t bl, bool fresh) {
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int kk = 0; kk < 2; ++kk)
+                    umma_bf16_lo(d, al + (uint32_t)(dy * kBigEdge * 8 + 2 * kk), kHi,
+                                 bl + (uint32_t)dy * bstep + 2u * (uint32_t)kk, kHi, idesc,
+                                 dy == 0 && kk == 0 && fresh ? 0u : 1u);
+        };
+        for (int t = blockIdx.x; t < p.items && ok; t += gridDim.x, ++kt) {
+            const int set = kt & 1;
+            const uint32_t d = tmem + (uint32_t)((set * 2 + half) * nco);
+            if (kt >= 2) ok = mbar_wait_bounded(&sempty[set], (uint32_t)((kt >> 1) - 1) & 1u, a.err);
+            for (int i = 0, c = 0; i < 3 * chunks && ok; ++i) {
+                ok = mbar_wait_bounded(&full[s], use & 1u, a.err) && ok;
+                ok = __all_sync(0xFFFFFFFFu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                if (leader) {
+                    const uint32_t st = slo + (uint32_t)(s * (stage_bytes >> 4)), bl = st + (uint32_t)(kBigXBytes >> 4);
+                    const uint32_t al = st + (uint32_t)(8 * half * kBigEdge * 8);
+                    chunk(d, al, bl, i == 0);
+                    if (2 * c + 1 < kc) chunk(d, al + 4u, bl + 4u, false);
+                    umma_commit(&empty[s]);
+                }
+                __syncwarp();
+                if (++s == p.stages) {
+                    s = 0;
+                    ++use;
+                }
+                if (++c == chunks) c = 0;
+            }
+            if (!ok) break;
+            if (leader) umma_commit(&sfull[set]);
+            __syncwarp();
+        }
+        if (!ok) *abort_flag = 1;
+        if (leader) {
+            umma_commit(fin);
+            mbar_wait_bounded(fin, 0u, a.err);   // nothing may be in flight when TMEM is freed
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3, group = (warp - 2) >> 2;
+        uint8_t* sbuf = stores + (warp - 2) * 64 * kG;
+        const uint32_t lane0 = tmem + ((uint32_t)(q * 32) << 16);
+        const bool relu = (a.flags & kConvRelu) != 0, leader = elect_one();
+        constexpr int kParts = kG / 8;   // 16-byte parts of a pixel's group of columns
+        const int sw = kG == 32 ? (lane >> 1) & 3 : (lane >> 2) & 1;
+        uint4* sb = reinterpret_cast<uint4*>(sbuf) + lane * kParts;
+        int kt = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < p.items && ok; t += gridDim.x, ++kt) {
+            const int set = kt & 1;
+            const int img = t / per_img, r = t - img * per_img, ty = r / p.nx, x0 = (r - ty * p.nx) * kBigEdge;
+            ok = mbar_wait_bounded(&sfull[set], (uint32_t)(kt >> 1) & 1u, a.err) && !*abort_flag;
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            for (int half = group; half < 2; half += p.groups) {
+                const int y0 = ty * kBigEdge + 8 * half + 2 * q;   // the warp's two rows of 16 pixels
+#pragma unroll 1
+                for (int c0 = 0; c0 < nco; c0 += kG) {
+                    uint32_t v[kG];
+                    const uint32_t col = lane0 + (uint32_t)((set * 2 + half) * nco + c0);
+                    if constexpr (kG == 32) tmem_ld32(col, v);
+                    else tmem_ld16(col, v);
+                    tmem_ld_wait();
+                    if (c0 + kG >= nco) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (leader) mbar_arrive(&sempty[set]);
+                    }
+                    const float4* b4 = reinterpret_cast<const float4*>(bsm + c0);
+                    uint32_t pk[kG / 2];
+#pragma unroll
+                    for (int j = 0; j < kG; j += 4) {
+                        const float4 b = b4[j / 4];
+                        pk[j / 2] = pack_bf16x2(__uint_as_float(v[j]) + b.x, __uint_as_float(v[j + 1]) + b.y);
+                        pk[j / 2 + 1] = pack_bf16x2(__uint_as_float(v[j + 2]) + b.z, __uint_as_float(v[j + 3]) + b.w);
+                    }
+                    if (relu) {   // of the rounded values: the same (a NaN becomes 0 either way)
+#pragma unroll
+                        for (int j = 0; j < kG / 2; ++j) pk[j] = relu2(pk[j]);
+                    }
+                    tma_store_wait_read<0>();   // the leader's last store has read the buffer
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < kParts; ++j)
+                        sb[j ^ sw] = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+                    fence_async_smem();
+                    __syncwarp();
+                    if (leader && y0 < a.H) {
+                        tma_store_4d(&mo, sbuf, c0, x0, y0, img);
+                        if (a.up_out)
+                            for (int k = 0; k < 8; ++k)
+                                if (y0 + (k >> 2) < a.H)
+                                    tma_store_5d(&mu, sbuf + (k >> 2) * 32 * kG, c0, k & 1, x0,
+                                                 2 * (y0 + (k >> 2)) + ((k >> 1) & 1), img);
+                        tma_store_commit();
+                    }
+                    if (kPool) {
+                        // the warp's 8 pooled pixels from their four stored values: lane l takes part
+                        // l % 4 of pixel l / 4 (8 channels of 32, 4 of 16)
+                        const int pp = lane >> 2, x = (x0 >> 1) + pp;
+                        float lo[kParts], hi[kParts];
+#pragma unroll
+                        for (int j = 0; j < kParts; ++j) lo[j] = hi[j] = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const int n = 2 * pp + (k & 1) + 16 * (k >> 1);
+                            const int nsw = kG == 32 ? (n >> 1) & 3 : (n >> 2) & 1;
+                            const int part = kG == 32 ? lane & 3 : (lane & 3) >> 1;
+                            const uint32_t* w = reinterpret_cast<const uint32_t*>(sbuf + n * 2 * kG + 16 * (part ^ nsw)) +
+                                                (kG == 32 ? 0 : 2 * (lane & 1));
+#pragma unroll
+                            for (int j = 0; j < kParts; ++j) {
+                                lo[j] = lo[j] + __uint_as_float(w[j] << 16);
+                                hi[j] = hi[j] + __uint_as_float(w[j] & 0xFFFF0000u);
+                            }
+                        }
+                        if ((y0 >> 1) < (a.H >> 1) && x < (a.W >> 1)) {
+                            uint32_t o[kParts];
+#pragma unroll
+                            for (int j = 0; j < kParts; ++j) o[j] = pack_bf16x2(lo[j] * 0.25f, hi[j] * 0.25f);
+                            __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(a.pool_out) +
+                                               (((size_t)img * (a.H >> 1) + (y0 >> 1)) * (a.W >> 1) + x) * a.pool_c +
+                                               a.pool_off + c0 + 2 * kParts * (lane & 3);
+                            if constexpr (kG == 32) *reinterpret_cast<uint4*>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+                            else *reinterpret_cast<uint2*>(d) = make_uint2(o[0], o[1]);
+                        }
+                        __syncwarp();
+                    }
+                }
             }
         }
         if (leader) tma_store_wait_all();
@@ -1067,6 +1336,8 @@ cudaError_t gkrt_encode_tmap_bf16(CUtensorMap* map, const void* base, uint32_t r
                                   const uint64_t* strides_bytes, const uint32_t* box);
 cudaError_t gkrt_encode_tmap_bf16_sw32(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims,
                                        const uint64_t* strides_bytes, const uint32_t* box);
+cudaError_t gkrt_encode_tmap_bf16_sw128(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims,
+                                        const uint64_t* strides_bytes, const uint32_t* box);
 cudaError_t gkrt_encode_tmap_bf16_dense(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims,
                                         const uint64_t* strides_bytes, const uint32_t* box);
 
@@ -1087,7 +1358,7 @@ constexpr int kRowSmemMin = 116 * 1024;   // more than half of an SM's: one CTA 
 static int row_rows(const ConvArgs& a, bool dx_outer) { return dx_outer || a.pool_out || a.cin > 32 ? 2 : 3; }
 
 static size_t row_smem(const ConvArgs& a, const RowPlan& p, int stage) {
-    return (size_t)9 * a.cin * p.nco * 2 + (size_t)2 * p.ring * stage + (size_t)p.groups * 4 * 64 * (p.nco % 32 ? 16 : 32) +
+    return (size_t)9 * a.cin * a.cout * 2 + (size_t)2 * p.ring * stage + (size_t)p.groups * 4 * 64 * (a.cout % 32 ? 16 : 32) +
            128 * 4 + (2 * kRowMaxStages + 2 * kRowMaxSets + 3 * kRowMaxChunks + 1) * 8 + 8 + 1024;
 }
 
@@ -1100,49 +1371,60 @@ static bool row_turns_ok(const RowPlan& p, int units) {
 }
 
 // The plan of a convolution on row tiles, or none (items 0) where it does not fit or the other kernels'
-// 16 x 8 tiles are estimated faster. The output channels are split over CTAs until the weights leave room
-// for each issuer's boxes (all of a tile's chunks where they stay, else two).
+// 16 x 8 tiles are estimated faster. Each issuer needs room for all of a tile's chunks where they stay,
+// else for two. (Splitting the output channels over CTAs to make room was slower than 16 x 16 tiles with
+// streamed weights: 64 -> 96 channels on 4 x 200 x 500 pixels 52 us, and 41.)
 // The estimate is in times of one 16 x 8 tile per SM, of which the other kernels take their tiles' number
-// over the SMs; a row tile was measured at 1.0 of those (128 x 2 pixels, sums by horizontal tap; 0.62
-// with the channels split), 1.8 (128 x 3, sums by chunk) and 1.5 (128 x 2), and whole waves count. Over
-// nine layers on 50 sizes from 16 x 32 to 4 x 200 x 500 either side of that line differs by at most 15%
-// (64 -> 64 channels: 200 x 128 pixels 8.2 us by tiles, 7.9 by rows; 4 x 200 x 140 14.8 and 16.4).
+// over the SMs; a row tile was measured at 1.0 of those (128 x 2 pixels, sums by horizontal tap), 1.8 (128
+// x 3, sums by chunk) and 1.5 (128 x 2), and whole waves count. Over the layers on 50 sizes from 16 x 32 to
+// 4 x 200 x 500 either side of that line differs by at most 15% (64 -> 64 channels: 200 x 128 pixels 8.2 us
+// by tiles, 7.9 by rows; 4 x 200 x 140 14.8 and 16.4).
 static RowPlan row_plan(const ConvArgs& a, int rb, int sms) {
     RowPlan p{};
     const int kc = a.cin / 32;
     const bool dx_outer = !conv_halo(a.cin, a.cout);
     const int R = row_rows(a, dx_outer), stage = row_stage_bytes(rb, R), need = dx_outer ? kc : 2;
-    if (a.cout > 128 || kc > kRowMaxChunks || (a.add_par && (a.pool_out || a.cout > 32))) return p;
+    if (a.cout > 128 || kc > kRowMaxChunks || (a.add_par && (a.pool_out || dx_outer))) return p;
     p.nxs = (a.W + 127) / 128;
     p.nyb = (a.H + R - 1) / R;
     const long long items = (long long)a.B * p.nxs * p.nyb;
     if (items > 0x7FFFFFFFLL / 4) return p;
-    for (int split = 1; split <= 4; ++split) {
-        if (split > 1 && a.cout % (32 * split)) continue;
-        p.nco = a.cout / split;
-        p.sets = std::min(kRowMaxSets, 512 / (R * p.nco)) & ~1;   // the issuers' in turn
-        for (p.groups = kRowGroups; p.groups > 0; p.groups /= 2) {
-            p.ring = 0;
-            const size_t fixed = row_smem(a, p, stage);
-            if (fixed < (size_t)kRowSmem)
-                p.ring = std::min(kRowMaxStages / 2, (int)(((size_t)kRowSmem - fixed) / (2 * (size_t)stage)));
-            if (p.ring >= need && row_turns_ok(p, R / (a.pool_out ? 2 : 1))) break;
-        }
-        if (!p.groups) continue;
-        const long long grid = std::max(1, sms / split), waves = (items + grid - 1) / grid;
-        const float rows = dx_outer ? (split == 1 ? 1.0f : 0.62f) * (float)waves + 0.3f
-                                    : (R == 3 ? 1.8f : 1.5f) * (float)waves + 1.6f;
-        const long long tiles = (long long)a.B * ((a.W + kTileX - 1) / kTileX) * ((a.H + kTileY - 1) / kTileY);
-        if (rows < (float)tiles / (float)sms) p.items = (int)items;
-        return p;
+    p.sets = std::min(kRowMaxSets, 512 / (R * a.cout)) & ~1;   // the issuers' in turn
+    for (p.groups = kRowGroups; p.groups > 0; p.groups /= 2) {
+        const size_t fixed = row_smem(a, p, 0);
+        p.ring = fixed < (size_t)kRowSmem
+                     ? std::min(kRowMaxStages / 2, (int)(((size_t)kRowSmem - fixed) / (2 * (size_t)stage)))
+                     : 0;
+        if (p.ring >= need && row_turns_ok(p, R / (a.pool_out ? 2 : 1))) break;
     }
+    if (!p.groups) return p;
+    const long long waves = (items + sms - 1) / sms;
+    const float rows = dx_outer ? (float)waves + 0.3f : (R == 3 ? 1.8f : 1.5f) * (float)waves + 1.6f;
+    const long long tiles = (long long)a.B * ((a.W + kTileX - 1) / kTileX) * ((a.H + kTileY - 1) / kTileY);
+    if (rows < (float)tiles / (float)sms) p.items = (int)items;
     return p;
+}
+
+// The tensor maps of a bf16 output's stores, kg channels of bx x by pixels, and of its nearest
+// upsampling's, bx pixels of a row to every other pixel.
+static cudaError_t encode_outputs(const ConvArgs& a, int kg, uint32_t bx, uint32_t by, CUtensorMap* mo, CUtensorMap* mu) {
+    auto encode = kg == 32 ? gkrt_encode_tmap_bf16 : gkrt_encode_tmap_bf16_sw32;
+    const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B, oc = (uint64_t)a.out_c * 2;
+    const uint64_t od[4] = {(uint64_t)a.cout, W, H, B}, os[3] = {oc, W * oc, H * W * oc};
+    const uint32_t ob[4] = {(uint32_t)kg, bx, by, 1};
+    cudaError_t e = encode(mo, static_cast<uint8_t*>(a.out) + (size_t)a.out_off * 2, 4, od, os, ob);
+    *mu = *mo;
+    if (e != cudaSuccess || !a.up_out) return e;
+    const uint64_t uc = (uint64_t)a.up_c * 2;
+    const uint64_t ud[5] = {(uint64_t)a.cout, 2, W, 2 * H, B}, us[4] = {uc, 2 * uc, 2 * W * uc, 4 * H * W * uc};
+    const uint32_t ub[5] = {(uint32_t)kg, 1, bx, 1, 1};
+    return encode(mu, static_cast<uint8_t*>(a.up_out) + (size_t)a.up_off * 2, 5, ud, us, ub);
 }
 
 static cudaError_t launch_rows(const void* xbase, int xv, uint64_t xc, const void* w, const ConvArgs& a, const RowPlan& p,
                                int rb, int sms, int dev, cudaStream_t st) {
     const bool f32 = (a.flags & kConvF32Out) != 0, dx_outer = !conv_halo(a.cin, a.cout);
-    const int kg = p.nco % 32 ? 16 : 32, R = row_rows(a, dx_outer);
+    const int kg = a.cout % 32 ? 16 : 32, R = row_rows(a, dx_outer);
     const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B;
     CUtensorMap mx, mw, mo, mu;
     const uint64_t xd[4] = {(uint64_t)xv, W, H, B};
@@ -1153,22 +1435,10 @@ static cudaError_t launch_rows(const void* xbase, int xv, uint64_t xc, const voi
     if (e != cudaSuccess) return e;
     const uint64_t wd[2] = {(uint64_t)9 * a.cin, (uint64_t)a.cout};
     const uint64_t ws[1] = {(uint64_t)9 * a.cin * 2};
-    const uint32_t wb[2] = {32, (uint32_t)p.nco};
+    const uint32_t wb[2] = {32, (uint32_t)a.cout};
     if ((e = gkrt_encode_tmap_bf16(&mw, w, 2, wd, ws, wb)) != cudaSuccess) return e;
     mo = mu = mw;
-    auto encode = kg == 32 ? gkrt_encode_tmap_bf16 : gkrt_encode_tmap_bf16_sw32;
-    if (!f32) {
-        const uint64_t oc = (uint64_t)a.out_c * 2;
-        const uint64_t od[4] = {(uint64_t)a.cout, W, H, B}, os[3] = {oc, W * oc, H * W * oc};
-        const uint32_t ob[4] = {(uint32_t)kg, 32, 1, 1};
-        if ((e = encode(&mo, static_cast<uint8_t*>(a.out) + (size_t)a.out_off * 2, 4, od, os, ob)) != cudaSuccess) return e;
-    }
-    if (a.up_out) {
-        const uint64_t uc = (uint64_t)a.up_c * 2;
-        const uint64_t ud[5] = {(uint64_t)a.cout, 2, W, 2 * H, B}, us[4] = {uc, 2 * uc, 2 * W * uc, 4 * H * W * uc};
-        const uint32_t ub[5] = {(uint32_t)kg, 1, 32, 1, 1};
-        if ((e = encode(&mu, static_cast<uint8_t*>(a.up_out) + (size_t)a.up_off * 2, 5, ud, us, ub)) != cudaSuccess) return e;
-    }
+    if (!f32 && (e = encode_outputs(a, kg, 32, 1, &mo, &mu)) != cudaSuccess) return e;
     typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ConvArgs, RowPlan);
     // by pixel bytes, rows and order of the sums; column group; mode
 #define GK_ROWS(rb, kg, r, dxo, add) \
@@ -1191,10 +1461,72 @@ static cudaError_t launch_rows(const void* xbase, int xv, uint64_t xc, const voi
                 return e;
         attr[dev] = true;
     }
-    const int split = a.cout / p.nco;
     const size_t smem = row_smem(a, p, row_stage_bytes(rb, R));
-    const unsigned grid = (unsigned)std::min(p.items, std::max(1, sms / split));
-    kernel<<<dim3(grid, (unsigned)split), 96 + p.groups * kEpiThreads, std::max(smem, (size_t)kRowSmemMin), st>>>(mx, mw, mo, mu, a, p);
+    kernel<<<std::min(p.items, sms), 96 + p.groups * kEpiThreads, std::max(smem, (size_t)kRowSmemMin), st>>>(mx, mw, mo, mu, a,
+                                                                                                          p);
+    return cudaGetLastError();
+}
+
+static size_t big_smem(const ConvArgs& a, const BigPlan& p) {
+    return (size_t)p.stages * (kBigXBytes + 3 * a.cout * 128) + (size_t)p.groups * 4 * 64 * (a.cout % 32 ? 16 : 32) +
+           128 * 4 + (2 * kBigMaxStages + 5) * 8 + 8 + 1024;
+}
+
+// The 16 x 16-tile plan of a convolution whose sums are taken by horizontal tap, or none (items 0) where
+// 16 x 8 tiles are estimated faster: a wave of these was measured at 1.4 to 1.65 times one of those per
+// SM (seven layers, sizes from 16 x 32 to 4 x 200 x 500), which lose where the second wave is nearly
+// empty (160 -> 64 channels on 200 x 192 pixels 12.4 us by 16 x 8 tiles, 14.7 by these; 500 wide 24.4 and
+// 20.5) and never where there is one wave (9.3 and 11.0).
+static BigPlan big_plan(const ConvArgs& a, int sms) {
+    BigPlan p{};
+    if (a.cout > 128 || conv_halo(a.cin, a.cout) || a.add_par || (a.flags & kConvF32Out)) return p;
+    // two epilogue groups, unless one leaves room for a third stage
+    for (p.stages = 4, p.groups = 2; big_smem(a, p) > (size_t)kRowSmem;) {
+        if (p.groups == 2 && p.stages == 3) p.groups = 1;
+        else {
+            p.groups = 2;
+            --p.stages;
+        }
+    }
+    p.nx = (a.W + kBigEdge - 1) / kBigEdge;
+    p.ny = (a.H + kBigEdge - 1) / kBigEdge;
+    const long long items = (long long)a.B * p.nx * p.ny;
+    if (items > 0x7FFFFFFFLL / 4) return p;
+    const long long waves = (items + sms - 1) / sms;
+    const long long tiles = (long long)a.B * ((a.W + kTileX - 1) / kTileX) * ((a.H + kTileY - 1) / kTileY);
+    if (waves == 1 || 1.6f * (float)waves <= (float)tiles / (float)sms + 0.7f) p.items = (int)items;
+    return p;
+}
+
+static cudaError_t launch_big(const void* xbase, int xv, uint64_t xc, const void* w, const ConvArgs& a, const BigPlan& p,
+                              int sms, int dev, cudaStream_t st) {
+    const int kg = a.cout % 32 ? 16 : 32;
+    const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B;
+    CUtensorMap mx, mw, mo, mu;
+    const uint64_t xd[4] = {(uint64_t)xv, W, H, B};
+    const uint64_t xs[3] = {xc * 2, W * xc * 2, H * W * xc * 2};
+    const uint32_t xb[4] = {64, kBigEdge, kBigEdge + 2, 1};
+    cudaError_t e = gkrt_encode_tmap_bf16_sw128(&mx, xbase, 4, xd, xs, xb);
+    if (e != cudaSuccess) return e;
+    const uint64_t wd[2] = {(uint64_t)9 * a.cin, (uint64_t)a.cout};
+    const uint64_t ws[1] = {(uint64_t)9 * a.cin * 2};
+    const uint32_t wb[2] = {64, (uint32_t)a.cout};
+    if ((e = gkrt_encode_tmap_bf16_sw128(&mw, w, 2, wd, ws, wb)) != cudaSuccess) return e;
+    if ((e = encode_outputs(a, kg, 16, 2, &mo, &mu)) != cudaSuccess) return e;
+    typedef void (*Kernel)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ConvArgs, BigPlan);
+    static const Kernel kernels[2][2] = {{k_conv_tiles<16, false>, k_conv_tiles<16, true>},
+                                         {k_conv_tiles<32, false>, k_conv_tiles<32, true>}};
+    static bool attr[kMaxDevices] = {};
+    if (!attr[dev]) {
+        for (int i = 0; i < 4; ++i)
+            if ((e = cudaFuncSetAttribute((const void*)kernels[i / 2][i % 2], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          kRowSmem)) != cudaSuccess)
+                return e;
+        attr[dev] = true;
+    }
+    const size_t smem = std::max(big_smem(a, p), (size_t)kRowSmemMin);
+    kernels[kg == 32][a.pool_out != nullptr]<<<std::min(p.items, sms), 96 + p.groups * kEpiThreads, smem, st>>>(mx, mw, mo,
+                                                                                                      mu, a, p);
     return cudaGetLastError();
 }
 
@@ -1322,6 +1654,8 @@ cudaError_t gkrt_launch_conv3x3(const void* x, const void* w, const ConvArgs& ar
     const uint32_t wb[2] = {32, (uint32_t)args.cout};
     e = gkrt_encode_tmap_bf16(&mw, w, 2, wd, ws, wb);
     if (e != cudaSuccess) return e;
+    const BigPlan big = big_plan(args, sms);
+    if (big.items) return launch_big(xbase, xv, xc, w, args, big, sms, dev, st);
     const size_t smem = gkrt_conv_smem_bytes(args.cout);
     // launch geometry per output width, computed once per device (host calls kept off the
     // per-launch path)

@@ -7,6 +7,7 @@ import pytest
 from gknextengine_gb300 import abi, native
 from gknextengine_gb300.denoiser import Unet
 from gknextengine_gb300.renderer import PathTracingRenderer
+import test_gpu_conv as base
 from test_gpu_conv import _torch
 
 pytestmark = pytest.mark.gpu
@@ -75,3 +76,15 @@ def test_unet_batch_equals_single_images():
             one = torch.zeros((1, H, W, 4), device="cuda")
             net.forward(x[i:i + 1].contiguous(), out_raw=one)
             assert torch.equal(raw[i], one[0])
+
+
+# 16 x 16 tiles: one pixel short of, at and past an edge and a half; channels that end in half a stage;
+# groups of 32 and of 16 output channels; two and three stages
+@pytest.mark.parametrize("B,H,W,cin,cout", [(2, 15, 17, 96, 96), (1, 33, 31, 160, 64), (1, 9, 16, 224, 96),
+                                            (3, 24, 48, 128, 128), (1, 17, 15, 160, 48), (1, 8, 8, 320, 80),
+                                            (1, 1, 1, 96, 128), (2, 200, 130, 192, 64)])
+def test_tiles_match_torch(B, H, W, cin, cout):
+    """As the other convolutions' tests, with their tolerances."""
+    base.test_conv_matches_torch(B, H, W, cin, cout, True)
+    if H > 1:
+        base.test_conv_fused_pool_and_upsample(B, H, W, cin, cout)
