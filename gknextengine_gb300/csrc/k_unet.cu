@@ -17,51 +17,41 @@ namespace {
 // ---- weight gradient with TMA-fed MN-major operands ----
 // dW[cout][tap][cin] = sum over pixels of dP[p][cout] X[p + tap][cin] with K = pixels: NHWC rows hold
 // the channels of one pixel contiguously, which is the MN-major layout of both operands for K along
-// pixels, so TMA loads them unchanged, in boxes of 32 channels x 32 pixels x some image rows, 64-byte
-// swizzled (atoms of 8 pixels x 64 bytes). All nine taps of 32 x 32 channels are one MMA of 128 x 96:
-//   M  rows are four boxes of X: the pairs (dx, 32-channel group) in order, four to an M block, each
-//      box loaded at its horizontal shift;
+// pixels, so TMA loads them unchanged, 64-byte swizzled (atoms of 8 pixels x 64 bytes; an operand may
+// start at any pixel of a box). All nine taps of 32 x 32 channels are one MMA of 128 x 96:
+//   M  rows are the box of one 32-channel group of X, {32 channels, 34 pixels, 4 image rows}, at
+//      pixel offsets 0, 1 and 2 (the taps dx): atoms one pixel apart. The fourth is not used;
 //   N  columns are the dP rows r - 1, r, r + 1 of one 32-channel group against X's row r (the taps
 //      dy = 1, 0, -1): consecutive rows of one box with a halo row on each side.
-// So an X element is loaded three times (once per dx) instead of nine, a dP element 1.5 times, and no
-// MMA is issued per tap. TMA's zero fill is the padding, and the channels past the tensors' ends. A
-// CTA takes up to kWgCombos pairs of M block and dP group (their accumulators fill the 512 TMEM
-// columns) and a run of tiles; warp 0 issues the loads into a ring of stages, warp 1 the MMAs, and
-// all four warps add the accumulators to dW: a warp's 32 lanes hold 32 consecutive input
-// channels, and through shared memory each lane gets four of them for one 16-byte addition (a
-// quarter of the additions at L2: 224 x 96 took 43.5 us with one value per addition, now 39; a dW that
-// is not 16-byte aligned keeps the single ones). Every wait is bounded.
-// What bounds it: L2 reads of the boxes, the tensor core at three quarters of its rows. One tap of one
-// 64-channel atom per MMA, every operand read once per tap (or dP once per step for up to 32
-// input channels), took 119 us for 32 x 32 channels on 8 x 256 x 256 pixels (now 31), 261 for 96 x 32
-// (90), 75 for 64 x 64 on 8 x 128 x 128 (29), 72 for 224 x 96 on 8 x 64 x 64 (39).
+// So an X element is loaded once and a dP element 1.5 times. TMA's zero fill is the
+// padding, and the channels past the tensors' ends. A CTA takes up to kWgCombos pairs of X and dP
+// groups (their accumulators fill the 512 TMEM columns) and a run of tiles; warp 0 issues the loads
+// into a ring of stages, a lane to a box, warps 1 and 2 the MMAs of every other pair, and the
+// warps 0-2 (dx) add the accumulators to dW: a warp's 32 lanes hold 32 consecutive input channels, and
+// through shared memory each lane gets four of them for one 16-byte addition (a quarter of the
+// additions at L2: 224 x 96 took 43.5 us with one value per addition, 39 with these; a dW that is not
+// 16-byte aligned keeps the single ones). Every wait is bounded.
+// What bounds it: the operand reads of shared memory (56 cycles an MMA) and the TMA unit (1.6 cycles a
+// box row of 64 bytes).
+// Before and after, on 8 x 256 x 256 pixels: 32 x 32 channels 119 us with one tap of one 64-channel atom
+// per MMA, every operand read once per tap; 31 with four X boxes, each at its shift, as an M block; now
+// 21. 96 x 32: 261, 90, 37. On 8 x 128 x 128: 64 x 64 75, 29, 22; on 8 x 64 x 64: 224 x 96 72, 39, 31.
+// Of those now the additions to dW at L2 are 2 to 12 us. Tiles of 8 rows: 19, 40, 25, 25.
 
 constexpr int kWtThreads = 128;
-constexpr int kWgPix = 32;                       // pixels of a tile row
-constexpr int kWgRows = 4;                       // X rows of a tile
-constexpr int kWgRow = kWgPix * 64;              // one box row: 32 pixels x 32 channels
-constexpr int kWgXBox = kWgRows * kWgRow;        // 8 KB
-constexpr int kWgDBox = (kWgRows + 2) * kWgRow;  // 12 KB
+constexpr int kWgPix = 32;            // pixels of a tile row
+constexpr int kWgXPix = kWgPix + 2;   // of X
+constexpr int kWgRows = 4;            // X rows of a tile
+constexpr int kWgXBox = kWgXPix * kWgRows * 64;        // 8.5 KB
+constexpr int kWgDBox = kWgPix * (kWgRows + 2) * 64;   // 12 KB
 constexpr int kWgCombos = 5;
-constexpr int kWgSmem = 200 * 1024;              // stages
-constexpr int kWgMaxStages = 4;
-constexpr int kWgExtra = 1024 + 256 + 4 * 2048;  // alignment, barriers, the epilogue's exchange
+constexpr int kWgSmem = 200 * 1024;   // stages
+constexpr int kWgMaxStages = 6;
+constexpr int kWgExtra = 1024 + 256 + 4 * 2048;   // alignment, barriers, the epilogue's exchange
 
-// Descriptor of an MN-major, 64-byte-swizzled operand: the leading byte offset is the stride between
-// 32-channel atoms along M (or N), the stride byte offset the one between 8-pixel groups along K.
-__device__ __forceinline__ uint64_t wg_desc(uint32_t saddr, uint32_t atom_stride) {
-    uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((atom_stride >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((512u >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1u << 46;   // version
-    d |= (uint64_t)4u << 61;   // SWIZZLE_64B
-    return d;
-}
-
-// How the pairs of M block and dP group are split over CTAs: mb x gb pairs per CTA.
+// How the pairs of X and dP group are split over CTAs: mb x gb pairs per CTA.
 struct WgPlan {
-    int na;            // 32-channel groups of X
-    int nblk, ng;      // M blocks, dP groups in all
+    int na, ng;        // X groups, dP groups in all
     int mb, gb;        // per CTA
     int stages;
     int xt, yt;        // tiles per image row, row tiles per image
@@ -79,7 +69,7 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
                                                            const __grid_constant__ CUtensorMap mx, WgradArgs a, WgPlan p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    const int stage_bytes = 4 * p.mb * kWgXBox + p.gb * kWgDBox;
+    const int stage_bytes = p.mb * kWgXBox + p.gb * kWgDBox;
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
     uint64_t* empty = full + kWgMaxStages;
     uint64_t* accb = empty + kWgMaxStages;
@@ -87,10 +77,9 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float* tb = reinterpret_cast<float*>(smem + p.stages * stage_bytes + 256) + warp * 512;   // 2 KB per warp
-    const int msplit = (p.nblk + p.mb - 1) / p.mb;
+    const int msplit = (p.na + p.mb - 1) / p.mb;
     const int blk0 = ((int)blockIdx.y % msplit) * p.mb, g0 = ((int)blockIdx.y / msplit) * p.gb;
-    const int nb = min(p.mb, p.nblk - blk0), ng = min(p.gb, p.ng - g0);
-    const int atoms = min(4 * nb, 3 * p.na - 4 * blk0);   // X boxes of this CTA's blocks
+    const int nb = min(p.mb, p.na - blk0), ng = min(p.gb, p.ng - g0);
     const int i0 = (int)((long long)p.items * blockIdx.x / gridDim.x);
     const int i1 = (int)((long long)p.items * (blockIdx.x + 1) / gridDim.x);
     const int combos = p.mb * p.gb;
@@ -99,9 +88,9 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
     if (tid == 0) {
         for (int st = 0; st < p.stages; ++st) {
             mbar_init(&full[st], 1);
-            mbar_init(&empty[st], 1);
+            mbar_init(&empty[st], 2);   // both issuers
         }
-        mbar_init(accb, 1);
+        mbar_init(accb, 2);
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -114,72 +103,102 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
+    // the producer's lane: its box's map, place in a stage, channels and offset from the tile's corner
+    const bool is_x = lane < nb, loads = lane < nb + ng;
+    const CUtensorMap* map = is_x ? &mx : &mdp;
+    const int place = is_x ? lane * kWgXBox : p.mb * kWgXBox + (lane - nb) * kWgDBox;
+    const int ch = 32 * (is_x ? blk0 + lane : g0 + lane - nb);
+    int tx = 0, ty = 0, img = 0;   // the next tile's
+    if (warp == 0) {
+        const int per_img = p.xt * p.yt, rem = i0 % per_img;
+        img = i0 / per_img;
+        ty = rem / p.xt;
+        tx = rem - ty * p.xt;
+    }
+    int s = 0;          // the next stage, and its uses so far
+    uint32_t use = 0;
+
     for (int seg = 0; seg < p.segs; ++seg) {
         const int k0 = (int)((long long)(i1 - i0) * seg / p.segs), k1 = (int)((long long)(i1 - i0) * (seg + 1) / p.segs);
-        if (warp == 0) {
-            if (lane == 0) {   // producer
-                const uint32_t bytes = (uint32_t)(atoms * kWgXBox + ng * kWgDBox);
-                for (int k = k0; k < k1 && !*abort_flag; ++k) {
-                    const int s = k % p.stages;
-                    const uint32_t use = (uint32_t)(k / p.stages);
-                    if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1u) & 1u, a.err)) {
-                        *abort_flag = 1;
-                        break;
+        if (warp == 0) {   // producer
+            const uint32_t bytes = (uint32_t)(nb * kWgXBox + ng * kWgDBox);
+            for (int k = k0; k < k1; ++k) {
+                bool ok = !*abort_flag;
+                if (use > 0) ok = mbar_wait_bounded(&empty[s], (use - 1u) & 1u, a.err) && ok;
+                if (!__all_sync(0xFFFFFFFFu, ok)) {
+                    *abort_flag = 1;
+                    break;
+                }
+                if (lane == 0) mbar_expect_tx(&full[s], bytes);
+                __syncwarp();
+                if (loads)
+                    tma_load_4d(smem + s * stage_bytes + place, map, ch, tx * kWgPix - (is_x ? 1 : 0),
+                                ty * kWgRows - (is_x ? 0 : 1), img, &full[s]);
+                if (++tx == p.xt) {
+                    tx = 0;
+                    if (++ty == p.yt) {
+                        ty = 0;
+                        ++img;
                     }
-                    const int it = i0 + k, per_img = p.xt * p.yt, img = it / per_img, rem = it - img * per_img;
-                    const int y0 = (rem / p.xt) * kWgRows, x0 = (rem % p.xt) * kWgPix;
-                    uint8_t* st = smem + s * stage_bytes;
-                    mbar_expect_tx(&full[s], bytes);
-                    for (int j = 0; j < atoms; ++j) {
-                        const int q = 4 * blk0 + j, dx = q / p.na, c = q - dx * p.na;
-                        tma_load_4d(st + j * kWgXBox, &mx, 32 * c, x0 + dx - 1, y0, img, &full[s]);
-                    }
-                    for (int g = 0; g < ng; ++g)
-                        tma_load_4d(st + 4 * p.mb * kWgXBox + g * kWgDBox, &mdp, 32 * (g0 + g), x0, y0 - 1, img, &full[s]);
+                }
+                if (++s == p.stages) {
+                    s = 0;
+                    ++use;
                 }
             }
-        } else if (warp == 1) {
-            if (lane == 0) {   // MMA issuer
-                const uint32_t idesc = umma_idesc_bf16(128u, 96u) | (1u << 15) | (1u << 16);   // MN-major A, B
-                bool ok = true;
-                for (int k = k0; k < k1 && ok; ++k) {
-                    const int s = k % p.stages;
-                    if (!mbar_wait_bounded(&full[s], (uint32_t)(k / p.stages) & 1u, a.err)) {
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t sx = smem_u32(smem + s * stage_bytes), sd = sx + (uint32_t)(4 * p.mb * kWgXBox);
-                    for (int m = 0; m < nb; ++m)
-                        for (int g = 0; g < ng; ++g) {
-                            const uint32_t d = tmem + (uint32_t)((m * p.gb + g) * 96);
-                            const uint64_t da = wg_desc(sx + (uint32_t)(4 * m * kWgXBox), (uint32_t)kWgXBox);
-                            const uint64_t db = wg_desc(sd + (uint32_t)(g * kWgDBox), (uint32_t)kWgRow);
+        } else if (warp < 3) {   // MMA issuers
+            constexpr uint32_t kHi = (512u >> 4) | (1u << 14) | (4u << 29);   // 8-pixel groups 512 bytes apart, SWIZZLE_64B
+            const bool leader = elect_one();
+            const uint32_t idesc = umma_idesc_bf16(128u, 96u) | (1u << 15) | (1u << 16);   // MN-major A, B
+            const uint32_t base = smem_u32(smem) >> 4;
+            bool ok = true;
+            for (int k = k0; k < k1; ++k) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&full[s], use & 1u, a.err));
+                if (!ok) {
+                    *abort_flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                if (leader) {
+                    // atoms along M: one pixel apart; along N: one dP row apart
+                    const uint32_t st = base + (uint32_t)(s * (stage_bytes >> 4));
+                    const uint32_t sx = st | ((64u >> 4) << 16), sd = (st + (uint32_t)(p.mb * (kWgXBox >> 4))) |
+                                                                      ((uint32_t)(kWgPix * 64 / 16) << 16);
+                    for (int m = 0, c = 0; m < nb; ++m)
+                        for (int g = 0; g < ng; ++g, ++c) {
+                            if ((c & 1) != warp - 1) continue;
+                            const uint32_t d = tmem + (uint32_t)(c * 96);
+                            const uint32_t al = sx + (uint32_t)(m * (kWgXBox >> 4)), bl = sd + (uint32_t)(g * (kWgDBox >> 4));
 #pragma unroll
-                            for (int r = 0; r < kWgRows * 2; ++r)   // 16 pixels (two 8-pixel groups) per MMA
-                                umma_bf16(d, da + (uint64_t)(r * 64), db + (uint64_t)(r * 64), idesc,
-                                          k != k0 || r != 0 ? 1u : 0u);
+                            for (int r = 0; r < 2 * kWgRows; ++r)   // 16 pixels (two 8-pixel groups) per MMA
+                                umma_bf16_lo(d, al + (uint32_t)((r >> 1) * (kWgXPix * 4) + (r & 1) * 64), kHi,
+                                             bl + (uint32_t)(r * 64), kHi, idesc, k != k0 || r != 0 ? 1u : 0u);
                         }
                     umma_commit(&empty[s]);
                 }
+                __syncwarp();
+                if (++s == p.stages) {
+                    s = 0;
+                    ++use;
+                }
             }
-            if (lane == 0) umma_commit(accb);
+            if (leader) umma_commit(accb);
+            __syncwarp();
         }
         __syncwarp();
         const bool summed = mbar_wait_bounded(accb, (uint32_t)seg & 1u, a.err);
         if (!summed) *abort_flag = 1;
-        const bool ready = summed && k1 > k0 && !*abort_flag;
-        __syncwarp();
+        const bool ready = __all_sync(0xFFFFFFFFu, summed && k1 > k0 && !*abort_flag) != 0;
         tc_fence_after();
-        // lane `lane` of warp w: input channel 32 c + lane of box 4 (blk0 + m) + w
+        // lane `lane` of warp dx: input channel 32 (blk0 + m) + lane
+        const int dx = warp;
         for (int part = 0; part < nb * ng * 6; ++part) {
-            const int m = part / (ng * 6), g = (part / 6) % ng, n0 = (part % 6) * 16;
-            const int q = 4 * (blk0 + m) + warp, dx = q / p.na, ci = 32 * (q - dx * p.na) + lane;
+            const int c = part / 6, n0 = (part - 6 * c) * 16, m = c / ng, g = c - m * ng;
+            const int ci = 32 * (blk0 + m) + lane;
             uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((m * p.gb + g) * 96 + n0), v);
+            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 96 + n0), v);
             tmem_ld_wait();
-            if (!ready || q >= 3 * p.na) continue;   // the same for the whole warp
+            if (!ready || dx > 2) continue;   // the same for the whole warp
             const int dy = 2 - n0 / 32;   // tap row: dP's row r - 1 is tap dy = +1
             const int co = 32 * (g0 + g) + (n0 & 31);
             float* d = a.dw + ((size_t)co * 9 + 3 * dy + dx) * a.cin + (ci - lane);
@@ -206,6 +225,12 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
         if (__syncthreads_or(*abort_flag)) break;   // the next sums start in the accumulators read here
         tc_fence_after();
     }
+    if (warp == 0)   // no load may be in flight when the CTA ends, whoever gave up
+        for (int i = 0; i < p.stages; ++i) {
+            const uint32_t uses = use + (i < s ? 1u : 0u);
+            if (uses > 0) mbar_wait_bounded(&full[i], (uses - 1u) & 1u, a.err);
+        }
+    __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, ncols);
 }
 
@@ -315,18 +340,18 @@ cudaError_t gkrt_encode_tmap_bf16(CUtensorMap* map, const void* base, uint32_t r
 
 // The split that loads least: each CTA of a pixel run loads 4 mb boxes of X and gb of dP (1.5 times
 // as tall), at least two stages in shared memory.
+// The split with the fewest cycles a tile, over all groups of pairs: MMAs, or box rows if those are more.
 static WgPlan wgrad_plan(const WgradArgs& a) {
     WgPlan p{};
     p.na = (a.cin + 31) / 32;
-    p.nblk = (3 * p.na + 3) / 4;
     p.ng = (a.cout + 31) / 32;
     double best = 1e30;
-    for (int mb = 1; mb <= std::min(p.nblk, kWgCombos); ++mb)
+    for (int mb = 1; mb <= std::min(p.na, kWgCombos); ++mb)
         for (int gb = 1; gb <= std::min(p.ng, kWgCombos / mb); ++gb) {
-            const int bytes = 4 * mb * kWgXBox + gb * kWgDBox;
+            const int bytes = mb * kWgXBox + gb * kWgDBox;
             if (2 * bytes > kWgSmem) continue;
-            const int groups = ((p.nblk + mb - 1) / mb) * ((p.ng + gb - 1) / gb);
-            const double cost = groups * (double)bytes;
+            const int groups = ((p.na + mb - 1) / mb) * ((p.ng + gb - 1) / gb);
+            const double cost = groups * (150.0 + std::max(mb * gb * kWgRows * 2 * 56.0, bytes / 64 * 1.6));
             if (cost < best) {
                 best = cost;
                 p.mb = mb;
@@ -359,8 +384,9 @@ cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
         if (e != cudaSuccess) return e;
     }
     const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B;
+    WgPlan p = wgrad_plan(a);
     const uint32_t dbox[4] = {32u, (uint32_t)kWgPix, (uint32_t)(kWgRows + 2), 1u};
-    const uint32_t xbox[4] = {32u, (uint32_t)kWgPix, (uint32_t)kWgRows, 1u};
+    const uint32_t xbox[4] = {32u, (uint32_t)kWgXPix, (uint32_t)kWgRows, 1u};
     CUtensorMap mdp, mx;
     const uint64_t dd[4] = {(uint64_t)a.cout, W, H, B};
     const uint64_t ds[3] = {(uint64_t)a.dp_c * 2, W * a.dp_c * 2, H * W * a.dp_c * 2};
@@ -369,12 +395,11 @@ cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
     const uint64_t xd[4] = {(uint64_t)xv, W, H, B};   // channels past xv: TMA's zero fill
     const uint64_t xs[3] = {(uint64_t)a.x_c * 2, W * a.x_c * 2, H * W * a.x_c * 2};
     if ((e = gkrt_encode_tmap_bf16(&mx, a.x + a.x_off, 4, xd, xs, xbox)) != cudaSuccess) return e;
-    WgPlan p = wgrad_plan(a);
-    const int stage_bytes = 4 * p.mb * kWgXBox + p.gb * kWgDBox;
-    const int groups = ((p.nblk + p.mb - 1) / p.mb) * ((p.ng + p.gb - 1) / p.gb);
+    const int stage_bytes = p.mb * kWgXBox + p.gb * kWgDBox;
+    const int groups = ((p.na + p.mb - 1) / p.mb) * ((p.ng + p.gb - 1) / p.gb);
     // one CTA per SM (its stages fill the shared memory), at least two tiles each. An FP32 sum covers at
-    // most a 34th of the pixels: with 30 CTAs, 224 x 96 on 8 x 64 x 64 was off by 1.3e-6 of the largest
-    // value in one sum each (27 us) and is by 6.2e-7 in two (39 us).
+    // most a 34th of the pixels: with 21 CTAs, 224 x 96 on 8 x 64 x 64 was off by 1.6e-6 of dW's norm in
+    // one sum each (25 us) and is by 7.4e-7 in two (31 us).
     const int grid = std::max(1, std::min((p.items + 1) / 2, sms_dev[dev] / groups));
     p.segs = (34 + grid - 1) / grid;
     if (p.items < 34 * 4) p.segs = 1;
