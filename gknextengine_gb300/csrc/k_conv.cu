@@ -267,6 +267,8 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3(const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
@@ -460,6 +462,8 @@ __global__ void __launch_bounds__(kConvThreads) k_conv3x3_halo(const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
@@ -741,11 +745,14 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_conv_rows(const __grid_const
         tmem_alloc(tslot, 512u);
         tmem_relinquish();
     }
-    // -0 adds nothing, not even to a -0
-    for (int i = tid; i < nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + i) : -0.0f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    // -0 adds nothing, not even to a -0
+    for (int i = tid; i < nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + i) : -0.0f;
+    __syncthreads();
     const uint32_t tmem = *tslot;
     const int per_img = p.nxs * p.nyb;
 
@@ -1133,10 +1140,14 @@ __global__ void __launch_bounds__(kBigThreads, 1) k_conv_tiles(const __grid_cons
         tmem_alloc(tslot, 512u);
         tmem_relinquish();
     }
-    for (int i = tid; i < nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + i) : -0.0f;   // -0 adds nothing
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
+    // -0 adds nothing, not even to a -0
+    for (int i = tid; i < nco; i += blockDim.x) bsm[i] = a.bias ? __ldg(a.bias + i) : -0.0f;
+    __syncthreads();
     const uint32_t tmem = *tslot;
     const int per_img = p.nx * p.ny;
 
@@ -1462,9 +1473,8 @@ static cudaError_t launch_rows(const void* xbase, int xv, uint64_t xc, const voi
         attr[dev] = true;
     }
     const size_t smem = row_smem(a, p, row_stage_bytes(rb, R));
-    kernel<<<std::min(p.items, sms), 96 + p.groups * kEpiThreads, std::max(smem, (size_t)kRowSmemMin), st>>>(mx, mw, mo, mu, a,
-                                                                                                          p);
-    return cudaGetLastError();
+    return launch_after(kernel, dim3((unsigned)std::min(p.items, sms)), 96 + p.groups * kEpiThreads, std::max(smem, (size_t)kRowSmemMin), st,
+                        mx, mw, mo, mu, a, p);
 }
 
 static size_t big_smem(const ConvArgs& a, const BigPlan& p) {
@@ -1525,9 +1535,8 @@ static cudaError_t launch_big(const void* xbase, int xv, uint64_t xc, const void
         attr[dev] = true;
     }
     const size_t smem = std::max(big_smem(a, p), (size_t)kRowSmemMin);
-    kernels[kg == 32][a.pool_out != nullptr]<<<std::min(p.items, sms), 96 + p.groups * kEpiThreads, smem, st>>>(mx, mw, mo,
-                                                                                                      mu, a, p);
-    return cudaGetLastError();
+    return launch_after(kernels[kg == 32][a.pool_out != nullptr], dim3((unsigned)std::min(p.items, sms)),
+                        96 + p.groups * kEpiThreads, smem, st, mx, mw, mo, mu, a, p);
 }
 
 // Outputs of up to 128 channels use the row-box stages (three vertical taps per box); the
@@ -1634,12 +1643,8 @@ cudaError_t gkrt_launch_conv3x3(const void* x, const void* w, const ConvArgs& ar
         const int tiles_x = (args.W + kHaloX - 1) / kHaloX, tiles_y = (args.H + kHaloY - 1) / kHaloY;
         const int ntiles = tiles_x * tiles_y * args.B;
         const int grid = std::min(ntiles, sms * per_sm);
-        if (rb == 64)
-            k_conv3x3_halo<64><<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles);
-        else if (rb == 32)
-            k_conv3x3_halo<32><<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles);
-        else
-            k_conv3x3_halo<16><<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles);
+        const auto kernel = rb == 64 ? k_conv3x3_halo<64> : rb == 32 ? k_conv3x3_halo<32> : k_conv3x3_halo<16>;
+        kernel<<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles);
         return cudaGetLastError();
     }
     const uint64_t xd[4] = {(uint64_t)xv, (uint64_t)args.W, (uint64_t)args.H, (uint64_t)args.B};
@@ -1682,10 +1687,7 @@ cudaError_t gkrt_launch_conv3x3(const void* x, const void* w, const ConvArgs& ar
     const int tiles_x = (args.W + kTileX - 1) / kTileX, tiles_y = (args.H + kTileY - 1) / kTileY;
     const int ntiles = tiles_x * tiles_y * args.B;
     const int grid = std::min(ntiles, sms * per_sm);
-    if (rows)
-        k_conv3x3<true><<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles, conv_stages(args.cout));
-    else
-        k_conv3x3<false><<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles,
-                                                           conv_stages(args.cout));
+    const auto kernel = rows ? k_conv3x3<true> : k_conv3x3<false>;
+    kernel<<<grid, kConvThreads, smem, st>>>(mx, mw, args, tiles_x, tiles_y, ntiles, conv_stages(args.cout));
     return cudaGetLastError();
 }

@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dep_launch();
+    grid_dep_wait();
     const uint32_t tmem = *tslot;
 
     // the producer's lane: its box's map, place in a stage, channels and offset from the tile's corner
@@ -271,6 +273,8 @@ enum GradMode { kGradPlain = 0, kGradPool = 1, kGradUpsample = 2 };
 template <int kMode>
 __global__ void __launch_bounds__(256) k_layer_grad(LayerGradArgs a, int run) {
     __shared__ float part[256 * 8];
+    grid_dep_launch();
+    grid_dep_wait();
     const int G = a.C / 8, per = 256 / G;
     const int g = threadIdx.x % G, k = threadIdx.x / G;
     float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -403,9 +407,8 @@ cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
     const int grid = std::max(1, std::min((p.items + 1) / 2, sms_dev[dev] / groups));
     p.segs = (34 + grid - 1) / grid;
     if (p.items < 34 * 4) p.segs = 1;
-    k_conv_wgrad<<<dim3((unsigned)grid, (unsigned)groups), kWtThreads, (size_t)p.stages * stage_bytes + kWgExtra, st>>>(
-        mdp, mx, a, p);
-    return cudaGetLastError();
+    return launch_after(k_conv_wgrad, dim3((unsigned)grid, (unsigned)groups), kWtThreads,
+                        (size_t)p.stages * stage_bytes + kWgExtra, st, mdp, mx, a, p);
 }
 
 cudaError_t gkrt_launch_layer_grad(const LayerGradArgs& a, int mode, cudaStream_t st) {
@@ -417,8 +420,9 @@ cudaError_t gkrt_launch_layer_grad(const LayerGradArgs& a, int mode, cudaStream_
     const int per = 256 / (a.C / 8);
     const int run = (int)std::max<long long>(4 * per, (npix + 607) / 608);
     const unsigned blocks = (unsigned)((npix + run - 1) / run);
-    if (mode == kGradPool) k_layer_grad<kGradPool><<<blocks, 256, 0, st>>>(a, run);
-    else if (mode == kGradUpsample) k_layer_grad<kGradUpsample><<<blocks, 256, 0, st>>>(a, run);
-    else k_layer_grad<kGradPlain><<<blocks, 256, 0, st>>>(a, run);
+    const auto kernel = mode == kGradPool       ? k_layer_grad<kGradPool>
+                        : mode == kGradUpsample ? k_layer_grad<kGradUpsample>
+                                                : k_layer_grad<kGradPlain>;
+    kernel<<<blocks, 256, 0, st>>>(a, run);
     return cudaGetLastError();
 }

@@ -48,6 +48,8 @@ constexpr int kXc = 16;
 // memory (pixel-per-thread loads of 40-byte records touch every line ten times).
 __global__ void __launch_bounds__(256) k_pack_input(const float* in, long long npix, __nv_bfloat16* x0) {
     __shared__ __align__(16) float rec[256 * 10];
+    grid_dep_launch();
+    grid_dep_wait();
     const long long p0 = blockIdx.x * 256LL;
     const int n = (int)(npix - p0 < 256 ? npix - p0 : 256);
     const float* src = in + p0 * 10;
@@ -88,6 +90,8 @@ __global__ void __launch_bounds__(256) k_pack_frame(const float4* sd, const floa
                                                     const float4* nrm, const float* depth, int W, int H, int P,
                                                     __nv_bfloat16* x0) {
     __shared__ __align__(16) uint4 packed[256 * (kXc / 8)];
+    grid_dep_launch();
+    grid_dep_wait();
     const long long i0 = blockIdx.x * 256LL, i = i0 + threadIdx.x;
     const long long npix = (long long)W * H;
     const int n = (int)(npix - i0 < 256 ? npix - i0 : 256);
@@ -130,6 +134,8 @@ __device__ __forceinline__ void store_grad(__nv_bfloat16* gy, long long p, float
 __global__ void __launch_bounds__(256) k_loss(const float4* y, const float* target, long long npix, float gscale,
                                               __nv_bfloat16* gy, double* loss) {
     __shared__ double part[8];
+    grid_dep_launch();
+    grid_dep_wait();
     const long long p = blockIdx.x * 256LL + threadIdx.x;
     double l = 0.0;
     if (p < npix) {
@@ -156,11 +162,15 @@ __global__ void __launch_bounds__(256) k_loss(const float4* y, const float* targ
 
 // caller-supplied gradient of the raw output (f32, 4 channels) to the bf16 32-channel layout
 __global__ void __launch_bounds__(256) k_grad_in(const float* d, long long npix, __nv_bfloat16* gy) {
+    grid_dep_launch();
+    grid_dep_wait();
     const long long p = blockIdx.x * 256LL + threadIdx.x;
     if (p < npix) store_grad(gy, p, d[p * 4], d[p * 4 + 1], d[p * 4 + 2]);
 }
 
 __global__ void k_out_linear(const float* y, long long npix, float* out) {
+    grid_dep_launch();
+    grid_dep_wait();
     const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (p >= npix) return;
     for (int c = 0; c < 3; ++c) out[p * 4 + c] = fmaxf(expm1f(fminf(y[p * 4 + c], kUnetMaxLog)), 0.0f);
@@ -182,6 +192,8 @@ struct AdamStep {
 template <bool kStep>
 __global__ void __launch_bounds__(256) k_params(ParamMap map, float* p, const float* g, float* m, float* v, AdamStep s,
                                                 __nv_bfloat16* wb, __nv_bfloat16* wf) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= map.n) return;
     float w = p[i];
@@ -217,6 +229,8 @@ __global__ void __launch_bounds__(256) k_params(ParamMap map, float* p, const fl
 // summed in FP32 and rounded to bf16; we0b[co][tap][ci] = w[co][tap][64 + ci].
 __device__ __forceinline__ int floor_half(int v) { return (v + 2) / 2 - 1; }   // v in -1..2
 __global__ void k_weights_subpixel(const float* w, __nv_bfloat16* wup, __nv_bfloat16* we0b) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 128 * 9 * 64) {
         const int ci = i % 64, lt = (i / 64) % 9, n = i / (64 * 9);
@@ -312,10 +326,10 @@ struct Unet {
 
     // the weights' bf16 copies from the FP32 masters, after an Adam step if given
     cudaError_t update_params(const AdamStep* s, cudaStream_t st) {
-        if (s) k_params<true><<<nb((long long)nparams), 256, 0, st>>>(param_map(), p, g, m, v, *s, wb, wf);
-        else k_params<false><<<nb((long long)nparams), 256, 0, st>>>(param_map(), p, g, m, v, AdamStep{}, wb, wf);
-        k_weights_subpixel<<<nb(128 * 9 * 64), 256, 0, st>>>(p + woff[D0A], wup, we0b);
-        return cudaGetLastError();
+        const cudaError_t e = launch_after(s ? k_params<true> : k_params<false>, nb((long long)nparams), 256, 0, st,
+                                           param_map(), p, g, m, v, s ? *s : AdamStep{}, wb, wf);
+        if (e != cudaSuccess) return e;
+        return launch_after(k_weights_subpixel, nb(128 * 9 * 64), 256, 0, st, p + woff[D0A], wup, we0b);
     }
 
     cudaError_t ensure_size(int b, int h, int w) {
@@ -562,9 +576,9 @@ static cudaError_t forward_dev(Unet* u, const float* input, int b, int h, int w,
     cudaError_t e = u->ensure_size(b, h, w);
     if (e != cudaSuccess) return e;
     const long long npix = (long long)b * h * w;
-    if (input) k_pack_input<<<nb(npix), 256, 0, st>>>(input, npix, u->x0);
+    if (input && (e = launch_after(k_pack_input, nb(npix), 256, 0, st, input, npix, u->x0)) != cudaSuccess) return e;
     if ((e = u->forward(st, train)) != cudaSuccess) return e;
-    if (out_linear) k_out_linear<<<nb(npix), 256, 0, st>>>(u->y, npix, out_linear);
+    if (out_linear && (e = launch_after(k_out_linear, nb(npix), 256, 0, st, u->y, npix, out_linear)) != cudaSuccess) return e;
     if (out_raw) e = cudaMemcpyAsync(out_raw, u->y, npix * 16, cudaMemcpyDeviceToDevice, st);
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
@@ -580,7 +594,7 @@ cudaError_t gkrt_unet_backward_dev(Unet* u, const float* d_raw, cudaStream_t st)
     const long long npix = (long long)u->B * u->H * u->W;
     cudaError_t e;
     if (!u->train_acts && (e = u->forward(st, true)) != cudaSuccess) return e;
-    k_grad_in<<<nb(npix), 256, 0, st>>>(d_raw, npix, u->gy);
+    if ((e = launch_after(k_grad_in, nb(npix), 256, 0, st, d_raw, npix, u->gy)) != cudaSuccess) return e;
     return u->backward(st);
 }
 
@@ -592,7 +606,9 @@ cudaError_t gkrt_unet_train_step_dev(Unet* u, const float* input, const float* t
     if ((e = cudaMemsetAsync(u->d_loss, 0, sizeof(double), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(u->g, 0, u->nparams * 4, st)) != cudaSuccess) return e;
     // gradients of the per-image sum of squared log errors (Adam does not see the scale)
-    k_loss<<<nb(npix), 256, 0, st>>>(reinterpret_cast<const float4*>(u->y), target, npix, 1.0f, u->gy, u->d_loss);
+    if ((e = launch_after(k_loss, nb(npix), 256, 0, st, reinterpret_cast<const float4*>(u->y), target, npix, 1.0f, u->gy,
+                          u->d_loss)) != cudaSuccess)
+        return e;
     if ((e = u->backward(st)) != cudaSuccess) return e;
     u->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
@@ -615,7 +631,9 @@ cudaError_t gkrt_unet_denoise_frame(Unet* u, const float4* sd, const float4* ss,
                                     const float* depth, int W, int H, int P, float* y_out_raw, cudaStream_t st) {
     cudaError_t e = u->ensure_size(1, H, W);
     if (e != cudaSuccess) return e;
-    k_pack_frame<<<nb((long long)W * H), 256, 0, st>>>(sd, ss, alb, nrm, depth, W, H, P, u->x0);
+    if ((e = launch_after(k_pack_frame, nb((long long)W * H), 256, 0, st, sd, ss, alb, nrm, depth, W, H, P, u->x0)) !=
+        cudaSuccess)
+        return e;
     if ((e = u->forward(st, false)) != cudaSuccess) return e;
     (void)y_out_raw;
     return cudaGetLastError();

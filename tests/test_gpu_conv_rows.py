@@ -88,3 +88,42 @@ def test_tiles_match_torch(B, H, W, cin, cout):
     base.test_conv_matches_torch(B, H, W, cin, cout, True)
     if H > 1:
         base.test_conv_fused_pool_and_upsample(B, H, W, cin, cout)
+
+
+def test_chain_in_a_graph():
+    """Kernels that start while their predecessors end, captured: a chain on one stream, replayed on new
+    inputs, equals the same calls outside."""
+    torch = _torch()
+    L = native.load()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn((4, 100, 256, 64), device="cuda", generator=g).bfloat16()
+    w = (torch.randn((64, 3, 3, 64), device="cuda", generator=g) / 24.0).bfloat16()
+    w2 = (torch.randn((96, 3, 3, 64), device="cuda", generator=g) / 24.0).bfloat16()
+    y, z, dw = torch.zeros_like(x), torch.zeros((4, 100, 256, 96), device="cuda").bfloat16(), torch.zeros((64, 3, 3, 64),
+                                                                                                          device="cuda")
+
+    def chain(stream):
+        p = lambda t: C.c_void_p(t.data_ptr())
+        st = C.c_void_p(stream.cuda_stream)
+        for src, dst, k in ((x, y, w), (y, z, w2)):
+            assert L.gkrt_conv3x3_bf16(p(src), 4, 100, 256, 64, p(k), None, dst.shape[3], p(dst), dst.shape[3], 0, 0, 1,
+                                       st) == abi.GKRT_OK
+        assert L.gkrt_conv3x3_wgrad_bf16(p(y), p(x), 4, 100, 256, 64, 64, p(dw), st) == abi.GKRT_OK
+
+    chain(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(torch.cuda.current_stream())
+    for _ in range(3):
+        x.copy_(torch.randn(x.shape, device="cuda", generator=g))
+        dw.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        got, got_dw = z.clone(), dw.clone()
+        dw.zero_()
+        chain(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        assert torch.equal(got, z)
+        # FP32 sums over 102,400 pixels, added in any order
+        torch.testing.assert_close(got_dw, dw, rtol=1e-3, atol=1e-3 * float(dw.abs().max()))
