@@ -189,11 +189,12 @@ GK_D f3 hemisphere_cos(Rng& s) {
     float r = sqrt_(u.y);
     return F3(r * cs, r * sn, sqrt_(1.0f - u.y));
 }
+GK_D float cone_z(float cos_theta, float u) { return fmaf_(u, cos_theta - 1.0f, 1.0f); }
 GK_D f3 cone(Rng& s, float cos_theta) {
     f2 u = rnd2(s);
     float sn, cs;
     sincos2pi(u.x, sn, cs);
-    float ct = fmaf_(u.y, cos_theta - 1.0f, 1.0f);
+    float ct = cone_z(cos_theta, u.y);
     float r = sqrt_(fmaf_(-ct, ct, 1.0f));
     return F3(r * cs, r * sn, ct);
 }
@@ -215,8 +216,7 @@ GK_D f2 unit_disk(Rng& s) {
     return r;
 }
 // Bounded VNDF sampling of GGX (Eto and Tokuyoshi 2023), Const_Func.slang:310-328
-GK_D f3 ggx_vndf(float alpha, f3 wi_, f2 uv) {
-    f3 wi = normalize3(F3(wi_.x * alpha, wi_.y * alpha, wi_.z));
+GK_D float ggx_vndf_z(float alpha, f3 wi_, f3 wi, float u) {   // wi: wi_ stretched by alpha, normalized
     float b = wi.z;
     if (wi_.z > 0.0f) {
         float a = sat(alpha);
@@ -224,7 +224,11 @@ GK_D f3 ggx_vndf(float alpha, f3 wi_, f2 uv) {
         float aw = div_(a * wi_.z, 1.0f + lxy);
         b = b * div_(fmaf_(-a, a, 1.0f), fmaf_(aw, aw, 1.0f));
     }
-    float z = fmaf_(1.0f - uv.y, 1.0f + b, -b);
+    return fmaf_(1.0f - u, 1.0f + b, -b);
+}
+GK_D f3 ggx_vndf(float alpha, f3 wi_, f2 uv) {
+    f3 wi = normalize3(F3(wi_.x * alpha, wi_.y * alpha, wi_.z));
+    float z = ggx_vndf_z(alpha, wi_, wi, uv.y);
     float sn, cs;
     sincos2pi(uv.x, sn, cs);
     float r = sqrt_(sat(fmaf_(-z, z, 1.0f)));

@@ -151,10 +151,12 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
     // finished rays that the shading phase takes mixed (94 hold a warp's worth of one of the three
     // kinds); a pool of one warp's worth is traced to its end
     const int enough = np >= 64u ? min(94, (int)np - 32) : (int)np + 1;
+    bool alone = false;             // node tests for fewer lanes than kNodeLanes, for want of other work
     for (;;) {
         unsigned mn = __ballot_sync(0xFFFFFFFFu, st == kStNode);
         // node tests
-        if (__popc(mn) >= kNodeLanes) {
+        if (__popc(mn) >= kNodeLanes || alone) {
+            alone = false;
             do {
                 if (st == kStNode) st = trav_node(T, S, stk, kPoolThreads, cn, cap);
                 mn = __ballot_sync(0xFFFFFFFFu, st == kStNode);
@@ -162,36 +164,9 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
         }
         const unsigned md = __ballot_sync(0xFFFFFFFFu, st == kStDone);
         const bool more = waiting < queue.n;
-        if ((more && __popc(md) >= kRefillLanes) || (md == 0xFFFFFFFFu)) {
-            // finished rays to their paths, the next rays of the queue to the free lanes
-            const bool fin = have && st == kStDone;
-            if (fin) {
-                __stcg(pool + slot + PF_HIT * np,
-                       make_float4(__uint_as_float(T.hit ? T.inst : 0xFFFFFFFFu), __uint_as_float(T.prim),
-                                   __uint_as_float(T.tri), 0.0f));
-                have = false;
-            }
-            done.add(fin, kind, slot);
-            const int k = waiting + __popc(md & ((1u << (threadIdx.x & 31u)) - 1u));
-            if (st == kStDone && k < queue.n) {
-                slot = queue.l[k];
-                const float4 o = __ldcg(pool + slot + PF_RAYO * np), d = __ldcg(pool + slot + PF_RAYD * np);
-                kind = __float_as_uint(d.w);
-                trav_init(T, S, F3(o.x, o.y, o.z), F3(d.x, d.y, d.z), o.w, kind == kRayAny ? kAny : kClosest);
-                wray[0] = o.x; wray[kPoolThreads] = o.y; wray[2 * kPoolThreads] = o.z;
-                wray[3 * kPoolThreads] = d.x; wray[4 * kPoolThreads] = d.y; wray[5 * kPoolThreads] = d.z;
-                st = T.done ? kStDone : kStNode;
-                have = true;
-            }
-            waiting = min(queue.n, waiting + __popc(md));
-            if (waiting >= queue.n) {
-                const unsigned live = __ballot_sync(0xFFFFFFFFu, have);
-                if (live == 0u) break;
-            }
-            continue;
-        }
-        if (!more) {
-            // the finished rays that found no refill, then back to the shading phase if it has work
+        const bool refill = more && (__popc(md) >= kRefillLanes || md == 0xFFFFFFFFu);
+        if (refill || !more) {
+            // finished rays to their paths
             const bool fin = have && st == kStDone;
             if (__any_sync(0xFFFFFFFFu, fin)) {
                 if (fin) {
@@ -201,7 +176,23 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
                 }
                 done.add(fin, kind, slot);
             }
-            if (done.largest() >= 32 || done.total() >= enough) break;
+            if (refill) {   // the next rays of the queue to the free lanes
+                const int k = waiting + __popc(md & ((1u << (threadIdx.x & 31u)) - 1u));
+                if (st == kStDone && k < queue.n) {
+                    slot = queue.l[k];
+                    const float4 o = __ldcg(pool + slot + PF_RAYO * np), d = __ldcg(pool + slot + PF_RAYD * np);
+                    kind = __float_as_uint(d.w);
+                    trav_init(T, S, F3(o.x, o.y, o.z), F3(d.x, d.y, d.z), o.w, kind == kRayAny ? kAny : kClosest);
+                    wray[0] = o.x; wray[kPoolThreads] = o.y; wray[2 * kPoolThreads] = o.z;
+                    wray[3 * kPoolThreads] = d.x; wray[4 * kPoolThreads] = d.y; wray[5 * kPoolThreads] = d.z;
+                    st = T.done ? kStDone : kStNode;
+                    have = true;
+                }
+                waiting = min(queue.n, waiting + __popc(md));
+                continue;
+            }
+            // no ray left, or back to the shading phase if it has work
+            if (md == 0xFFFFFFFFu || done.largest() >= 32 || done.total() >= enough) break;
         }
         const unsigned mx = __ballot_sync(0xFFFFFFFFu, st == kStTrans), ml = __ballot_sync(0xFFFFFFFFu, st == kStLeaf);
         if (__popc(mx) >= kTransLanes || (mx != 0u && mn == 0u && __popc(mx) >= __popc(ml))) {
@@ -216,8 +207,8 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
                 T.wd = F3(wray[3 * kPoolThreads], wray[4 * kPoolThreads], wray[5 * kPoolThreads]);
                 st = trav_tris(T, S, stk, kPoolThreads, cn);
             }
-        } else if (st == kStNode) {     // mn != 0 here: mx and ml below their thresholds
-            st = trav_node(T, S, stk, kPoolThreads, cn, cap);
+        } else {
+            alone = true;   // mn != 0 here: mx and ml below their thresholds
         }
     }
     queue.n = 0;

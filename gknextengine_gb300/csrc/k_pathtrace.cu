@@ -22,9 +22,9 @@ constexpr int kPtThreads = kPoolThreads;
 constexpr int kPtWarps = kPoolWarps;
 constexpr int kPtMaxBlocks = 8;    // resident blocks per SM, at most
 // Resident blocks per SM: the traversal phase fits 128 registers, the shading phase spills below.
-// Trace pass with 4 / 5 / 6 blocks (ms): 1080p bricks 2.97 / 3.11 / 3.25, Cornell 256 x 256
-// 0.146 / 0.159 / 0.175, 720p on the probe grid 1.25 / 1.18 / -, 4K city 53.9 / 54.3 / 58.9, textured
-// 1277 x 713 at 8 samples 8.0 / 9.5 / 11.0.
+// Trace pass with 3 / 4 / 5 blocks (ms): 1080p bricks 3.12 / 2.84 / 3.03, Cornell 256 x 256
+// 0.160 / 0.134 / 0.150, 720p on the probe grid 1.31 / 1.16 / 1.14, 4K city 52.3 / 48.7 / 48.4, textured
+// 1277 x 713 at 8 samples 6.8 / 6.6 / 7.7.
 constexpr int kPtBlocks = 4;
 constexpr float kCosCone = 0.999990482f;   // cos(0.25 deg), Shading.slang:897
 
@@ -130,7 +130,9 @@ __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
     const uint32_t stage = L.stage;
     bool emitted = false, need_begin = false, need_pre = false, pre_first = false;
     bool need_end = false, need_after_sun = false, need_finish = false;
+    bool need_probe = false, need_sun = false;
     float shadow = 0.0f;
+    f3 sunO;   // where the sun ray starts
 
     // 0. the vertex a closest-hit ray met
     HitVtx hv;
@@ -237,18 +239,16 @@ __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
             const uint32_t maxB = (loop >> 16) & 0x7FFFu;
             const bool pdiel = (loop >> 31) != 0u;
             if (fc.fast_gather && !pdiel) {
-                L.rc = L.rc * probe_term(c.sc, L.vs.P, L.vs.N);
-                need_end = true;
+                need_probe = true;
             } else {
                 L.b = 1;
                 if (L.b < maxB) need_pre = true;
                 else need_end = true;
             }
         } else if (fc.has_sun && rnd1(L.seed) < 0.5f) {
-            const f3 cd = align_normal(cone(L.seed, kCosCone), sunDir);
             L.stage = ST_SUN;
-            emit(T, c, L.vs.P, cd, true);
-            emitted = true;
+            sunO = L.vs.P;
+            need_sun = true;
         } else {
             need_after_sun = true;
         }
@@ -271,12 +271,15 @@ __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
         const bool pdiel = (loop >> 31) != 0u;
         const bool early = !pdiel && rnd1(L.seed) < 0.5f;
         if (L.b == maxB - 1u || early) {
-            L.rc = L.rc * probe_term(c.sc, L.vs.P, L.vs.N);
-            need_end = true;
+            need_probe = true;
         } else {
             ++L.b;
             need_pre = true;
         }
+    }
+    if (need_probe) {
+        L.rc = L.rc * probe_term(c.sc, L.vs.P, L.vs.N);
+        need_end = true;
     }
 
     // 5. end of a sample (Shading.slang:1159-1176), then the next sample or DirectIlluminate
@@ -288,10 +291,9 @@ __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
         if (++L.i < samples) {
             need_begin = true;
         } else if (fc.has_sun) {
-            const f3 cd = align_normal(cone(L.seed, kCosCone), sunDir);
             L.stage = ST_DIRECT;
-            emit(T, c, xyz(c.get(PF_PP)), cd, true);
-            emitted = true;
+            sunO = xyz(c.get(PF_PP));
+            need_sun = true;
         } else {
             shadow = 0.0f;
             need_finish = true;
@@ -345,40 +347,78 @@ __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
         pre_first = true;
     }
 
-    // 9. GetRayColor up to its trace (Shading.slang:1007-1039)
-    if (need_pre) {
-        const MatV mat = load_mat(c.sc, L.vs.mat);
-        const bool diel = mat.model == GKRT_MAT_DIELECTRIC;
-        const float startPosOffset = diel ? 0.0f : 1.0f;
-        const float dotValue = dot3(L.dir, L.vs.N);
-        const bool back = dotValue > 0.0f;
-        const f3 outward = back ? -L.vs.N : L.vs.N;
-        const float niOverNt = back ? mat.ri2 : div_(1.0f, mat.ri2);
-        const float cosine = dotValue > 0.0f ? mat.ri * dotValue : -dotValue;
-        const float reflectProb = schlick(cosine, mat.ri);
-        const bool chanceReflect = rnd1(L.seed) < reflectProb;
-        const bool chanceMetal = rnd1(L.seed) < mat.metal;
-        const bool chanceGGX = chanceReflect || chanceMetal;
-        f3 tdir;
-        if (chanceGGX) tdir = ggx_sample(L.seed, sqrt_(mat.fuzz), reflect3(L.dir, outward));
-        else tdir = align_normal(hemisphere_cos(L.seed), outward);
-        if (pre_first) { L.hitReflect = chanceGGX; L.hitMetal = chanceMetal; }
-        if (diel && !chanceReflect) tdir = refract3(L.dir, outward, niOverNt);
-        L.dir = tdir;
-        L.chanceReflect = chanceReflect;
-        L.back = back;
-        L.diel = diel;
-        L.neeLobe = kNee && !back && !diel && !chanceGGX;
-        NeeSample ns;
-        if (kNee && L.neeLobe && nee_sample(c.sc, L.seed, L.vs.P, L.vs.N, L.rc, ns)) {
-            f4 contrib = ns.contrib;
-            if (L.hitMetal) contrib = contrib * pv_albedo<kTex>(c);
-            c.put(PF_NEE, contrib);
-            L.stage = pre_first ? ST_NEE_FIRST : ST_NEE_BOUNCE;
-            emit(T, c, ns.o, ns.dir, true, ns.tmax);
+    // 9. GetRayColor up to its trace (Shading.slang:1007-1039), or a ray in the sun's cone: one sampled
+    // direction about one axis for either (GGX, cosine hemisphere, cone)
+    if (need_pre || need_sun) {
+        MatV mat;
+        bool diel = false, chanceReflect = false, chanceMetal = false, chanceGGX = false, back = false;
+        float startPosOffset = 0.0f, niOverNt = 0.0f;
+        f3 outward, axis = sunDir;
+        if (need_pre) {
+            mat = load_mat(c.sc, L.vs.mat);
+            diel = mat.model == GKRT_MAT_DIELECTRIC;
+            startPosOffset = diel ? 0.0f : 1.0f;
+            const float dotValue = dot3(L.dir, L.vs.N);
+            back = dotValue > 0.0f;
+            outward = back ? -L.vs.N : L.vs.N;
+            niOverNt = back ? mat.ri2 : div_(1.0f, mat.ri2);
+            const float cosine = dotValue > 0.0f ? mat.ri * dotValue : -dotValue;
+            const float reflectProb = schlick(cosine, mat.ri);
+            chanceReflect = rnd1(L.seed) < reflectProb;
+            chanceMetal = rnd1(L.seed) < mat.metal;
+            chanceGGX = chanceReflect || chanceMetal;
+            axis = chanceGGX ? reflect3(L.dir, outward) : outward;
+        }
+        f3 tb, bb;
+        onb(axis, tb, bb);
+        f3 wi, v;
+        float alpha = 0.0f, r, z;
+        if (chanceGGX) {
+            const float roughness = sqrt_(mat.fuzz);
+            alpha = roughness * roughness;
+            v = F3(dot3(tb, axis), dot3(bb, axis), dot3(axis, axis));
+            wi = normalize3(F3(v.x * alpha, v.y * alpha, v.z));
+        }
+        const f2 u = rnd2(L.seed);
+        float sn, cs;
+        sincos2pi(u.x, sn, cs);
+        if (chanceGGX) {
+            z = ggx_vndf_z(alpha, v, wi, u.y);
+            r = sqrt_(sat(fmaf_(-z, z, 1.0f)));
+        } else if (need_pre) {
+            r = sqrt_(u.y);
+            z = sqrt_(1.0f - u.y);
         } else {
-            L.stage = pre_first ? ST_FIRST : ST_BOUNCE;
-            emit(T, c, fma3(L.vs.N, 0.001f * startPosOffset, L.vs.P), tdir, false);
+            z = cone_z(kCosCone, u.y);
+            r = sqrt_(fmaf_(-z, z, 1.0f));
+        }
+        v = F3(r * cs, r * sn, z);
+        if (chanceGGX) {
+            const f3 m = wi + v;
+            v = normalize3(F3(m.x * alpha, m.y * alpha, m.z));
+        }
+        f3 tdir = to_world(v, tb, bb, axis);
+        if (need_sun) {
+            emit(T, c, sunO, tdir, true);
+        } else {
+            if (pre_first) { L.hitReflect = chanceGGX; L.hitMetal = chanceMetal; }
+            if (diel && !chanceReflect) tdir = refract3(L.dir, outward, niOverNt);
+            L.dir = tdir;
+            L.chanceReflect = chanceReflect;
+            L.back = back;
+            L.diel = diel;
+            L.neeLobe = kNee && !back && !diel && !chanceGGX;
+            NeeSample ns;
+            if (kNee && L.neeLobe && nee_sample(c.sc, L.seed, L.vs.P, L.vs.N, L.rc, ns)) {
+                f4 contrib = ns.contrib;
+                if (L.hitMetal) contrib = contrib * pv_albedo<kTex>(c);
+                c.put(PF_NEE, contrib);
+                L.stage = pre_first ? ST_NEE_FIRST : ST_NEE_BOUNCE;
+                emit(T, c, ns.o, ns.dir, true, ns.tmax);
+            } else {
+                L.stage = pre_first ? ST_FIRST : ST_BOUNCE;
+                emit(T, c, fma3(L.vs.N, 0.001f * startPosOffset, L.vs.P), tdir, false);
+            }
         }
         emitted = true;
     }
@@ -457,9 +497,11 @@ __device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
 // What bounds it: instruction issue with too few warps to cover it (1080p bricks: 310 warp
 // instructions per ray at 16.3 of 32 lanes, 419 at 12.4 when a warp traced its 32 rays to the end
 // before shading them all in registers; an issue in 38 % of the cycles, waits for instruction
-// fetch, node loads and fixed latencies in equal parts). Trace pass before / now, ms: 1080p bricks
-// 3.43 / 2.97, 4K city 91.9 / 51.0, textured 17.7 / 8.0, Cornell 256 x 256 0.164 / 0.146, 720p on
-// the probe grid 1.98 / 1.25.
+// fetch, node loads and fixed latencies in equal parts). So the code is kept small: one copy of the node
+// test, of the finished rays' hand-over, of the probe lookup and of the sampled direction (3 % to 17 % of
+// the pass). Trace pass in registers / on the pools / with one copy of each, ms: 1080p bricks 3.43 /
+// 2.97 / 2.84, 4K city 91.9 / 51.0 / 48.7, textured 17.7 / 8.2 / 6.6, Cornell 256 x 256 0.164 / 0.146 /
+// 0.134, 720p on the probe grid 1.98 / 1.25 / 1.16.
 //
 // Shared memory (dynamic): per-thread traversal stacks of stack_words entries (the scene's
 // depth bound), the world rays in flight, then each warp's path lists. A stack no larger than the
