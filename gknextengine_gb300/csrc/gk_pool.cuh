@@ -25,9 +25,22 @@ constexpr uint32_t kPoolMax = 256;
 // The traversal's schedule, in lanes: node tests run while at least kNodeLanes lanes have one, then
 // instance transitions (kTransLanes waiting) or triangle leaves (kLeafLanes), and finished rays make
 // room for new ones kRefillLanes at a time. kNodeLanes 8 / 12 / 16: 4K city 56.7 / 55.1 / 57;
-// kTransLanes 4 / 8 / 12: 57.2 / 52.6 / 54.9; kLeafLanes 10 / 14: 52.6 / 55.2; kRefillLanes 2 / 4 / 8:
-// 54.0 / 53.3 / 55.2.
-constexpr int kNodeLanes = 12, kTransLanes = 8, kLeafLanes = 10, kRefillLanes = 4;
+// kTransLanes 4 / 8 / 12: 57.2 / 52.6 / 54.9; kLeafLanes 10 / 14: 52.6 / 55.2; kRefillLanes
+// 4 / 6 / 8: 48.7 / 48.0 / 47.9 (1080p bricks 2.85 / 2.82 / 2.79, textured 6.38 / 6.30 / 6.23).
+constexpr int kNodeLanes = 12, kTransLanes = 8, kLeafLanes = 10, kRefillLanes = 8;
+
+// kOne: pools of one warp's worth of paths, which trace all their rays to the end before they shade again.
+// Latency is all there is to the small frames that use them: their fields go through L1 (a few pools per
+// SM; larger pools would drive out the nodes), there is no stash, and work runs for the fewer lanes the
+// fewer are left. (Frames of bricks with fixed thresholds, then shares: 300 x 200 at 1 sample 324 -> 288 us,
+// at 8 samples 1642 -> 1470.)
+template <bool kOne>
+__device__ __forceinline__ float4 pool_get(const float4* p) { return kOne ? *p : __ldcg(p); }
+template <bool kOne>
+__device__ __forceinline__ void pool_put(float4* p, float4 v) {
+    if (kOne) *p = v;
+    else __stcg(p, v);
+}
 
 // The paths of a warp's pool whose rays are finished, in three lists by the kind of ray (camera,
 // bounce, any-hit): the shading phase takes full warps of one kind, so that its sections run for
@@ -138,40 +151,54 @@ __device__ __forceinline__ void stash_empty(float4* s, const SceneView& S) {
 // at least kNodeLanes lanes have one, else instance transitions or triangle leaves, whichever
 // enough lanes wait for; lanes without a ray take one from the queue. The rays the lanes are in the
 // middle of at the end stay in the stash, so that a warp never waits for its longest ray.
+template <bool kOne = false>
 __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue, DoneLists& done, float4* pool, uint32_t np,
                                             float4* stash, float* wray, uint32_t* stk, int cap, Counters& cn) {
+    int kN = kNodeLanes, kT = kTransLanes, kL = kLeafLanes;
     Trav T;
     int st;
     uint32_t slot;
-    stash_load(stash, T, st, slot);
+    if (kOne) {   // every ray of the last time was finished
+        st = kStDone;
+        slot = kNoSlot;
+    } else {
+        stash_load(stash, T, st, slot);
+    }
     uint32_t kind = slot >> 10;
     slot &= kNoSlot;
     bool have = slot != kNoSlot;
     int waiting = 0;                // entries taken from the queue's front
     // finished rays that the shading phase takes mixed (94 hold a warp's worth of one of the three
     // kinds); a pool of one warp's worth is traced to its end
-    const int enough = np >= 64u ? min(94, (int)np - 32) : (int)np + 1;
+    const int enough = !kOne && np >= 64u ? min(94, (int)np - 32) : (int)np + 1;
     bool alone = false;             // node tests for fewer lanes than kNodeLanes, for want of other work
     for (;;) {
         unsigned mn = __ballot_sync(0xFFFFFFFFu, st == kStNode);
         // node tests
-        if (__popc(mn) >= kNodeLanes || alone) {
+        if (__popc(mn) >= kN || alone) {
             alone = false;
             do {
                 if (st == kStNode) st = trav_node(T, S, stk, kPoolThreads, cn, cap);
                 mn = __ballot_sync(0xFFFFFFFFu, st == kStNode);
-            } while (__popc(mn) >= kNodeLanes);
+            } while (__popc(mn) >= kN);
         }
         const unsigned md = __ballot_sync(0xFFFFFFFFu, st == kStDone);
         const bool more = waiting < queue.n;
+        if (kOne && !more) {   // no ray will join: the thresholds are shares of the rays left
+            const int n = 32 - __popc(md);
+            kN = max(1, n >> 1);
+            kT = max(1, (3 * n) >> 3);
+            kL = max(1, (5 * n) >> 4);
+        }
         const bool refill = more && (__popc(md) >= kRefillLanes || md == 0xFFFFFFFFu);
         if (refill || !more) {
             // finished rays to their paths
             const bool fin = have && st == kStDone;
             if (__any_sync(0xFFFFFFFFu, fin)) {
                 if (fin) {
-                    __stcg(pool + slot + PF_HIT * np, make_float4(__uint_as_float(T.hit ? T.inst : 0xFFFFFFFFu),
-                                                                  __uint_as_float(T.prim), __uint_as_float(T.tri), 0.0f));
+                    pool_put<kOne>(pool + slot + PF_HIT * np,
+                                   make_float4(__uint_as_float(T.hit ? T.inst : 0xFFFFFFFFu), __uint_as_float(T.prim),
+                                               __uint_as_float(T.tri), 0.0f));
                     have = false;
                 }
                 done.add(fin, kind, slot);
@@ -180,7 +207,7 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
                 const int k = waiting + __popc(md & ((1u << (threadIdx.x & 31u)) - 1u));
                 if (st == kStDone && k < queue.n) {
                     slot = queue.l[k];
-                    const float4 o = __ldcg(pool + slot + PF_RAYO * np), d = __ldcg(pool + slot + PF_RAYD * np);
+                    const float4 o = pool_get<kOne>(pool + slot + PF_RAYO * np), d = pool_get<kOne>(pool + slot + PF_RAYD * np);
                     kind = __float_as_uint(d.w);
                     trav_init(T, S, F3(o.x, o.y, o.z), F3(d.x, d.y, d.z), o.w, kind == kRayAny ? kAny : kClosest);
                     wray[0] = o.x; wray[kPoolThreads] = o.y; wray[2 * kPoolThreads] = o.z;
@@ -192,16 +219,16 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
                 continue;
             }
             // no ray left, or back to the shading phase if it has work
-            if (md == 0xFFFFFFFFu || done.largest() >= 32 || done.total() >= enough) break;
+            if (md == 0xFFFFFFFFu || (!kOne && (done.largest() >= 32 || done.total() >= enough))) break;
         }
         const unsigned mx = __ballot_sync(0xFFFFFFFFu, st == kStTrans), ml = __ballot_sync(0xFFFFFFFFu, st == kStLeaf);
-        if (__popc(mx) >= kTransLanes || (mx != 0u && mn == 0u && __popc(mx) >= __popc(ml))) {
+        if (__popc(mx) >= kT || (mx != 0u && mn == 0u && __popc(mx) >= __popc(ml))) {
             if (st == kStTrans) {
                 T.wo = F3(wray[0], wray[kPoolThreads], wray[2 * kPoolThreads]);
                 T.wd = F3(wray[3 * kPoolThreads], wray[4 * kPoolThreads], wray[5 * kPoolThreads]);
                 st = trav_trans(T, S, stk, kPoolThreads, cap);
             }
-        } else if (__popc(ml) >= kLeafLanes || (ml != 0u && mn == 0u)) {
+        } else if (__popc(ml) >= kL || (ml != 0u && mn == 0u)) {
             if (st == kStLeaf) {
                 T.wo = F3(wray[0], wray[kPoolThreads], wray[2 * kPoolThreads]);
                 T.wd = F3(wray[3 * kPoolThreads], wray[4 * kPoolThreads], wray[5 * kPoolThreads]);
@@ -212,7 +239,7 @@ __device__ __forceinline__ void trace_queue(const SceneView& S, PathList& queue,
         }
     }
     queue.n = 0;
-    stash_save(stash, T, have ? st : kStDone, have ? (slot | (kind << 10)) : kNoSlot);
+    if (!kOne) stash_save(stash, T, have ? st : kStDone, have ? (slot | (kind << 10)) : kNoSlot);
     __syncwarp();
 }
 

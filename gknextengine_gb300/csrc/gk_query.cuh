@@ -13,6 +13,7 @@ namespace gk {
 
 constexpr int kQueryThreads = 128;
 constexpr int kQueryWarps = kQueryThreads / 32;
+constexpr int kQueryRefillLanes = 4;   // finished rays make room for new ones so many at a time
 constexpr int kQueryRing = 64;      // finished rays per warp: fewer than 32 kept, up to 32 more per step
 // Shared memory of a block: stacks and world rays per thread, a ring of 16-byte entries per warp.
 constexpr size_t query_smem(int stack_words) {
@@ -108,7 +109,7 @@ __device__ __forceinline__ void query_run(const SceneView& S, const Source& src,
             } while (__popc(mn) >= thr);
         }
         const unsigned md = __ballot_sync(0xFFFFFFFFu, st == kStDone);
-        if (__popc(md) >= kRefillLanes && (run < n || md == 0xFFFFFFFFu || __any_sync(0xFFFFFFFFu, have && st == kStDone))) {
+        if (__popc(md) >= kQueryRefillLanes && (run < n || md == 0xFFFFFFFFu || __any_sync(0xFFFFFFFFu, have && st == kStDone))) {
             // finished rays to the ring, complete entries written, the next rays to the free lanes
             const bool fin = have && st == kStDone;
             const unsigned mf = __ballot_sync(0xFFFFFFFFu, fin);

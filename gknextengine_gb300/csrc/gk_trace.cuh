@@ -4,10 +4,9 @@
 // Shading.slang:737-826). GB300 has no RT cores, so traversal is software, over either of
 // the two node formats the builders produce from the same SAH trees:
 //   * four-child nodes (128 bytes, one cache line, seven 16-byte loads per node, a stack of
-//     node refs): used by the rt pass and the adjoint, whose node step stays short;
+//     node refs): used by the rt pass, the adjoint, the ray queries and the probe bake;
 //   * compressed 8-wide nodes (96 bytes, six loads test eight 8-bit child boxes, a stack of
-//     sorted node groups): used by the ray-query kernels, where traversal runs alone and the
-//     wide nodes halve the node steps of incoherent rays.
+//     sorted node groups): used by the probe voxelization.
 // Both keep 48-byte triangles in leaf order, a per-thread stack in shared memory (strided
 // by the block size, conflict-free) and a marker entry for the hand-over from the instance
 // level to the mesh level.

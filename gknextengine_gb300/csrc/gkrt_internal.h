@@ -211,7 +211,7 @@ bool gpu_bvh_cooperative_supported();   // the current device takes cooperative 
 // Four-child nodes [base, base + count) of `quad` from the same slots of the two-child array.
 cudaError_t gpu_bvh_quads(const BvhNode* nodes, QuadNode* quad, uint32_t base, uint32_t count, cudaStream_t st);
 // Collapse of two-child trees (device array bin, roots: node refs, -1 for none) into the
-// compressed 8-wide nodes the kernels traverse, at out[wide_base ...) of an array of out_cap
+// compressed 8-wide nodes (probe voxelization), at out[wide_base ...) of an array of out_cap
 // nodes. wroots: wide root per tree (-1 for none); count: wide nodes written; depth: levels.
 // links: when non-null, the collapse also records what a refit of these trees needs.
 struct RefitLinks;

@@ -26,6 +26,12 @@ constexpr int kPtMaxBlocks = 8;    // resident blocks per SM, at most
 // 0.160 / 0.134 / 0.150, 720p on the probe grid 1.31 / 1.16 / 1.14, 4K city 52.3 / 48.7 / 48.4, textured
 // 1277 x 713 at 8 samples 6.8 / 6.6 / 7.7.
 constexpr int kPtBlocks = 4;
+// Pools of one warp's worth (kOne) serve frames of up to kPtOneWarps warps' worth of pixels per SM, with
+// three blocks per SM, whose registers hold a path without spills. Whole frames of bricks with 2 / 3 / 4 /
+// 5 blocks, us: 100 x 70 pixels 215 / 220 / 231 / 272, 300 x 200 250 / 269 / 288 / 330, 400 x 300 358 / 305 /
+// 333 / 406; Cornell 256 x 256 158 / 131 / 156 / 176. Larger pools on 640 x 360: bricks 537 us (504),
+// Cornell 289 (277), city 4853 (4532), textured 429 (471), probe grid 1002 (1027).
+constexpr int kPtOneBlocks = 3, kPtOneWarps = 64;
 constexpr float kCosCone = 0.999990482f;   // cos(0.25 deg), Shading.slang:897
 
 // Warp-aggregated flush: one atomic per counter per warp. Slots 0-5 are per pass
@@ -83,6 +89,7 @@ struct Lane {
     f3 dir;           // current path direction
 };
 
+template <bool kOne>
 struct Ctx {
     const ShadeScene& sc;
     const GkrtFrameConstants& fc;
@@ -92,20 +99,23 @@ struct Ctx {
     uint32_t np;      // paths per pool: the stride between fields
     Counters& cn;
     __device__ f4 get(int f) const {
-        const float4 v = __ldcg(path + (uint32_t)f * np);
+        const float4 v = pool_get<kOne>(path + (uint32_t)f * np);
         return F4(v.x, v.y, v.z, v.w);
     }
-    __device__ void put(int f, f4 v) const { __stcg(path + (uint32_t)f * np, make_float4(v.x, v.y, v.z, v.w)); }
+    __device__ void put(int f, f4 v) const {
+        pool_put<kOne>(path + (uint32_t)f * np, make_float4(v.x, v.y, v.z, v.w));
+    }
     __device__ void put(int f, f3 v, uint32_t w) const { put(f, F4(v.x, v.y, v.z, __uint_as_float(w))); }
 };
 
+template <class Ctx>
 __device__ __forceinline__ void emit(PathRay& R, const Ctx& c, f3 o, f3 d, bool any, float tmax = 1000.0f) {
     ++c.cn.rays;
     R.wo = o; R.wd = d; R.tmax = tmax; R.any = any;
 }
 
 // primaryAlbedo_ of the reference: the material's diffuse, times its diffuse texture (kTex)
-template <bool kTex>
+template <bool kTex, class Ctx>
 __device__ __forceinline__ f4 pv_albedo(const Ctx& c) {
     if (kTex) return c.get(PF_ALB);
     return load_mat(c.sc, __float_as_uint(c.get(PF_PP).w)).diffuse;
@@ -123,7 +133,7 @@ __device__ __forceinline__ f4 pv_albedo(const Ctx& c) {
 // next) run once per warp for all the lanes that need them.
 // kTex: textured materials and the textured sky compiled in (the scene has texture ids or the
 // frame samples a sky texture).
-template <bool kNee, bool kTex>
+template <bool kNee, bool kTex, class Ctx>
 __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
     const GkrtFrameConstants& fc = c.fc;
     const f3 sunDir = F3(fc.sun_direction[0], fc.sun_direction[1], fc.sun_direction[2]);
@@ -426,6 +436,7 @@ __device__ __forceinline__ bool advance(Lane& L, PathRay& T, const Ctx& c) {
 }
 
 // Camera ray of FHardwarePrimaryRayCaster (Shading.slang:286-304) for pixel index pix.
+template <class Ctx>
 __device__ __forceinline__ void start_pixel(Lane& L, PathRay& T, const Ctx& c, int x, int y) {
     const GkrtFrameConstants& fc = c.fc;
     L.pix = y * c.P + x;
@@ -450,6 +461,7 @@ __device__ __forceinline__ void start_pixel(Lane& L, PathRay& T, const Ctx& c, i
 }
 
 // State word pair of a path: stage and flags, sample and bounce indices.
+template <class Ctx>
 __device__ __forceinline__ void store_path(const Ctx& c, const Lane& L, const PathRay& R) {
     c.put(PF_RAYO, F4(R.wo.x, R.wo.y, R.wo.z, R.tmax));
     c.put(PF_RAYD, R.wd, R.any ? kRayAny : L.stage == ST_PRIMARY ? kRayCamera : kRayBounce);
@@ -466,6 +478,7 @@ __device__ __forceinline__ void store_path(const Ctx& c, const Lane& L, const Pa
     }
 }
 
+template <class Ctx>
 __device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
     const f4 o = c.get(PF_RAYO), d = c.get(PF_RAYD), h = c.get(PF_HIT), sd = c.get(PF_SEED), st = c.get(PF_STATE);
     R.wo = xyz(o); R.wd = xyz(d); R.tmax = o.w; R.any = __float_as_uint(d.w) == kRayAny;
@@ -500,14 +513,14 @@ __device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
 // fetch, node loads and fixed latencies in equal parts). So the code is kept small: one copy of the node
 // test, of the finished rays' hand-over, of the probe lookup and of the sampled direction (3 % to 17 % of
 // the pass). Trace pass in registers / on the pools / with one copy of each, ms: 1080p bricks 3.43 /
-// 2.97 / 2.84, 4K city 91.9 / 51.0 / 48.7, textured 17.7 / 8.2 / 6.6, Cornell 256 x 256 0.164 / 0.146 /
+// 2.97 / 2.84, 4K city 91.9 / 51.0 / 48.7, textured 17.7 / 8.2 / 6.4, Cornell 256 x 256 0.164 / 0.146 /
 // 0.134, 720p on the probe grid 1.98 / 1.25 / 1.16.
 //
 // Shared memory (dynamic): per-thread traversal stacks of stack_words entries (the scene's
 // depth bound), the world rays in flight, then each warp's path lists. A stack no larger than the
 // scene needs leaves the rest of the SM's 256 KB to L1, which serves the node fetches.
-template <bool kNee, bool kTex>
-__global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
+template <bool kNee, bool kTex, bool kOne>
+__global__ void __launch_bounds__(kPtThreads, kOne ? kPtOneBlocks : kPtBlocks) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
                                                            int P, PixelImages im, unsigned long long* counters,
                                                            unsigned int* work, int stack_words, float4* pools,
                                                            uint32_t np) {
@@ -527,7 +540,7 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_trace_pass(ShadeScene
     for (uint32_t k = lane; k < np; k += 32u) spare.l[k] = (PathId)k;
     PathList queue{lists + 3u * np, 0};
     DoneLists done{lists, np, {0, 0, 0}};
-    stash_empty(stash, sc.S);
+    if (!kOne) stash_empty(stash, sc.S);
     __syncwarp();
     bool exhausted = false;
     int live = 0;                                  // paths with a ray queued, in flight or finished
@@ -545,7 +558,7 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_trace_pass(ShadeScene
             uint32_t slot = 0;
             if (k < n) {
                 slot = done.at(k, take);
-                const Ctx c{sc, fc, im, W, H, P, pool + slot, np, cn};
+                const Ctx<kOne> c{sc, fc, im, W, H, P, pool + slot, np, cn};
                 Lane L;
                 PathRay R;
                 load_path(c, L, R);
@@ -574,7 +587,7 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_trace_pass(ShadeScene
                 const int y = (int)((tile / (unsigned)tiles_x) * 4u + (in >> 3));
                 ray = k < total && x < W && y < H;
                 if (ray) {
-                    const Ctx c{sc, fc, im, W, H, P, pool + slot, np, cn};
+                    const Ctx<kOne> c{sc, fc, im, W, H, P, pool + slot, np, cn};
                     Lane L;
                     PathRay R;
                     start_pixel(L, R, c, x, y);
@@ -591,7 +604,7 @@ __global__ void __launch_bounds__(kPtThreads, kPtBlocks) k_trace_pass(ShadeScene
         }
         live += queue.n;
         if (live == 0) break;
-        trace_queue(sc.S, queue, done, pool, np, stash, wray, stack, stack_words, cn);
+        trace_queue<kOne>(sc.S, queue, done, pool, np, stash, wray, stack, stack_words, cn);
     }
     flush_counters(cn, counters);
 }
@@ -639,13 +652,19 @@ cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstant
     const size_t smem = (size_t)(stack_words + kPoolRayWords) * kPtThreads * 4u + pool_list_bytes(kPoolMax);
     using Kernel = void (*)(ShadeScene, GkrtFrameConstants, int, int, int, PixelImages, unsigned long long*, unsigned int*,
                             int, float4*, uint32_t);
-    const Kernel f = nee ? (tex ? k_trace_pass<true, true> : k_trace_pass<true, false>)
-                         : (tex ? k_trace_pass<false, true> : k_trace_pass<false, false>);
+    static const Kernel kernels[2][2][2] = {
+        {{k_trace_pass<false, false, false>, k_trace_pass<false, false, true>},
+         {k_trace_pass<false, true, false>, k_trace_pass<false, true, true>}},
+        {{k_trace_pass<true, false, false>, k_trace_pass<true, false, true>},
+         {k_trace_pass<true, true, false>, k_trace_pass<true, true, true>}}};
+    const uint32_t pixels = (uint32_t)W * (uint32_t)H;
+    const bool one = pixels <= (uint32_t)num_sms * kPtOneWarps * 32u;
+    const Kernel f = kernels[nee][tex][one];
     // resident blocks per SM of each instantiation and stack size, queried once per device
-    static int occ[kMaxDevices][2][2][kQuadStackMax + 1] = {};
+    static int occ[kMaxDevices][2][2][2][kQuadStackMax + 1] = {};
     const int dev = current_device_slot();
     if (dev < 0) return cudaErrorInvalidDevice;
-    int* o = &occ[dev][nee][tex][stack_words];
+    int* o = &occ[dev][nee][tex][one][stack_words];
     cudaError_t e = cudaSuccess;
     if (!*o) {
         const int most = (kQuadStackMax + kPoolRayWords) * kPtThreads * 4 + (int)pool_list_bytes(kPoolMax);   // the deepest trees a build accepts
@@ -653,10 +672,9 @@ cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstant
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, f, kPtThreads, smem);
         if (e != cudaSuccess) return e;
     }
-    const uint32_t pixels = (uint32_t)W * (uint32_t)H;
     uint32_t blocks = (uint32_t)(num_sms * std::max(1, std::min(*o, kPtMaxBlocks)));
     blocks = std::min(blocks, (pixels + kPtThreads - 1) / kPtThreads);
-    const uint32_t np = paths_per_pool(pixels, blocks * kPtWarps);
+    const uint32_t np = one ? 32u : paths_per_pool(pixels, blocks * kPtWarps);
     if ((size_t)blocks * kPtWarps * (np * PF_COUNT + kStashFields * 32u) * sizeof(float4) > pool_bytes) return cudaErrorInvalidValue;
     e = cudaMemsetAsync(work, 0, sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
