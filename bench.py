@@ -13,7 +13,7 @@ reprojection and the joint bilateral filter. The scene is synthetic (seeded nump
 * roofline: the trace kernel against its binding resource, instruction issue: warp
             instructions per ray (ncu) x the frame's rays over the event-timed duration,
             against SMs x 4 issue slots x the sampled SM clock. Beside it (roofline.hbm) the
-            algorithmic bytes (node visits x 64 B + triangle tests x 48 B + rays x 32 B +
+            algorithmic bytes (node visits x 112 B + triangle tests x 48 B + rays x 32 B +
             hit fetches x 236 B + outputs, all device-counted) and the DRAM traffic (ncu)
             against the measured HBM copy bandwidth.
 * city    : 3 timed 4K frames of the 10.5 M-triangle city with the per-frame instance rebuild.
@@ -41,24 +41,29 @@ METRIC = "Mrays/s and ms/frame 1080p 1spp; denoised RelMSE vs 4096 spp vs bilate
 UNIT = "Mrays/s"
 W_, H_ = 1920, 1080
 HIT_FETCH_BYTES = 3 * 4 + 3 * 16 + 64 + 64 + 48   # indices, normals, material, instance, triangle
-NODE_BYTES, TRI_BYTES, RAY_BYTES = 64, 48, 32
+NODE_BYTES, TRI_BYTES, RAY_BYTES = 112, 48, 32   # seven 16-byte words of a four-child node
 # ncu counters of one 1080p k_trace_pass launch of the default workload (one capture of
 # `python bench.py --steps 3 --warmup 3 --no-cpu-baseline --no-relmse --no-city`, fifth launch):
 # warp instructions issued (sm__inst_executed.sum), thread instructions
 # (smsp__thread_inst_executed.sum), DRAM bytes read + written, and the rays of that launch.
 # The node and triangle reads of the algorithmic bytes are served by L1/L2.
+# TRACE_NCU_1080P: the kernel that held a path in registers; TRACE_NCU_POOLS: the one on path pools,
+# which the benchmark's line uses.
 TRACE_NCU_1080P = {"inst": 1876796969, "thread_inst": 23252036915, "dram_bytes": 7515904 + 116706048,
+                   "rays": 4483043}
+TRACE_NCU_POOLS = {"inst": 1348093445, "thread_inst": 21990874094, "dram_bytes": 668959744 + 908498176,
                    "rays": 4483043}
 ISSUE_PER_SM_PER_CLOCK = 4   # four schedulers per SM, one warp instruction each per cycle
 
 
-def trace_roofline(st, trace_ms, alg_bytes, alg_gbs, hbm_peak, peak_kind, num_sms, clocks):
+def trace_roofline(st, trace_ms, alg_bytes, alg_gbs, hbm_peak, peak_kind, num_sms, clocks,
+                   counters=TRACE_NCU_1080P):
     """Roofline of the rt-pass kernel against the bound that holds: issue slots. The BVH is
     cache-resident, so DRAM carries little more than the output images (dram_frac), and the
     kernel is bound by instruction issue and SIMT efficiency (divergent traversal and shading).
     achieved: warp instructions per ray (ncu, one 1080p launch) x the rays of the timed frame over
     its event-timed duration; peak: SMs x 4 issue slots x the SM clock sampled during the run."""
-    n = TRACE_NCU_1080P
+    n = counters
     full = WORKLOAD == "bricks" and (W_, H_) == (1920, 1080)
     sm_mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 2070.0
     issue_peak = num_sms * ISSUE_PER_SM_PER_CLOCK * sm_mhz * 1e6 / 1e9
@@ -732,7 +737,7 @@ def run_gkrt(args):
                         "h2d_bytes_per_step": ctypes.sizeof(abi.GkrtFrameConstants),
                         "d2h_bytes_per_step": W_ * H_ * 16, "ms_per_frame": e2e_s / K * 1e3},
                 "roofline": trace_roofline(st_last, trace_avg_ms, alg_bytes, achieved, peak, peak_kind, num_sms,
-                                           clk.summary()),
+                                           clk.summary(), TRACE_NCU_POOLS),
                 "clocks": clk.summary()}
         if world == 1 and WORKLOAD == "bricks" and not args.no_city:
             line["city"] = city_measure(local)

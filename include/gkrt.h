@@ -279,7 +279,7 @@ typedef struct GkrtStats {
     uint32_t tlas_nodes;
     uint32_t emitters;          /* emissive triangles in the GKRT_NEE_EMISSIVE table      */
     uint32_t build_launches;    /* kernels launched by GPU BVH builds since creation      */
-    uint32_t wide_nodes;        /* compressed 8-wide nodes traversed (mesh + instance)    */
+    uint32_t wide_nodes;        /* compressed 8-wide nodes of the mesh + instance levels  */
     uint32_t wide_depth;        /* wide levels, deepest mesh tree + instance tree         */
     uint32_t tlas_refits;       /* instance-level refits since creation                   */
     uint32_t hit_fetches;       /* closest hits whose vertex, normal, material and instance
