@@ -40,6 +40,11 @@ namespace {
 // Resident blocks per SM (128 registers); 3 / 4 / 5 blocks took 19.9 / 17.8 / 16.6 ms forward and
 // 20.1 / 18.6 / 18.5 backward with pools of 80 / 96 / 64 paths (4 blocks with 64: 16.5 / 17.5).
 constexpr int kAdjBlocks = 4;
+// Pools of one warp's worth of paths (kOne): at 3 blocks per SM up to 16 warps' worth of pixels per SM, at
+// 4 up to 48. Forward and backward, us, pools of more / 3 / 4 blocks: 100 x 100 pixels at 16 samples 13953 /
+// 10340 / 10755, 256 x 256 at 8 9811 / 7023 / 7706, 300 x 400 at 4 5866 / 5415 / 4618, 400 x 500 8798 /
+// 7783 / 6959, 512 x 512 9670 / 11323 / 10217.
+constexpr int kAdjOneWarps3 = 16, kAdjOneWarps4 = 48;
 // Records of one sample: a factor per ray's hit and one for a metallic first bounce, a score per
 // GGX bounce. The entry points take at most 16 bounces, a ray each.
 constexpr int kMaxRays = 16;
@@ -103,14 +108,17 @@ struct AdjArgs {
     double* g_rough;
 };
 
+template <bool kOne>
 struct AdjPath {
     float4* p;        // field 0
     uint32_t np;      // stride between fields
     __device__ f4 get(int f) const {
-        const float4 v = __ldcg(p + (uint32_t)f * np);
+        const float4 v = pool_get<kOne>(p + (uint32_t)f * np);
         return F4(v.x, v.y, v.z, v.w);
     }
-    __device__ void put(int f, f4 v) const { __stcg(p + (uint32_t)f * np, make_float4(v.x, v.y, v.z, v.w)); }
+    __device__ void put(int f, f4 v) const {
+        pool_put<kOne>(p + (uint32_t)f * np, make_float4(v.x, v.y, v.z, v.w));
+    }
     __device__ void put(int f, f3 v, uint32_t w) const { put(f, F4(v.x, v.y, v.z, __uint_as_float(w))); }
     __device__ float2* ggx(int k) const {
         return reinterpret_cast<float2*>(p + (uint32_t)(AF_GGX + (k >> 1)) * np) + (k & 1);
@@ -124,7 +132,7 @@ __device__ __forceinline__ void add_grad(double* g, float v) {
 // Runs a path on the answer of its ray, up to its next ray (true) or the end of its pixel (false):
 // FPathTracingRendererV2::Render and GetRayColor (Shading.slang:1003-1184) with detached GGX
 // sampling and, backward, the sample's records.
-template <bool kBackward>
+template <bool kBackward, class AdjPath>
 __device__ __forceinline__ bool adj_advance(const ShadeScene& sc, const GkrtFrameConstants& fc, const AdjArgs& a,
                                             const AdjPath& c, Counters& cn) {
     const f4 ro = c.get(PF_RAYO), rd = c.get(PF_RAYD), h = c.get(PF_HIT), sd = c.get(AF_SEED), state = c.get(AF_STATE);
@@ -359,10 +367,12 @@ __device__ __forceinline__ bool adj_advance(const ShadeScene& sc, const GkrtFram
 // Persistent warps over the frame's pixels (row-major, 32 at a time). What bounds it: as the rt pass,
 // instruction issue; one thread per pixel, every warp waiting for its longest path at each ray of
 // each sample, took 40.7 ms forward and 51 backward at 512 x 512 and 16 samples; now 16.5 and 17.5.
-template <bool kBackward>
-__global__ void __launch_bounds__(kPoolThreads, kAdjBlocks) k_adjoint(ShadeScene sc, GkrtFrameConstants fc, AdjArgs a,
+// kOneBlocks: pools of one warp's worth, blocks per SM (0: larger pools)
+template <bool kBackward, int kOneBlocks>
+__global__ void __launch_bounds__(kPoolThreads, kOneBlocks ? kOneBlocks : kAdjBlocks) k_adjoint(ShadeScene sc, GkrtFrameConstants fc, AdjArgs a,
                                                                       unsigned long long* counters, unsigned int* work,
                                                                       int stack_words, float4* pools, uint32_t np) {
+    constexpr bool kOne = kOneBlocks != 0;
     extern __shared__ uint32_t adj_smem[];
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = tid & 31u;
@@ -379,7 +389,7 @@ __global__ void __launch_bounds__(kPoolThreads, kAdjBlocks) k_adjoint(ShadeScene
     for (uint32_t k = lane; k < np; k += 32u) spare.l[k] = (PathId)k;
     PathList queue{lists + 3u * np, 0};
     DoneLists done{lists, np, {0, 0, 0}};
-    stash_empty(stash, sc.S);
+    if (!kOne) stash_empty(stash, sc.S);
     __syncwarp();
     bool exhausted = false;
     int live = 0;
@@ -396,7 +406,7 @@ __global__ void __launch_bounds__(kPoolThreads, kAdjBlocks) k_adjoint(ShadeScene
             uint32_t slot = 0;
             if (k < n) {
                 slot = done.at(k, take);
-                ray = adj_advance<kBackward>(sc, fc, a, AdjPath{pool + slot, np}, cn);
+                ray = adj_advance<kBackward>(sc, fc, a, AdjPath<kOne>{pool + slot, np}, cn);
             }
             __syncwarp();
             queue.add(ray, slot);
@@ -422,7 +432,7 @@ __global__ void __launch_bounds__(kPoolThreads, kAdjBlocks) k_adjoint(ShadeScene
                     f3 o, d;
                     camera_ray(fc, x, y, a.W, a.H, seed, o, d);
                     ++cn.rays;
-                    const AdjPath c{pool + slot, np};
+                    const AdjPath<kOne> c{pool + slot, np};
                     c.put(PF_RAYO, F4(o.x, o.y, o.z, 1000.0f));
                     c.put(PF_RAYD, d, kRayCamera);
                     c.put(AF_SEED, F4(__uint_as_float(seed.v[0]), __uint_as_float(seed.v[1]),
@@ -438,7 +448,7 @@ __global__ void __launch_bounds__(kPoolThreads, kAdjBlocks) k_adjoint(ShadeScene
         }
         live += queue.n;
         if (live == 0) break;
-        trace_queue(sc.S, queue, done, pool, np, stash, wray, stack, stack_words, cn);
+        trace_queue<kOne>(sc.S, queue, done, pool, np, stash, wray, stack, stack_words, cn);
     }
     // ray counters: warp sums, one atomic per warp
     unsigned long long r = cn.rays;
@@ -474,13 +484,18 @@ cudaError_t gkrt_launch_adjoint(const ShadeScene& sc, const GkrtFrameConstants& 
     if (stack_words < 1 || stack_words > kQuadStackMax) return cudaErrorInvalidValue;
     using Kernel = void (*)(ShadeScene, GkrtFrameConstants, AdjArgs, unsigned long long*, unsigned int*, int, float4*,
                             uint32_t);
-    const Kernel f = dimage ? (Kernel)k_adjoint<true> : (Kernel)k_adjoint<false>;
+    static const Kernel kernels[2][3] = {{k_adjoint<false, 0>, k_adjoint<false, 3>, k_adjoint<false, 4>},
+                                         {k_adjoint<true, 0>, k_adjoint<true, 3>, k_adjoint<true, 4>}};
+    const uint32_t pixels = (uint32_t)W * (uint32_t)H;
+    const uint32_t sm_warps = pixels / (uint32_t)num_sms / 32u;
+    const int one = sm_warps < (uint32_t)kAdjOneWarps3 ? 1 : sm_warps < (uint32_t)kAdjOneWarps4 ? 2 : 0;
+    const Kernel f = kernels[dimage != nullptr][one];
     const uint32_t fields = dimage ? adj_fields<true>() : adj_fields<false>();
     const size_t smem = (size_t)(stack_words + kPoolRayWords) * kPoolThreads * 4u + pool_list_bytes(kPoolMax);
-    static int occ[kMaxDevices][2][kQuadStackMax + 1] = {};
+    static int occ[kMaxDevices][2][3][kQuadStackMax + 1] = {};
     const int dev = current_device_slot();
     if (dev < 0) return cudaErrorInvalidDevice;
-    int* o = &occ[dev][dimage ? 1 : 0][stack_words];
+    int* o = &occ[dev][dimage ? 1 : 0][one][stack_words];
     cudaError_t e = cudaSuccess;
     if (!*o) {
         const int most = (kQuadStackMax + kPoolRayWords) * kPoolThreads * 4 + (int)pool_list_bytes(kPoolMax);
@@ -488,14 +503,13 @@ cudaError_t gkrt_launch_adjoint(const ShadeScene& sc, const GkrtFrameConstants& 
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, f, kPoolThreads, smem);
         if (e != cudaSuccess) return e;
     }
-    const uint32_t pixels = (uint32_t)W * (uint32_t)H;
     uint32_t blocks = (uint32_t)(num_sms * std::max(1, std::min(*o, kAdjBlocks)));
     blocks = std::min(blocks, (pixels + kPoolThreads - 1) / kPoolThreads);
     const uint32_t warps = blocks * kPoolWarps;
     // A pixel's samples are a long chain of rays: pools of two thirds of a warp's share of the pixels
     // leave the rest to the warps that end early (512 x 512 at 16 samples, a share of 107: pools of
     // 32 / 64 / 96 paths 21.2 / 16.5 / 17.8 ms forward).
-    const uint32_t np = std::max(32u, std::min(kPoolMax, pixels / warps * 2u / 3u / 32u * 32u));
+    const uint32_t np = one ? 32u : std::max(32u, std::min(kPoolMax, pixels / warps * 2u / 3u / 32u * 32u));
     // scratch of this call alone (calls may overlap on several streams): the pools, then the pixel counter
     const size_t bytes = (size_t)warps * (fields * np + kStashFields * 32u) * sizeof(float4);
     float4* pools = nullptr;

@@ -4,7 +4,7 @@ import pytest
 
 from gknextengine_gb300 import abi, scenes
 from gknextengine_gb300.renderer import PathTracingRenderer
-from test_gpu_path_pools import _pass
+from test_gpu_path_pools import _pass, test_adjoint_sizes as adjoint_sizes
 
 pytestmark = pytest.mark.gpu
 
@@ -20,3 +20,9 @@ def test_one_warp_pools(W, H, samples, nee):
     with PathTracingRenderer(0) as r:
         r.load_scene(sc)
         _pass(r, sc, cam, st, W, H)
+
+
+# up to 16 warps' worth of pixels per SM, up to 48 and beyond (152 SMs: 77,824 and 233,472 pixels)
+@pytest.mark.parametrize("W,H,spp,bounces", [(304, 255, 1, 2), (304, 257, 1, 2), (456, 513, 1, 2), (9, 31, 5, 4)])
+def test_adjoint_one_warp_pools(W, H, spp, bounces):
+    adjoint_sizes(W, H, spp, bounces, False)
