@@ -189,15 +189,8 @@ GK_D f3 hemisphere_cos(Rng& s) {
     float r = sqrt_(u.y);
     return F3(r * cs, r * sn, sqrt_(1.0f - u.y));
 }
+// cosine to the axis of a direction of the cone, uniform over its solid angle
 GK_D float cone_z(float cos_theta, float u) { return fmaf_(u, cos_theta - 1.0f, 1.0f); }
-GK_D f3 cone(Rng& s, float cos_theta) {
-    f2 u = rnd2(s);
-    float sn, cs;
-    sincos2pi(u.x, sn, cs);
-    float ct = cone_z(cos_theta, u.y);
-    float r = sqrt_(fmaf_(-ct, ct, 1.0f));
-    return F3(r * cs, r * sn, ct);
-}
 GK_D f2 unit_disk(Rng& s) {
     f2 u = rnd2(s);
     float ox = u.x + (u.x - 1.0f), oy = u.y + (u.y - 1.0f);
