@@ -27,11 +27,12 @@ constexpr int kPtMaxBlocks = 8;    // resident blocks per SM, at most
 // 1277 x 713 at 8 samples 6.8 / 6.6 / 7.7.
 constexpr int kPtBlocks = 4;
 // Pools of one warp's worth (kOne) serve frames of up to kPtOneWarps warps' worth of pixels per SM, with
-// three blocks per SM, whose registers hold a path without spills. Whole frames of bricks with 2 / 3 / 4 /
+// three blocks per SM, whose registers hold a path without spills, or two where those have a lane for
+// every pixel. Whole frames of bricks with 2 / 3 / 4 /
 // 5 blocks, us: 100 x 70 pixels 215 / 220 / 231 / 272, 300 x 200 250 / 269 / 288 / 330, 400 x 300 358 / 305 /
 // 333 / 406; Cornell 256 x 256 158 / 131 / 156 / 176. Larger pools on 640 x 360: bricks 537 us (504),
 // Cornell 289 (277), city 4853 (4532), textured 429 (471), probe grid 1002 (1027).
-constexpr int kPtOneBlocks = 3, kPtOneWarps = 64;
+constexpr uint32_t kPtOneWarps = 64;
 constexpr float kCosCone = 0.999990482f;   // cos(0.25 deg), Shading.slang:897
 
 // Warp-aggregated flush: one atomic per counter per warp. Slots 0-5 are per pass
@@ -519,11 +520,13 @@ __device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
 // Shared memory (dynamic): per-thread traversal stacks of stack_words entries (the scene's
 // depth bound), the world rays in flight, then each warp's path lists. A stack no larger than the
 // scene needs leaves the rest of the SM's 256 KB to L1, which serves the node fetches.
-template <bool kNee, bool kTex, bool kOne>
-__global__ void __launch_bounds__(kPtThreads, kOne ? kPtOneBlocks : kPtBlocks) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
+// kOneBlocks: pools of one warp's worth, blocks per SM (0: larger pools)
+template <bool kNee, bool kTex, int kOneBlocks>
+__global__ void __launch_bounds__(kPtThreads, kOneBlocks ? kOneBlocks : kPtBlocks) k_trace_pass(ShadeScene sc, GkrtFrameConstants fc, int W, int H,
                                                            int P, PixelImages im, unsigned long long* counters,
                                                            unsigned int* work, int stack_words, float4* pools,
                                                            uint32_t np) {
+    constexpr bool kOne = kOneBlocks != 0;
     extern __shared__ uint32_t dyn_smem[];
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = tid & 31u;
@@ -652,16 +655,16 @@ cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstant
     const size_t smem = (size_t)(stack_words + kPoolRayWords) * kPtThreads * 4u + pool_list_bytes(kPoolMax);
     using Kernel = void (*)(ShadeScene, GkrtFrameConstants, int, int, int, PixelImages, unsigned long long*, unsigned int*,
                             int, float4*, uint32_t);
-    static const Kernel kernels[2][2][2] = {
-        {{k_trace_pass<false, false, false>, k_trace_pass<false, false, true>},
-         {k_trace_pass<false, true, false>, k_trace_pass<false, true, true>}},
-        {{k_trace_pass<true, false, false>, k_trace_pass<true, false, true>},
-         {k_trace_pass<true, true, false>, k_trace_pass<true, true, true>}}};
+#define GK_PASSES(nee, tex) {k_trace_pass<nee, tex, 0>, k_trace_pass<nee, tex, 2>, k_trace_pass<nee, tex, 3>}
+    static const Kernel kernels[2][2][3] = {{GK_PASSES(false, false), GK_PASSES(false, true)},
+                                            {GK_PASSES(true, false), GK_PASSES(true, true)}};
+#undef GK_PASSES
     const uint32_t pixels = (uint32_t)W * (uint32_t)H;
-    const bool one = pixels <= (uint32_t)num_sms * kPtOneWarps * 32u;
+    const uint32_t per_sm = pixels / (uint32_t)num_sms;
+    const int one = per_sm <= 2u * kPtThreads ? 1 : per_sm <= kPtOneWarps * 32u ? 2 : 0;
     const Kernel f = kernels[nee][tex][one];
     // resident blocks per SM of each instantiation and stack size, queried once per device
-    static int occ[kMaxDevices][2][2][2][kQuadStackMax + 1] = {};
+    static int occ[kMaxDevices][2][2][3][kQuadStackMax + 1] = {};
     const int dev = current_device_slot();
     if (dev < 0) return cudaErrorInvalidDevice;
     int* o = &occ[dev][nee][tex][one][stack_words];

@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 # 64 warps' worth of pixels per SM on 152 SMs: 311,296 pixels = 608 x 512
 @pytest.mark.parametrize("W,H,samples,nee", [(608, 512, 1, abi.NEE_REFERENCE), (609, 512, 1, abi.NEE_REFERENCE),
-                                             (130, 3, 8, abi.NEE_REFERENCE), (255, 129, 4, abi.NEE_EMISSIVE),
+                                             (130, 3, 8, abi.NEE_REFERENCE), (304, 128, 1, abi.NEE_REFERENCE),
+                                             (305, 129, 1, abi.NEE_EMISSIVE), (255, 129, 4, abi.NEE_EMISSIVE),
                                              (456, 128, 2, abi.NEE_REFERENCE)])
 def test_one_warp_pools(W, H, samples, nee):
     sc, cam, st = scenes.cornell()
