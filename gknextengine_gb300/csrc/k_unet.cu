@@ -22,10 +22,13 @@ namespace {
 //   M  rows are the box of one 32-channel group of X, {32 channels, 34 pixels, 4 image rows}, at
 //      pixel offsets 0, 1 and 2 (the taps dx): atoms one pixel apart. The fourth is not used;
 //   N  columns are the dP rows r - 1, r, r + 1 of one 32-channel group against X's row r (the taps
-//      dy = 1, 0, -1): consecutive rows of one box with a halo row on each side.
-// So an X element is loaded once and a dP element 1.5 times. TMA's zero fill is the
+//      dy = 1, 0, -1): consecutive rows of one box with a halo row on each side. At an image's first and
+//      last row N leaves out the dP row outside it, whose zeros times an infinite X would be NaN in a tap
+//      that this row has no part in; and X rows past the image take no MMA.
+// So an X element is loaded once and a dP element 1.5 times. TMA's zero fill is the horizontal
 // padding, and the channels past the tensors' ends. A CTA takes up to kWgCombos pairs of X and dP
-// groups (their accumulators fill the 512 TMEM columns) and a run of tiles; warp 0 issues the loads
+// groups (their accumulators fill the 512 TMEM columns; they are zeroed first, and every MMA adds,
+// whichever columns it covers) and a run of tiles; warp 0 issues the loads
 // into a ring of stages, a lane to a box, warps 1 and 2 the MMAs of every other pair, and the
 // warps 0-2 (dx) add the accumulators to dW: a warp's 32 lanes hold 32 consecutive input channels, and
 // through shared memory each lane gets four of them for one 16-byte addition (a quarter of the
@@ -102,8 +105,13 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
     __syncthreads();
     tc_fence_after();
     grid_dep_launch();
+    const uint32_t tmem = *tslot, mine = tmem + ((uint32_t)(warp * 32) << 16);   // this warp's lanes
+    for (int n = 0; n < nb * ng * 96; n += 16) tmem_zero16(mine + (uint32_t)n);
+    tmem_st_wait();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
     grid_dep_wait();
-    const uint32_t tmem = *tslot;
 
     // the producer's lane: its box's map, place in a stage, channels and offset from the tile's corner
     const bool is_x = lane < nb, loads = lane < nb + ng;
@@ -111,7 +119,7 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
     const int place = is_x ? lane * kWgXBox : p.mb * kWgXBox + (lane - nb) * kWgDBox;
     const int ch = 32 * (is_x ? blk0 + lane : g0 + lane - nb);
     int tx = 0, ty = 0, img = 0;   // the next tile's
-    if (warp == 0) {
+    if (warp < 3) {
         const int per_img = p.xt * p.yt, rem = i0 % per_img;
         img = i0 / per_img;
         ty = rem / p.xt;
@@ -152,9 +160,12 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
             constexpr uint32_t kHi = (512u >> 4) | (1u << 14) | (4u << 29);   // 8-pixel groups 512 bytes apart, SWIZZLE_64B
             const bool leader = elect_one();
             const uint32_t idesc = umma_idesc_bf16(128u, 96u) | (1u << 15) | (1u << 16);   // MN-major A, B
+            constexpr uint32_t kDRow = kWgPix * 64 / 16;   // a row of a dP box
             const uint32_t base = smem_u32(smem) >> 4;
             bool ok = true;
             for (int k = k0; k < k1; ++k) {
+                const int rows = a.H - ty * kWgRows;   // of the image, from the tile's first on
+                const bool inner = ty > 0 && rows > kWgRows;
                 ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&full[s], use & 1u, a.err));
                 if (!ok) {
                     *abort_flag = 1;
@@ -165,20 +176,61 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
                     // atoms along M: one pixel apart; along N: one dP row apart
                     const uint32_t st = base + (uint32_t)(s * (stage_bytes >> 4));
                     const uint32_t sx = st | ((64u >> 4) << 16), sd = (st + (uint32_t)(p.mb * (kWgXBox >> 4))) |
-                                                                      ((uint32_t)(kWgPix * 64 / 16) << 16);
-                    for (int m = 0, c = 0; m < nb; ++m)
-                        for (int g = 0; g < ng; ++g, ++c) {
-                            if ((c & 1) != warp - 1) continue;
-                            const uint32_t d = tmem + (uint32_t)(c * 96);
-                            const uint32_t al = sx + (uint32_t)(m * (kWgXBox >> 4)), bl = sd + (uint32_t)(g * (kWgDBox >> 4));
+                                                                      (kDRow << 16);
+                    if (inner) {
+                        for (int m = 0, c = 0; m < nb; ++m)
+                            for (int g = 0; g < ng; ++g, ++c) {
+                                if ((c & 1) != warp - 1) continue;
+                                const uint32_t d = tmem + (uint32_t)(c * 96);
+                                const uint32_t al = sx + (uint32_t)(m * (kWgXBox >> 4)), bl = sd + (uint32_t)(g * (kWgDBox >> 4));
+                                auto mma = [&](int r, uint32_t dd, uint32_t bb, uint32_t id) {   // 16 pixels (two 8-pixel groups)
+                                    umma_bf16_lo(dd, al + (uint32_t)((r >> 1) * (kWgXPix * 4) + (r & 1) * 64), kHi,
+                                                 bb + (uint32_t)(r * 64), kHi, id, 1u);
+                                };
 #pragma unroll
-                            for (int r = 0; r < 2 * kWgRows; ++r)   // 16 pixels (two 8-pixel groups) per MMA
-                                umma_bf16_lo(d, al + (uint32_t)((r >> 1) * (kWgXPix * 4) + (r & 1) * 64), kHi,
-                                             bl + (uint32_t)(r * 64), kHi, idesc, k != k0 || r != 0 ? 1u : 0u);
-                        }
+                                for (int r = 0; r < 2 * kWgRows; ++r) mma(r, d, bl, idesc);
+                            }
+                    } else {
+                        // the image's first row has no dP row above, its last none below: 32 columns less (N / 8
+                        // starts at bit 17). A loop of its own: with these operands in registers for every tile
+                        // 96 x 32 channels on 2 x 509 x 517 pixels took 42.0 us; 41.0 so, as before the outer rows
+                        // were told apart
+                        const uint32_t up = ty == 0 ? 1u : 0u, down = rows == kWgRows ? 1u : 0u;
+                        const uint32_t id0 = idesc - (up << 19), id3 = idesc - (down << 19), up_d = up * 32u, up_b = up * kDRow;
+                        for (int m = 0, c = 0; m < nb; ++m)
+                            for (int g = 0; g < ng; ++g, ++c) {
+                                if ((c & 1) != warp - 1) continue;
+                                const uint32_t d = tmem + (uint32_t)(c * 96);
+                                const uint32_t al = sx + (uint32_t)(m * (kWgXBox >> 4)), bl = sd + (uint32_t)(g * (kWgDBox >> 4));
+                                auto mma = [&](int r, uint32_t dd, uint32_t bb, uint32_t id) {
+                                    umma_bf16_lo(dd, al + (uint32_t)((r >> 1) * (kWgXPix * 4) + (r & 1) * 64), kHi,
+                                                 bb + (uint32_t)(r * 64), kHi, id, 1u);
+                                };
+                                if (rows >= kWgRows) {
+                                    mma(0, d + up_d, bl + up_b, id0);
+                                    mma(1, d + up_d, bl + up_b, id0);
+                                    mma(2, d, bl, idesc);
+                                    mma(3, d, bl, idesc);
+                                    mma(4, d, bl, idesc);
+                                    mma(5, d, bl, idesc);
+                                    mma(6, d, bl, id3);
+                                    mma(7, d, bl, id3);
+                                } else {
+                                    for (int r = 0; r < 2 * rows; ++r) {
+                                        const uint32_t u = r < 2 ? up : 0u;
+                                        mma(r, d + 32u * u, bl + kDRow * u,
+                                            idesc - ((u + ((r >> 1) == rows - 1 ? 1u : 0u)) << 19));
+                                    }
+                                }
+                            }
+                    }
                     umma_commit(&empty[s]);
                 }
                 __syncwarp();
+                if (++tx == p.xt) {
+                    tx = 0;
+                    if (++ty == p.yt) ty = 0;
+                }
                 if (++s == p.stages) {
                     s = 0;
                     ++use;
@@ -200,6 +252,7 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
             uint32_t v[16];
             tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 96 + n0), v);
             tmem_ld_wait();
+            if (seg + 1 < p.segs) tmem_zero16(mine + (uint32_t)(c * 96 + n0));
             if (!ready || dx > 2) continue;   // the same for the whole warp
             const int dy = 2 - n0 / 32;   // tap row: dP's row r - 1 is tap dy = +1
             const int co = 32 * (g0 + g) + (n0 & 31);
@@ -223,6 +276,7 @@ __global__ void __launch_bounds__(kWtThreads) k_conv_wgrad(const __grid_constant
                 }
             }
         }
+        tmem_st_wait();
         tc_fence_before();
         if (__syncthreads_or(*abort_flag)) break;   // the next sums start in the accumulators read here
         tc_fence_after();
