@@ -287,7 +287,8 @@ GK_D Fp32Hit fp32_test(f3 o, const Shear& s, f3 v0, f3 v1, f3 v2) {
 // 7, e2 . q 8; the constants below are rounded up for the second order and the sums' own
 // rounding (and 1e-37 covers products that underflow). x adds the three errors and 2 roundings. As in the FP32 shading test, edges that are
 // not certain, or errors above half of det, leave the decision to FP64. The reciprocals are
-// approximate (2 ulps, inside the slack of 1.25 and 8u |t|). The last term covers the FP64
+// approximate (2 ulps, inside the slack of 1.25 and 8u |t|) and flushed to zero for a determinant above
+// 2^126, which is left to FP64 too. The last term covers the FP64
 // test's own error: 2^-29 of an FP32 evaluation's, itself below the farthest vertex's distance.
 struct TriTest { int kind; float t, e; };   // kind: 0 certain miss, 1 certain hit, 2 undecided
 GK_D TriTest tri_test(f3 o, f3 d, f3 v0, f3 v1, f3 v2) {
@@ -316,7 +317,7 @@ GK_D TriTest tri_test(f3 o, f3 d, f3 v0, f3 v1, f3 v2) {
     const bool allneg = (u < -eu) && (v < -ev) && (x < -ex);
     const float adet = fabsf(det);
     r.kind = 2;
-    if (!(allpos || allneg) || !(ex < 0.5f * adet)) return r;
+    if (!(allpos || allneg) || !(ex < 0.5f * adet) || !(adet < 0x1p126f)) return r;
     const float ed = (8.0f * kU) * sd;
     const float t = dot3(e2, q) * rcp_approx(det);
     const float et = (10.0f * kU) * fmaf_(fabsf(e2.z), B.z, fmaf_(fabsf(e2.y), B.y, fabsf(e2.x) * B.x));
