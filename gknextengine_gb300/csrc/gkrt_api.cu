@@ -144,7 +144,8 @@ struct GkrtContext {
     unsigned int* d_work = nullptr;             // pixel counter of the persistent trace kernel
     int num_sms = 1;
     // stream-ordered scratch of calls that may overlap on several streams (adjoint, bake): what is freed
-    // stays reserved for the next call, until the context ends
+    // stays reserved for the next call, until the images are resized or the context ends. Made with the
+    // context, because a stream capture refuses it (the scratch of captured calls belongs to the graph).
     cudaMemPool_t mem_pool = nullptr;
 };
 
@@ -964,6 +965,19 @@ int gkrt_internal_ready_view(GkrtContext* ctx, SceneView* view, unsigned long lo
     return GKRT_OK;
 }
 
+static cudaError_t make_mem_pool(int device, cudaMemPool_t* pool) {
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaError_t e = cudaMemPoolCreate(pool, &props);
+    uint64_t keep = UINT64_MAX;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    return e;
+}
+
 extern "C" {
 
 int gkrt_abi_version(void) { return GKRT_ABI_VERSION; }
@@ -994,6 +1008,7 @@ int gkrt_context_create(const GkrtDeviceDesc* desc, GkrtContext** out) {
     if (e == cudaSuccess) e = cudaMalloc((void**)&ctx->d_work, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMalloc((void**)&ctx->d_tex, GKRT_MAX_TEXTURES * sizeof(DevTex));
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    if (e == cudaSuccess) e = make_mem_pool(ctx->device, &ctx->mem_pool);
     if (e == cudaSuccess) e = cudaMemset(ctx->d_counters, 0, 8 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_error, 0, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_tex, 0, GKRT_MAX_TEXTURES * sizeof(DevTex));
@@ -1005,6 +1020,7 @@ int gkrt_context_create(const GkrtDeviceDesc* desc, GkrtContext** out) {
         for (auto& pe : ctx->pass_ev)
             for (cudaEvent_t& ev : pe)
                 if (ev) cudaEventDestroy(ev);
+        if (ctx->mem_pool) cudaMemPoolDestroy(ctx->mem_pool);
         delete ctx;
         return e == cudaErrorMemoryAllocation ? GKRT_ERR_OOM : GKRT_ERR_CUDA;
     }
@@ -1054,6 +1070,7 @@ int gkrt_resize(GkrtContext* ctx, uint32_t width, uint32_t height) {
         return fail(ctx, GKRT_ERR_INVALID_ARG, "image size must be 1..16384");
     DeviceGuard device_guard(ctx->device);
     free_images(ctx);
+    GK_CUDA(cudaMemPoolTrimTo(ctx->mem_pool, 0));   // scratch of the old size
     const uint32_t pitch = (width + 3u) & ~3u;
     const size_t px = (size_t)pitch * height;
     for (int i = 0; i < GKRT_IMG_COUNT; ++i) {
@@ -1649,26 +1666,6 @@ int gkrt_trace_rays(GkrtContext* ctx, const GkrtRay* rays, GkrtHit* hits, uint32
     return GKRT_OK;
 }
 
-static int ensure_mem_pool(GkrtContext* ctx) {
-    if (ctx->mem_pool) return GKRT_OK;
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = ctx->device;
-    cudaMemPool_t pool = nullptr;
-    GK_CUDA(cudaMemPoolCreate(&pool, &props));
-    uint64_t keep = UINT64_MAX;
-    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-        cudaMemPoolDestroy(pool);
-        return cuda_fail(ctx, e, "cudaMemPoolSetAttribute");
-    }
-    ctx->mem_pool = pool;
-    return GKRT_OK;
-}
-
 // ---- ambient-cube probe grid ----
 
 namespace {
@@ -1703,7 +1700,6 @@ int gkrt_probe_bake(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_t fir
     cudaStream_t st = (cudaStream_t)stream;
     int rc = ensure_bvh(ctx, 0, st);
     if (rc != GKRT_OK) return rc;
-    if ((rc = ensure_mem_pool(ctx)) != GKRT_OK) return rc;
     const uint32_t* cubes_read = ctx->d_cubes;
     if (gkrt_probe_bake_needs_snapshot(count)) {
         if (!ctx->d_cubes_prev) GK_CUDA(cudaMalloc((void**)&ctx->d_cubes_prev, kProbeCount * 14 * sizeof(uint32_t)));
@@ -1821,7 +1817,6 @@ int gkrt_adjoint_forward(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32_
     if (!image) return fail(ctx, GKRT_ERR_INVALID_ARG, "null image");
     DeviceGuard device_guard(ctx->device);
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = ensure_mem_pool(ctx)) != GKRT_OK) return rc;
     if ((rc = ensure_bvh(ctx, 0, st)) != GKRT_OK) return rc;
     GK_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), st));
     GK_CUDA(gkrt_launch_adjoint(shade_scene(ctx), *fc, (int)ctx->W, (int)ctx->H, spp, sample_roughness,
@@ -1837,7 +1832,6 @@ int gkrt_adjoint_backward(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32
     if (!d_image || !grad_albedo || !grad_roughness) return fail(ctx, GKRT_ERR_INVALID_ARG, "null buffer");
     DeviceGuard device_guard(ctx->device);
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = ensure_mem_pool(ctx)) != GKRT_OK) return rc;
     if ((rc = ensure_bvh(ctx, 0, st)) != GKRT_OK) return rc;
     GK_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 6 * sizeof(unsigned long long), st));
     GK_CUDA(gkrt_launch_adjoint(shade_scene(ctx), *fc, (int)ctx->W, (int)ctx->H, spp, sample_roughness, nullptr,

@@ -442,7 +442,8 @@ int  gkrt_trace_rays_noalloc(GkrtContext* ctx, const GkrtRay* rays, GkrtHit* hit
  * sky_index (computed by gkrt_texture_upload for RGBA32F textures, zero for 8-bit ones:
  * SampleIBLRough, Shading.slang:188-192), else the constant sky colour. The reference's
  * schedule bakes slice (frame % F) of size (27648 / F) * 64 with F = 30, 120 or 300.
- * Neighbour probes are read as they were before the call.
+ * Neighbour probes are read as they were before the call. Scratch as the adjoint's, below; the
+ * first call of a context for more than 65,536 probes allocates, which a stream capture refuses.
  *
  * gkrt_probe_download: the grid to host memory (either pointer may be NULL); synchronous. */
 int  gkrt_probe_voxelize(GkrtContext* ctx, void* stream);
@@ -460,6 +461,9 @@ int  gkrt_probe_download(GkrtContext* ctx, uint32_t* cubes, uint32_t* voxels);
  * sampler's densities at the current and the sampling roughness, which is 1 when they are
  * equal. Gradients are ADDED to grad_albedo (3 doubles per material) and grad_roughness
  * (1 double per material), device arrays the caller zeroes.
+ * Calls on several streams may overlap: each takes scratch of its own, in stream order, from a
+ * pool of the context's (kept until gkrt_resize or the context's end). A captured call's scratch
+ * belongs to the graph.
  * gkrt_set_material_params overwrites diffuse rgb (3 floats each) and fuzziness of
  * materials [first, first + count) from device arrays (either may be NULL); emitter
  * radiance changes need gkrt_scene_upload. */
