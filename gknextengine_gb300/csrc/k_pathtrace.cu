@@ -30,9 +30,10 @@ constexpr int kPtBlocks = 4;
 // three blocks per SM, whose registers hold a path without spills, or two where those have a lane for
 // every pixel. Whole frames of bricks with 2 / 3 / 4 /
 // 5 blocks, us: 100 x 70 pixels 215 / 220 / 231 / 272, 300 x 200 250 / 269 / 288 / 330, 400 x 300 358 / 305 /
-// 333 / 406; Cornell 256 x 256 158 / 131 / 156 / 176. Larger pools on 640 x 360: bricks 537 us (504),
-// Cornell 289 (277), city 4853 (4532), textured 429 (471), probe grid 1002 (1027).
-constexpr uint32_t kPtOneWarps = 64;
+// 333 / 406; Cornell 256 x 256 158 / 131 / 156 / 176. One-warp pools / larger ones, us, at 640 x 400 (53
+// warps' worth per SM): bricks 554 / 560, Cornell 325 / 312, textured 556 / 482, field of bricks on the probe
+// grid 515 / 533, city 1545 / 1548; at 700 x 400 (58): 602 / 588, 339 / 325, 586 / 501, 557 / 549, 1664 / 1648.
+constexpr uint32_t kPtOneWarps = 56;
 constexpr float kCosCone = 0.999990482f;   // cos(0.25 deg), Shading.slang:897
 
 // Warp-aggregated flush: one atomic per counter per warp. Slots 0-5 are per pass
@@ -633,9 +634,12 @@ __global__ void __launch_bounds__(kQueryThreads, kRqBlocks) k_trace_rays(SceneVi
 using namespace gk;
 
 // Paths per pool and the pools' size: as many paths per warp as the frame has pixels for, in whole
-// warps, up to kPoolMax.
+// warps, up to kPoolMax. A share that ends within a warp's worth is rounded up, so that every pixel starts at
+// once though some warps get none, but below 128 down: 640 x 480 with 128 / 96 paths: bricks 632 / 619 us, Cornell
+// 385 / 371, field of bricks 579 / 573 (textured 587 / 651, city 1705 / 1785); 700 x 400 with 128 / 96:
+// 620 / 588. Above, 720 x 480 with 160 / 128: city 1885 / 1946, bricks 700 / 671.
 static uint32_t paths_per_pool(uint32_t pixels, uint32_t warps) {
-    const uint32_t want = (pixels / std::max(1u, warps) + 31u) / 32u * 32u;
+    const uint32_t share = pixels / std::max(1u, warps), want = (share < 128u ? share : share + 31u) / 32u * 32u;
     return std::max(32u, std::min(kPoolMax, want));
 }
 size_t gkrt_trace_pool_bytes(uint32_t pixels, int num_sms) {
