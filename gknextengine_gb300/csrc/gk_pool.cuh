@@ -104,9 +104,14 @@ struct PathList {
     }
 };
 
-// The rays that a warp's lanes are in the middle of, kept over the shading phase: 9 float4 fields of
+// The rays that a warp's lanes are in the middle of, kept over the shading phase: 8 float4 fields of
 // 32 lanes each in device memory (the world ray and the stack stay in shared memory).
-constexpr int kStashFields = 9;
+constexpr int kStashFields = 8;
+// Device memory of a warp, in float4: its pool of np paths, and the stash that pools of one warp's worth
+// do without.
+__host__ __device__ constexpr uint32_t warp_pool_size(uint32_t fields, uint32_t np, bool one) {
+    return fields * np + (one ? 0u : kStashFields * 32u);
+}
 __device__ __forceinline__ void stash_save(float4* s, const Trav& T, int st, uint32_t slot) {
     const unsigned flags = (unsigned)st | (T.hit ? 4u : 0u) | (T.best_exact ? 8u : 0u) | (T.inblas ? 16u : 0u) |
                            ((unsigned)T.mode << 5) | (slot << 8);

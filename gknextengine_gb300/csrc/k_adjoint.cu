@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kPoolThreads, kOneBlocks ? kOneBlocks : kAdjBl
     float* wray = reinterpret_cast<float*>(adj_smem + stack_words * kPoolThreads) + tid;
     PathId* lists = reinterpret_cast<PathId*>(adj_smem + (stack_words + kPoolRayWords) * kPoolThreads) +
                     (uint32_t)warp * 5u * np;
-    float4* pool = pools + (size_t)(blockIdx.x * kPoolWarps + warp) * (adj_fields<kBackward>() * np + kStashFields * 32u);
+    float4* pool = pools + (size_t)(blockIdx.x * kPoolWarps + warp) * warp_pool_size(adj_fields<kBackward>(), np, kOne);
     float4* stash = pool + adj_fields<kBackward>() * np + lane;
     Counters cn;
     cn.rays = 0; cn.fallbacks = 0; cn.retraces = 0; cn.nodes = 0; cn.tris = 0; cn.hits = 0;
@@ -511,7 +511,7 @@ cudaError_t gkrt_launch_adjoint(const ShadeScene& sc, const GkrtFrameConstants& 
     // 32 / 64 / 96 paths 21.2 / 16.5 / 17.8 ms forward).
     const uint32_t np = one ? 32u : std::max(32u, std::min(kPoolMax, pixels / warps * 2u / 3u / 32u * 32u));
     // scratch of this call alone (calls may overlap on several streams): the pools, then the pixel counter
-    const size_t bytes = (size_t)warps * (fields * np + kStashFields * 32u) * sizeof(float4);
+    const size_t bytes = (size_t)warps * warp_pool_size(fields, np, one != 0) * sizeof(float4);
     float4* pools = nullptr;
     e = cudaMallocFromPoolAsync((void**)&pools, bytes + 16u, mem, st);
     if (e != cudaSuccess) return e;

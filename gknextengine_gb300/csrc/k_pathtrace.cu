@@ -20,8 +20,8 @@ namespace gk {
 
 constexpr int kPtThreads = kPoolThreads;
 constexpr int kPtWarps = kPoolWarps;
-constexpr int kPtMaxBlocks = 8;    // resident blocks per SM, at most
-// Resident blocks per SM: the traversal phase fits 128 registers, the shading phase spills below.
+// Resident blocks per SM, at most (what the pools are sized for): the traversal phase fits 128 registers, the
+// shading phase spills below.
 // Trace pass with 3 / 4 / 5 blocks (ms): 1080p bricks 3.12 / 2.84 / 3.03, Cornell 256 x 256
 // 0.160 / 0.134 / 0.150, 720p on the probe grid 1.31 / 1.16 / 1.14, 4K city 52.3 / 48.7 / 48.4, textured
 // 1277 x 713 at 8 samples 6.8 / 6.6 / 7.7.
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kPtThreads, kOneBlocks ? kOneBlocks : kPtBlock
     uint32_t* stack = dyn_smem + tid;
     float* wray = reinterpret_cast<float*>(dyn_smem + stack_words * kPtThreads) + tid;
     PathId* lists = reinterpret_cast<PathId*>(dyn_smem + (stack_words + kPoolRayWords) * kPtThreads) + (uint32_t)warp * 5u * np;
-    float4* pool = pools + (size_t)(blockIdx.x * kPtWarps + warp) * (PF_COUNT * np + kStashFields * 32u);
+    float4* pool = pools + (size_t)(blockIdx.x * kPtWarps + warp) * warp_pool_size(PF_COUNT, np, kOne);
     float4* stash = pool + PF_COUNT * np + lane;
     Counters cn;
     cn.rays = 0; cn.fallbacks = 0; cn.retraces = 0; cn.nodes = 0; cn.tris = 0; cn.hits = 0;
@@ -642,10 +642,12 @@ static uint32_t paths_per_pool(uint32_t pixels, uint32_t warps) {
     const uint32_t share = pixels / std::max(1u, warps), want = (share < 128u ? share : share + 31u) / 32u * 32u;
     return std::max(32u, std::min(kPoolMax, want));
 }
+static bool one_warp_pools(uint32_t pixels, int num_sms) { return pixels / (uint32_t)num_sms <= kPtOneWarps * 32u; }
 size_t gkrt_trace_pool_bytes(uint32_t pixels, int num_sms) {
-    const size_t warps = std::min<size_t>((size_t)num_sms * kPtMaxBlocks, (size_t)pixels / kPtThreads + 1u) * kPtWarps;
-    return (std::min<size_t>(warps * kPoolMax, (size_t)pixels + 32u * warps) * PF_COUNT + warps * kStashFields * 32u) *
-           sizeof(float4);
+    const size_t warps = std::min<size_t>((size_t)num_sms * kPtBlocks, (size_t)pixels / kPtThreads + 1u) * kPtWarps;
+    const bool one = one_warp_pools(pixels, num_sms);
+    const size_t paths = one ? 32u * warps : std::min<size_t>(warps * kPoolMax, (size_t)pixels + 32u * warps);
+    return (paths * PF_COUNT + warps * warp_pool_size(0, 0, one)) * sizeof(float4);
 }
 
 cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstants& fc, int W, int H, int P,
@@ -665,7 +667,7 @@ cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstant
 #undef GK_PASSES
     const uint32_t pixels = (uint32_t)W * (uint32_t)H;
     const uint32_t per_sm = pixels / (uint32_t)num_sms;
-    const int one = per_sm <= 2u * kPtThreads ? 1 : per_sm <= kPtOneWarps * 32u ? 2 : 0;
+    const int one = per_sm <= 2u * kPtThreads ? 1 : one_warp_pools(pixels, num_sms) ? 2 : 0;
     const Kernel f = kernels[nee][tex][one];
     // resident blocks per SM of each instantiation and stack size, queried once per device
     static int occ[kMaxDevices][2][2][3][kQuadStackMax + 1] = {};
@@ -679,10 +681,10 @@ cudaError_t gkrt_launch_trace_pass(const ShadeScene& sc, const GkrtFrameConstant
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, f, kPtThreads, smem);
         if (e != cudaSuccess) return e;
     }
-    uint32_t blocks = (uint32_t)(num_sms * std::max(1, std::min(*o, kPtMaxBlocks)));
+    uint32_t blocks = (uint32_t)(num_sms * std::max(1, std::min(*o, kPtBlocks)));
     blocks = std::min(blocks, (pixels + kPtThreads - 1) / kPtThreads);
     const uint32_t np = one ? 32u : paths_per_pool(pixels, blocks * kPtWarps);
-    if ((size_t)blocks * kPtWarps * (np * PF_COUNT + kStashFields * 32u) * sizeof(float4) > pool_bytes) return cudaErrorInvalidValue;
+    if ((size_t)blocks * kPtWarps * warp_pool_size(PF_COUNT, np, one != 0) * sizeof(float4) > pool_bytes) return cudaErrorInvalidValue;
     e = cudaMemsetAsync(work, 0, sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
     f<<<blocks, kPtThreads, smem, st>>>(sc, fc, W, H, P, im, counters, work, stack_words, pool, np);
