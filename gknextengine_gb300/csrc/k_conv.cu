@@ -1416,6 +1416,14 @@ static RowPlan row_plan(const ConvArgs& a, int rb, int sms) {
     return p;
 }
 
+// For the tests: the row tiles that a convolution takes on a device of `sms`, 0 where it takes others.
+extern "C" int gkrt_internal_conv_row_tiles(int B, int H, int W, int cin, int cout, int pooled, int sms) {
+    ConvArgs a{};
+    a.B = B; a.H = H; a.W = W; a.cin = cin; a.cout = cout;
+    a.pool_out = pooled ? &a : nullptr;
+    return row_plan(a, 64, sms).items;
+}
+
 // The tensor maps of a bf16 output's stores, kg channels of bx x by pixels, and of its nearest
 // upsampling's, bx pixels of a row to every other pixel.
 static cudaError_t encode_outputs(const ConvArgs& a, int kg, uint32_t bx, uint32_t by, CUtensorMap* mo, CUtensorMap* mu) {
