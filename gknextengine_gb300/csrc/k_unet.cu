@@ -59,6 +59,7 @@ struct WgPlan {
     int stages;
     int xt, yt;        // tiles per image row, row tiles per image
     int items;         // tiles in all
+    int groups, grid;  // of pairs, CTAs each
     int segs;          // partial sums per CTA: the accumulators are added to dW and restarted
     int vec;           // dW takes 16-byte additions (16-byte aligned; cin is a multiple of 16)
 };
@@ -396,10 +397,9 @@ using namespace gk;
 cudaError_t gkrt_encode_tmap_bf16(CUtensorMap* map, const void* base, uint32_t rank, const uint64_t* dims,
                                   const uint64_t* strides_bytes, const uint32_t* box);
 
-// The split that loads least: each CTA of a pixel run loads 4 mb boxes of X and gb of dP (1.5 times
-// as tall), at least two stages in shared memory.
-// The split with the fewest cycles a tile, over all groups of pairs: MMAs, or box rows if those are more.
-static WgPlan wgrad_plan(const WgradArgs& a) {
+// The split with the fewest cycles a tile, over all groups of pairs: MMAs, or box rows if those are more. At
+// least two stages (a box of X per group, and one of dP, 1.5 times as tall) fit in shared memory.
+static WgPlan wgrad_plan(const WgradArgs& a, int sms) {
     WgPlan p{};
     p.na = (a.cin + 31) / 32;
     p.ng = (a.cout + 31) / 32;
@@ -421,7 +421,20 @@ static WgPlan wgrad_plan(const WgradArgs& a) {
     p.yt = (a.H + kWgRows - 1) / kWgRows;
     p.items = a.B * p.xt * p.yt;
     p.vec = ((uintptr_t)a.dw & 15u) == 0u;
+    p.groups = ((p.na + p.mb - 1) / p.mb) * ((p.ng + p.gb - 1) / p.gb);
+    // one CTA per SM (its stages fill the shared memory), at least two tiles each. From 136 tiles on an FP32
+    // sum covers at most a 34th of the pixels: with 21 CTAs, 224 x 96 on 8 x 64 x 64 was off by 1.6e-6 of dW's
+    // norm in one sum each (25 us) and is by 7.4e-7 in two (31 us). (Fewer tiles are at most 17,280 pixels
+    // in all: a sum may cover more than a 34th of them, of fewer terms.)
+    p.grid = std::max(1, std::min((p.items + 1) / 2, sms / p.groups));
+    p.segs = p.items < 34 * 4 ? 1 : (34 + p.grid - 1) / p.grid;
     return p;
+}
+// For the tests: the partial sums of each CTA, on a device of `sms`.
+extern "C" int gkrt_internal_wgrad_sums(int B, int H, int W, int cin, int cout, int sms) {
+    WgradArgs a{};
+    a.B = B; a.H = H; a.W = W; a.cin = cin; a.cout = cout;
+    return wgrad_plan(a, sms).segs;
 }
 
 cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
@@ -442,7 +455,7 @@ cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
         if (e != cudaSuccess) return e;
     }
     const uint64_t W = (uint64_t)a.W, H = (uint64_t)a.H, B = (uint64_t)a.B;
-    WgPlan p = wgrad_plan(a);
+    const WgPlan p = wgrad_plan(a, sms_dev[dev]);
     const uint32_t dbox[4] = {32u, (uint32_t)kWgPix, (uint32_t)(kWgRows + 2), 1u};
     const uint32_t xbox[4] = {32u, (uint32_t)kWgXPix, (uint32_t)kWgRows, 1u};
     CUtensorMap mdp, mx;
@@ -454,14 +467,7 @@ cudaError_t gkrt_launch_conv_wgrad(const WgradArgs& a, cudaStream_t st) {
     const uint64_t xs[3] = {(uint64_t)a.x_c * 2, W * a.x_c * 2, H * W * a.x_c * 2};
     if ((e = gkrt_encode_tmap_bf16(&mx, a.x + a.x_off, 4, xd, xs, xbox)) != cudaSuccess) return e;
     const int stage_bytes = p.mb * kWgXBox + p.gb * kWgDBox;
-    const int groups = ((p.na + p.mb - 1) / p.mb) * ((p.ng + p.gb - 1) / p.gb);
-    // one CTA per SM (its stages fill the shared memory), at least two tiles each. An FP32 sum covers at
-    // most a 34th of the pixels: with 21 CTAs, 224 x 96 on 8 x 64 x 64 was off by 1.6e-6 of dW's norm in
-    // one sum each (25 us) and is by 7.4e-7 in two (31 us).
-    const int grid = std::max(1, std::min((p.items + 1) / 2, sms_dev[dev] / groups));
-    p.segs = (34 + grid - 1) / grid;
-    if (p.items < 34 * 4) p.segs = 1;
-    return launch_after(k_conv_wgrad, dim3((unsigned)grid, (unsigned)groups), kWtThreads,
+    return launch_after(k_conv_wgrad, dim3((unsigned)p.grid, (unsigned)p.groups), kWtThreads,
                         (size_t)p.stages * stage_bytes + kWgExtra, st, mdp, mx, a, p);
 }
 
