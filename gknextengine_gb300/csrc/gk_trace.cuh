@@ -219,13 +219,13 @@ static __device__ __noinline__ ExactHit exact_test(f3 o, f3 d, f3 v0, f3 v1, f3 
     return r;
 }
 
-struct Fp32Hit { int kind; float t, e, b1, b2; };   // kind: 0 certain miss, 1 certain hit, 2 undecided
+struct Fp32Hit { int kind; float t, b1, b2; };   // kind: 0 certain miss, 1 certain hit, 2 undecided
 
 // FP32 test with certified bounds on U, V, W (first order: 3.02u x magnitude x lateral
-// offset) and on t. Unit roundoff u = 2^-24.
+// offset), for the shading values of a hit. Unit roundoff u = 2^-24.
 GK_D Fp32Hit fp32_test(f3 o, const Shear& s, f3 v0, f3 v1, f3 v2) {
     const float kU = 5.9604645e-08f;
-    Fp32Hit r; r.kind = 0; r.t = 0.0f; r.e = 0.0f; r.b1 = 0.0f; r.b2 = 0.0f;
+    Fp32Hit r; r.kind = 0; r.t = 0.0f; r.b1 = 0.0f; r.b2 = 0.0f;
     f3 a = v0 - o, b = v1 - o, c = v2 - o;
     float akx = pick(a, s.kx), aky = pick(a, s.ky), akz = pick(a, s.kz);
     float bkx = pick(b, s.kx), bky = pick(b, s.ky), bkz = pick(b, s.kz);
@@ -261,16 +261,8 @@ GK_D Fp32Hit fp32_test(f3 o, const Shear& s, f3 v0, f3 v1, f3 v2) {
     if (ED >= 0.5f * adet) { r.kind = 2; return r; }
     float Az = s.Sz * akz, Bz = s.Sz * bkz, Cz = s.Sz * ckz;
     float T = fmaf_(W, Cz, fmaf_(V, Bz, U * Az));
-    float t = div_(T, det);
-    float aAz = fabsf(Az), aBz = fabsf(Bz), aCz = fabsf(Cz);
-    float sumUZ = fmaf_(fabsf(W), aCz, fmaf_(fabsf(V), aBz, fabsf(U) * aAz));
-    float ET = fmaf_(6.1f * kU, sumUZ, fmaf_(eW, aCz, fmaf_(eV, aBz, eU * aAz)));
-    float at = fabsf(t);
-    float e = 1.25f * div_(fmaf_(at, ED, ET), adet - ED);
-    e = fmaf_(4.0f * kU, at, e);
     r.kind = 1;
-    r.t = t;
-    r.e = e;
+    r.t = div_(T, det);
     r.b1 = div_(V, det);
     r.b2 = div_(W, det);
     return r;

@@ -654,13 +654,6 @@ __device__ __forceinline__ void tma_store_wait_read() {   // at most kPending gr
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// (a, b) += (x, y)
-__device__ __forceinline__ void add2(uint32_t& a, uint32_t& b, float x, float y) {
-    asm("{\n\t.reg .b64 s, t;\n\tmov.b64 s, {%0, %1};\n\tmov.b64 t, {%2, %3};\n\tadd.rn.f32x2 s, s, t;\n\t"
-        "mov.b64 {%0, %1}, s;\n\t}"
-        : "+r"(a), "+r"(b)
-        : "f"(x), "f"(y));
-}
 __device__ __forceinline__ uint32_t relu2(uint32_t v) {
     __nv_bfloat162 h = *reinterpret_cast<__nv_bfloat162*>(&v);
     h = __hmax2(h, __nv_bfloat162{__nv_bfloat16_raw{0}, __nv_bfloat16_raw{0}});
