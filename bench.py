@@ -47,8 +47,9 @@ NODE_BYTES, TRI_BYTES, RAY_BYTES = 112, 48, 32   # seven 16-byte words of a four
 # warp instructions issued (sm__inst_executed.sum), thread instructions
 # (smsp__thread_inst_executed.sum), DRAM bytes read + written, and the rays of that launch.
 # The node and triangle reads of the algorithmic bytes are served by L1/L2.
-# TRACE_NCU_1080P: the kernel that held a path in registers; TRACE_NCU_POOLS: the one on path pools,
-# which the benchmark's line uses.
+# TRACE_NCU_POOLS: the kernel on path pools, which the benchmark's line uses. TRACE_NCU_1080P: the one
+# before it, which held a path in registers; only the CPU test of the arithmetic reads it, as
+# trace_roofline's default.
 TRACE_NCU_1080P = {"inst": 1876796969, "thread_inst": 23252036915, "dram_bytes": 7515904 + 116706048,
                    "rays": 4483043}
 TRACE_NCU_POOLS = {"inst": 1348093445, "thread_inst": 21990874094, "dram_bytes": 668959744 + 908498176,
@@ -59,8 +60,9 @@ ISSUE_PER_SM_PER_CLOCK = 4   # four schedulers per SM, one warp instruction each
 def trace_roofline(st, trace_ms, alg_bytes, alg_gbs, hbm_peak, peak_kind, num_sms, clocks,
                    counters=TRACE_NCU_1080P):
     """Roofline of the rt-pass kernel against the bound that holds: issue slots. The BVH is
-    cache-resident, so DRAM carries little more than the output images (dram_frac), and the
-    kernel is bound by instruction issue and SIMT efficiency (divergent traversal and shading).
+    cache-resident; DRAM carries the output images and the path pools, which outgrow L2 (dram_frac
+    0.08), and the kernel is bound by instruction issue and SIMT efficiency (divergent traversal and
+    shading).
     achieved: warp instructions per ray (ncu, one 1080p launch) x the rays of the timed frame over
     its event-timed duration; peak: SMs x 4 issue slots x the SM clock sampled during the run."""
     n = counters

@@ -1804,7 +1804,8 @@ static int adjoint_checks(GkrtContext* ctx, const GkrtFrameConstants* fc, uint32
         return fail(ctx, GKRT_ERR_UNSUPPORTED, "the adjoint covers the reference NEE mode without sun");
     if (fc->number_of_bounces > 16 || fc->max_number_of_bounces > 16)
         return fail(ctx, GKRT_ERR_UNSUPPORTED, "the adjoint records at most 16 bounces");
-    if (ctx->nmat > 8192) return fail(ctx, GKRT_ERR_UNSUPPORTED, "the adjoint sums at most 8192 materials per block");
+    // part of the interface (the gradient kernel itself has no limit)
+    if (ctx->nmat > 8192) return fail(ctx, GKRT_ERR_UNSUPPORTED, "the adjoint takes at most 8192 materials");
     if (ctx->textured || (fc->flags & GKRT_FRAME_SKY_TEXTURE))
         return fail(ctx, GKRT_ERR_UNSUPPORTED, "the adjoint covers untextured scenes under the constant sky");
     return GKRT_OK;

@@ -4,7 +4,7 @@
 // FPathTracingRendererV2 (assets/shaders/common/Shading.slang:1084-1241, with the traced
 // camera ray of FHardwarePrimaryRayCaster, :283-334) as a state machine that stops
 // whenever it needs a ray traced. Each warp owns a pool of paths in device memory (a few per
-// lane, L2-resident) and alternates two phases over it: all rays of the pool are traced, a lane
+// lane; the pools of a large frame are larger than L2) and alternates two phases over it: all rays of the pool are traced, a lane
 // whose ray is finished taking the next one, then every path runs its state machine to its next
 // ray, 32 paths of one kind at a time, and pixels from a global counter (8 x 4 pixel tiles) take
 // the places of paths that ended. A warp thus waits for its longest ray once per pool instead of
@@ -27,8 +27,8 @@ constexpr int kPtWarps = kPoolWarps;
 // 1277 x 713 at 8 samples 6.8 / 6.6 / 7.7.
 constexpr int kPtBlocks = 4;
 // Pools of one warp's worth (kOne) serve frames of up to kPtOneWarps warps' worth of pixels per SM, with
-// three blocks per SM, whose registers hold a path without spills, or two where those have a lane for
-// every pixel. Whole frames of bricks with 2 / 3 / 4 /
+// three blocks per SM, whose registers hold a path almost without spills (32 to 56 bytes), or two, which have
+// none, where those have a lane for every pixel. Whole frames of bricks with 2 / 3 / 4 /
 // 5 blocks, us: 100 x 70 pixels 215 / 220 / 231 / 272, 300 x 200 250 / 269 / 288 / 330, 400 x 300 358 / 305 /
 // 333 / 406; Cornell 256 x 256 158 / 131 / 156 / 176. One-warp pools / larger ones, us, at 640 x 400 (53
 // warps' worth per SM): bricks 554 / 560, Cornell 325 / 312, textured 556 / 482, field of bricks on the probe
@@ -509,10 +509,10 @@ __device__ __forceinline__ void load_path(const Ctx& c, Lane& L, PathRay& R) {
 // kNee: emissive-triangle NEE compiled in (GKRT_NEE_EMISSIVE with a non-empty table); the
 // reference mode runs the instantiation without it.
 //
-// What bounds it: instruction issue with too few warps to cover it (1080p bricks: 310 warp
+// What bounds it: instruction issue with too few warps to cover it (1080p bricks: 301 warp
 // instructions per ray at 16.3 of 32 lanes, 419 at 12.4 when a warp traced its 32 rays to the end
-// before shading them all in registers; an issue in 38 % of the cycles, waits for instruction
-// fetch, node loads and fixed latencies in equal parts). So the code is kept small: one copy of the node
+// before shading them all in registers; an issue in 42 % of the cycles, waits per issue for node loads and
+// pool fields 2.6, fixed latencies 1.7, instruction fetch 1.5; 1.6 GB of pools through DRAM). So the code is kept small: one copy of the node
 // test, of the finished rays' hand-over, of the probe lookup and of the sampled direction (3 % to 17 % of
 // the pass). Trace pass in registers / on the pools / with one copy of each, ms: 1080p bricks 3.43 /
 // 2.97 / 2.84, 4K city 91.9 / 51.0 / 48.7, textured 17.7 / 8.2 / 6.4, Cornell 256 x 256 0.164 / 0.146 /

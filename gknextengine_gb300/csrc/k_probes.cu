@@ -424,7 +424,7 @@ cudaError_t gkrt_launch_probe_voxelize(const ShadeScene& sc, uint32_t first, uin
     return cudaGetLastError();
 }
 
-// Probes per batch: 170 MB of scratch at most.
+// Probes per batch: 108 MB of scratch at most.
 static constexpr uint32_t kBakeBatch = 1u << 16;
 bool gkrt_probe_bake_needs_snapshot(uint32_t count) { return count > kBakeBatch; }
 

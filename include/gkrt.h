@@ -454,7 +454,7 @@ int  gkrt_probe_download(GkrtContext* ctx, uint32_t* cubes, uint32_t* voxels);
  * `spp` samples per pixel from the primary hit, composed as the compose pass composes it
  * (diffuse x primary albedo + specular, no filter), and its path-replay adjoint.
  * Reference NEE mode without sun, untextured materials and the constant sky (else
- * GKRT_ERR_UNSUPPORTED), at most 16 bounces.
+ * GKRT_ERR_UNSUPPORTED), at most 16 bounces and 8192 materials.
  * image / d_image: dense width x height float4 device arrays (the context's size).
  * sample_roughness: per material, the roughness GGX directions are sampled with (detached);
  * NULL samples with the current roughness. GGX bounces are weighted by the ratio of the
